@@ -41,12 +41,17 @@ AHEAD_HD uint32_t ht_mix(uint64_t k) {
     return (uint32_t)k;
 }
 
+// A slot's key is read before it is claimed: a key that is already there (all
+// but the first rows of a group) costs a cached load, not a CAS on a word that
+// every other row of the group also fights for.  A stale read can only show an
+// empty slot, and the CAS then decides.
 AHEAD_DEV uint32_t ht_insert(const HashTab& h, uint64_t k) {
     if (k == kEmptyKey) return h.mask + 1;
     uint32_t s = ht_mix(k) & h.mask;
     for (uint32_t i = 0; i <= h.mask; ++i) {
-        const uint64_t prev = atomicCAS((unsigned long long*)&h.keys[s], (unsigned long long)kEmptyKey,
-                                        (unsigned long long)k);
+        uint64_t prev = h.keys[s];
+        if (prev == kEmptyKey)
+            prev = atomicCAS((unsigned long long*)&h.keys[s], (unsigned long long)kEmptyKey, (unsigned long long)k);
         if (prev == kEmptyKey || prev == k) return s;
         s = (s + 1) & h.mask;
     }

@@ -114,6 +114,89 @@ inline void run_colcheck(OpScope& s, const ahead_col& c, uint64_t n, uint64_t ai
     });
 }
 
+// ------------------------------------------------------- rare error rows
+// Corrupt codes are rare, so the kernels that read a column anyway append the
+// rows of corrupt codes to a short list (in any order); only when a list is
+// not empty is it sorted into the error vector, and only when it overflows is
+// the vector made by a compaction of the column.
+constexpr uint32_t kFastErrCap = 4096;
+
+// Block c sorts list c (at most kFastErrCap rows, bitonic in shared memory)
+// and writes row * aoid into the error vector, up to its capacity; block 0
+// also writes its sorted rows to `sorted` when given.
+static __global__ void __launch_bounds__(1024) sort_err_rows_kernel(const unsigned long long* cnt, const uint64_t* rows1,
+                                                             const uint64_t* rows2, uint64_t* e1, uint64_t cap1,
+                                                             uint64_t* e2, uint64_t cap2, uint64_t aoid,
+                                                             uint64_t* sorted = nullptr) {
+    __shared__ uint64_t s_r[kFastErrCap];
+    const int c = blockIdx.x;
+    const unsigned long long k = cnt[c];
+    uint64_t* e = c == 0 ? e1 : e2;
+    const uint64_t cap = c == 0 ? cap1 : cap2;
+    if (k == 0 || k > kFastErrCap) return;
+    const uint64_t* rows = c == 0 ? rows1 : rows2;
+    uint32_t m = 1;
+    while (m < k) m <<= 1;
+    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) s_r[i] = i < k ? rows[i] : ~0ull;
+    __syncthreads();
+    for (uint32_t size = 2; size <= m; size <<= 1)
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
+                const uint32_t j = i ^ stride;
+                if (j > i) {
+                    const bool up = (i & size) == 0;
+                    const uint64_t x = s_r[i], y = s_r[j];
+                    if ((x > y) == up) {
+                        s_r[i] = y;
+                        s_r[j] = x;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    if (e)
+        for (uint32_t i = threadIdx.x; i < k && i < cap; i += blockDim.x) e[i] = s_r[i] * aoid;
+    if (sorted && c == 0)
+        for (uint32_t i = threadIdx.x; i < k; i += blockDim.x) sorted[i] = s_r[i];
+}
+
+// One column's short error list: its count is counter `ci` of the call.
+struct ErrList {
+    unsigned long long* cnt;
+    uint64_t* rows;  // [kFastErrCap]
+    AHEAD_DEV void add(uint64_t row) const {
+        if (*(volatile unsigned long long*)cnt > kFastErrCap) return;  // (a column of errors: no queue on one word)
+        const unsigned long long k = atomicAdd(cnt, 1ull);
+        if (k < kFastErrCap) rows[k] = row;
+    }
+};
+constexpr size_t kErrListBytes = kFastErrCap * 8 + 256;
+
+inline ErrList err_list(OpScope& s, int ci) {
+    ErrList l;
+    l.cnt = (unsigned long long*)(s.d_counters + ci);
+    l.rows = (uint64_t*)s.alloc(kFastErrCap * 8);
+    return l;
+}
+
+// After finish() has read the counters back: writes the error vector of a list
+// with a few rows (a launch, no wait: the stream orders it before any reader)
+// and returns false when the list overflowed, so that the caller runs the
+// column's compaction.
+inline bool settle_err_list(OpScope& s, const ErrList& l, int ci, uint64_t aoid, ahead_errvec* e) {
+    const uint64_t k = s.counter(ci);
+    if (k > kFastErrCap) return false;
+    if (e) {
+        e->count = k;
+        if (k && edata(e)) {
+            sort_err_rows_kernel<<<1, 1024, 0, s.ctx->stream>>>(l.cnt, l.rows, nullptr, edata(e), ecap(e), nullptr, 0,
+                                                                aoid);
+            s.launched();
+        }
+    }
+    return true;
+}
+
 }  // namespace ahead
 
 namespace ahead {

@@ -4,10 +4,11 @@
 //
 // Group ids are assigned in order of first occurrence, as the reference's
 // dictionary loop does (lib/column_operators/AN/groupbyAN.tcc:70-91,
-// 127-160).  On the GPU: every row inserts its key into the hash table of
-// hash.cuh and atomicMin's its row index into the slot's first-row word; a
-// stable compaction of the rows that are their key's first row ranks the
-// groups by first occurrence; a last pass writes every row's encoded group id.
+// 127-160).  On the GPU: every row lowers its key's first-row word (indexed by
+// the key itself while the keys are small, else a slot of the hash table of
+// hash.cuh); the groups are ranked by first row (a sort of the few, or a stable
+// compaction of the rows that are their key's first row); a last pass writes
+// every row's encoded group id.
 #include "hash.cuh"
 #include "ops_common.cuh"
 
@@ -33,7 +34,7 @@ __global__ void gb_insert_kernel(HashTab h, GbKey k, uint64_t n, uint32_t* slot_
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t s = ht_insert(h, gb_key(k, i));
         slot_of[i] = s;
-        atomicMin(&first[s], (uint32_t)i);
+        if ((uint32_t)i < first[s]) atomicMin(&first[s], (uint32_t)i);  // (a stale word is only larger)
     }
 }
 
@@ -79,6 +80,254 @@ __global__ void gb_assign_kernel(const uint32_t* slot_of, const uint32_t* first,
         const uint64_t v = (uint64_t)gid_of_slot[s] * aoid;
         gids[i] = (binary && first[s] != (uint32_t)i) ? (uint64_t)(uint32_t)v : v;
     }
+}
+
+// ---------------------------------------------------- small-key group-by
+// Group keys are dictionary codes (years, categories, brands) or such a code
+// times the number of groups so far plus a group id: small integers.  So the
+// key indexes a table of first rows directly (`limit` 4-byte words: twice the
+// rows, between 2^16 and 2^22, so clearing it costs no more than reading the
+// inputs), without hashing, key words or probing, and neighbouring keys share
+// L1 lines.  A row reads its key's word first and only lowers it when it would:
+// once the seed block has seen the first rows, almost no row does an atomic.
+// At 12M rows, year (7) then category (40): the hash table's one CAS and one
+// atomicMin per row on a few words took 1,876 us for the two insert passes; the
+// seed, insert, rank and assign kernels here take 61 us unary and 95 us binary
+// (insert 22.8 and 46.2: 8 and 16 bytes a row at 4.2 TB/s, bound by HBM and
+// the L1 gathers).  The columns' AN checks ride along: corrupt rows go to short
+// lists.  A key at or above `limit` raises `over`, and the hash table takes the
+// call.
+constexpr uint32_t kGbMinLimit = 1u << 16, kGbMaxLimit = 1u << 22;
+constexpr uint32_t kGbSort = 4096;  // groups ranked by one block's sort; more are ranked by the compaction
+constexpr uint32_t kGbSeedRows = 4096;
+constexpr uint32_t kNoRow = 0xffffffffu;
+
+struct SmallGb {
+    GbKey k;
+    uint64_t n, gmax;        // gmax: largest valid grouping id (binary)
+    uint32_t* slot_of;       // [n] the row's key
+    uint32_t* first;         // [limit] first row of each key
+    uint32_t* gid_of_slot;   // [limit]
+    uint32_t* found;         // [kGbSort] the keys that occur, in any order
+    unsigned long long* count;  // keys that occur
+    uint32_t* over;          // a key did not fit
+    uint32_t limit;
+    int check;               // AN inputs: report corrupt codes
+    ErrList terr, gerr;
+};
+
+AHEAD_DEV uint32_t ld_ca(const uint32_t* p) {  // cached: a stale word only shows a later row, or none
+    uint32_t v;
+    asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
+template <bool TENC>
+AHEAD_DEV uint32_t small_gb_row(const SmallGb& g, uint64_t row, uint64_t tv, uint64_t gv) {
+    const uint64_t t = TENC ? mulw(tv, g.k.tail.ainv, g.k.tail.width) : tv;
+    if (TENC && t > g.k.tail.umax) g.terr.add(row);
+    uint64_t key = t & g.k.keymask;
+    if (g.k.binary) {
+        const uint64_t gd = gv * g.k.gainv;
+        if (g.check && gd > g.gmax) g.gerr.add(row);
+        key = ((t & g.k.lmask) * (g.k.ngroups & g.k.lmask) + (gd & g.k.lmask)) & g.k.lmask;
+    }
+    if (key >= g.limit) {
+        *g.over = 1;
+        return 0;
+    }
+    const uint32_t s = (uint32_t)key, r = (uint32_t)row;
+    if (r < ld_ca(g.first + s) && r < *(volatile uint32_t*)(g.first + s) && atomicMin(&g.first[s], r) == kNoRow) {
+        const unsigned long long i = atomicAdd(g.count, 1ull);
+        if (i < kGbSort) g.found[i] = s;
+    }
+    return s;
+}
+
+// The first rows, by one block in rounds: the keys that repeat are all in the
+// table before the grid starts.
+template <bool TENC>
+__global__ void __launch_bounds__(1024) small_gb_seed_kernel(SmallGb g) {
+    const uint64_t m = g.n < kGbSeedRows ? g.n : kGbSeedRows;
+    for (uint64_t i = threadIdx.x; i < m; i += blockDim.x) {
+        g.slot_of[i] = small_gb_row<TENC>(g, i, load_at(g.k.tail, i), g.k.binary ? load_at(g.k.grp, i) : 0);
+        __syncwarp();
+    }
+}
+
+// Four consecutive rows per thread and step (their loads in flight together;
+// 16-byte loads where the columns are aligned).
+template <int W>
+AHEAD_DEV void load4(const DCol& c, uint64_t i, bool vec, uint64_t (&v)[4]) {
+    if (c.type != AHEAD_VOID && vec) {
+        if constexpr (W == 8) {
+            const ulonglong2* q = reinterpret_cast<const ulonglong2*>((const char*)c.data + i * 8);
+            const ulonglong2 a = __ldg(q), b = __ldg(q + 1);
+            v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+            return;
+        } else if constexpr (W == 4) {
+            const uint4 a = __ldg(reinterpret_cast<const uint4*>((const char*)c.data + i * 4));
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+            return;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = load_at(c, i + q);
+}
+
+// TW, GW: the tail's and the grouping's width (GW 0: unary).
+template <int TW, int GW, bool TENC>
+__global__ void __launch_bounds__(256) small_gb_insert_kernel(SmallGb g, bool vec) {
+    const uint64_t r0 = kGbSeedRows, m = (g.n - r0) / 4, stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += stride) {
+        const uint64_t row = r0 + 4 * i;
+        uint64_t t[4], gv[4] = {0, 0, 0, 0};
+        load4<TW>(g.k.tail, row, vec, t);
+        if constexpr (GW) load4<GW>(g.k.grp, row, vec, gv);
+        uint32_t s[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s[q] = small_gb_row<TENC>(g, row + q, t[q], gv[q]);
+        *reinterpret_cast<uint4*>(g.slot_of + row) = make_uint4(s[0], s[1], s[2], s[3]);
+    }
+    if (blockIdx.x == 0 && threadIdx.x < (g.n - r0) % 4) {
+        const uint64_t row = r0 + 4 * m + threadIdx.x;
+        g.slot_of[row] = small_gb_row<TENC>(g, row, load_at(g.k.tail, row), GW ? load_at(g.k.grp, row) : 0);
+    }
+}
+
+// One block ranks up to kGbSort groups by first row (bitonic in shared memory)
+// and writes each group's first head; more groups are left to the compaction.
+template <bool AN>
+__global__ void __launch_bounds__(1024) small_gb_rank_kernel(SmallGb g, DCol head, int decode_head, uint64_t aoid,
+                                                             void* firsts, uint64_t cap) {
+    __shared__ uint64_t s_k[kGbSort];
+    const unsigned long long c = *g.count;
+    if (c > kGbSort || *g.over) return;
+    uint32_t m = 1;
+    while (m < c) m <<= 1;
+    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
+        const uint32_t s = i < c ? g.found[i] : 0;
+        s_k[i] = i < c ? ((uint64_t)g.first[s] << 32 | s) : ~0ull;
+    }
+    __syncthreads();
+    for (uint32_t size = 2; size <= m; size <<= 1)
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
+                const uint32_t j = i ^ stride;
+                if (j > i) {
+                    const uint64_t x = s_k[i], y = s_k[j];
+                    if ((x > y) == ((i & size) == 0)) {
+                        s_k[i] = y;
+                        s_k[j] = x;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    for (uint32_t i = threadIdx.x; i < c; i += blockDim.x) {
+        const uint64_t x = s_k[i];
+        g.gid_of_slot[(uint32_t)x] = i;
+        if (i < cap) {
+            const uint64_t h = load_at(head, x >> 32);
+            if (AN) ((uint64_t*)firsts)[i] = (decode_head ? dec_if(head, h, head.ainv) : h) * aoid;
+            else ((uint32_t*)firsts)[i] = (uint32_t)h;
+        }
+    }
+}
+
+// Every row's group id, four rows per thread and step (8 x 4 bytes read and
+// written per row: bound by HBM).  SORTED: only when the rank kernel ranked the groups.
+template <bool AN, bool SORTED>
+__global__ void __launch_bounds__(256) small_gb_assign_kernel(SmallGb g, uint64_t aoid, int binary, void* gids,
+                                                              uint64_t cap) {
+    if (SORTED && (*g.count > kGbSort || *g.over)) return;
+    const uint64_t n = g.n < cap ? g.n : cap, m = n / 4, stride = (uint64_t)gridDim.x * blockDim.x;
+    auto gid = [&](uint64_t row, uint32_t s) -> uint64_t {
+        const uint32_t id = g.gid_of_slot[s];
+        if (!AN) return id;
+        const uint64_t v = (uint64_t)id * aoid;
+        // (the binary dictionary keeps the code in an oid_t: see gb_assign_kernel)
+        return (binary && (v >> 32) && g.first[s] != (uint32_t)row) ? (uint64_t)(uint32_t)v : v;
+    };
+    const bool vec = ((uintptr_t)gids & 15) == 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += stride) {
+        const uint4 s = *reinterpret_cast<const uint4*>(g.slot_of + 4 * i);
+        const uint64_t v[4] = {gid(4 * i, s.x), gid(4 * i + 1, s.y), gid(4 * i + 2, s.z), gid(4 * i + 3, s.w)};
+        if (AN && vec) {
+            ulonglong2* o = reinterpret_cast<ulonglong2*>((uint64_t*)gids + 4 * i);
+            o[0] = make_ulonglong2(v[0], v[1]);
+            o[1] = make_ulonglong2(v[2], v[3]);
+        } else if (!AN && vec) {
+            reinterpret_cast<uint4*>(gids)[i] = make_uint4((uint32_t)v[0], (uint32_t)v[1], (uint32_t)v[2],
+                                                           (uint32_t)v[3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) store_at(gids, AN ? 8 : 4, 4 * i + q, v[q]);
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x < n % 4) {
+        const uint64_t row = 4 * m + threadIdx.x;
+        store_at(gids, AN ? 8 : 4, row, gid(row, g.slot_of[row]));
+    }
+}
+
+inline uint32_t gb_limit(uint64_t n) {
+    uint64_t l = kGbMinLimit;
+    while (l < 2 * n && l < kGbMaxLimit) l <<= 1;
+    return (uint32_t)l;
+}
+
+inline size_t small_gb_scratch(uint64_t n) {
+    return (size_t)gb_limit(n) * 8 + n * 4 + kGbSort * 4 + 2 * kErrListBytes + 4096;
+}
+
+// Counters 10-13 of the call: groups, `over`, corrupt tails, corrupt grouping codes.
+constexpr int kGbCount = 10, kGbOver = 11, kGbTail = 12, kGbGrp = 13, kGbCounters = 14;
+
+// The group-by through the first-row table: everything up to the group ids of
+// up to kGbSort groups.
+template <bool AN>
+SmallGb launch_small_gb(OpScope& s, const GbKey& k, uint64_t n, uint64_t gmax, const DCol& head, int decode_head,
+                        uint64_t aoid, ahead_bat* gids, ahead_bat* firsts, uint64_t cap) {
+    cudaStream_t st = s.ctx->stream;
+    SmallGb g;
+    g.k = k;
+    g.n = n;
+    g.gmax = gmax;
+    g.limit = gb_limit(n);
+    g.first = (uint32_t*)s.alloc((size_t)g.limit * 4);
+    g.gid_of_slot = (uint32_t*)s.alloc((size_t)g.limit * 4);
+    g.slot_of = (uint32_t*)s.alloc(n * 4);
+    g.found = (uint32_t*)s.alloc(kGbSort * 4);
+    g.count = (unsigned long long*)(s.d_counters + kGbCount);
+    g.over = (uint32_t*)(s.d_counters + kGbOver);
+    g.check = AN;
+    g.terr = err_list(s, kGbTail);
+    g.gerr = err_list(s, kGbGrp);
+    cudaMemsetAsync(g.first, 0xff, (size_t)g.limit * 4, st);
+    const bool vec = ((uintptr_t)k.tail.data & 15) == 0 && (!k.binary || ((uintptr_t)k.grp.data & 15) == 0);
+    small_gb_seed_kernel<AN><<<1, 1024, 0, st>>>(g);
+    s.launched();
+    if (n > kGbSeedRows) {
+        const uint32_t blocks = grid_for((n - kGbSeedRows + 3) / 4, 256);
+        const uint32_t grid = blocks < (uint32_t)s.ctx->num_sms * 8 ? blocks : (uint32_t)s.ctx->num_sms * 8;
+        by_width(k.tail.width, [&](auto tag) -> int {
+            constexpr int TW = decltype(tag)::value;
+            if (k.binary) small_gb_insert_kernel<TW, AN ? 8 : 4, AN><<<grid, 256, 0, st>>>(g, vec);
+            else small_gb_insert_kernel<TW, 0, AN><<<grid, 256, 0, st>>>(g, vec);
+            return 0;
+        });
+        s.launched();
+    }
+    small_gb_rank_kernel<AN><<<1, 1024, 0, st>>>(g, head, decode_head, aoid, firsts->tail.data,
+                                                 firsts->tail.data ? cap : 0);
+    s.launched();
+    if (gids->tail.data) {
+        small_gb_assign_kernel<AN, true><<<grid_for((n + 3) / 4, 256), 256, 0, st>>>(g, aoid, k.binary,
+                                                                                     gids->tail.data, cap);
+        s.launched();
+    }
+    return g;
 }
 
 // Grouped sums: sum[gid] += t * (AResult * AT^-1) over rows with a valid
@@ -131,7 +380,7 @@ __global__ void gb_insert_str_kernel(HashTab h, const char* strs, uint64_t width
         const uint64_t key = str_hash(strs + i * width, width) * ngroups + load_at(grp, i) * gainv;
         const uint32_t s = ht_insert(h, key);
         slot_of[i] = s;
-        atomicMin(&first[s], (uint32_t)i);
+        if ((uint32_t)i < first[s]) atomicMin(&first[s], (uint32_t)i);  // (a stale word is only larger)
     }
 }
 
@@ -153,58 +402,102 @@ int run_groupby(ahead_ctx* ctx, const ahead_bat* in, const ahead_bat* grouping, 
     }
     gids->count = n;
     firsts->count = 0;
+    if (!n) return AHEAD_OK;
+    GbKey k;
+    k.tail = dcol(in->tail);
+    k.grp = binary ? dcol(grouping->tail) : dcol(in->tail);
+    k.keymask = wmask(type_base_width(T));
+    k.lmask = wmask(type_width(type_larger_of(T)));
+    k.ngroups = ngroups;
+    k.gainv = binary ? grouping->tail.Ainv : 0;
+    k.binary = binary;
+    const DCol hc = dcol(in->head);
     OpScope s(ctx);
-    const uint32_t cap_slots = ht_capacity(n);
-    size_t need = (size_t)(cap_slots + 1) * (8 + 4 + 4) + n * 4 + compact_scratch<FirstOp>(n) + 3 * colcheck_scratch(n) +
-                  4096;
-    int rc = s.reserve(need);
-    if (rc) return rc;
-    if (n) {
-        cudaStream_t st = ctx->stream;
-        HashTab h{};
-        h.mask = cap_slots - 1;
-        h.keys = (uint64_t*)s.alloc((size_t)(cap_slots + 1) * 8);
-        uint32_t* first = (uint32_t*)s.alloc((size_t)(cap_slots + 1) * 4);
-        uint32_t* gid_of_slot = (uint32_t*)s.alloc((size_t)(cap_slots + 1) * 4);
-        uint32_t* slot_of = (uint32_t*)s.alloc(n * 4);
-        cudaMemsetAsync(h.keys, 0xff, (size_t)(cap_slots + 1) * 8, st);
-        cudaMemsetAsync(first, 0xff, (size_t)(cap_slots + 1) * 4, st);
-        GbKey k;
-        k.tail = dcol(in->tail);
-        k.grp = binary ? dcol(grouping->tail) : dcol(in->tail);
-        k.keymask = wmask(type_base_width(T));
-        k.lmask = wmask(type_width(type_larger_of(T)));
-        k.ngroups = ngroups;
-        k.gainv = binary ? grouping->tail.Ainv : 0;
-        k.binary = binary;
-        gb_insert_kernel<<<grid_for(n, 256), 256, 0, st>>>(h, k, n, slot_of, first);
+    auto check_head = [&] {
+        if (eH) run_colcheck(s, in->head, n, hc.ainv, hc.umax, hc.width, aoid, ev(errs, 0), 1);
+    };
+    auto check_tail = [&] { run_colcheck(s, in->tail, n, k.tail.ainv, k.tail.umax, k.tail.width, aoid, ev(errs, 1), 2); };
+    auto check_grp = [&] {
+        run_colcheck(s, grouping->tail, n, grouping->tail.Ainv, grouping->tail.unenc_max, 8, aoid, ev(errs, 2), 3);
+    };
+    auto first_op = [&](const uint32_t* slot_of, const uint32_t* first, uint32_t* gid_of_slot) {
         FirstOp op;
         op.base = (const char*)slot_of;
         op.status = s.d_status;
         op.first = first;
         op.gid_of_slot = gid_of_slot;
-        op.head = dcol(in->head);
+        op.head = hc;
         op.aoid = aoid;
         op.cap = firsts->tail.data ? cap : 0;
         op.firsts = (uint64_t*)firsts->tail.data;
         op.acc = nullptr;
         op.decode_head = binary;
-        run_compact(s, op, n, 0);
-        if (gids->tail.data)
-            gb_assign_kernel<<<grid_for(n, 256), 256, 0, st>>>(slot_of, first, gid_of_slot, n, aoid, binary,
-                                                                (uint64_t*)gids->tail.data, cap);
-        s.launched(2);
-        if (eH) {
-            const DCol hc = dcol(in->head);
-            run_colcheck(s, in->head, n, hc.ainv, hc.umax, hc.width, aoid, ev(errs, 0), 1);
+        return op;
+    };
+    int rc = s.reserve(small_gb_scratch(n) + compact_scratch<FirstOp>(n) + (eH ? colcheck_scratch(n) : 0));
+    if (rc) return rc;
+    const SmallGb g = launch_small_gb<true>(s, k, n, binary ? grouping->tail.unenc_max : 0, hc, binary, aoid, gids,
+                                            firsts, cap);
+    check_head();
+    rc = s.finish(kGbCounters);
+    if (rc) return rc;
+    if (!s.counter(kGbOver)) {
+        const uint64_t groups = s.counter(kGbCount);
+        if (errs && eH) errs[0].count = s.counter(1);
+        if (groups > kGbSort) {  // ranked by the compaction of the rows that are their key's first
+            run_compact(s, first_op(g.slot_of, g.first, g.gid_of_slot), n, 0);
+            if (gids->tail.data) {
+                small_gb_assign_kernel<true, false><<<grid_for((n + 3) / 4, 256), 256, 0, ctx->stream>>>(
+                    g, aoid, binary, gids->tail.data, cap);
+                s.launched();
+            }
         }
-        run_colcheck(s, in->tail, n, k.tail.ainv, k.tail.umax, k.tail.width, aoid, ev(errs, 1), 2);
-        if (binary) run_colcheck(s, grouping->tail, n, grouping->tail.Ainv, grouping->tail.unenc_max, 8, aoid, ev(errs, 2), 3);
+        const bool ok_t = settle_err_list(s, g.terr, kGbTail, aoid, ev(errs, 1));
+        const bool ok_g = !binary || settle_err_list(s, g.gerr, kGbGrp, aoid, ev(errs, 2));
+        if (groups > kGbSort) {
+            rc = s.finish(1);
+            if (rc) return rc;
+        }
+        if (!ok_t || !ok_g) {  // a column with many corrupt codes
+            rc = s.reserve(2 * colcheck_scratch(n));
+            if (rc) return rc;
+            if (!ok_t) check_tail();
+            if (!ok_g) check_grp();
+            rc = s.finish(4);
+            if (rc) return rc;
+            if (errs && !ok_t) errs[1].count = s.counter(2);
+            if (errs && !ok_g) errs[2].count = s.counter(3);
+        }
+        firsts->count = groups;
+        return (n > cap || groups > cap) ? AHEAD_CAPACITY : AHEAD_OK;
     }
+    // keys beyond the first-row table: the hash table
+    const uint32_t cap_slots = ht_capacity(n);
+    rc = s.reserve((size_t)(cap_slots + 1) * (8 + 4 + 4) + n * 4 + compact_scratch<FirstOp>(n) +
+                   3 * colcheck_scratch(n) + 4096);
+    if (rc) return rc;
+    cudaStream_t st = ctx->stream;
+    HashTab h{};
+    h.mask = cap_slots - 1;
+    h.keys = (uint64_t*)s.alloc((size_t)(cap_slots + 1) * 8);
+    uint32_t* first = (uint32_t*)s.alloc((size_t)(cap_slots + 1) * 4);
+    uint32_t* gid_of_slot = (uint32_t*)s.alloc((size_t)(cap_slots + 1) * 4);
+    uint32_t* slot_of = (uint32_t*)s.alloc(n * 4);
+    cudaMemsetAsync(h.keys, 0xff, (size_t)(cap_slots + 1) * 8, st);
+    cudaMemsetAsync(first, 0xff, (size_t)(cap_slots + 1) * 4, st);
+    gb_insert_kernel<<<grid_for(n, 256), 256, 0, st>>>(h, k, n, slot_of, first);
+    run_compact(s, first_op(slot_of, first, gid_of_slot), n, 0);
+    if (gids->tail.data)
+        gb_assign_kernel<<<grid_for(n, 256), 256, 0, st>>>(slot_of, first, gid_of_slot, n, aoid, binary,
+                                                            (uint64_t*)gids->tail.data, cap);
+    s.launched(2);
+    check_head();
+    check_tail();
+    if (binary) check_grp();
     rc = s.finish(4);
     if (rc) return rc;
-    firsts->count = n ? s.counter(0) : 0;
-    if (errs && n) {
+    firsts->count = s.counter(0);
+    if (errs) {
         if (eH) errs[0].count = s.counter(1);
         errs[1].count = s.counter(2);
         if (binary) errs[2].count = s.counter(3);
@@ -265,31 +558,18 @@ int run_groupby_plain(ahead_ctx* ctx, const ahead_bat* in, const ahead_bat* grou
     default_meta(&firsts->tail, AHEAD_OID);
     gids->count = n;
     firsts->count = 0;
+    if (!n) return AHEAD_OK;
+    GbKey k;
+    k.tail = dcol(in->tail);
+    k.tail.enc = 0;  // the raw tail: an encoded tail is grouped by its codes
+    k.grp = binary ? dcol(grouping->tail) : dcol(in->tail);
+    k.keymask = wmask(type_width(T));
+    k.lmask = wmask(type_width(type_larger_of(T)));
+    k.ngroups = ngroups;
+    k.gainv = 1;
+    k.binary = binary;
     OpScope s(ctx);
-    const uint32_t cap_slots = ht_capacity(n);
-    const size_t need = (size_t)(cap_slots + 1) * (8 + 4 + 4) + n * 4 + compact_scratch<FirstPlainOp>(n) + 4096;
-    int rc = s.reserve(need);
-    if (rc) return rc;
-    if (n) {
-        cudaStream_t st = ctx->stream;
-        HashTab h{};
-        h.mask = cap_slots - 1;
-        h.keys = (uint64_t*)s.alloc((size_t)(cap_slots + 1) * 8);
-        uint32_t* first = (uint32_t*)s.alloc((size_t)(cap_slots + 1) * 4);
-        uint32_t* gid_of_slot = (uint32_t*)s.alloc((size_t)(cap_slots + 1) * 4);
-        uint32_t* slot_of = (uint32_t*)s.alloc(n * 4);
-        cudaMemsetAsync(h.keys, 0xff, (size_t)(cap_slots + 1) * 8, st);
-        cudaMemsetAsync(first, 0xff, (size_t)(cap_slots + 1) * 4, st);
-        GbKey k;
-        k.tail = dcol(in->tail);
-        k.tail.enc = 0;  // the raw tail: an encoded tail is grouped by its codes
-        k.grp = binary ? dcol(grouping->tail) : dcol(in->tail);
-        k.keymask = wmask(type_width(T));
-        k.lmask = wmask(type_width(type_larger_of(T)));
-        k.ngroups = ngroups;
-        k.gainv = 1;
-        k.binary = binary;
-        gb_insert_kernel<<<grid_for(n, 256), 256, 0, st>>>(h, k, n, slot_of, first);
+    auto first_op = [&](const uint32_t* slot_of, const uint32_t* first, uint32_t* gid_of_slot) {
         FirstPlainOp op;
         op.base = (const char*)slot_of;
         op.status = s.d_status;
@@ -299,15 +579,49 @@ int run_groupby_plain(ahead_ctx* ctx, const ahead_bat* in, const ahead_bat* grou
         op.cap = firsts->tail.data ? cap : 0;
         op.firsts = (uint32_t*)firsts->tail.data;
         op.acc = nullptr;
-        run_compact(s, op, n, 0);
-        if (gids->tail.data)
-            gb_assign_plain_kernel<<<grid_for(n, 256), 256, 0, st>>>(slot_of, gid_of_slot, n,
-                                                                      (uint32_t*)gids->tail.data, cap);
-        s.launched(2);
+        return op;
+    };
+    int rc = s.reserve(small_gb_scratch(n) + compact_scratch<FirstPlainOp>(n));
+    if (rc) return rc;
+    const SmallGb g = launch_small_gb<false>(s, k, n, 0, dcol(in->head), 0, 1, gids, firsts, cap);
+    rc = s.finish(kGbCounters);
+    if (rc) return rc;
+    if (!s.counter(kGbOver)) {
+        const uint64_t groups = s.counter(kGbCount);
+        if (groups > kGbSort) {
+            run_compact(s, first_op(g.slot_of, g.first, g.gid_of_slot), n, 0);
+            if (gids->tail.data) {
+                small_gb_assign_kernel<false, false><<<grid_for((n + 3) / 4, 256), 256, 0, ctx->stream>>>(
+                    g, 1, binary, gids->tail.data, cap);
+                s.launched();
+            }
+            rc = s.finish(1);
+            if (rc) return rc;
+        }
+        firsts->count = groups;
+        return (n > cap || groups > cap) ? AHEAD_CAPACITY : AHEAD_OK;
     }
+    const uint32_t cap_slots = ht_capacity(n);
+    rc = s.reserve((size_t)(cap_slots + 1) * (8 + 4 + 4) + n * 4 + compact_scratch<FirstPlainOp>(n) + 4096);
+    if (rc) return rc;
+    cudaStream_t st = ctx->stream;
+    HashTab h{};
+    h.mask = cap_slots - 1;
+    h.keys = (uint64_t*)s.alloc((size_t)(cap_slots + 1) * 8);
+    uint32_t* first = (uint32_t*)s.alloc((size_t)(cap_slots + 1) * 4);
+    uint32_t* gid_of_slot = (uint32_t*)s.alloc((size_t)(cap_slots + 1) * 4);
+    uint32_t* slot_of = (uint32_t*)s.alloc(n * 4);
+    cudaMemsetAsync(h.keys, 0xff, (size_t)(cap_slots + 1) * 8, st);
+    cudaMemsetAsync(first, 0xff, (size_t)(cap_slots + 1) * 4, st);
+    gb_insert_kernel<<<grid_for(n, 256), 256, 0, st>>>(h, k, n, slot_of, first);
+    run_compact(s, first_op(slot_of, first, gid_of_slot), n, 0);
+    if (gids->tail.data)
+        gb_assign_plain_kernel<<<grid_for(n, 256), 256, 0, st>>>(slot_of, gid_of_slot, n, (uint32_t*)gids->tail.data,
+                                                                  cap);
+    s.launched(2);
     rc = s.finish(1);
     if (rc) return rc;
-    firsts->count = n ? s.counter(0) : 0;
+    firsts->count = s.counter(0);
     return (n > cap || firsts->count > cap) ? AHEAD_CAPACITY : AHEAD_OK;
 }
 

@@ -372,8 +372,6 @@ struct MulSumOp {
 // (ascending rows, as the reference's loop pushes them) into the error
 // vectors.  More than kFastErrCap errors in either column: the caller runs
 // the compaction instead.
-constexpr uint32_t kFastErrCap = 4096;
-
 template <int W>
 AHEAD_DEV void load8(const char* p, uint64_t chunk, uint64_t (&v)[8]) {
     const uint4* q = reinterpret_cast<const uint4*>(p + chunk * 8 * W);
@@ -461,45 +459,6 @@ __global__ void __launch_bounds__(256) check_fast_kernel(const char* a, uint64_t
         for (int q = 0; q < R; ++q) check(R * c + q, x0[q]);
     }
     if (blockIdx.x == 0 && threadIdx.x < n % R) check(R * nv + threadIdx.x, gmem_ld<W>(a, R * nv + threadIdx.x));
-}
-
-// Block c sorts list c (at most kFastErrCap rows, bitonic in shared memory)
-// and writes row * aoid into the error vector, up to its capacity; block 0
-// also writes its sorted rows to `sorted` when given.
-__global__ void __launch_bounds__(1024) sort_err_rows_kernel(const unsigned long long* cnt, const uint64_t* rows1,
-                                                             const uint64_t* rows2, uint64_t* e1, uint64_t cap1,
-                                                             uint64_t* e2, uint64_t cap2, uint64_t aoid,
-                                                             uint64_t* sorted = nullptr) {
-    __shared__ uint64_t s_r[kFastErrCap];
-    const int c = blockIdx.x;
-    const unsigned long long k = cnt[c];
-    uint64_t* e = c == 0 ? e1 : e2;
-    const uint64_t cap = c == 0 ? cap1 : cap2;
-    if (k == 0 || k > kFastErrCap) return;
-    const uint64_t* rows = c == 0 ? rows1 : rows2;
-    uint32_t m = 1;
-    while (m < k) m <<= 1;
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) s_r[i] = i < k ? rows[i] : ~0ull;
-    __syncthreads();
-    for (uint32_t size = 2; size <= m; size <<= 1)
-        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-                const uint32_t j = i ^ stride;
-                if (j > i) {
-                    const bool up = (i & size) == 0;
-                    const uint64_t x = s_r[i], y = s_r[j];
-                    if ((x > y) == up) {
-                        s_r[i] = y;
-                        s_r[j] = x;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    if (e)
-        for (uint32_t i = threadIdx.x; i < k && i < cap; i += blockDim.x) e[i] = s_r[i] * aoid;
-    if (sorted && c == 0)
-        for (uint32_t i = threadIdx.x; i < k; i += blockDim.x) sorted[i] = s_r[i];
 }
 
 // checkAndDecodeAN of a void-head column once its corrupt rows are known:
