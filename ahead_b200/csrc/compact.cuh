@@ -1,4 +1,4 @@
-// compact.cuh -- stable multi-stream compaction in three streaming passes.
+// compact.cuh -- stable multi-stream compaction in streaming passes.
 //
 // Every AN operator that filters rows (selectAN, checkAndDecodeAN, the
 // positional matchjoinAN / fetchjoinAN ...) produces up to five output
@@ -6,18 +6,30 @@
 // error-position vectors (rare).  The reference builds them with push_back in
 // one sequential loop (e.g. lib/column_operators/AN/selectAN_scalar.tcc:84-92).
 //
-//   pass 1  classify: each 4096-row tile is read once; a warp walks its
-//           512 rows one row per lane per step, the per-step ballot of
-//           stream 0 is stored as a 32-row bitmap word, and every stream is
-//           counted per tile.  No inter-block waiting of any kind.
-//   pass 2  two small scans turn the per-tile counts into offsets.
-//   pass 3  emit: stream 0 is written from the bitmap words (ranks are
-//           popcounts, consecutive lanes write consecutive addresses), or,
-//           for a tile whose every row is in it, as a plain transform; the
-//           sparse streams are recomputed only for tiles whose count is > 0.
+// The unit of work is a tile of 32 * K rows that one warp owns in every pass,
+// so no pass waits on another warp:
+//   pass 1  classify: a lane reads 16-byte vectors of consecutive rows, sets a
+//           bit per row of stream 0 in a register of its own, and three or so
+//           shuffles turn the lanes' bits into row-ordered bitmap words.  A
+//           vector's registers take the next load as soon as its rows have been
+//           evaluated, so that loads are always in flight.
+//   pass 2  scan: the per-tile counts become offsets (blocks of 1024 tiles; the
+//           last block to finish scans the group totals).
+//   pass 3  emit: the warp lists its kept rows in shared memory and writes
+//           stream 0 with consecutive lanes on consecutive positions; a tile
+//           whose every row is kept is a plain transform; the sparse streams are
+//           recomputed only for tiles that hold any.
+// Up to 32 small tiles one block does all three in one launch.
 //
-// Traffic beyond the input and the outputs: one bit per row written and read
-// back, plus re-reading the few tiles that hold errors.
+// K is 32 for long columns (fewest instructions per row) and 8 below 2^23 rows
+// (enough warps to fill the chip) and for operators whose every row waits on a
+// gather.  Measured on 600M 32-bit codes, a fifth selected: classify 367 us, the
+// copy bandwidth (2.4 GB; 459 us with a ballot per 32 rows, 20 instructions a
+// row instead of 8, and 450 fed through a shared-memory ring); emit 268 us for
+// 0.96 GB (660 us when a block walked 4096-row tiles without looking ahead): it
+// is bound by its ~380 instructions per 1024 rows.  Traffic beyond the input and the outputs: one bit per row, and 20
+// bytes per tile and stream, written and read back, plus re-reading the few
+// tiles with errors.
 #pragma once
 
 #include <type_traits>
@@ -26,12 +38,23 @@
 
 namespace ahead {
 
-constexpr int kCThreads = 256;  // threads per tile block
+constexpr int kCThreads = 256;  // threads per block
 constexpr int kCWarps = kCThreads / 32;
-constexpr int kCSteps = 16;  // rows per lane per tile
-constexpr int kTileRows = kCThreads * kCSteps;  // 4096
-constexpr int kTileWords = kTileRows / 32;      // 128 bitmap words per tile
-constexpr int kWarpWords = kTileWords / kCWarps;  // 16
+constexpr uint64_t kLongColumn = 1ull << 23;  // rows from which tiles are long
+constexpr uint32_t kOneBlockTiles = 32;       // up to here one block runs the whole compaction
+
+// Rows per lane of a tile: long ones, and short ones (at least one 16-byte vector).
+constexpr int kLongK = 32;
+constexpr int short_k(int w) { return w == 1 ? 16 : 8; }
+template <class Op>
+AHEAD_HD constexpr bool long_tiles(uint64_t n) {
+    return !Op::GATHER && n >= kLongColumn;
+}
+template <class Op>
+inline uint32_t compact_tiles(uint64_t n) {
+    const uint64_t r = 32 * (long_tiles<Op>(n) ? kLongK : short_k(Op::W));
+    return (uint32_t)((n + r - 1) / r);
+}
 
 template <int W>
 AHEAD_DEV uint64_t gmem_ld(const char* p, uint64_t i) {
@@ -41,70 +64,14 @@ AHEAD_DEV uint64_t gmem_ld(const char* p, uint64_t i) {
     return __ldg((const unsigned long long*)p + i);
 }
 
-// ------------------------------------------------------------ mbarrier / TMA
-AHEAD_DEV uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-AHEAD_DEV void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-AHEAD_DEV void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-AHEAD_DEV void mbar_arrive_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-                 "r"(bytes)
-                 : "memory");
-}
-AHEAD_DEV void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-AHEAD_DEV bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, "
-        "p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait (try_wait suspends for a hardware time slice per call); false
-// when it gave up.
-AHEAD_DEV bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    for (uint32_t i = 0; i < (1u << 22); ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
-// Bulk copy global -> shared (16-byte aligned addresses, size multiple of 16),
-// completion signalled on `bar` as transaction bytes.
-AHEAD_DEV void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_addr(dst)),
-        "l"(src), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
-}
-template <int W>
-AHEAD_DEV uint64_t smem_ld(const char* p, int i) {
-    if (W == 1) return ((const uint8_t*)p)[i];
-    if (W == 2) return ((const uint16_t*)p)[i];
-    if (W == 4) return ((const uint32_t*)p)[i];
-    return ((const unsigned long long*)p)[i];
-}
-
-// Stage ring of the TMA-fed classify pass: 64 KB per block.
-template <int W>
-struct RingCfg {
-    static constexpr int TILE_BYTES = kTileRows * W;
-    static constexpr int RAW = (64 * 1024) / TILE_BYTES;
-    static constexpr int STAGES = RAW < 2 ? 2 : (RAW > 8 ? 8 : RAW);
-    static constexpr int SMEM = STAGES * TILE_BYTES;
-};
-
 // Scratch of one compaction: bitmap words, per-tile counts and offsets.
 struct CompactBufs {
-    uint32_t* words;    // [ntiles * 128] stream-0 bitmap
-    uint32_t* counts;   // [ntiles][NCH], zeroed before pass 1
+    uint32_t* words;    // [ntiles * K] stream-0 bitmap
+    uint32_t* counts;   // [ntiles][NCH]
     uint64_t* offsets;  // [ntiles][NCH] exclusive offset within the tile's group
     uint64_t* gbase;    // [ngroups][NCH] exclusive offset of each group of 1024 tiles
     uint64_t* totals;   // [NCH]
+    uint32_t* done;     // blocks of the scan that have finished; zero between scans
     uint32_t ntiles;
     uint32_t nchan;
 };
@@ -113,33 +80,27 @@ constexpr int kScanGroup = 1024;  // tiles per first-level scan block
 
 AHEAD_HD uint32_t scan_groups(uint32_t ntiles) { return (ntiles + kScanGroup - 1) / kScanGroup; }
 
-inline size_t compact_bytes(uint32_t ntiles, uint32_t nchan) {
-    return (size_t)ntiles * kTileWords * 4 + (size_t)ntiles * nchan * 12 + (size_t)scan_groups(ntiles) * nchan * 8 +
-           2048;
+inline size_t compact_bytes(uint64_t n, uint32_t ntiles, uint32_t nchan) {
+    return (size_t)(n + 1023) / 1024 * 128 + (size_t)ntiles * nchan * 12 + (size_t)scan_groups(ntiles) * nchan * 8 +
+           4096;
 }
 
 // `Op` supplies
 //   static constexpr int W;     width in bytes of the driving column `base`
 //   static constexpr int NCH;   number of output streams (0 = kept rows)
 //   static constexpr bool ACC;  sum the eval accumulator into *op.acc
+//   static constexpr bool GATHER; eval loads from other places than row `row`
 //   static constexpr bool EMIT_V; stream 0 emission needs the driving value
 //   static constexpr int NOUT;  output columns written per stream-0 row
 //   const char* base;
-//   uint32_t* status;           device status word (timeouts)
 //   uint32_t eval(uint64_t v, uint64_t row, uint64_t& acc) const;  bit c = stream c
 //   uint64_t out0(int k, uint64_t v, uint64_t row) const;  k-th output of a kept row
-//   void put0(int k, uint64_t pos, uint64_t val) const;    store it at pos
+//   uint64_t cap0() const;      positions below it are stored
+//   void put0(int k, uint64_t pos, uint64_t val) const;    store it at pos < cap0()
 //   void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const;  streams c >= 1
 //
-// Row layout of a tile: warp w owns rows [512w, 512w+512); in step s each lane
-// holds one 16-byte vector of VEC = 16/W consecutive rows, row =
-// 512w + s*32*VEC + lane*VEC + k.  Stream 0's bitmap is kept in row order: bit
-// b of the warp's word j is row 512w + 32j + b.
-template <int W>
-struct Vec {
-    static constexpr int VEC = 16 / W;
-    static constexpr int STEPS = 512 / (32 * VEC);  // steps per warp per tile
-};
+// Row layout of a tile: with VEC = 16 / W rows per vector, lane l holds in
+// vector s the rows 32 * VEC * s + VEC * l + (0 .. VEC - 1) of the tile.
 
 template <int W>
 AHEAD_DEV void unpack16(const uint4 q, uint64_t (&v)[16 / W]) {
@@ -153,124 +114,200 @@ AHEAD_DEV void unpack16(const uint4 q, uint64_t (&v)[16 / W]) {
     }
 }
 
-// Pass 1: a persistent grid walks the tiles (tile = block + k * grid).  With
-// BULK, one thread streams the tiles into a ring of shared-memory stages with
-// cp.async.bulk several tiles ahead, so the bytes in flight cost no
-// registers; without it (unaligned column) lanes load rows directly.  Per-warp
-// counts go to the tile's counters with one atomic each.
-template <class Op, bool BULK>
-__global__ void __launch_bounds__(kCThreads) classify_kernel(Op op, uint64_t n, CompactBufs cb) {
-    constexpr int W = Op::W;
-    constexpr int NCH = Op::NCH;
-    constexpr int VEC = Vec<W>::VEC;
-    constexpr int STEPS = Vec<W>::STEPS;
-    typedef RingCfg<W> Ring;
-    extern __shared__ __align__(128) char s_ring[];
-    __shared__ __align__(8) uint64_t s_bar[8];
-    __shared__ int s_abort;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t total_bytes = n * W;
-    const uint32_t nmine = blockIdx.x < cb.ntiles ? (cb.ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+// The vectors a lane has in flight: half a long tile, all of a short one.
+template <int W, int K>
+struct Flight {
+    static constexpr int VEC = 16 / W;
+    static constexpr int NV = K / VEC;                       // vectors per tile
+    static constexpr int NF = NV > 1 && K == kLongK ? NV / 2 : NV;  // in flight
+    uint4 q[NF];
+    AHEAD_DEV static uint4 get(const char* base, uint64_t row, bool vec) {
+        if (vec) return __ldg(reinterpret_cast<const uint4*>(base + row * W));
+        uint32_t w[4] = {0, 0, 0, 0};  // a column that starts off a 16-byte boundary
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) {
+            const uint64_t x = gmem_ld<W>(base, row + k);
+            if (W == 8) {
+                w[2 * k] = (uint32_t)x;
+                w[2 * k + 1] = (uint32_t)(x >> 32);
+            } else {
+                w[k * W / 4] |= (uint32_t)x << (8 * (k * W % 4));
+            }
+        }
+        return make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    AHEAD_DEV void load(const char* base, uint64_t row, bool vec) {
+#pragma unroll
+        for (int s = 0; s < NF; ++s) q[s] = get(base, row + 32 * VEC * s, vec);
+    }
+};
 
-    auto issue = [&](uint32_t k) {  // start the copy of my k-th tile
-        const int st = k % Ring::STAGES;
-        const uint64_t off = (uint64_t)(blockIdx.x + k * gridDim.x) * Ring::TILE_BYTES;
-        const uint64_t rem = total_bytes - off;
-        const uint32_t bytes = (uint32_t)((rem < (uint64_t)Ring::TILE_BYTES ? rem : Ring::TILE_BYTES) & ~15ull);
-        if (bytes) {
-            mbar_arrive_tx(&s_bar[st], bytes);
-            bulk_g2s(s_ring + st * Ring::TILE_BYTES, op.base + off, bytes, &s_bar[st]);
-        } else {
-            mbar_arrive(&s_bar[st]);
+// Lanes' bits to row-ordered words.  Bit VEC * s + q of lane l's `bits` is row
+// 32 * VEC * s + VEC * l + q, so swapping the lane's low bits with s leaves the
+// word of 32 rows number (32 / LPW) * s + l / LPW, LPW = 32 / VEC lanes a word, in
+// lane LPW * (l / LPW) + s; a last shuffle brings word w to lane w.
+template <int VEC>
+AHEAD_DEV uint32_t words_of(uint32_t bits) {
+    constexpr int LPW = 32 / VEC;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 1; d < LPW; d <<= 1) {
+        const int j = VEC * d;  // the bit distance that lane distance d swaps with
+        // positions whose index has bit j clear
+        constexpr uint32_t all = 0xffffffffu;
+        const uint32_t m = j == 16 ? 0x0000ffffu : j == 8 ? 0x00ff00ffu : j == 4 ? 0x0f0f0f0fu : j == 2 ? 0x33333333u : all;
+        const uint32_t o = __shfl_xor_sync(kFull, bits, d);
+        bits = (lane & d) ? ((bits & ~m) | ((o >> j) & m)) : ((bits & m) | ((o & m) << j));
+    }
+    if (LPW == 1) return bits;
+    // word w = VEC * s + h (h = lane / LPW) sits in lane LPW * h + s
+    return __shfl_sync(kFull, bits, LPW * (lane % VEC) + lane / VEC);
+}
+
+// One tile's stream-0 words (lane s < K returns word s) and its counts (lane c
+// returns stream c's).  A whole tile's first vectors are in `f`; the tile
+// `next` (0: none) is loaded as registers free up.
+template <class Op, int K>
+AHEAD_DEV void tile_classify(const Op& op, uint64_t n, uint32_t tile, Flight<Op::W, K>& f, uint32_t next, bool vec,
+                             uint64_t& acc, uint32_t& word, uint32_t& count) {
+    typedef Flight<Op::W, K> F;
+    constexpr int VEC = F::VEC;
+    constexpr int NCH = Op::NCH;
+    const int lane = threadIdx.x & 31;
+    const uint64_t row0 = (uint64_t)tile * (32 * K) + VEC * lane;
+    uint32_t mine = 0, sparse[NCH];
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) sparse[c] = 0;
+    auto take = [&](uint32_t bits, int at) {
+        if (bits & 1u) mine |= 1u << at;
+#pragma unroll
+        for (int c = 1; c < NCH; ++c)
+            if (bits & (1u << c)) ++sparse[c];
+    };
+    if ((uint64_t)(tile + 1) * (32 * K) <= n) {
+#pragma unroll
+        for (int s = 0; s < F::NV; ++s) {
+            const uint64_t row = row0 + 32 * VEC * s;
+            uint64_t v[VEC];
+            unpack16<Op::W>(f.q[s % F::NF], v);
+            if (s + F::NF < F::NV) f.q[s % F::NF] = F::get(op.base, row + 32 * VEC * F::NF, vec);
+            else if (next)
+                f.q[s % F::NF] = F::get(op.base, (uint64_t)next * (32 * K) + VEC * lane + 32 * VEC * (s % F::NF), vec);
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) take(op.eval(v[q], row + q, acc), VEC * s + q);
+        }
+    } else {
+#pragma unroll
+        for (int s = 0; s < F::NV; ++s)
+            for (int q = 0; q < VEC; ++q) {
+                const uint64_t row = row0 + 32 * VEC * s + q;
+                if (row < n) take(op.eval(gmem_ld<Op::W>(op.base, row), row, acc), VEC * s + q);
+            }
+    }
+    word = words_of<VEC>(mine);
+    count = __reduce_add_sync(kFull, (uint32_t)__popc(mine));
+#pragma unroll
+    for (int c = 1; c < NCH; ++c) {
+        const uint32_t t = __reduce_add_sync(kFull, sparse[c]);
+        if (lane == c) count = t;
+    }
+}
+
+// Writes one tile's stream-0 rows to positions base, base + 1, ...: lane s < K
+// holds word s, `cnt` rows are kept, `list` is this warp's 32 * K half-words of
+// shared memory.  Four rows per lane are in flight at a time, since an output
+// may be a chain of gathers.
+template <class Op, int K>
+AHEAD_DEV void tile_emit(const Op& op, uint64_t n, uint32_t tile, uint32_t word, uint32_t cnt, uint64_t base,
+                         uint16_t* list) {
+    constexpr int W = Op::W;
+    constexpr int U = 4;
+    const int lane = threadIdx.x & 31;
+    const uint64_t trow0 = (uint64_t)tile * (32 * K);
+    const uint32_t trows = trow0 + 32 * K <= n ? (uint32_t)(32 * K) : (uint32_t)(n - trow0);
+    const bool all = cnt == trows;  // every row: position i is row i
+    if (!all) {  // lane l lists the kept ones of rows [K * l, K * l + K), the last one first
+        uint32_t h = word;
+        if (K < 32) h = (__shfl_sync(kFull, word, lane * K / 32) >> (lane * K % 32)) & ((1u << (K & 31)) - 1u);
+        uint16_t* at = list + warp_incl_scan(__popc(h));
+        while (h) {
+            const uint32_t b = 31 - __clz(h);
+            *--at = (uint16_t)(K * lane + b);
+            h ^= 1u << b;
+        }
+        __syncwarp();
+    }
+    const bool fits = base + cnt <= op.cap0();
+    auto rows = [&](auto fits_tag) {
+        constexpr bool FITS = decltype(fits_tag)::value;
+        for (uint32_t i0 = lane; i0 < cnt; i0 += 32 * U) {
+            uint64_t row[U], val[U][Op::NOUT];
+            typename std::conditional<W == 8, uint64_t, uint32_t>::type v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const uint32_t i = i0 + 32 * u;
+                row[u] = trow0 + (i < cnt ? (all ? i : list[i]) : 0u);
+                v[u] = Op::EMIT_V ? gmem_ld<W>(op.base, row[u]) : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i0 + 32 * u < cnt) {
+#pragma unroll
+                    for (int o = 0; o < Op::NOUT; ++o) val[u][o] = op.out0(o, v[u], row[u]);
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i0 + 32 * u < cnt && (FITS || base + i0 + 32 * u < op.cap0())) {
+#pragma unroll
+                    for (int o = 0; o < Op::NOUT; ++o) op.put0(o, base + i0 + 32 * u, val[u][o]);
+                }
         }
     };
-    if (BULK) {
-        if (threadIdx.x == 0) {
-            s_abort = 0;
-            for (int i = 0; i < Ring::STAGES; ++i) mbar_init(&s_bar[i], 1);
-            mbar_fence_init();
-            for (uint32_t k = 0; k < nmine && k < (uint32_t)Ring::STAGES; ++k) issue(k);
+    if (fits) rows(std::true_type());
+    else rows(std::false_type());
+    if (!all) __syncwarp();  // the list is reused
+}
+
+// Writes one tile's sparse streams: lane c holds stream c's count and position.
+template <class Op, int K>
+AHEAD_DEV void tile_emit_sparse(const Op& op, uint64_t n, uint32_t tile, uint64_t base) {
+    constexpr int W = Op::W;
+    const int lane = threadIdx.x & 31;
+    const uint64_t row0 = (uint64_t)tile * (32 * K) + lane;
+    uint64_t pos[Op::NCH];
+#pragma unroll
+    for (int c = 1; c < Op::NCH; ++c) pos[c] = __shfl_sync(kFull, base, c);
+    uint64_t dummy = 0;
+    for (int s = 0; s < K; ++s) {
+        const uint64_t row = row0 + 32 * s;
+        const uint64_t v = row < n ? gmem_ld<W>(op.base, row) : 0;
+        const uint32_t bits = row < n ? op.eval(v, row, dummy) : 0u;
+        if (!__any_sync(kFull, bits > 1u)) continue;
+#pragma unroll
+        for (int c = 1; c < Op::NCH; ++c) {
+            const uint32_t b = __ballot_sync(kFull, (bits >> c) & 1u);
+            if ((bits >> c) & 1u) op.emit(c, pos[c] + __popc(b & ((1u << lane) - 1u)), v, row);
+            pos[c] += __popc(b);
         }
-        __syncthreads();
     }
+}
+
+// Pass 1, `per` tiles per warp.
+template <class Op, int K>
+__global__ void __launch_bounds__(kCThreads) classify_kernel(Op op, uint64_t n, CompactBufs cb, int per) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool vec = ((uintptr_t)op.base & 15) == 0;
     uint64_t acc = 0;
-    for (uint32_t k = 0; k < nmine; ++k) {
-        const uint32_t tile = blockIdx.x + k * gridDim.x;
-        const uint64_t trow0 = (uint64_t)tile * kTileRows;
-        const char* tb = s_ring + (k % Ring::STAGES) * Ring::TILE_BYTES;
-        uint32_t in_smem = 0;  // rows of this tile that the bulk copy brought in
-        if (BULK) {
-            if (!mbar_wait(&s_bar[k % Ring::STAGES], (k / Ring::STAGES) & 1)) {
-                atomicOr(op.status, kDevStatusTimeout);
-                s_abort = 1;
-            }
-            const uint64_t rem = total_bytes - trow0 * W;
-            in_smem = (uint32_t)(((rem < (uint64_t)Ring::TILE_BYTES ? rem : Ring::TILE_BYTES) & ~15ull) / W);
-        }
-        uint32_t sparse[NCH];  // this lane's rows per stream
-#pragma unroll
-        for (int c = 0; c < NCH; ++c) sparse[c] = 0;
-        // Word j of the warp covers rows [32j, 32j+32) of its 512-row segment:
-        // in step s the lanes of group g = lane / (32/VEC) contribute word
-        // s*VEC + g, each its VEC bits at bit position VEC * (lane % (32/VEC)).
-        constexpr int LPW = 32 / VEC;  // lanes per word
-        uint32_t mine = 0;  // lane (s*VEC + g) keeps word (s, g)
-        auto step = [&](auto full_tag) {
-            constexpr bool FULL = decltype(full_tag)::value;
-#pragma unroll
-            for (int s = 0; s < STEPS; ++s) {
-                const uint32_t lr = warp * 512 + s * 32 * VEC + lane * VEC;
-                const uint64_t row0 = trow0 + lr;
-                uint64_t v[VEC];
-                if (BULK && (FULL || lr + VEC <= in_smem)) {
-                    unpack16<W>(*(const uint4*)(tb + (size_t)lr * W), v);
-                } else if (!BULK && (FULL || row0 + VEC <= n) && (((uintptr_t)op.base + row0 * W) & 15) == 0) {
-                    unpack16<W>(__ldg((const uint4*)(op.base + row0 * W)), v);
-                } else {
-#pragma unroll
-                    for (int q = 0; q < VEC; ++q) v[q] = (FULL || row0 + q < n) ? gmem_ld<W>(op.base, row0 + q) : 0;
-                }
-                uint32_t m0 = 0;
-#pragma unroll
-                for (int q = 0; q < VEC; ++q) {
-                    const uint32_t bits = (FULL || row0 + q < n) ? op.eval(v[q], row0 + q, acc) : 0u;
-                    m0 |= (bits & 1u) << q;
-#pragma unroll
-                    for (int c = 1; c < NCH; ++c) sparse[c] += (bits >> c) & 1u;
-                }
-                sparse[0] += __popc(m0);
-                uint32_t word = m0 << (VEC * (lane % LPW));
-#pragma unroll
-                for (int d = 1; d < LPW; d <<= 1) word |= __shfl_xor_sync(kFull, word, d);
-                // group g's word sits in all its lanes; lane s*VEC+g takes it
-                const uint32_t g = (uint32_t)(lane - s * VEC);
-                const uint32_t wv = __shfl_sync(kFull, word, (g < (uint32_t)VEC ? g : 0) * LPW);
-                if (g < (uint32_t)VEC) mine = wv;
-            }
-        };
-        const bool full = (BULK ? in_smem == (uint32_t)kTileRows : trow0 + kTileRows <= n);
-        if (full) step(std::true_type());
-        else step(std::false_type());
-        if (lane < kWarpWords) cb.words[(size_t)tile * kTileWords + warp * kWarpWords + lane] = mine;
-        const uint32_t c0 = __reduce_add_sync(kFull, sparse[0]);
-        uint32_t mycnt = (lane == 0) ? c0 : 0;
-#pragma unroll
-        for (int c = 1; c < NCH; ++c) {
-            const uint32_t t = __reduce_add_sync(kFull, sparse[c]);
-            if (lane == c) mycnt = t;
-        }
-        if (lane < NCH && mycnt) atomicAdd(&cb.counts[(size_t)tile * NCH + lane], mycnt);
-        if (BULK) {
-            __syncthreads();  // every warp is done with this stage
-            if (s_abort) {
-                // Wait (bounded) for the copies still in flight before leaving.
-                if (threadIdx.x == 0)
-                    for (uint32_t q = k + 1; q < nmine && q < k + Ring::STAGES; ++q)
-                        mbar_wait(&s_bar[q % Ring::STAGES], (q / Ring::STAGES) & 1);
-                break;
-            }
-            if (threadIdx.x == 0 && k + Ring::STAGES < nmine) issue(k + Ring::STAGES);
-        }
+    const uint32_t whole = (uint32_t)(n / (32 * K));  // whole tiles
+    uint32_t tile = blockIdx.x * per * kCWarps + warp;
+    Flight<Op::W, K> f;
+    if (tile < whole) f.load(op.base, (uint64_t)tile * (32 * K) + 16 / Op::W * lane, vec);
+    for (int k = 0; k < per && tile < cb.ntiles; ++k, tile += kCWarps) {
+        const uint32_t next = k + 1 < per && tile + kCWarps < whole ? tile + kCWarps : 0;
+        uint32_t word, count;
+        tile_classify<Op, K>(op, n, tile, f, next, vec, acc, word, count);
+        if (lane < K) cb.words[(size_t)tile * K + lane] = word;
+        if (lane < Op::NCH) cb.counts[(size_t)tile * Op::NCH + lane] = count;
     }
     if constexpr (Op::ACC) {
         acc = warp_sum64(acc);
@@ -278,184 +315,158 @@ __global__ void __launch_bounds__(kCThreads) classify_kernel(Op op, uint64_t n, 
     }
 }
 
-// Pass 2a: each block scans the counts of 1024 consecutive tiles per channel
-// (exclusive, within the group) and writes the group totals to gbase.
-static __global__ void __launch_bounds__(kScanGroup) tile_scan_kernel(CompactBufs cb) {
-    __shared__ uint64_t s_part[32];
-    const uint32_t nch = cb.nchan;
+// Exclusive scan of one value per thread over a block of 1024; *total by every thread.
+AHEAD_DEV uint64_t block_scan_1024(uint64_t x, uint64_t* s_part, uint64_t* total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t t = blockIdx.x * kScanGroup + threadIdx.x;
-    for (uint32_t c = 0; c < nch; ++c) {
-        const uint64_t x = t < cb.ntiles ? cb.counts[(size_t)t * nch + c] : 0;
-        const uint64_t incl = warp_incl_scan64(x);
-        if (lane == 31) s_part[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            const uint64_t p = s_part[lane];
-            const uint64_t pi = warp_incl_scan64(p);
-            s_part[lane] = pi - p;
-            if (lane == 31) cb.gbase[(size_t)blockIdx.x * nch + c] = pi;
-        }
-        __syncthreads();
-        if (t < cb.ntiles) cb.offsets[(size_t)t * nch + c] = s_part[warp] + incl - x;
-        __syncthreads();
+    const uint64_t incl = warp_incl_scan64(x);
+    if (lane == 31) s_part[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        const uint64_t p = s_part[lane];
+        const uint64_t pi = warp_incl_scan64(p);
+        s_part[lane] = pi - p;
+        if (lane == 31) s_part[32] = pi;
     }
+    __syncthreads();
+    const uint64_t r = s_part[warp] + incl - x;
+    *total = s_part[32];
+    __syncthreads();
+    return r;
 }
 
-// Pass 2b: one block turns the group totals into exclusive group offsets.
-static __global__ void __launch_bounds__(1024) group_scan_kernel(CompactBufs cb) {
-    __shared__ uint64_t s_part[32];
-    const uint32_t ng = scan_groups(cb.ntiles), nch = cb.nchan;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// Pass 2: each block scans the counts of 1024 consecutive tiles per stream
+// (exclusive, within the group; three streams' counts of at most 1024 share a
+// 64-bit word, 21 bits each) and writes the group totals to gbase; the last
+// block to finish turns those into exclusive group offsets, a warp per stream
+// while they are few.  (As two kernels, each scanning stream after stream, this
+// took 10-14 us of every operator with up to a few thousand tiles.)
+static __global__ void __launch_bounds__(kScanGroup) tile_scan_kernel(CompactBufs cb) {
+    __shared__ uint64_t s_part[33];
+    __shared__ bool s_last;
+    const uint32_t nch = cb.nchan, ng = scan_groups(cb.ntiles);
+    const uint32_t t = blockIdx.x * kScanGroup + threadIdx.x;
+    for (uint32_t c0 = 0; c0 < nch; c0 += 3) {
+        const uint32_t m = nch - c0 < 3 ? nch - c0 : 3;
+        const uint64_t part = m == 1 ? ~0ull : (1ull << 21) - 1;  // (a single stream's counts may be larger)
+        uint64_t x = 0;
+        if (t < cb.ntiles)
+            for (uint32_t c = 0; c < m; ++c) x |= (uint64_t)cb.counts[(size_t)t * nch + c0 + c] << (21 * c);
+        uint64_t total;
+        const uint64_t ex = block_scan_1024(x, s_part, &total);
+        if (t < cb.ntiles)
+            for (uint32_t c = 0; c < m; ++c) cb.offsets[(size_t)t * nch + c0 + c] = (ex >> (21 * c)) & part;
+        if (threadIdx.x < m) {
+            const uint64_t tot = (total >> (21 * threadIdx.x)) & part;
+            cb.gbase[(size_t)blockIdx.x * nch + c0 + threadIdx.x] = ng == 1 ? 0 : tot;
+            if (ng == 1) cb.totals[c0 + threadIdx.x] = tot;
+        }
+    }
+    if (ng == 1) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(cb.done, 1u) == gridDim.x - 1;
+        if (s_last) *cb.done = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (ng <= 128) {
+        if (warp >= nch) return;
+        uint64_t carry = 0;
+        for (uint32_t g0 = 0; g0 < ng; g0 += 32) {
+            const uint32_t g = g0 + lane;
+            uint64_t* p = cb.gbase + (size_t)g * nch + warp;
+            const uint64_t x = g < ng ? __ldcg((const unsigned long long*)p) : 0;
+            const uint64_t incl = warp_incl_scan64(x);
+            if (g < ng) *p = carry + incl - x;
+            carry += __shfl_sync(kFull, incl, 31);
+        }
+        if (lane == 0) cb.totals[warp] = carry;
+        return;
+    }
     for (uint32_t c = 0; c < nch; ++c) {
         uint64_t carry = 0;
-        for (uint32_t g0 = 0; g0 < ng; g0 += 1024) {
+        for (uint32_t g0 = 0; g0 < ng; g0 += kScanGroup) {
             const uint32_t g = g0 + threadIdx.x;
-            const uint64_t x = g < ng ? cb.gbase[(size_t)g * nch + c] : 0;
-            const uint64_t incl = warp_incl_scan64(x);
-            if (lane == 31) s_part[warp] = incl;
-            __syncthreads();
-            if (warp == 0) {
-                const uint64_t p = s_part[lane];
-                s_part[lane] = warp_incl_scan64(p) - p;
-            }
-            __syncthreads();
-            const uint64_t ex = carry + s_part[warp] + incl - x;
-            __syncthreads();
-            if (g < ng) cb.gbase[(size_t)g * nch + c] = ex;
-            if (threadIdx.x == blockDim.x - 1) s_part[0] = ex + x;
-            __syncthreads();
-            carry = s_part[0];
-            __syncthreads();
+            const uint64_t x = g < ng ? __ldcg((const unsigned long long*)&cb.gbase[(size_t)g * nch + c]) : 0;
+            uint64_t total;
+            const uint64_t ex = block_scan_1024(x, s_part, &total);
+            if (g < ng) cb.gbase[(size_t)g * nch + c] = carry + ex;
+            carry += total;
         }
         if (threadIdx.x == 0) cb.totals[c] = carry;
     }
 }
 
-// Pass 3: a persistent grid writes the streams.  Stream 0 comes from the
-// bitmap; each warp derives its offset inside the tile from the popcounts of
-// the preceding warps' words, ranks the rows of a step with one warp scan of
-// the lanes' counts, stages the outputs in shared memory and writes them with
-// full-width stores.  Sparse streams are recomputed only for tiles that hold
-// any (block-uniform branch).
-template <class Op>
-__global__ void __launch_bounds__(kCThreads, 4) emit_kernel(Op op, uint64_t n, CompactBufs cb) {
-    constexpr int W = Op::W;
+// Pass 3, `per` tiles per warp; the next tile's header and words are loaded
+// before this one's rows are written.
+template <class Op, int K>
+__global__ void __launch_bounds__(kCThreads) emit_kernel(Op op, uint64_t n, CompactBufs cb, int per) {
     constexpr int NCH = Op::NCH;
-    constexpr int VEC = Vec<W>::VEC;
-    constexpr int STEPS = Vec<W>::STEPS;
-    __shared__ uint32_t s_sc[NCH][kCWarps];
-    __shared__ uint16_t s_rows[kCWarps][512];
+    __shared__ uint16_t s_rows[kCWarps][32 * K];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t tile = blockIdx.x; tile < cb.ntiles; tile += gridDim.x) {
-        const uint32_t* counts = cb.counts + (size_t)tile * NCH;
-        const uint64_t* offs = cb.offsets + (size_t)tile * NCH;
-        const uint64_t* gb = cb.gbase + (size_t)(tile / kScanGroup) * NCH;
-        const uint64_t trow0 = (uint64_t)tile * kTileRows;
-        // the tile's header and bitmap words in one round trip
-        const uint32_t* tw = cb.words + (size_t)tile * kTileWords;
-        const uint32_t cnt0 = counts[0];
-        const uint64_t base0 = offs[0] + gb[0];
-        uint32_t tws[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) tws[q] = tw[lane + 32 * q];
-        const uint32_t hw = tw[warp * kWarpWords + (lane >> 1)];
-        const uint32_t trows = trow0 + kTileRows <= n ? (uint32_t)kTileRows : (uint32_t)(n - trow0);
-        if (cnt0 == trows) {
-            // every row of the tile is in stream 0: output i is row i, a plain
-            // coalesced transform with all of a thread's loads in flight together
-            uint64_t v[kCSteps];
-#pragma unroll
-            for (int k = 0; k < kCSteps; ++k) {
-                const uint32_t i = threadIdx.x + k * kCThreads;
-                v[k] = (Op::EMIT_V && i < trows) ? gmem_ld<W>(op.base, trow0 + i) : 0;
-            }
-#pragma unroll
-            for (int k = 0; k < kCSteps; ++k) {
-                const uint32_t i = threadIdx.x + k * kCThreads;
-                if (i < trows)
-#pragma unroll
-                    for (int o = 0; o < Op::NOUT; ++o) op.put0(o, base0 + i, op.out0(o, v[k], trow0 + i));
-            }
-        } else if (cnt0) {
-            uint32_t before = 0;  // kept rows of the preceding warps
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int wi = lane + 32 * q;
-                if (wi < warp * kWarpWords) before += __popc(tws[q]);
-            }
-            before = __reduce_add_sync(kFull, before);
-            // Lane l owns rows [16l, 16l+16) of the warp's segment: half of word l/2.
-            uint32_t h = (hw >> (16 * (lane & 1))) & 0xffffu;
-            const uint32_t c = __popc(h);
-            const uint32_t incl = warp_incl_scan(c);
-            const uint32_t tot = __shfl_sync(kFull, incl, 31);
-            uint32_t r = incl - c;
-            while (h) {  // stage the kept rows' segment offsets in row order
-                const uint32_t bit = __ffs(h) - 1;
-                h &= h - 1;
-                s_rows[warp][r++] = (uint16_t)(16 * lane + bit);
-            }
-            __syncwarp();
-            const uint64_t base = base0 + before;
-            const uint64_t srow = trow0 + (uint64_t)warp * 512;
-            for (uint32_t i = lane; i < tot; i += 32) {
-                const uint64_t row = srow + s_rows[warp][i];
-                const uint64_t v = Op::EMIT_V ? gmem_ld<W>(op.base, row) : 0;
-#pragma unroll
-                for (int o = 0; o < Op::NOUT; ++o) op.put0(o, base + i, op.out0(o, v, row));
-            }
-            __syncwarp();
+    auto tile_of = [&](int k) { return (blockIdx.x * per + k) * kCWarps + warp; };
+    uint32_t word = 0, count = 0;
+    uint64_t base = 0;
+    auto head = [&](uint32_t tile) {
+        word = count = 0;
+        base = 0;
+        if (tile >= cb.ntiles) return;
+        if (lane < K) word = __ldg(cb.words + (size_t)tile * K + lane);
+        if (lane < NCH) {
+            count = __ldg(cb.counts + (size_t)tile * NCH + lane);
+            base = __ldg((const unsigned long long*)cb.offsets + (size_t)tile * NCH + lane) +
+                   __ldg((const unsigned long long*)cb.gbase + (size_t)(tile / kScanGroup) * NCH + lane);
         }
-        if constexpr (NCH > 1) {
-            bool any = false;
+    };
+    head(tile_of(0));
+    for (int k = 0; k < per; ++k) {
+        const uint32_t tile = tile_of(k);
+        if (tile >= cb.ntiles) break;
+        const uint32_t w = word, c = count;
+        const uint64_t b = base;
+        if (k + 1 < per) head(tile_of(k + 1));
+        const uint32_t c0 = __shfl_sync(kFull, c, 0);
+        if (c0) tile_emit<Op, K>(op, n, tile, w, c0, __shfl_sync(kFull, b, 0), s_rows[warp]);
+        if constexpr (NCH > 1)
+            if (__any_sync(kFull, lane > 0 && c)) tile_emit_sparse<Op, K>(op, n, tile, b);
+    }
+}
+
+// All passes in one block, for up to kOneBlockTiles short tiles: warp w owns tile w.
+template <class Op>
+__global__ void __launch_bounds__(kOneBlockTiles * 32) compact_one_kernel(Op op, uint64_t n, CompactBufs cb) {
+    constexpr int NCH = Op::NCH;
+    constexpr int K = short_k(Op::W);
+    __shared__ uint16_t s_rows[kOneBlockTiles][32 * K];
+    __shared__ uint32_t s_cnt[NCH][kOneBlockTiles];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool vec = ((uintptr_t)op.base & 15) == 0;
+    uint32_t word = 0, count = 0;
+    uint64_t acc = 0;
+    Flight<Op::W, K> f;
+    if ((uint64_t)(warp + 1) * (32 * K) <= n) f.load(op.base, (uint64_t)warp * (32 * K) + 16 / Op::W * lane, vec);
+    tile_classify<Op, K>(op, n, warp, f, 0, vec, acc, word, count);
+    if (lane < NCH) s_cnt[lane][warp] = count;
+    __syncthreads();
+    uint64_t base = 0;
 #pragma unroll
-            for (int c = 1; c < NCH; ++c) any |= counts[c] != 0;
-            if (any) {
-                // Recompute the tile; bits[s] holds, per slot q, the stream bits.
-                uint32_t bits[STEPS][VEC];
-                uint32_t wc[NCH];
-#pragma unroll
-                for (int c = 0; c < NCH; ++c) wc[c] = 0;
-                uint64_t dummy = 0;
-#pragma unroll
-                for (int s = 0; s < STEPS; ++s) {
-                    const uint64_t row0 = trow0 + warp * 512 + s * 32 * VEC + lane * VEC;
-#pragma unroll
-                    for (int q = 0; q < VEC; ++q) {
-                        bits[s][q] = row0 + q < n ? op.eval(gmem_ld<W>(op.base, row0 + q), row0 + q, dummy) : 0u;
-#pragma unroll
-                        for (int c = 1; c < NCH; ++c) wc[c] += (bits[s][q] >> c) & 1u;
-                    }
-                }
-#pragma unroll
-                for (int c = 1; c < NCH; ++c) wc[c] = __reduce_add_sync(kFull, wc[c]);
-                __syncthreads();
-                if (lane == 0)
-#pragma unroll
-                    for (int c = 1; c < NCH; ++c) s_sc[c][warp] = wc[c];
-                __syncthreads();
-#pragma unroll
-                for (int c = 1; c < NCH; ++c) {
-                    if (!counts[c]) continue;
-                    uint64_t pos = offs[c] + gb[c];
-                    for (int k = 0; k < warp; ++k) pos += s_sc[c][k];
-#pragma unroll
-                    for (int s = 0; s < STEPS; ++s) {
-                        uint32_t cl = 0;
-#pragma unroll
-                        for (int q = 0; q < VEC; ++q) cl += (bits[s][q] >> c) & 1u;
-                        const uint32_t incl = warp_incl_scan(cl);
-                        uint64_t p = pos + incl - cl;
-                        const uint64_t row0 = trow0 + warp * 512 + s * 32 * VEC + lane * VEC;
-#pragma unroll
-                        for (int q = 0; q < VEC; ++q)
-                            if ((bits[s][q] >> c) & 1u) op.emit(c, p++, gmem_ld<W>(op.base, row0 + q), row0 + q);
-                        pos += __shfl_sync(kFull, incl, 31);
-                    }
-                }
-            }
-        }
+    for (int c = 0; c < NCH; ++c) {
+        const uint32_t x = lane < (int)(blockDim.x >> 5) ? s_cnt[c][lane] : 0;
+        const uint32_t before = __reduce_add_sync(kFull, lane < warp ? x : 0u);
+        const uint32_t total = __reduce_add_sync(kFull, x);
+        if (lane == c) base = before;
+        if (threadIdx.x == 0) cb.totals[c] = total;
+    }
+    const uint32_t c0 = __shfl_sync(kFull, count, 0);
+    if (c0) tile_emit<Op, K>(op, n, warp, word, c0, __shfl_sync(kFull, base, 0), s_rows[warp]);
+    if constexpr (NCH > 1)
+        if (__any_sync(kFull, lane > 0 && lane < NCH && count)) tile_emit_sparse<Op, K>(op, n, warp, base);
+    if constexpr (Op::ACC) {
+        acc = warp_sum64(acc);
+        if (lane == 0 && acc) atomicAdd((unsigned long long*)op.acc, (unsigned long long)acc);
     }
 }
 

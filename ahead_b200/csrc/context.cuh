@@ -30,6 +30,7 @@ struct ahead_ctx {
 namespace ahead {
 
 constexpr int kStageWords = 64;
+constexpr int kScanDone = 61;  // counter word of tile_scan_kernel
 
 // noalloc.cu: drop the cached scratch address of a device (a new context may
 // follow a device reset).
@@ -92,19 +93,19 @@ struct OpScope {
         return p;
     }
 
-    // Compaction scratch for `ntiles` tiles and `nchan` streams; the stream
-    // totals land in d_counters[first_counter ...].  Only the per-tile counts
-    // need clearing; every other word is written before it is read.
-    CompactBufs compact_bufs(uint32_t ntiles, uint32_t nchan, int first_counter) {
+    // Compaction scratch for n rows in `ntiles` tiles and `nchan` streams; the stream
+    // totals land in d_counters[first_counter ...].  Every word is written
+    // before it is read; the scan's `done` word leaves each scan as zero.
+    CompactBufs compact_bufs(uint64_t n, uint32_t ntiles, uint32_t nchan, int first_counter) {
         CompactBufs cb;
-        cb.words = (uint32_t*)alloc((size_t)ntiles * kTileWords * 4);
+        cb.words = (uint32_t*)alloc((size_t)(n + 1023) / 1024 * 128);
         cb.counts = (uint32_t*)alloc((size_t)ntiles * nchan * 4);
         cb.offsets = (uint64_t*)alloc((size_t)ntiles * nchan * 8);
         cb.gbase = (uint64_t*)alloc((size_t)scan_groups(ntiles) * nchan * 8);
         cb.totals = d_counters + first_counter;
+        cb.done = (uint32_t*)(d_counters + kScanDone);
         cb.ntiles = ntiles;
         cb.nchan = nchan;
-        cudaMemsetAsync(cb.counts, 0, (size_t)ntiles * nchan * 4, ctx->stream);
         return cb;
     }
 
@@ -179,8 +180,6 @@ inline uint64_t inv_pow2(uint64_t a, int bits) {
     return x & wmask(bits / 8);
 }
 
-inline uint32_t compact_tiles(uint64_t n) { return (uint32_t)((n + kTileRows - 1) / kTileRows); }
-
 // A kernel's dynamic shared-memory limit is a function attribute of each
 // device: set it once per device (the context's, current in the calling
 // thread), tracked per kernel in a set of devices 0..63 (beyond that it is
@@ -199,42 +198,47 @@ inline bool dyn_smem_ready(const ahead_ctx* ctx, int bytes) {
     return true;
 }
 
-// Pass 1 of a compaction: the bulk-copy fed classify kernel for 16-byte
-// aligned columns (when its shared memory could be granted), else the one
-// that loads rows directly.
+// Launch one compaction over n rows with its scratch in `cb`; returns the
+// number of launches.  Few tiles: one block does everything (the separate
+// launches of almost no work each cost 15 us at 2,556 rows, the one 5).  Else 1
+// to 8 tiles per warp, so that the grid keeps about eight blocks per SM busy.
 template <class Op>
-inline void launch_classify(const ahead_ctx* ctx, cudaStream_t st, const Op& op, uint64_t n, const CompactBufs& cb) {
+inline int launch_compact(const ahead_ctx* ctx, cudaStream_t st, const Op& op, uint64_t n, const CompactBufs& cb) {
     const uint32_t nt = cb.ntiles;
-    constexpr int smem = RingCfg<Op::W>::SMEM;
-    if (((uintptr_t)op.base & 15) == 0 && dyn_smem_ready<classify_kernel<Op, true>>(ctx, smem)) {
-        const uint32_t g2 = nt < (uint32_t)ctx->num_sms * 3 ? nt : (uint32_t)ctx->num_sms * 3;
-        classify_kernel<Op, true><<<g2, kCThreads, smem, st>>>(op, n, cb);
-    } else {
-        const uint32_t cap = (uint32_t)ctx->num_sms * 8;
-        classify_kernel<Op, false><<<nt < cap ? nt : cap, kCThreads, 0, st>>>(op, n, cb);
+    if (nt <= kOneBlockTiles && !long_tiles<Op>(n)) {
+        compact_one_kernel<Op><<<1, nt * 32, 0, st>>>(op, n, cb);
+        return 1;
     }
+    const uint32_t fill = (uint32_t)ctx->num_sms * 8 * kCWarps;
+    const uint32_t per = nt / fill < 1 ? 1 : nt / fill > 8 ? 8 : nt / fill;
+    const uint32_t grid = (nt + per * kCWarps - 1) / (per * kCWarps);
+    auto passes = [&](auto k_tag) {
+        constexpr int K = decltype(k_tag)::value;
+        classify_kernel<Op, K><<<grid, kCThreads, 0, st>>>(op, n, cb, (int)per);
+        tile_scan_kernel<<<scan_groups(nt), kScanGroup, 0, st>>>(cb);
+        emit_kernel<Op, K><<<grid, kCThreads, 0, st>>>(op, n, cb, (int)per);
+    };
+    if constexpr (!Op::GATHER)
+        if (long_tiles<Op>(n)) {
+            passes(std::integral_constant<int, kLongK>());
+            return 3;
+        }
+    passes(std::integral_constant<int, short_k(Op::W)>());
+    return 3;
 }
 
-// Launch one compaction over n rows (classify, scan, emit); totals land in
-// counters [c0, c0+NCH).
+// A compaction of an operator call; totals land in counters [c0, c0 + NCH).
 template <class Op>
 inline void run_compact(OpScope& s, const Op& op, uint64_t n, int c0) {
     if (n == 0) return;
-    const uint32_t nt = compact_tiles(n);
-    CompactBufs cb = s.compact_bufs(nt, Op::NCH, c0);
-    const uint32_t cap = (uint32_t)s.ctx->num_sms * 8;
-    const uint32_t grid = nt < cap ? nt : cap;
-    launch_classify(s.ctx, s.ctx->stream, op, n, cb);
-    tile_scan_kernel<<<scan_groups(nt), kScanGroup, 0, s.ctx->stream>>>(cb);
-    group_scan_kernel<<<1, 1024, 0, s.ctx->stream>>>(cb);
-    emit_kernel<Op><<<grid, kCThreads, 0, s.ctx->stream>>>(op, n, cb);
-    s.launched(4);
+    const CompactBufs cb = s.compact_bufs(n, compact_tiles<Op>(n), Op::NCH, c0);
+    s.launched(launch_compact(s.ctx, s.ctx->stream, op, n, cb));
 }
 
 template <class Op>
 inline size_t compact_scratch(uint64_t n) {
     if (n == 0) return 0;
-    return compact_bytes(compact_tiles(n), Op::NCH) + 1024;
+    return compact_bytes(n, compact_tiles<Op>(n), Op::NCH) + 1024;
 }
 
 }  // namespace ahead

@@ -26,8 +26,8 @@
 //     (one stream, or wait for the previous call to return -- each call
 //     returns only after its stream has finished); overlapping calls race;
 //   * what must start at zero: the status word and the counters (first 512
-//     bytes) and the per-tile counts; each call clears them with
-//     cudaMemsetAsync on the context's stream before its kernels run.
+//     bytes); each call clears them with cudaMemsetAsync on the context's
+//     stream before its kernels run.
 // Results are those of ahead_gpu_check_an (checkAN, encdecAN_scalar.tcc:
 // 69-94): the positions row * AOID of the codes whose decoded value exceeds the
 // largest unencoded value.  The reference has no such entry point.
@@ -40,10 +40,12 @@ using namespace ahead;
 namespace {
 
 constexpr uint64_t kNoAllocMaxRows = 1ull << 24;
-constexpr uint32_t kNoAllocTiles = (uint32_t)(kNoAllocMaxRows / kTileRows);
+// tiles of the longest column in short tiles, of the longest below the long ones' first length
+constexpr uint32_t kNoAllocTiles = (uint32_t)(kLongColumn / (32 * short_k(8)));
+static_assert(kNoAllocMaxRows / (32 * kLongK) <= kNoAllocTiles, "long tiles need no more");
 constexpr size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 constexpr size_t kHeadBytes = 512;  // status word (8 B) + counters
-constexpr size_t kWordsBytes = align256((size_t)kNoAllocTiles * kTileWords * 4);
+constexpr size_t kWordsBytes = align256((size_t)(kNoAllocMaxRows / 8));
 constexpr size_t kCountsBytes = align256((size_t)kNoAllocTiles * 4);
 constexpr size_t kOffsetsBytes = align256((size_t)kNoAllocTiles * 8);
 constexpr size_t kGbaseBytes = align256(((kNoAllocTiles + kScanGroup - 1) / kScanGroup) * 8);
@@ -99,17 +101,16 @@ int check_noalloc(ahead_ctx* ctx, unsigned char* scratch, const ahead_bat* in, u
     cudaError_t e = cudaMemsetAsync(scratch, 0, kHeadBytes, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemsetAsync");
     if (n) {
-        const uint32_t nt = compact_tiles(n);
+        const uint32_t nt = compact_tiles<Op>(n);
         CompactBufs cb;
         cb.words = reinterpret_cast<uint32_t*>(scratch + kHeadBytes);
         cb.counts = reinterpret_cast<uint32_t*>(scratch + kHeadBytes + kWordsBytes);
         cb.offsets = reinterpret_cast<uint64_t*>(scratch + kHeadBytes + kWordsBytes + kCountsBytes);
         cb.gbase = reinterpret_cast<uint64_t*>(scratch + kHeadBytes + kWordsBytes + kCountsBytes + kOffsetsBytes);
         cb.totals = counters;
+        cb.done = reinterpret_cast<uint32_t*>(counters + kScanDone);
         cb.ntiles = nt;
         cb.nchan = Op::NCH;
-        e = cudaMemsetAsync(cb.counts, 0, (size_t)nt * Op::NCH * 4, st);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemsetAsync");
         Op op;
         op.base = (const char*)in->tail.data;
         op.status = status;
@@ -119,13 +120,7 @@ int check_noalloc(ahead_ctx* ctx, unsigned char* scratch, const ahead_bat* in, u
         op.err = edata(err);
         op.errcap = ecap(err);
         op.acc = nullptr;
-        const uint32_t cap = (uint32_t)ctx->num_sms * 8;
-        const uint32_t grid = nt < cap ? nt : cap;
-        launch_classify(ctx, st, op, n, cb);
-        tile_scan_kernel<<<scan_groups(nt), kScanGroup, 0, st>>>(cb);
-        group_scan_kernel<<<1, 1024, 0, st>>>(cb);
-        emit_kernel<Op><<<grid, kCThreads, 0, st>>>(op, n, cb);
-        ctx->launches += 4;
+        ctx->launches += launch_compact(ctx, st, op, n, cb);
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");

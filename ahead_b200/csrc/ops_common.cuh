@@ -46,6 +46,7 @@ struct CheckOp {
     static constexpr int W = WW;
     static constexpr int NCH = 1;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = false;
     const char* base;
     uint32_t* status;
     uint64_t ainv, umax, aoid, errcap;
@@ -57,8 +58,9 @@ struct CheckOp {
         return mulw(v, ainv, W) > umax ? 1u : 0u;
     }
     AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row * aoid; }
+    AHEAD_DEV uint64_t cap0() const { return errcap; }
     AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        if (pos < errcap) err[pos] = val;
+        err[pos] = val;
     }
     AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
         if (pos < errcap) err[pos] = row * aoid;
@@ -74,6 +76,7 @@ struct ColCheckOp {
     static constexpr int W = WW;
     static constexpr int NCH = 1;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = false;
     static constexpr bool EMIT_V = false;
     static constexpr int NOUT = 1;
     const char* base;
@@ -83,15 +86,16 @@ struct ColCheckOp {
     uint64_t* acc;
     AHEAD_DEV uint32_t eval(uint64_t v, uint64_t, uint64_t&) const { return ((v * ainv) & wmaskenc) > umax ? 1u : 0u; }
     AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row * aoid; }
+    AHEAD_DEV uint64_t cap0() const { return errcap; }
     AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        if (pos < errcap) err[pos] = val;
+        err[pos] = val;
     }
     AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
         if (pos < errcap) err[pos] = row * aoid;
     }
 };
 
-inline size_t colcheck_scratch(uint64_t n) { return n ? compact_bytes(compact_tiles(n), 1) + 1024 : 0; }
+inline size_t colcheck_scratch(uint64_t n) { return compact_scratch<ColCheckOp<8>>(n); }
 
 // Launch the column check; the error count lands in counter `ci`.
 inline void run_colcheck(OpScope& s, const ahead_col& c, uint64_t n, uint64_t ainv, uint64_t umax, int wenc,

@@ -44,6 +44,7 @@ struct FirstOp {
     static constexpr int W = 4;
     static constexpr int NCH = 1;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = true;
     static constexpr bool EMIT_V = false;
     static constexpr int NOUT = 1;
     const char* base;
@@ -57,6 +58,7 @@ struct FirstOp {
     int decode_head;
     AHEAD_DEV uint32_t eval(uint64_t v, uint64_t row, uint64_t&) const { return first[v] == (uint32_t)row ? 1u : 0u; }
     AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row; }
+    AHEAD_DEV uint64_t cap0() const { return ~0ull; }  // (every group gets its id)
     AHEAD_DEV void put0(int, uint64_t pos, uint64_t row) const {
         const uint32_t s = ((const uint32_t*)base)[row];
         gid_of_slot[s] = (uint32_t)pos;
@@ -516,6 +518,7 @@ struct FirstPlainOp {
     static constexpr int W = 4;
     static constexpr int NCH = 1;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = true;
     static constexpr bool EMIT_V = false;
     static constexpr int NOUT = 1;
     const char* base;
@@ -528,6 +531,7 @@ struct FirstPlainOp {
     uint64_t* acc;
     AHEAD_DEV uint32_t eval(uint64_t v, uint64_t row, uint64_t&) const { return first[v] == (uint32_t)row ? 1u : 0u; }
     AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row; }
+    AHEAD_DEV uint64_t cap0() const { return ~0ull; }  // (every group gets its id)
     AHEAD_DEV void put0(int, uint64_t pos, uint64_t row) const {
         const uint32_t s = ((const uint32_t*)base)[row];
         gid_of_slot[s] = (uint32_t)pos;

@@ -94,6 +94,7 @@ AHEAD_DEV void join_emit(const JoinOut& o, uint64_t pos, uint64_t prow, uint64_t
 }
 
 constexpr int kProbeRowsPerThread = 16;
+constexpr int kProbeTile = 256 * kProbeRowsPerThread;  // probe rows per block and step
 // a probe row's entry: kNoSlot, the single matching build row | kDirect, or
 // the slot of a key with several build rows
 constexpr uint32_t kDirect = 0x80000000u;
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(256) probe_count_kernel(const ProbeSlot* __res
         uint32_t c = 0;
 #pragma unroll 4
         for (int k = 0; k < kProbeRowsPerThread; ++k) {
-            const uint64_t row = (uint64_t)tile * kTileRows + k * 256 + threadIdx.x;
+            const uint64_t row = (uint64_t)tile * kProbeTile + k * 256 + threadIdx.x;
             if (row >= n) break;
             uint64_t key = 0;
             uint32_t s = kNoSlot;
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(256) probe_emit_kernel(const ProbeSlot* __rest
     __shared__ uint32_t s_w[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (uint32_t tile = blockIdx.x; tile < cb.ntiles; tile += gridDim.x) {
-        const uint64_t r0 = (uint64_t)tile * kTileRows + (uint64_t)threadIdx.x * kProbeRowsPerThread;
+        const uint64_t r0 = (uint64_t)tile * kProbeTile + (uint64_t)threadIdx.x * kProbeRowsPerThread;
         uint32_t c = 0;
         for (int k = 0; k < kProbeRowsPerThread; ++k) {
             const uint64_t row = r0 + k;
@@ -180,8 +181,9 @@ __global__ void __launch_bounds__(256) probe_emit_kernel(const ProbeSlot* __rest
 
 size_t join_scratch(uint64_t nb, uint64_t np) {
     const uint64_t cap = ht_capacity(nb) + 1;
-    return cap * (8 + 4 + 4 + 4 + 8 + 16) + 256 + nb * 8 + np * 4 + compact_bytes(compact_tiles(cap), 1) +
-           compact_bytes(compact_tiles(np), 1) + 8 * 1024;
+    const uint64_t nt = (np + kProbeTile - 1) / kProbeTile;
+    return cap * (8 + 4 + 4 + 4 + 8 + 16) + 256 + nb * 8 + np * 4 + (scan_groups(cap) + 1) * 8 + nt * 12 +
+           (scan_groups(nt) + 1) * 8 + 16 * 1024;
 }
 
 // Build on `bk` (nb rows), probe with `pk` (np rows); the output total lands
@@ -211,10 +213,10 @@ void run_hash_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk, 
     sb.offsets = (uint64_t*)s.alloc((size_t)(cap + 1) * 8);
     sb.gbase = (uint64_t*)s.alloc((size_t)scan_groups(cap + 1) * 8);
     sb.totals = s.d_counters + 60;
+    sb.done = (uint32_t*)(s.d_counters + kScanDone);
     sb.ntiles = cap + 1;
     sb.nchan = 1;
     tile_scan_kernel<<<scan_groups(cap + 1), kScanGroup, 0, st>>>(sb);
-    group_scan_kernel<<<1, 1024, 0, st>>>(sb);
     ht_offsets_kernel<<<grid_for(cap + 1, 256), 256, 0, st>>>(h, sb);
     ht_fill_kernel<<<grid_for(nb, 256), 256, 0, st>>>(h, slot_of, nb);
     ht_order_kernel<<<grid_for(cap + 1, 256), 256, 0, st>>>(h, cap + 1);
@@ -222,23 +224,23 @@ void run_hash_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk, 
     const bool direct = nb < (uint64_t)(kDirect - 1);
     ProbeSlot* pt = (ProbeSlot*)s.alloc((size_t)(cap + 1) * sizeof(ProbeSlot));
     ht_pack_kernel<<<grid_for(cap + 1, 256), 256, 0, st>>>(h, pt, cap + 1, direct);
-    s.launched(7);
+    s.launched(6);
     if (!np) return;
-    const uint32_t nt = compact_tiles(np);
+    const uint32_t nt = (uint32_t)((np + kProbeTile - 1) / kProbeTile);
     CompactBufs pb;
     pb.words = nullptr;
     pb.counts = (uint32_t*)s.alloc((size_t)nt * 4);
     pb.offsets = (uint64_t*)s.alloc((size_t)nt * 8);
     pb.gbase = (uint64_t*)s.alloc((size_t)scan_groups(nt) * 8);
     pb.totals = s.d_counters + ci;
+    pb.done = sb.done;
     pb.ntiles = nt;
     pb.nchan = 1;
     const uint32_t pg = nt < (uint32_t)g ? nt : (uint32_t)g;
     probe_count_kernel<<<pg, 256, 0, st>>>(pt, h.mask, direct, pk, np, pslot, pb);
     tile_scan_kernel<<<scan_groups(nt), kScanGroup, 0, st>>>(pb);
-    group_scan_kernel<<<1, 1024, 0, st>>>(pb);
     probe_emit_kernel<<<pg, 256, 0, st>>>(pt, h.rows, np, pslot, pb, o);
-    s.launched(4);
+    s.launched(3);
 }
 
 bool small_res(int t) { return t == AHEAD_RESTINY || t == AHEAD_RESSHORT || t == AHEAD_RESINT; }
@@ -265,6 +267,7 @@ struct MjPosOp {
     static constexpr int W = CHECKED ? 8 : 4;
     static constexpr int NCH = CHECKED ? 4 : 1;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = true;
     static constexpr bool EMIT_V = true;
     static constexpr int NOUT = 2;
     const char* base;
@@ -291,8 +294,9 @@ struct MjPosOp {
         const uint64_t t = load_at(t2c, pos2(v));
         return reenc ? dec_if(t2c, t, ft) : t;
     }
+    AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void put0(int k, uint64_t pos, uint64_t val) const {
-        if (pos < cap) store_at(k == 0 ? oh : ot, k == 0 ? ohw : otw, pos, val);
+        store_at(k == 0 ? oh : ot, k == 0 ? ohw : otw, pos, val);
     }
     AHEAD_DEV void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const {
         if (c == 1) {
@@ -312,6 +316,7 @@ struct FetchOp {
     static constexpr int W = CHECKED ? 8 : 4;
     static constexpr int NCH = CHECKED ? 3 : 1;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = true;
     static constexpr bool EMIT_V = true;
     static constexpr int NOUT = 1;
     const char* base;
@@ -337,8 +342,9 @@ struct FetchOp {
         const uint64_t t = load_at(t2c, pos(v));
         return reenc ? mulw(t, fac, w2) : t;
     }
+    AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void put0(int, uint64_t p, uint64_t val) const {
-        if (p < cap) store_at(ot, otw, p, val);
+        store_at(ot, otw, p, val);
     }
     AHEAD_DEV void emit(int c, uint64_t p, uint64_t v, uint64_t row) const {
         if (c == 1) {
@@ -584,6 +590,7 @@ struct IsectOp {
     static constexpr int W = 8;
     static constexpr int NCH = 1;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = true;
     static constexpr bool EMIT_V = false;
     static constexpr int NOUT = 2;
     const char* base;
@@ -622,8 +629,9 @@ struct IsectOp {
         const uint64_t t = load_at(t2c, find(row));
         return reenc ? dec_if(t2c, t, ft) : t;
     }
+    AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void put0(int k, uint64_t pos, uint64_t val) const {
-        if (pos < cap) store_at(k == 0 ? oh : ot, k == 0 ? ohw : otw, pos, val);
+        store_at(k == 0 ? oh : ot, k == 0 ? ohw : otw, pos, val);
     }
     AHEAD_DEV void emit(int, uint64_t, uint64_t, uint64_t) const {}
 };
@@ -636,6 +644,7 @@ struct IsectPlainOp {
     static constexpr int W = WW;
     static constexpr int NCH = 1;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = true;
     static constexpr bool EMIT_V = false;
     static constexpr int NOUT = 2;
     const char* base;
@@ -659,8 +668,9 @@ struct IsectPlainOp {
     AHEAD_DEV uint64_t out0(int k, uint64_t, uint64_t row) const {
         return k == 0 ? load_at(h1c, row) : load_at(t2c, find(row));
     }
+    AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void put0(int k, uint64_t pos, uint64_t val) const {
-        if (pos < cap) store_at(k == 0 ? oh : ot, k == 0 ? ohw : otw, pos, val);
+        store_at(k == 0 ? oh : ot, k == 0 ? ohw : otw, pos, val);
     }
     AHEAD_DEV void emit(int, uint64_t, uint64_t, uint64_t) const {}
 };
@@ -795,6 +805,7 @@ struct FetchStrOp {
     static constexpr int W = 8;
     static constexpr int NCH = 2;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = false;
     static constexpr bool EMIT_V = true;
     static constexpr int NOUT = 1;
     const char* base;
@@ -805,8 +816,9 @@ struct FetchStrOp {
     uint64_t* acc;
     AHEAD_DEV uint32_t eval(uint64_t v, uint64_t, uint64_t&) const { return v * ainv < count ? 1u : 2u; }
     AHEAD_DEV uint64_t out0(int, uint64_t v, uint64_t) const { return v * ainv; }
+    AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        if (pos < cap) rows[pos] = (uint32_t)val;
+        rows[pos] = (uint32_t)val;
     }
     AHEAD_DEV void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const {
         if (c == 0) put0(0, pos, out0(0, v, row));
@@ -820,6 +832,7 @@ struct FetchStrPlainOp {
     static constexpr int W = 4;
     static constexpr int NCH = 1;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = false;
     static constexpr bool EMIT_V = true;
     static constexpr int NOUT = 1;
     const char* base;
@@ -829,8 +842,9 @@ struct FetchStrPlainOp {
     uint64_t* acc;
     AHEAD_DEV uint32_t eval(uint64_t v, uint64_t, uint64_t&) const { return v < count ? 1u : 0u; }
     AHEAD_DEV uint64_t out0(int, uint64_t v, uint64_t) const { return v; }
+    AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        if (pos < cap) rows[pos] = (uint32_t)val;
+        rows[pos] = (uint32_t)val;
     }
     AHEAD_DEV void emit(int, uint64_t pos, uint64_t v, uint64_t) const { put0(0, pos, v); }
 };

@@ -21,6 +21,7 @@ struct SelectOp {
     static constexpr int W = WW;
     static constexpr int NCH = AN ? 2 : 1;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = false;
     const char* base;
     uint32_t* status;
     uint64_t seqbase, ainv, umax, aoid, cap, errcap;
@@ -35,11 +36,10 @@ struct SelectOp {
         const uint32_t oid = (uint32_t)(seqbase + row);
         return AN ? (uint64_t)oid * kResoidAMax : (uint64_t)oid;
     }
+    AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        if (pos < cap) {
-            if (AN) out_an[pos] = val;
-            else out_oid[pos] = (uint32_t)val;
-        }
+        if (AN) out_an[pos] = val;
+        else out_oid[pos] = (uint32_t)val;
     }
     AHEAD_DEV uint32_t eval(uint64_t v, uint64_t, uint64_t&) const {
         if constexpr (W <= 4) {
@@ -231,6 +231,7 @@ struct CadVoidOp {
     static constexpr int W = WW;
     static constexpr int NCH = 2;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = false;
     const char* base;
     uint32_t* status;
     void* out;
@@ -244,8 +245,9 @@ struct CadVoidOp {
         return mulw(v, ainv, W) > umax ? 2u : 1u;
     }
     AHEAD_DEV uint64_t out0(int, uint64_t v, uint64_t) const { return mulw(v, ainv, W); }
+    AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        if (pos < cap) store_at(out, ow, pos, val);
+        store_at(out, ow, pos, val);
     }
     AHEAD_DEV void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const {
         if (c == 0) {
@@ -264,6 +266,7 @@ struct CadGenOp {
     static constexpr int W = WW;
     static constexpr int NCH = 3;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = false;
     const char* base;
     uint32_t* status;
     DCol hc, tc;
@@ -277,8 +280,9 @@ struct CadGenOp {
     AHEAD_DEV uint64_t out0(int k, uint64_t t, uint64_t row) const {
         return k == 0 ? dec_if(hc, load_at(hc, row), hc.ainv) : mulw(t, tc.ainv, W);
     }
+    AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void put0(int k, uint64_t pos, uint64_t val) const {
-        if (pos < cap) store_at(k == 0 ? oh : ot, k == 0 ? ohw : otw, pos, val);
+        store_at(k == 0 ? oh : ot, k == 0 ? ohw : otw, pos, val);
     }
     AHEAD_DEV uint32_t eval(uint64_t t, uint64_t row, uint64_t&) const {
         const uint64_t h = load_at(hc, row);
@@ -306,6 +310,7 @@ struct DecodeOp {
     static constexpr int W = WW;
     static constexpr int NCH = 1;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = false;
     const char* base;
     uint32_t* status;
     DCol hc, tc;
@@ -317,8 +322,9 @@ struct DecodeOp {
     static constexpr bool EMIT_V = false;
     static constexpr int NOUT = 1;
     AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row * aoid; }
+    AHEAD_DEV uint64_t cap0() const { return errcap; }
     AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        if (pos < errcap) err[pos] = val;
+        err[pos] = val;
     }
     AHEAD_DEV uint32_t eval(uint64_t t, uint64_t row, uint64_t&) const {
         const uint64_t d = mulw(t, tc.ainv, W);
@@ -339,6 +345,7 @@ struct MulSumOp {
     static constexpr int W = WW;
     static constexpr int NCH = 2;
     static constexpr bool ACC = true;
+    static constexpr bool GATHER = false;
     const char* base;
     uint32_t* status;
     DCol ac, bc;
@@ -348,8 +355,9 @@ struct MulSumOp {
     static constexpr bool EMIT_V = false;
     static constexpr int NOUT = 1;
     AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row * aoid; }
+    AHEAD_DEV uint64_t cap0() const { return ecap1; }
     AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        if (pos < ecap1) e1[pos] = val;
+        e1[pos] = val;
     }
     AHEAD_DEV uint32_t eval(uint64_t a, uint64_t row, uint64_t& s) const {
         const uint64_t b = load_at(bc, row);
@@ -575,6 +583,7 @@ struct ArithOp {
     static constexpr int W = WW;
     static constexpr int NCH = 2;
     static constexpr bool ACC = false;
+    static constexpr bool GATHER = false;
     const char* base;
     uint32_t* status;
     DCol ac, bc;
@@ -586,8 +595,9 @@ struct ArithOp {
     static constexpr bool EMIT_V = false;
     static constexpr int NOUT = 1;
     AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row * aoid; }
+    AHEAD_DEV uint64_t cap0() const { return ecap1; }
     AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        if (pos < ecap1) e1[pos] = val;
+        e1[pos] = val;
     }
     AHEAD_DEV uint32_t eval(uint64_t a, uint64_t row, uint64_t&) const {
         const uint64_t t1 = mulw(a, ac.ainv, W), t2 = mulw(load_at(bc, row), bc.ainv, bc.width);
