@@ -99,8 +99,17 @@ inline size_t compact_bytes(uint64_t n, uint32_t ntiles, uint32_t nchan) {
 //   void put0(int k, uint64_t pos, uint64_t val) const;    store it at pos < cap0()
 //   void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const;  streams c >= 1
 //
+//   void begin();  optional: loads what eval and out0 need from device memory, once per thread
+//
 // Row layout of a tile: with VEC = 16 / W rows per vector, lane l holds in
 // vector s the rows 32 * VEC * s + VEC * l + (0 .. VEC - 1) of the tile.
+
+template <class Op>
+AHEAD_DEV auto begin_op(Op& op, int) -> decltype(op.begin(), void()) {
+    op.begin();
+}
+template <class Op>
+AHEAD_DEV void begin_op(Op&, long) {}
 
 template <int W>
 AHEAD_DEV void unpack16(const uint4 q, uint64_t (&v)[16 / W]) {
@@ -297,6 +306,7 @@ template <class Op, int K>
 __global__ void __launch_bounds__(kCThreads) classify_kernel(Op op, uint64_t n, CompactBufs cb, int per) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool vec = ((uintptr_t)op.base & 15) == 0;
+    begin_op(op, 0);
     uint64_t acc = 0;
     const uint32_t whole = (uint32_t)(n / (32 * K));  // whole tiles
     uint32_t tile = blockIdx.x * per * kCWarps + warp;
@@ -407,6 +417,7 @@ __global__ void __launch_bounds__(kCThreads) emit_kernel(Op op, uint64_t n, Comp
     constexpr int NCH = Op::NCH;
     __shared__ uint16_t s_rows[kCWarps][32 * K];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    begin_op(op, 0);
     auto tile_of = [&](int k) { return (blockIdx.x * per + k) * kCWarps + warp; };
     uint32_t word = 0, count = 0;
     uint64_t base = 0;
@@ -444,6 +455,7 @@ __global__ void __launch_bounds__(kOneBlockTiles * 32) compact_one_kernel(Op op,
     __shared__ uint32_t s_cnt[NCH][kOneBlockTiles];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool vec = ((uintptr_t)op.base & 15) == 0;
+    begin_op(op, 0);
     uint32_t word = 0, count = 0;
     uint64_t acc = 0;
     Flight<Op::W, K> f;

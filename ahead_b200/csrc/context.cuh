@@ -198,6 +198,11 @@ inline bool dyn_smem_ready(const ahead_ctx* ctx, int bytes) {
     return true;
 }
 
+inline uint32_t tiles_per_warp(const ahead_ctx* ctx, uint32_t nt) {
+    const uint32_t k = nt / ((uint32_t)ctx->num_sms * 8 * kCWarps);
+    return k < 1 ? 1 : k > 8 ? 8 : k;
+}
+
 // Launch one compaction over n rows with its scratch in `cb`; returns the
 // number of launches.  Few tiles: one block does everything (the separate
 // launches of almost no work each cost 15 us at 2,556 rows, the one 5).  Else 1
@@ -209,8 +214,7 @@ inline int launch_compact(const ahead_ctx* ctx, cudaStream_t st, const Op& op, u
         compact_one_kernel<Op><<<1, nt * 32, 0, st>>>(op, n, cb);
         return 1;
     }
-    const uint32_t fill = (uint32_t)ctx->num_sms * 8 * kCWarps;
-    const uint32_t per = nt / fill < 1 ? 1 : nt / fill > 8 ? 8 : nt / fill;
+    const uint32_t per = tiles_per_warp(ctx, nt);
     const uint32_t grid = (nt + per * kCWarps - 1) / (per * kCWarps);
     auto passes = [&](auto k_tag) {
         constexpr int K = decltype(k_tag)::value;
@@ -225,6 +229,16 @@ inline int launch_compact(const ahead_ctx* ctx, cudaStream_t st, const Op& op, u
         }
     passes(std::integral_constant<int, short_k(Op::W)>());
     return 3;
+}
+
+// Passes 2 and 3 of a compaction in short tiles whose pass 1 has its own kernel.
+template <class Op>
+inline int launch_compact_tail(const ahead_ctx* ctx, cudaStream_t st, const Op& op, uint64_t n, const CompactBufs& cb) {
+    constexpr int K = short_k(Op::W);
+    const uint32_t per = tiles_per_warp(ctx, cb.ntiles);
+    tile_scan_kernel<<<scan_groups(cb.ntiles), kScanGroup, 0, st>>>(cb);
+    emit_kernel<Op, K><<<(cb.ntiles + per * kCWarps - 1) / (per * kCWarps), kCThreads, 0, st>>>(op, n, cb, (int)per);
+    return 2;
 }
 
 // A compaction of an operator call; totals land in counters [c0, c0 + NCH).

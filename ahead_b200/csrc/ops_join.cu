@@ -1,12 +1,13 @@
 // ops_join.cu -- hashjoinAN / hashjoin, matchjoinAN / matchjoin and
 // fetchjoinAN / fetchjoin.
 //
-// Hash joins build the table of hash.cuh on the build side (the right BAT by
-// default) with keys decoded and cast to the unencoded base type, probe in
-// probe-row order and emit every match in build order
-// (lib/column_operators/AN/hashjoinAN.tcc:54-223).  Rows with detected errors
-// are still built and probed, exactly as in the reference; the four error
-// vectors are column checks of the four inputs.
+// Hash joins key the build side (the right BAT by default) by its decoded keys
+// cast to the unencoded base type, probe in probe-row order and emit every match
+// in build order (lib/column_operators/AN/hashjoinAN.tcc:54-223).  Unique keys
+// of a bounded range (a dimension's keys) index a bitmap and a value array
+// directly, and the probe is a compaction; anything else takes the hash table
+// of hash.cuh.  Rows with detected errors are still built and probed, exactly
+// as in the reference; the four error vectors are checks of the four inputs.
 //
 // Positional match/fetch joins are compactions over the OID list with a gather
 // (matchjoinAN.tcc:226-354).  The merge matchjoin (matchjoinAN.tcc:46-144) is
@@ -177,6 +178,262 @@ __global__ void __launch_bounds__(256) probe_emit_kernel(const ProbeSlot* __rest
             for (uint32_t j = 0; j < e.cnt; ++j) join_emit(o, pos++, row, rows[e.first + j]);
         }
     }
+}
+
+// --------------------------------------------------------- direct join
+// A dimension's keys are unique and dense enough that key - smallest key can
+// index an array: one bit says whether the key is there, one 8-byte word holds
+// what the join emits for it (the build side's OID, re-encoded).  The probe is
+// then a compaction of the probe rows whose bit is set -- a key has at most one
+// match -- with the AN checks of the probe's columns as its sparse streams, so
+// the probe column is read once per pass and nothing per row is stored between
+// the passes.  The bitmap is copied into shared memory (up to kDjSmem bytes:
+// 1.6M keys), where 32 lanes' lookups cost a few bank conflicts, not 32 L2
+// requests; only the matches touch the value array in L2.
+//
+// Three things send the join to the hash table instead, found by the build
+// kernels and read back with the counts: a key range above the limit (2^24 at
+// most: the value array then stays near L2's size), or a repeated key; and
+// 8-byte raw codes as keys are not tried (multiples of A: far too wide).
+// At 60M probe rows against 320K of 800K keys: hash probe 512 + 559 us (one
+// 16-byte slot request to L2 per row, then thread-serial output) and 110 us of
+// separate column checks, against 15 us to build, 124 to classify and 289 to emit
+// (DRAM floor of the two passes: 205).
+constexpr uint64_t kDjMaxSpan = 1ull << 24;
+constexpr int kDjSmem = 200 * 1024;
+constexpr int kDjBounds = 20, kDjBad = 22, kDjBuildKey = 23, kDjBuildVal = 24, kDjCounters = 25;  // counters
+
+inline uint64_t dj_limit(uint64_t nb, uint64_t np) {
+    const uint64_t l = (1ull << 20) + 64 * nb + np;
+    return (l < kDjMaxSpan ? l : kDjMaxSpan) & ~31ull;
+}
+
+struct DjBuild {
+    KeyCfg bk;
+    DCol bcol;        // build-side output column
+    uint64_t nb, limit, factor;
+    int reenc, check; // check: report corrupt keys and values
+    uint64_t* bounds; // [0] the largest ~key, [1] the largest key
+    uint32_t* bad;
+    uint32_t* bits;   // [limit / 32]
+    uint64_t* val;    // [limit]
+    ErrList kerr, verr;
+    AHEAD_DEV uint64_t kmin() const { return ~bounds[0]; }
+    AHEAD_DEV uint64_t span() const { return bounds[1] - kmin() + 1; }
+};
+
+// Key bounds, the AN checks of the build columns, and the bitmap cleared.
+__global__ void __launch_bounds__(256) dj_bounds_kernel(DjBuild b) {
+    __shared__ uint64_t s_lo[8], s_hi[8];
+    const uint64_t first = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t w = first; w < b.limit / 32; w += stride) b.bits[w] = 0;
+    uint64_t nlo = 0, hi = 0;
+    for (uint64_t i = first; i < b.nb; i += stride) {
+        const uint64_t v = load_at(b.bk.col, i);
+        const uint64_t d = b.bk.dec ? mulw(v, b.bk.ainv, b.bk.width) : v;
+        if (b.check && b.bk.col.enc && mulw(v, b.bk.col.ainv, b.bk.width) > b.bk.col.umax) b.kerr.add(i);
+        if (b.check && b.bcol.enc && mulw(load_at(b.bcol, i), b.bcol.ainv, b.bcol.width) > b.bcol.umax) b.verr.add(i);
+        const uint64_t k = d & b.bk.keymask;
+        nlo = ~k > nlo ? ~k : nlo;
+        hi = k > hi ? k : hi;
+    }
+    for (int d = 16; d > 0; d >>= 1) {
+        const uint64_t a = __shfl_xor_sync(kFull, nlo, d), c = __shfl_xor_sync(kFull, hi, d);
+        nlo = a > nlo ? a : nlo;
+        hi = c > hi ? c : hi;
+    }
+    if ((threadIdx.x & 31) == 0) {
+        s_lo[threadIdx.x >> 5] = nlo;
+        s_hi[threadIdx.x >> 5] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) {
+            nlo = s_lo[w] > nlo ? s_lo[w] : nlo;
+            hi = s_hi[w] > hi ? s_hi[w] : hi;
+        }
+        if (nlo) {  // (a block without rows holds 0)
+            atomicMax((unsigned long long*)&b.bounds[0], (unsigned long long)nlo);
+            atomicMax((unsigned long long*)&b.bounds[1], (unsigned long long)hi);
+        }
+    }
+}
+
+// Sets each key's bit and value.  Neighbouring lanes hold neighbouring keys
+// (dimension tables are in key order), so the lanes of one word share one atomic.
+__global__ void __launch_bounds__(256) dj_insert_kernel(DjBuild b) {
+    const uint64_t kmin = b.kmin(), span = b.span(), stride = (uint64_t)gridDim.x * blockDim.x;
+    if (span > b.limit) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *b.bad = 1;
+        return;
+    }
+    const uint64_t rounds = (b.nb + stride - 1) / stride;
+    for (uint64_t r = 0; r < rounds; ++r) {
+        const uint64_t i = r * stride + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+        const bool live = i < b.nb;
+        uint64_t d = 0;
+        if (live) {
+            const uint64_t v = load_at(b.bk.col, i);
+            d = ((b.bk.dec ? mulw(v, b.bk.ainv, b.bk.width) : v) & b.bk.keymask) - kmin;
+            const uint64_t x = load_at(b.bcol, i);
+            b.val[d] = b.reenc ? x * b.factor : x;
+        }
+        const uint32_t word = live ? (uint32_t)(d >> 5) : ~0u, bit = live ? 1u << (d & 31) : 0u;
+        const uint32_t peers = __match_any_sync(kFull, word);
+        const uint32_t set = __reduce_or_sync(peers, bit);
+        if (live && (threadIdx.x & 31) == __ffs(peers) - 1) {
+            const uint32_t old = atomicOr(&b.bits[word], set);
+            if ((old & set) || __popc(set) != __popc(peers)) *b.bad = 1;  // a key twice
+        }
+    }
+}
+
+// The probe.  Streams: 0 matching rows, 1 corrupt probe keys, 2 corrupt values
+// of the probe side's output column.
+template <int WW, bool AN>
+struct DjOp {
+    static constexpr int W = WW;
+    static constexpr int NCH = AN ? 3 : 1;
+    static constexpr bool ACC = false;
+    static constexpr bool GATHER = true;
+    static constexpr bool EMIT_V = true;
+    static constexpr int NOUT = 2;
+    const char* base;
+    KeyCfg pk;
+    JoinOut o;
+    const uint64_t* bounds;
+    const uint32_t* bad;
+    const uint32_t* bits;
+    const uint64_t* val;
+    uint64_t limit, kmin, span;  // kmin, span: set by begin
+    uint64_t aoid, eck, eco;
+    uint64_t *ek, *eo, *acc;
+    AHEAD_DEV void begin() {
+        kmin = ~__ldg((const unsigned long long*)bounds);
+        span = __ldg((const unsigned long long*)bounds + 1) - kmin + 1;
+        if (__ldg(bad) || span > limit) span = 0;
+    }
+    AHEAD_DEV uint64_t dec(uint64_t v) const { return pk.dec ? mulw(v, pk.ainv, W) : v; }
+    AHEAD_DEV uint32_t eval(uint64_t v, uint64_t row, uint64_t&) const {
+        const uint64_t d = dec(v);
+        uint32_t b = 0;
+        if (AN) {
+            if (d > pk.col.umax) b |= 2u;
+            if (o.pcol.enc && mulw(load_at(o.pcol, row), o.pcol.ainv, o.pcol.width) > o.pcol.umax) b |= 4u;
+        }
+        const uint64_t k = (d & pk.keymask) - kmin;
+        if ((d & pk.largermask) <= pk.condmax && k < span && ((bits[(uint32_t)k >> 5] >> (k & 31)) & 1u)) b |= 1u;
+        return b;
+    }
+    AHEAD_DEV uint64_t out0(int k, uint64_t v, uint64_t row) const {
+        if ((k == 0) == (o.probe_is_head != 0)) {
+            const uint64_t x = load_at(o.pcol, row);
+            return k == 0 ? (o.rh ? x * o.fh : x) : (o.rt ? x * o.ft : x);
+        }
+        return __ldg((const unsigned long long*)val + ((dec(v) & pk.keymask) - kmin));
+    }
+    AHEAD_DEV uint64_t cap0() const { return o.cap; }
+    AHEAD_DEV void put0(int k, uint64_t pos, uint64_t x) const { store_at(k == 0 ? o.oh : o.ot, k == 0 ? o.ohw : o.otw, pos, x); }
+    AHEAD_DEV void emit(int c, uint64_t pos, uint64_t, uint64_t row) const {
+        if (c == 1) {
+            if (pos < eck) ek[pos] = row * aoid;
+        } else if (pos < eco) {
+            eo[pos] = row * aoid;
+        }
+    }
+};
+
+// Pass 1 with the bitmap in shared memory: one block of 32 warps per SM walks
+// the tiles (a bitmap that does not fit is read through L1 and L2).
+template <class Op>
+__global__ void __launch_bounds__(1024, 1) dj_classify_kernel(Op op, uint64_t n, CompactBufs cb) {
+    extern __shared__ uint32_t s_bits[];
+    constexpr int K = short_k(Op::W);
+    const int lane = threadIdx.x & 31;
+    const bool vec = ((uintptr_t)op.base & 15) == 0;
+    op.begin();
+    const uint32_t whole = (uint32_t)(n / (32 * K)), nw = gridDim.x * 32;
+    uint32_t tile = blockIdx.x * 32 + (threadIdx.x >> 5);
+    Flight<Op::W, K> f;
+    if (tile < whole) f.load(op.base, (uint64_t)tile * (32 * K) + 16 / Op::W * lane, vec);
+    const uint32_t words = (uint32_t)((op.span + 31) / 32);
+    if (words <= kDjSmem / 4) {
+        for (uint32_t i = threadIdx.x; i < words; i += 1024) s_bits[i] = op.bits[i];
+        __syncthreads();
+        op.bits = s_bits;
+    }
+    uint64_t acc = 0;
+    for (; tile < cb.ntiles; tile += nw) {
+        const uint32_t next = tile + nw < whole ? tile + nw : 0;
+        uint32_t word, count;
+        tile_classify<Op, K>(op, n, tile, f, next, vec, acc, word, count);
+        if (lane < K) cb.words[(size_t)tile * K + lane] = word;
+        if (lane < Op::NCH) cb.counts[(size_t)tile * Op::NCH + lane] = count;
+    }
+}
+
+size_t dj_scratch(uint64_t nb, uint64_t np) {
+    const uint64_t limit = dj_limit(nb, np);
+    return limit / 8 + limit * 8 + 2 * kErrListBytes + compact_scratch<DjOp<8, true>>(np) + 4096;
+}
+
+// Builds and probes; totals in counters 0 (matches), 1 and 2 (probe errors).
+// `err_k`, `err_o`: the probe key's and the probe output column's vectors.
+template <bool AN>
+void run_direct_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk, uint64_t np, const JoinOut& o,
+                     uint64_t aoid, ahead_errvec* err_k, ahead_errvec* err_o, ErrList* kerr, ErrList* verr) {
+    cudaStream_t st = s.ctx->stream;
+    DjBuild b;
+    b.bk = bk;
+    b.bcol = o.bcol;
+    b.nb = nb;
+    b.limit = dj_limit(nb, np);
+    b.reenc = o.probe_is_head ? o.rt : o.rh;
+    b.factor = o.probe_is_head ? o.ft : o.fh;
+    b.check = AN;
+    b.bounds = s.d_counters + kDjBounds;
+    b.bad = (uint32_t*)(s.d_counters + kDjBad);
+    b.bits = (uint32_t*)s.alloc(b.limit / 8);
+    b.val = (uint64_t*)s.alloc(b.limit * 8);
+    *kerr = b.kerr = err_list(s, kDjBuildKey);
+    *verr = b.verr = err_list(s, kDjBuildVal);
+    const uint64_t most = b.limit / 32 > nb ? b.limit / 32 : nb;
+    const uint32_t g = (uint32_t)s.ctx->num_sms * 4, want = grid_for(most, 256);
+    dj_bounds_kernel<<<want < g ? want : g, 256, 0, st>>>(b);
+    dj_insert_kernel<<<grid_for(nb, 256), 256, 0, st>>>(b);
+    s.launched(2);
+    auto probe = [&](auto tag) -> int {
+        typedef DjOp<decltype(tag)::value, AN> Op;
+        Op op;
+        op.base = (const char*)pk.col.data;
+        op.pk = pk;
+        op.o = o;
+        op.bounds = b.bounds;
+        op.bad = b.bad;
+        op.bits = b.bits;
+        op.val = b.val;
+        op.limit = b.limit;
+        op.kmin = op.span = 0;
+        op.aoid = aoid;
+        op.ek = edata(err_k);
+        op.eo = edata(err_o);
+        op.eck = ecap(err_k);
+        op.eco = ecap(err_o);
+        op.acc = nullptr;
+        const uint32_t nt = compact_tiles<Op>(np);
+        const CompactBufs cb = s.compact_bufs(np, nt, Op::NCH, 0);
+        if (nt <= kOneBlockTiles || !dyn_smem_ready<dj_classify_kernel<Op>>(s.ctx, kDjSmem)) {
+            s.launched(launch_compact(s.ctx, st, op, np, cb));
+            return 0;
+        }
+        const uint32_t blocks = (nt + 31) / 32;
+        dj_classify_kernel<Op><<<blocks < (uint32_t)s.ctx->num_sms ? blocks : s.ctx->num_sms, 1024, kDjSmem, st>>>(
+            op, np, cb);
+        s.launched(1 + launch_compact_tail(s.ctx, st, op, np, cb));
+        return 0;
+    };
+    if constexpr (AN) by_width_enc(pk.width, probe);
+    else by_width(pk.width, probe);
 }
 
 size_t join_scratch(uint64_t nb, uint64_t np) {
@@ -953,49 +1210,75 @@ int ahead_gpu_hashjoin_an(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r
     OpScope s(ctx);
     const uint64_t nl = l->count, nr = r->count;
     const bool both = nl > 0 && nr > 0;
-    const uint64_t nb = side == AHEAD_HASH_LEFT ? nl : nr, np = side == AHEAD_HASH_LEFT ? nr : nl;
-    int rc = s.reserve((both ? join_scratch(nb, np) : 0) +
-                       (both ? colcheck_scratch(nl) * 2 + colcheck_scratch(nr) * 2 : 0));
+    if (!both) return AHEAD_OK;
+    const bool left = side == AHEAD_HASH_LEFT;
+    const uint64_t nb = left ? nl : nr, np = left ? nr : nl;
+    const int bt1 = type_base_width(T1), bh2 = type_base_width(H2);
+    const int larger = bt1 > bh2 ? bt1 : bh2;
+    JoinOut o;
+    o.fh = fH1;
+    o.ft = fT2;
+    o.cap = (out->head.data && out->tail.data) ? cap : 0;
+    o.oh = out->head.data;
+    o.ot = out->tail.data;
+    o.rh = reenc_head;
+    o.rt = reenc_tail;
+    o.ohw = type_width(oH);
+    o.otw = type_width(oT);
+    o.probe_is_head = !left;
+    o.pcol = dcol(left ? r->tail : l->head);
+    o.bcol = dcol(left ? l->head : r->tail);
+    const KeyCfg bk = left ? key_cfg(l->tail, 1, bt1, bt1, false) : key_cfg(r->head, 1, bh2, bh2, false);
+    const KeyCfg pk = left ? key_cfg(r->head, 1, bt1, larger, true) : key_cfg(l->tail, 1, bh2, larger, true);
+    // the column check of error vector k (head1, tail1, head2, tail2) into counter 1 + k
+    auto check = [&](int k) {
+        if (k == 0 && eH1)
+            run_colcheck(s, l->head, nl, AH1Inv, l->head.unenc_max & wmask(wh1e), wh1e, aoid, ev(errs, 0), 1);
+        if (k == 1)
+            run_colcheck(s, l->tail, nl, l->tail.Ainv & wmask(type_width(T1)),
+                         l->tail.unenc_max & wmask(type_width(T1)), type_width(T1), aoid, ev(errs, 1), 2);
+        if (k == 2)
+            run_colcheck(s, r->head, nr, r->head.Ainv & wmask(type_width(H2)),
+                         r->head.unenc_max & wmask(type_width(H2)), type_width(H2), aoid, ev(errs, 2), 3);
+        if (k == 3 && eT2)
+            run_colcheck(s, r->tail, nr, AT2Inv, r->tail.unenc_max & wmask(wt2e), wt2e, aoid, ev(errs, 3), 4);
+    };
+    int rc = s.reserve(dj_scratch(nb, np));
     if (rc) return rc;
-    if (both) {
-        const int bt1 = type_base_width(T1), bh2 = type_base_width(H2);
-        const int larger = bt1 > bh2 ? bt1 : bh2;
-        JoinOut o;
-        o.fh = fH1;
-        o.ft = fT2;
-        o.cap = (out->head.data && out->tail.data) ? cap : 0;
-        o.oh = out->head.data;
-        o.ot = out->tail.data;
-        o.rh = reenc_head;
-        o.rt = reenc_tail;
-        o.ohw = type_width(oH);
-        o.otw = type_width(oT);
-        if (side == AHEAD_HASH_LEFT) {
-            KeyCfg bk = key_cfg(l->tail, 1, bt1, bt1, false);
-            KeyCfg pk = key_cfg(r->head, 1, bt1, larger, true);
-            o.probe_is_head = 0;
-            o.pcol = dcol(r->tail);
-            o.bcol = dcol(l->head);
-            run_hash_join(s, bk, nl, pk, nr, o, 0);
-        } else {
-            KeyCfg bk = key_cfg(r->head, 1, bh2, bh2, false);
-            KeyCfg pk = key_cfg(l->tail, 1, bh2, larger, true);
-            o.probe_is_head = 1;
-            o.pcol = dcol(l->head);
-            o.bcol = dcol(r->tail);
-            run_hash_join(s, bk, nr, pk, nl, o, 0);
+    // error vectors of the probe's key and output column, and the build's
+    const int vpk = left ? 2 : 1, vpo = left ? 3 : 0, vbk = left ? 1 : 2, vbo = left ? 0 : 3;
+    ErrList kerr, verr;
+    run_direct_join<true>(s, bk, nb, pk, np, o, aoid, ev(errs, vpk), ev(errs, vpo), &kerr, &verr);
+    rc = s.finish(kDjCounters);
+    if (rc) return rc;
+    if (!s.counter(kDjBad)) {
+        out->count = s.counter(0);
+        if (errs) {
+            errs[vpk].count = s.counter(1);
+            if (errs[vpo].present) errs[vpo].count = s.counter(2);
+            const bool okk = settle_err_list(s, kerr, kDjBuildKey, aoid, ev(errs, vbk));
+            const bool okv = !errs[vbo].present || settle_err_list(s, verr, kDjBuildVal, aoid, ev(errs, vbo));
+            if (!okk || !okv) {  // a build column with many corrupt codes
+                rc = s.reserve(2 * colcheck_scratch(nb));
+                if (rc) return rc;
+                if (!okk) check(vbk);
+                if (!okv) check(vbo);
+                rc = s.finish(5);
+                if (rc) return rc;
+                if (!okk) errs[vbk].count = s.counter(1 + vbk);
+                if (!okv) errs[vbo].count = s.counter(1 + vbo);
+            }
         }
-        if (eH1) run_colcheck(s, l->head, nl, AH1Inv, l->head.unenc_max & wmask(wh1e), wh1e, aoid, ev(errs, 0), 1);
-        run_colcheck(s, l->tail, nl, l->tail.Ainv & wmask(type_width(T1)), l->tail.unenc_max & wmask(type_width(T1)),
-                     type_width(T1), aoid, ev(errs, 1), 2);
-        run_colcheck(s, r->head, nr, r->head.Ainv & wmask(type_width(H2)), r->head.unenc_max & wmask(type_width(H2)),
-                     type_width(H2), aoid, ev(errs, 2), 3);
-        if (eT2) run_colcheck(s, r->tail, nr, AT2Inv, r->tail.unenc_max & wmask(wt2e), wt2e, aoid, ev(errs, 3), 4);
+        return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
     }
+    rc = s.reserve(join_scratch(nb, np) + colcheck_scratch(nl) * 2 + colcheck_scratch(nr) * 2);
+    if (rc) return rc;
+    run_hash_join(s, bk, nb, pk, np, o, 0);
+    for (int k = 0; k < 4; ++k) check(k);
     rc = s.finish(5);
     if (rc) return rc;
-    out->count = both ? s.counter(0) : 0;
-    if (both && errs)
+    out->count = s.counter(0);
+    if (errs)
         for (int k = 0; k < 4; ++k)
             if (errs[k].present) errs[k].count = s.counter(1 + k);
     return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
@@ -1015,28 +1298,39 @@ int ahead_gpu_hashjoin(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r, i
     const uint64_t nl = l->count, nr = r->count;
     const bool both = nl > 0 && nr > 0;
     const uint64_t nb = side == AHEAD_HASH_LEFT ? nl : nr, np = side == AHEAD_HASH_LEFT ? nr : nl;
-    int rc = s.reserve(both ? join_scratch(nb, np) : 0);
-    if (rc) return rc;
-    if (both) {
-        const int w = type_width(T1);
-        JoinOut o;
-        o.fh = o.ft = 1;
-        o.cap = (out->head.data && out->tail.data) ? cap : 0;
-        o.oh = out->head.data;
-        o.ot = out->tail.data;
-        o.rh = o.rt = 0;
-        o.ohw = type_width(type_select_of(H1));
-        o.otw = type_width(type_select_of(T2));
-        KeyCfg bk = key_cfg(side == AHEAD_HASH_LEFT ? l->tail : r->head, 0, w, w, false);
-        KeyCfg pk = key_cfg(side == AHEAD_HASH_LEFT ? r->head : l->tail, 0, w, w, false);
-        o.probe_is_head = side != AHEAD_HASH_LEFT;
-        o.pcol = dcol(side == AHEAD_HASH_LEFT ? r->tail : l->head);
-        o.bcol = dcol(side == AHEAD_HASH_LEFT ? l->head : r->tail);
-        run_hash_join(s, bk, nb, pk, np, o, 0);
+    if (!both) return AHEAD_OK;
+    const int w = type_width(T1);
+    JoinOut o;
+    o.fh = o.ft = 1;
+    o.cap = (out->head.data && out->tail.data) ? cap : 0;
+    o.oh = out->head.data;
+    o.ot = out->tail.data;
+    o.rh = o.rt = 0;
+    o.ohw = type_width(type_select_of(H1));
+    o.otw = type_width(type_select_of(T2));
+    const KeyCfg bk = key_cfg(side == AHEAD_HASH_LEFT ? l->tail : r->head, 0, w, w, false);
+    const KeyCfg pk = key_cfg(side == AHEAD_HASH_LEFT ? r->head : l->tail, 0, w, w, false);
+    o.probe_is_head = side != AHEAD_HASH_LEFT;
+    o.pcol = dcol(side == AHEAD_HASH_LEFT ? r->tail : l->head);
+    o.bcol = dcol(side == AHEAD_HASH_LEFT ? l->head : r->tail);
+    if (w < 8) {  // (8-byte keys are raw codes)
+        int rc = s.reserve(dj_scratch(nb, np));
+        if (rc) return rc;
+        ErrList kerr, verr;
+        run_direct_join<false>(s, bk, nb, pk, np, o, 0, nullptr, nullptr, &kerr, &verr);
+        rc = s.finish(kDjCounters);
+        if (rc) return rc;
+        if (!s.counter(kDjBad)) {
+            out->count = s.counter(0);
+            return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
+        }
     }
+    int rc = s.reserve(join_scratch(nb, np));
+    if (rc) return rc;
+    run_hash_join(s, bk, nb, pk, np, o, 0);
     rc = s.finish(1);
     if (rc) return rc;
-    out->count = both ? s.counter(0) : 0;
+    out->count = s.counter(0);
     return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
 }
 
