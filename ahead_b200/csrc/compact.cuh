@@ -25,7 +25,7 @@
 // (enough warps to fill the chip) and for operators whose every row waits on a
 // gather.  Measured on 600M 32-bit codes, a fifth selected: classify 367 us, the
 // copy bandwidth (2.4 GB; 459 us with a ballot per 32 rows, 20 instructions a
-// row instead of 8, and 450 fed through a shared-memory ring); emit 268 us for
+// row instead of 8, and 450 fed through a shared-memory ring); emit 243 us for
 // 0.96 GB (660 us when a block walked 4096-row tiles without looking ahead): it
 // is bound by its ~380 instructions per 1024 rows.  Traffic beyond the input and the outputs: one bit per row, and 20
 // bytes per tile and stream, written and read back, plus re-reading the few
@@ -96,7 +96,10 @@ inline size_t compact_bytes(uint64_t n, uint32_t ntiles, uint32_t nchan) {
 //   uint32_t eval(uint64_t v, uint64_t row, uint64_t& acc) const;  bit c = stream c
 //   uint64_t out0(int k, uint64_t v, uint64_t row) const;  k-th output of a kept row
 //   uint64_t cap0() const;      positions below it are stored
+//   void* optr(int k) const; int owidth(int k) const;  where, and how wide, or instead
 //   void put0(int k, uint64_t pos, uint64_t val) const;    store it at pos < cap0()
+//   void rows0(v[U], row0, idx[U], val[NOUT][U]) const;    optional: the outputs of U kept
+//                               rows row0 + idx[u] at once, so that their loads overlap
 //   void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const;  streams c >= 1
 //
 //   void begin();  optional: loads what eval and out0 need from device memory, once per thread
@@ -222,6 +225,85 @@ AHEAD_DEV void tile_classify(const Op& op, uint64_t n, uint32_t tile, Flight<Op:
     }
 }
 
+// U rows' values of one column, at row0 + idx[u] or (gather) at p[u]: the type is
+// the same for all, so its branches are taken once for the U loads.
+template <int U>
+AHEAD_DEV void load_rows(const DCol& c, uint64_t row0, const uint32_t (&idx)[U], uint64_t (&x)[U]) {
+    if (c.type == AHEAD_VOID) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) x[u] = (uint32_t)(c.seqbase + row0 + idx[u]);
+        return;
+    }
+    auto ld = [&](auto* p) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) x[u] = __ldg(p + row0 + idx[u]);
+    };
+    if (c.width == 8) ld((const unsigned long long*)c.data);
+    else if (c.width == 4) ld((const uint32_t*)c.data);
+    else if (c.width == 2) ld((const uint16_t*)c.data);
+    else ld((const uint8_t*)c.data);
+}
+template <int U>
+AHEAD_DEV void gather_rows(const DCol& c, const uint64_t (&p)[U], uint64_t (&x)[U]) {
+    if (c.type == AHEAD_VOID) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) x[u] = (uint32_t)(c.seqbase + p[u]);
+        return;
+    }
+    auto ld = [&](auto* d) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) x[u] = __ldg(d + p[u]);
+    };
+    if (c.width == 8) ld((const unsigned long long*)c.data);
+    else if (c.width == 4) ld((const uint32_t*)c.data);
+    else if (c.width == 2) ld((const uint16_t*)c.data);
+    else ld((const uint8_t*)c.data);
+}
+
+template <class Op, class V, int U>
+AHEAD_DEV auto outputs_of(const Op& op, const V (&v)[U], uint64_t row0, const uint32_t (&idx)[U],
+                          uint64_t (&val)[Op::NOUT][U], int) -> decltype(op.rows0(v, row0, idx, val), void()) {
+    op.rows0(v, row0, idx, val);
+}
+template <class Op, class V, int U>
+AHEAD_DEV void outputs_of(const Op& op, const V (&v)[U], uint64_t row0, const uint32_t (&idx)[U],
+                          uint64_t (&val)[Op::NOUT][U], long) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int o = 0; o < Op::NOUT; ++o) val[o][u] = op.out0(o, v[u], row0 + idx[u]);
+}
+
+// Outputs u go to position base + i0 + 32 * u while i0 + 32 * u < room.
+template <class Op, int U>
+AHEAD_DEV auto store_outputs(const Op& op, uint64_t base, uint32_t i0, uint32_t room, const uint64_t (&val)[Op::NOUT][U],
+                             int) -> decltype(op.optr(0), void()) {
+#pragma unroll
+    for (int o = 0; o < Op::NOUT; ++o) {
+        auto st = [&](auto* p) {
+            p += base + i0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i0 + 32 * u < room) p[32 * u] = val[o][u];
+        };
+        const int w = op.owidth(o);
+        if (w == 8) st((uint64_t*)op.optr(o));
+        else if (w == 4) st((uint32_t*)op.optr(o));
+        else if (w == 2) st((uint16_t*)op.optr(o));
+        else st((uint8_t*)op.optr(o));
+    }
+}
+template <class Op, int U>
+AHEAD_DEV void store_outputs(const Op& op, uint64_t base, uint32_t i0, uint32_t room, const uint64_t (&val)[Op::NOUT][U],
+                             long) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (i0 + 32 * u < room) {
+#pragma unroll
+            for (int o = 0; o < Op::NOUT; ++o) op.put0(o, base + i0 + 32 * u, val[o][u]);
+        }
+}
+
 // Writes one tile's stream-0 rows to positions base, base + 1, ...: lane s < K
 // holds word s, `cnt` rows are kept, `list` is this warp's 32 * K half-words of
 // shared memory.  Four rows per lane are in flight at a time, since an output
@@ -246,34 +328,22 @@ AHEAD_DEV void tile_emit(const Op& op, uint64_t n, uint32_t tile, uint32_t word,
         }
         __syncwarp();
     }
-    const bool fits = base + cnt <= op.cap0();
-    auto rows = [&](auto fits_tag) {
-        constexpr bool FITS = decltype(fits_tag)::value;
-        for (uint32_t i0 = lane; i0 < cnt; i0 += 32 * U) {
-            uint64_t row[U], val[U][Op::NOUT];
-            typename std::conditional<W == 8, uint64_t, uint32_t>::type v[U];
+    const uint64_t fit = op.cap0() > base ? op.cap0() - base : 0;  // positions that are stored
+    const uint32_t room = fit < cnt ? (uint32_t)fit : cnt;
+    const uint32_t spare = all ? 0 : list[0];  // a kept row, for the lanes past the last one
+    for (uint32_t i0 = lane; i0 < cnt; i0 += 32 * U) {
+        uint32_t idx[U];
+        uint64_t val[Op::NOUT][U];
+        typename std::conditional<W == 8, uint64_t, uint32_t>::type v[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const uint32_t i = i0 + 32 * u;
-                row[u] = trow0 + (i < cnt ? (all ? i : list[i]) : 0u);
-                v[u] = Op::EMIT_V ? gmem_ld<W>(op.base, row[u]) : 0;
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (i0 + 32 * u < cnt) {
-#pragma unroll
-                    for (int o = 0; o < Op::NOUT; ++o) val[u][o] = op.out0(o, v[u], row[u]);
-                }
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (i0 + 32 * u < cnt && (FITS || base + i0 + 32 * u < op.cap0())) {
-#pragma unroll
-                    for (int o = 0; o < Op::NOUT; ++o) op.put0(o, base + i0 + 32 * u, val[u][o]);
-                }
+        for (int u = 0; u < U; ++u) {
+            const uint32_t i = i0 + 32 * u;
+            idx[u] = i < cnt ? (all ? i : list[i]) : spare;
+            v[u] = Op::EMIT_V ? gmem_ld<W>(op.base + trow0 * W, idx[u]) : 0;
         }
-    };
-    if (fits) rows(std::true_type());
-    else rows(std::false_type());
+        outputs_of(op, v, trow0, idx, val, 0);
+        store_outputs(op, base, i0, room, val, 0);
+    }
     if (!all) __syncwarp();  // the list is reused
 }
 

@@ -59,9 +59,8 @@ struct CheckOp {
     }
     AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row * aoid; }
     AHEAD_DEV uint64_t cap0() const { return errcap; }
-    AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        err[pos] = val;
-    }
+    AHEAD_DEV void* optr(int) const { return err; }
+    AHEAD_DEV int owidth(int) const { return 8; }
     AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
         if (pos < errcap) err[pos] = row * aoid;
     }
@@ -87,9 +86,8 @@ struct ColCheckOp {
     AHEAD_DEV uint32_t eval(uint64_t v, uint64_t, uint64_t&) const { return ((v * ainv) & wmaskenc) > umax ? 1u : 0u; }
     AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row * aoid; }
     AHEAD_DEV uint64_t cap0() const { return errcap; }
-    AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        err[pos] = val;
-    }
+    AHEAD_DEV void* optr(int) const { return err; }
+    AHEAD_DEV int owidth(int) const { return 8; }
     AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
         if (pos < errcap) err[pos] = row * aoid;
     }

@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256) probe_emit_kernel(const ProbeSlot* __rest
 // 8-byte raw codes as keys are not tried (multiples of A: far too wide).
 // At 60M probe rows against 320K of 800K keys: hash probe 512 + 559 us (one
 // 16-byte slot request to L2 per row, then thread-serial output) and 110 us of
-// separate column checks, against 15 us to build, 124 to classify and 289 to emit
+// separate column checks, against 15 us to build, 123 to classify and 219 to emit
 // (DRAM floor of the two passes: 205).
 constexpr uint64_t kDjMaxSpan = 1ull << 24;
 constexpr int kDjSmem = 200 * 1024;
@@ -325,15 +325,22 @@ struct DjOp {
         if ((d & pk.largermask) <= pk.condmax && k < span && ((bits[(uint32_t)k >> 5] >> (k & 31)) & 1u)) b |= 1u;
         return b;
     }
-    AHEAD_DEV uint64_t out0(int k, uint64_t v, uint64_t row) const {
-        if ((k == 0) == (o.probe_is_head != 0)) {
-            const uint64_t x = load_at(o.pcol, row);
-            return k == 0 ? (o.rh ? x * o.fh : x) : (o.rt ? x * o.ft : x);
+    // output 0: the probe side's value, output 1: the build side's
+    template <class V, int U>
+    AHEAD_DEV void rows0(const V (&v)[U], uint64_t row0, const uint32_t (&idx)[U], uint64_t (&x)[2][U]) const {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            x[1][u] = __ldg((const unsigned long long*)val + ((dec(v[u]) & pk.keymask) - kmin));
+        load_rows(o.pcol, row0, idx, x[0]);
+        if (o.probe_is_head ? o.rh : o.rt) {
+            const uint64_t f = o.probe_is_head ? o.fh : o.ft;
+#pragma unroll
+            for (int u = 0; u < U; ++u) x[0][u] *= f;
         }
-        return __ldg((const unsigned long long*)val + ((dec(v) & pk.keymask) - kmin));
     }
     AHEAD_DEV uint64_t cap0() const { return o.cap; }
-    AHEAD_DEV void put0(int k, uint64_t pos, uint64_t x) const { store_at(k == 0 ? o.oh : o.ot, k == 0 ? o.ohw : o.otw, pos, x); }
+    AHEAD_DEV void* optr(int k) const { return (k == 0) == (o.probe_is_head != 0) ? o.oh : o.ot; }
+    AHEAD_DEV int owidth(int k) const { return (k == 0) == (o.probe_is_head != 0) ? o.ohw : o.otw; }
     AHEAD_DEV void emit(int c, uint64_t pos, uint64_t, uint64_t row) const {
         if (c == 1) {
             if (pos < eck) ek[pos] = row * aoid;
@@ -543,18 +550,24 @@ struct MjPosOp {
         if (CHECKED && t2enc && dec_if(t2c, load_at(t2c, p), t2c.ainv) > t2c.umax) return bits | 8u;
         return bits | 1u;
     }
-    AHEAD_DEV uint64_t out0(int k, uint64_t v, uint64_t row) const {
-        if (k == 0) {
-            const uint64_t h = load_at(h1c, row);
-            return reenc ? dec_if(h1c, h, fh) : h;
+    template <class V, int U>
+    AHEAD_DEV void rows0(const V (&v)[U], uint64_t row0, const uint32_t (&idx)[U], uint64_t (&x)[2][U]) const {
+        uint64_t p[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) p[u] = pos2(v[u]);
+        gather_rows(t2c, p, x[1]);
+        load_rows(h1c, row0, idx, x[0]);
+        if (reenc) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                x[0][u] = dec_if(h1c, x[0][u], fh);
+                x[1][u] = dec_if(t2c, x[1][u], ft);
+            }
         }
-        const uint64_t t = load_at(t2c, pos2(v));
-        return reenc ? dec_if(t2c, t, ft) : t;
     }
     AHEAD_DEV uint64_t cap0() const { return cap; }
-    AHEAD_DEV void put0(int k, uint64_t pos, uint64_t val) const {
-        store_at(k == 0 ? oh : ot, k == 0 ? ohw : otw, pos, val);
-    }
+    AHEAD_DEV void* optr(int k) const { return k == 0 ? oh : ot; }
+    AHEAD_DEV int owidth(int k) const { return k == 0 ? ohw : otw; }
     AHEAD_DEV void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const {
         if (c == 1) {
             if (pos < ec1) e1[pos] = row * aoid;
@@ -595,14 +608,20 @@ struct FetchOp {
         if (CHECKED && bad(load_at(t2c, p))) return 4u;
         return 1u;
     }
-    AHEAD_DEV uint64_t out0(int, uint64_t v, uint64_t) const {
-        const uint64_t t = load_at(t2c, pos(v));
-        return reenc ? mulw(t, fac, w2) : t;
+    template <class V, int U>
+    AHEAD_DEV void rows0(const V (&v)[U], uint64_t, const uint32_t (&)[U], uint64_t (&x)[1][U]) const {
+        uint64_t p[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) p[u] = pos(v[u]);
+        gather_rows(t2c, p, x[0]);
+        if (reenc) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) x[0][u] = mulw(x[0][u], fac, w2);
+        }
     }
     AHEAD_DEV uint64_t cap0() const { return cap; }
-    AHEAD_DEV void put0(int, uint64_t p, uint64_t val) const {
-        store_at(ot, otw, p, val);
-    }
+    AHEAD_DEV void* optr(int) const { return ot; }
+    AHEAD_DEV int owidth(int) const { return otw; }
     AHEAD_DEV void emit(int c, uint64_t p, uint64_t v, uint64_t row) const {
         if (c == 1) {
             if (p < ec1) e1[p] = row * aoid;
@@ -887,9 +906,8 @@ struct IsectOp {
         return reenc ? dec_if(t2c, t, ft) : t;
     }
     AHEAD_DEV uint64_t cap0() const { return cap; }
-    AHEAD_DEV void put0(int k, uint64_t pos, uint64_t val) const {
-        store_at(k == 0 ? oh : ot, k == 0 ? ohw : otw, pos, val);
-    }
+    AHEAD_DEV void* optr(int k) const { return k == 0 ? oh : ot; }
+    AHEAD_DEV int owidth(int k) const { return k == 0 ? ohw : otw; }
     AHEAD_DEV void emit(int, uint64_t, uint64_t, uint64_t) const {}
 };
 
@@ -926,9 +944,8 @@ struct IsectPlainOp {
         return k == 0 ? load_at(h1c, row) : load_at(t2c, find(row));
     }
     AHEAD_DEV uint64_t cap0() const { return cap; }
-    AHEAD_DEV void put0(int k, uint64_t pos, uint64_t val) const {
-        store_at(k == 0 ? oh : ot, k == 0 ? ohw : otw, pos, val);
-    }
+    AHEAD_DEV void* optr(int k) const { return k == 0 ? oh : ot; }
+    AHEAD_DEV int owidth(int k) const { return k == 0 ? ohw : otw; }
     AHEAD_DEV void emit(int, uint64_t, uint64_t, uint64_t) const {}
 };
 
@@ -1074,12 +1091,10 @@ struct FetchStrOp {
     AHEAD_DEV uint32_t eval(uint64_t v, uint64_t, uint64_t&) const { return v * ainv < count ? 1u : 2u; }
     AHEAD_DEV uint64_t out0(int, uint64_t v, uint64_t) const { return v * ainv; }
     AHEAD_DEV uint64_t cap0() const { return cap; }
-    AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        rows[pos] = (uint32_t)val;
-    }
+    AHEAD_DEV void* optr(int) const { return rows; }
+    AHEAD_DEV int owidth(int) const { return 4; }
     AHEAD_DEV void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const {
-        if (c == 0) put0(0, pos, out0(0, v, row));
-        else if (pos < errcap) err[pos] = row * aoid;
+        if (c == 1 && pos < errcap) err[pos] = row * aoid;
     }
 };
 
@@ -1100,10 +1115,9 @@ struct FetchStrPlainOp {
     AHEAD_DEV uint32_t eval(uint64_t v, uint64_t, uint64_t&) const { return v < count ? 1u : 0u; }
     AHEAD_DEV uint64_t out0(int, uint64_t v, uint64_t) const { return v; }
     AHEAD_DEV uint64_t cap0() const { return cap; }
-    AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        rows[pos] = (uint32_t)val;
-    }
-    AHEAD_DEV void emit(int, uint64_t pos, uint64_t v, uint64_t) const { put0(0, pos, v); }
+    AHEAD_DEV void* optr(int) const { return rows; }
+    AHEAD_DEV int owidth(int) const { return 4; }
+    AHEAD_DEV void emit(int, uint64_t, uint64_t, uint64_t) const {}
 };
 
 // The slots of a compacted row list, into `out` (the second step of both string fetch-joins).

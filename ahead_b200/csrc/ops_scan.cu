@@ -37,10 +37,8 @@ struct SelectOp {
         return AN ? (uint64_t)oid * kResoidAMax : (uint64_t)oid;
     }
     AHEAD_DEV uint64_t cap0() const { return cap; }
-    AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        if (AN) out_an[pos] = val;
-        else out_oid[pos] = (uint32_t)val;
-    }
+    AHEAD_DEV void* optr(int) const { return AN ? (void*)out_an : (void*)out_oid; }
+    AHEAD_DEV int owidth(int) const { return AN ? 8 : 4; }
     AHEAD_DEV uint32_t eval(uint64_t v, uint64_t, uint64_t&) const {
         if constexpr (W <= 4) {
             // narrow codes: 32-bit arithmetic; a single plain interval is the common case
@@ -246,9 +244,8 @@ struct CadVoidOp {
     }
     AHEAD_DEV uint64_t out0(int, uint64_t v, uint64_t) const { return mulw(v, ainv, W); }
     AHEAD_DEV uint64_t cap0() const { return cap; }
-    AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        store_at(out, ow, pos, val);
-    }
+    AHEAD_DEV void* optr(int) const { return out; }
+    AHEAD_DEV int owidth(int) const { return ow; }
     AHEAD_DEV void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const {
         if (c == 0) {
             if (pos < cap) store_at(out, ow, pos, mulw(v, ainv, W));
@@ -281,9 +278,8 @@ struct CadGenOp {
         return k == 0 ? dec_if(hc, load_at(hc, row), hc.ainv) : mulw(t, tc.ainv, W);
     }
     AHEAD_DEV uint64_t cap0() const { return cap; }
-    AHEAD_DEV void put0(int k, uint64_t pos, uint64_t val) const {
-        store_at(k == 0 ? oh : ot, k == 0 ? ohw : otw, pos, val);
-    }
+    AHEAD_DEV void* optr(int k) const { return k == 0 ? oh : ot; }
+    AHEAD_DEV int owidth(int k) const { return k == 0 ? ohw : otw; }
     AHEAD_DEV uint32_t eval(uint64_t t, uint64_t row, uint64_t&) const {
         const uint64_t h = load_at(hc, row);
         const uint64_t dh = dec_if(hc, h, hc.ainv), dt = mulw(t, tc.ainv, W);
@@ -323,9 +319,8 @@ struct DecodeOp {
     static constexpr int NOUT = 1;
     AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row * aoid; }
     AHEAD_DEV uint64_t cap0() const { return errcap; }
-    AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        err[pos] = val;
-    }
+    AHEAD_DEV void* optr(int) const { return err; }
+    AHEAD_DEV int owidth(int) const { return 8; }
     AHEAD_DEV uint32_t eval(uint64_t t, uint64_t row, uint64_t&) const {
         const uint64_t d = mulw(t, tc.ainv, W);
         store_at(oh, ohw, row, load_at(hc, row));
@@ -356,9 +351,8 @@ struct MulSumOp {
     static constexpr int NOUT = 1;
     AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row * aoid; }
     AHEAD_DEV uint64_t cap0() const { return ecap1; }
-    AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        e1[pos] = val;
-    }
+    AHEAD_DEV void* optr(int) const { return e1; }
+    AHEAD_DEV int owidth(int) const { return 8; }
     AHEAD_DEV uint32_t eval(uint64_t a, uint64_t row, uint64_t& s) const {
         const uint64_t b = load_at(bc, row);
         s += a * b;
@@ -596,9 +590,8 @@ struct ArithOp {
     static constexpr int NOUT = 1;
     AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row * aoid; }
     AHEAD_DEV uint64_t cap0() const { return ecap1; }
-    AHEAD_DEV void put0(int, uint64_t pos, uint64_t val) const {
-        e1[pos] = val;
-    }
+    AHEAD_DEV void* optr(int) const { return e1; }
+    AHEAD_DEV int owidth(int) const { return 8; }
     AHEAD_DEV uint32_t eval(uint64_t a, uint64_t row, uint64_t&) const {
         const uint64_t t1 = mulw(a, ac.ainv, W), t2 = mulw(load_at(bc, row), bc.ainv, bc.width);
         const uint64_t x = t1 * ar, y = t2 * ar;
