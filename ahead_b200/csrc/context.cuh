@@ -60,6 +60,7 @@ struct OpScope {
     uint32_t* d_status = nullptr;
     uint64_t* d_counters = nullptr;  // [kStageWords - 1]
     int rc = AHEAD_OK;
+    bool pending = false;  // launches since the last wait
 
     explicit OpScope(ahead_ctx* c) : ctx(c) {}
 
@@ -109,11 +110,26 @@ struct OpScope {
         return cb;
     }
 
-    void launched(int n = 1) { ctx->launches += n; }
+    void launched(int n = 1) {
+        ctx->launches += n;
+        pending = true;
+    }
+
+    // Waits for launches made after the last finish(): a caller may read the
+    // outputs on any stream once a call has returned.
+    int wait() {
+        if (!pending) return AHEAD_OK;
+        pending = false;
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
+        e = cudaStreamSynchronize(ctx->stream);
+        return e == cudaSuccess ? AHEAD_OK : cuda_fail(ctx, e, "cudaStreamSynchronize");
+    }
 
     // Copy the status word and the first `ncounters` counters to the host and
     // wait for the stream.  Returns the call's status.
     int finish(int ncounters) {
+        pending = false;
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
         e = cudaMemcpyAsync(ctx->h_stage, ctx->arena, 8 + 8 * (size_t)ncounters, cudaMemcpyDeviceToHost,

@@ -124,12 +124,10 @@ inline void run_colcheck(OpScope& s, const ahead_col& c, uint64_t n, uint64_t ai
 constexpr uint32_t kFastErrCap = 4096;
 
 // Block c sorts list c (at most kFastErrCap rows, bitonic in shared memory)
-// and writes row * aoid into the error vector, up to its capacity; block 0
-// also writes its sorted rows to `sorted` when given.
+// and writes row * aoid into the error vector, up to its capacity.
 static __global__ void __launch_bounds__(1024) sort_err_rows_kernel(const unsigned long long* cnt, const uint64_t* rows1,
                                                              const uint64_t* rows2, uint64_t* e1, uint64_t cap1,
-                                                             uint64_t* e2, uint64_t cap2, uint64_t aoid,
-                                                             uint64_t* sorted = nullptr) {
+                                                             uint64_t* e2, uint64_t cap2, uint64_t aoid) {
     __shared__ uint64_t s_r[kFastErrCap];
     const int c = blockIdx.x;
     const unsigned long long k = cnt[c];
@@ -158,8 +156,6 @@ static __global__ void __launch_bounds__(1024) sort_err_rows_kernel(const unsign
         }
     if (e)
         for (uint32_t i = threadIdx.x; i < k && i < cap; i += blockDim.x) e[i] = s_r[i] * aoid;
-    if (sorted && c == 0)
-        for (uint32_t i = threadIdx.x; i < k; i += blockDim.x) sorted[i] = s_r[i];
 }
 
 // One column's short error list: its count is counter `ci` of the call.
@@ -182,9 +178,8 @@ inline ErrList err_list(OpScope& s, int ci) {
 }
 
 // After finish() has read the counters back: writes the error vector of a list
-// with a few rows (a launch, no wait: the stream orders it before any reader)
-// and returns false when the list overflowed, so that the caller runs the
-// column's compaction.
+// with a few rows (a launch: the caller waits) and returns false when the list
+// overflowed, so that the caller runs the column's compaction.
 inline bool settle_err_list(OpScope& s, const ErrList& l, int ci, uint64_t aoid, ahead_errvec* e) {
     const uint64_t k = s.counter(ci);
     if (k > kFastErrCap) return false;
@@ -197,6 +192,229 @@ inline bool settle_err_list(OpScope& s, const ErrList& l, int ci, uint64_t aoid,
         }
     }
     return true;
+}
+
+// ---------------------------------------------- rows dropped now and then
+// checkAndDecodeAN and the positional joins drop a row only when its code, OID
+// or fetched value is corrupt, which is rare.  So one pass writes every row's
+// output at the row's own position and lists the rows to drop (unordered; bit 0
+// of an entry is its kind, which error vector reports it).  With none listed
+// the outputs are done; with a few, the list is sorted into the error vectors
+// and the outputs are moved down in place; more than kMaxDrops (or than the scratch
+// holds the edges of): the caller
+// runs the compaction, which writes everything again.  (The compaction's two
+// passes gather every value twice.)
+constexpr uint32_t kMaxDrops = 2048;
+constexpr uint32_t kSureDrops = 256;  // scratch for the edges of this many is always there: an eighth of the outputs
+
+struct DropList {
+    unsigned long long *cnt, *kind1;  // entries, and those of kind 1
+    uint64_t* rows;                   // [kMaxDrops] row << 1 | kind
+    AHEAD_DEV void add(uint64_t row, uint32_t kind) const {
+        if (*(volatile unsigned long long*)cnt > kMaxDrops) return;
+        const unsigned long long k = atomicAdd(cnt, 1ull);
+        if (k < kMaxDrops) rows[k] = row << 1 | kind;
+        if (kind) atomicAdd(kind1, 1ull);
+    }
+};
+
+inline DropList drop_list(OpScope& s, int ci) {  // counters ci, ci + 1
+    DropList l;
+    l.cnt = (unsigned long long*)(s.d_counters + ci);
+    l.kind1 = l.cnt + 1;
+    l.rows = (uint64_t*)s.alloc(kMaxDrops * 8);
+    return l;
+}
+
+// One block sorts the k listed rows into `sorted` and writes the error vectors:
+// row * aoid (kind 0, and kind 1 without a position column), or the position the
+// row's OID names, times aoid (kind 1; `oid` holds the 8-byte codes).
+static __global__ void __launch_bounds__(1024) sort_drops_kernel(const uint64_t* rows, uint32_t k, uint64_t* sorted,
+                                                                 const uint64_t* oid, uint64_t ainv, uint64_t aoid,
+                                                                 uint64_t* e0, uint64_t cap0, uint64_t* e1,
+                                                                 uint64_t cap1) {
+    __shared__ uint64_t s_r[kMaxDrops];
+    __shared__ uint64_t s_part[33];
+    uint32_t m = 1;
+    while (m < k) m <<= 1;
+    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) s_r[i] = i < k ? rows[i] : ~0ull;
+    __syncthreads();
+    for (uint32_t size = 2; size <= m; size <<= 1)
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
+                const uint32_t j = i ^ stride;
+                if (j > i) {
+                    const uint64_t x = s_r[i], y = s_r[j];
+                    if ((x > y) == ((i & size) == 0)) {
+                        s_r[i] = y;
+                        s_r[j] = x;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    uint64_t ones = 0;  // entries of kind 1 before this round's
+    for (uint32_t i0 = 0; i0 < k; i0 += 1024) {
+        const uint32_t i = i0 + threadIdx.x;
+        const uint64_t x = i < k ? s_r[i] : 0;
+        uint64_t total;
+        const uint64_t before = ones + block_scan_1024(x & 1, s_part, &total);
+        if (i < k) {
+            const uint64_t row = x >> 1;
+            sorted[i] = row;
+            if (x & 1) {
+                if (e1 && before < cap1) e1[before] = (oid ? oid[row] * ainv : row) * aoid;
+            } else if (e0 && i - before < cap0) {
+                e0[i - before] = row * aoid;
+            }
+        }
+        ones += total;
+    }
+}
+
+// Moves the rows of one or two columns down over the k dropped ones, in place.
+// A chunk of 2048 rows (4096 of up to 4 bytes) moves by at most k of its rows:
+// the rows whose place lies in their own chunk go there directly, once all of
+// the chunk is in registers; the few that go to the chunk before wait in `edge`
+// (k per chunk) for shift_edges_kernel.  Together they read and write each row
+// behind the first dropped one once.  A chunk's loads are issued before it looks
+// for its place in the list, which the whole block does with one load per entry.
+// 60M 4-byte values move in 88 us (480 MB, 5.5 TB/s); with a binary search ahead
+// of the loads, or the rows spilled to local memory, it took 106 and 141.
+constexpr uint32_t kShiftChunk = 2048;
+constexpr uint32_t shift_chunk(int w) { return w == 8 ? kShiftChunk : 2 * kShiftChunk; }
+
+template <int W>
+struct UIntOf {
+    typedef typename std::conditional<W == 8, uint64_t, typename std::conditional<W == 4, uint32_t,
+        typename std::conditional<W == 2, uint16_t, uint8_t>::type>::type>::type type;
+};
+
+struct ShiftCols {
+    void* data[2];
+    void* edge[2];
+    uint64_t n;
+    const uint64_t* sorted;
+    uint32_t k;
+};
+
+AHEAD_DEV uint32_t drops_below(const uint64_t* sorted, uint32_t lo, uint32_t hi, uint64_t row) {
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (__ldg((const unsigned long long*)sorted + mid) < row) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+template <int W>
+__global__ void __launch_bounds__(256, 8) shift_rows_kernel(ShiftCols s) {
+    typedef typename UIntOf<W>::type T;
+    constexpr uint32_t C = shift_chunk(W);
+    constexpr uint32_t U = C / 256;
+    __shared__ T s_v[C];
+    const int col = blockIdx.y;
+    const uint64_t c0 = (uint64_t)blockIdx.x * C;
+    T* p = (T*)(col ? s.data[1] : s.data[0]) + c0;
+    const uint32_t m = s.n - c0 < C ? (uint32_t)(s.n - c0) : C, t = threadIdx.x;
+    typename std::conditional<W == 8, uint64_t, uint32_t>::type v[U];
+    if (m == C) {
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) v[u] = p[u * 256 + t];
+    } else {
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) v[u] = u * 256 + t < m ? p[u * 256 + t] : 0;
+    }
+    uint32_t lo = 0, hi = 0;  // dropped rows before the chunk, and before its end
+    for (uint32_t i0 = 0; i0 < s.k; i0 += 256) {
+        const uint64_t x = i0 + t < s.k ? __ldg((const unsigned long long*)s.sorted + i0 + t) : ~0ull;
+        lo += __syncthreads_count(x < c0);  // (also: the chunk is read before any of it is overwritten)
+        hi += __syncthreads_count(x < c0 + m);
+    }
+    if (hi == 0) return;
+    T* e = (T*)(col ? s.edge[1] : s.edge[0]) + (uint64_t)blockIdx.x * s.k;
+    if (lo == hi) {  // (nearly every chunk) the same move for all rows
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t r = u * 256 + t;
+            if (r < lo) {
+                if (r < m) e[lo - 1 - r] = (T)v[u];
+            } else if (r < m) {
+                p[r - lo] = (T)v[u];
+            }
+        }
+        return;
+    }
+    // a chunk with dropped rows: each row looks up how many lie before it (through
+    // shared memory: a loop of searches over a register array would spill it)
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) s_v[u * 256 + t] = (T)v[u];
+    __syncthreads();
+    for (uint32_t r = t; r < m; r += 256) {
+        const uint32_t d = drops_below(s.sorted, lo, hi, c0 + r);
+        if (d < hi && __ldg((const unsigned long long*)s.sorted + d) == c0 + r) continue;
+        if (r >= d) p[r - d] = s_v[r];
+        else e[d - 1 - r] = s_v[r];
+    }
+}
+
+template <int W>
+__global__ void __launch_bounds__(256) shift_edges_kernel(ShiftCols s) {  // a warp per chunk
+    const int col = blockIdx.y;
+    typedef typename UIntOf<W>::type T;
+    constexpr uint32_t C = shift_chunk(W);
+    const uint32_t lane = threadIdx.x & 31, chunk = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const uint64_t c0 = (uint64_t)chunk * C, c1 = c0 + C < s.n ? c0 + C : s.n;
+    if (c0 >= s.n) return;
+    uint32_t lo = 0, hi = 0;
+    for (uint32_t i = lane; i < s.k; i += 32) {
+        const uint64_t x = __ldg((const unsigned long long*)s.sorted + i);
+        lo += x < c0;
+        hi += x < c1;
+    }
+    lo = __reduce_add_sync(kFull, lo);
+    hi = __reduce_add_sync(kFull, hi);
+    const uint32_t clean = (uint32_t)(c1 - c0) - (hi - lo);
+    const T* e = (const T*)(col ? s.edge[1] : s.edge[0]) + (uint64_t)chunk * s.k;
+    T* p = (T*)(col ? s.data[1] : s.data[0]);
+    // the chunk's first clean row goes to c0 - lo, the next ones behind it
+    for (uint32_t i = lane; i < lo && i < clean; i += 32) p[c0 - lo + i] = e[lo - 1 - i];
+}
+
+// Scratch of the list, the sorted rows and the edges of columns of `row_bytes` together.
+inline size_t drop_scratch(uint64_t n, uint64_t row_bytes) {
+    return ((n + kShiftChunk - 1) / kShiftChunk) * kSureDrops * row_bytes + 2 * kMaxDrops * 8 + 4096;
+}
+// Whether k dropped rows' outputs (of `row_bytes` together) can be moved with the scratch at hand.
+inline bool shift_fits(const OpScope& s, uint64_t n, uint64_t k, uint64_t row_bytes) {
+    return k <= kMaxDrops &&
+           s.off + ((n + kShiftChunk - 1) / kShiftChunk) * k * row_bytes + 1024 <= s.ctx->arena_cap;
+}
+
+// Closes the k gaps in the columns o and, when given, ot.
+inline void launch_shift(OpScope& s, uint64_t n, const uint64_t* sorted, uint32_t k, void* o, int ow,
+                         void* ot = nullptr, int otw = 0) {
+    ShiftCols c;
+    c.n = n;
+    c.sorted = sorted;
+    c.k = k;
+    auto run = [&](int w, int cols) {
+        by_width(w, [&](auto tag) -> int {
+            constexpr int W = decltype(tag)::value;
+            const uint32_t chunks = (uint32_t)((n + shift_chunk(W) - 1) / shift_chunk(W));
+            for (int i = 0; i < cols; ++i) c.edge[i] = s.alloc((size_t)chunks * k * W);
+            shift_rows_kernel<W><<<dim3(chunks, cols), 256, 0, s.ctx->stream>>>(c);
+            shift_edges_kernel<W><<<dim3((chunks + 7) / 8, cols), 256, 0, s.ctx->stream>>>(c);
+            return 0;
+        });
+        s.launched(2);
+    };
+    c.data[0] = o;
+    c.data[1] = ot;
+    if (!ot || ow == otw) return run(ow, ot ? 2 : 1);
+    run(ow, 1);
+    c.data[0] = ot;
+    run(otw, 1);
 }
 
 }  // namespace ahead

@@ -456,10 +456,6 @@ int run_groupby(ahead_ctx* ctx, const ahead_bat* in, const ahead_bat* grouping, 
         }
         const bool ok_t = settle_err_list(s, g.terr, kGbTail, aoid, ev(errs, 1));
         const bool ok_g = !binary || settle_err_list(s, g.gerr, kGbGrp, aoid, ev(errs, 2));
-        if (groups > kGbSort) {
-            rc = s.finish(1);
-            if (rc) return rc;
-        }
         if (!ok_t || !ok_g) {  // a column with many corrupt codes
             rc = s.reserve(2 * colcheck_scratch(n));
             if (rc) return rc;
@@ -471,6 +467,8 @@ int run_groupby(ahead_ctx* ctx, const ahead_bat* in, const ahead_bat* grouping, 
             if (errs && !ok_g) errs[2].count = s.counter(3);
         }
         firsts->count = groups;
+        rc = s.wait();
+        if (rc) return rc;
         return (n > cap || groups > cap) ? AHEAD_CAPACITY : AHEAD_OK;
     }
     // keys beyond the first-row table: the hash table

@@ -305,15 +305,18 @@ struct DjOp {
     const uint32_t* bad;
     const uint32_t* bits;
     const uint64_t* val;
-    uint64_t limit, kmin, span;  // kmin, span: set by begin
+    uint64_t limit;
+    uint32_t kmin, span;  // set by begin (keys have at most 32 bits)
     uint64_t aoid, eck, eco;
     uint64_t *ek, *eo, *acc;
     AHEAD_DEV void begin() {
-        kmin = ~__ldg((const unsigned long long*)bounds);
-        span = __ldg((const unsigned long long*)bounds + 1) - kmin + 1;
-        if (__ldg(bad) || span > limit) span = 0;
+        const uint64_t lo = ~__ldg((const unsigned long long*)bounds);
+        const uint64_t m = __ldg((const unsigned long long*)bounds + 1) - lo + 1;
+        kmin = (uint32_t)lo;
+        span = (__ldg(bad) || m > limit) ? 0u : (uint32_t)m;
     }
     AHEAD_DEV uint64_t dec(uint64_t v) const { return pk.dec ? mulw(v, pk.ainv, W) : v; }
+    AHEAD_DEV uint32_t key(uint64_t d) const { return ((uint32_t)d & (uint32_t)pk.keymask) - kmin; }
     AHEAD_DEV uint32_t eval(uint64_t v, uint64_t row, uint64_t&) const {
         const uint64_t d = dec(v);
         uint32_t b = 0;
@@ -321,8 +324,10 @@ struct DjOp {
             if (d > pk.col.umax) b |= 2u;
             if (o.pcol.enc && mulw(load_at(o.pcol, row), o.pcol.ainv, o.pcol.width) > o.pcol.umax) b |= 4u;
         }
-        const uint64_t k = (d & pk.keymask) - kmin;
-        if ((d & pk.largermask) <= pk.condmax && k < span && ((bits[(uint32_t)k >> 5] >> (k & 31)) & 1u)) b |= 1u;
+        const uint32_t k = key(d);
+        // (the key's range check only where the other side's keys are wider)
+        if (pk.largermask > pk.condmax && (d & pk.largermask) > pk.condmax) return b;
+        if (k < span && ((bits[k >> 5] >> (k & 31)) & 1u)) b |= 1u;
         return b;
     }
     // output 0: the probe side's value, output 1: the build side's
@@ -330,7 +335,7 @@ struct DjOp {
     AHEAD_DEV void rows0(const V (&v)[U], uint64_t row0, const uint32_t (&idx)[U], uint64_t (&x)[2][U]) const {
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            x[1][u] = __ldg((const unsigned long long*)val + ((dec(v[u]) & pk.keymask) - kmin));
+            x[1][u] = __ldg((const unsigned long long*)val + key(dec(v[u])));
         load_rows(o.pcol, row0, idx, x[0]);
         if (o.probe_is_head ? o.rh : o.rt) {
             const uint64_t f = o.probe_is_head ? o.fh : o.ft;
@@ -630,6 +635,152 @@ struct FetchOp {
         }
     }
 };
+
+// The positional joins in one pass: almost every row is kept, so row i's output
+// goes to position i at once and the rows to drop are listed (see DropList).
+// kRows rows per lane, their list entries, then their gathers in flight
+// together.  What bounds it is the gather: at 12M OIDs of a fifth of a 60M-row
+// 8-byte column nearly 60 % of the column's sectors are read (571 MB with the
+// list and the outputs).
+struct PosArgs {
+    const char* base;   // the OID list's codes
+    uint64_t n, inv, sz;
+    DCol h1c, t2c;      // head of the list, fetched column
+    uint64_t fh, ft;    // re-encoding factors
+    void *oh, *ot;      // (oh null: fetchjoin, no head output)
+    int ohw, otw, reenc, head_err, t2enc, w2;
+    ErrList herr;       // corrupt heads
+    DropList drops;     // kind 0: OID past the column, kind 1: corrupt value
+};
+constexpr int kPosRows = 4;
+
+template <bool CHECKED, bool FETCH>
+__global__ void __launch_bounds__(256) pos_join_kernel(PosArgs a) {
+    constexpr int W = CHECKED ? 8 : 4;
+    typedef typename std::conditional<W == 8, uint64_t, uint32_t>::type V;
+    const int lane = threadIdx.x & 31;
+    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5, span = 32 * kPosRows;
+    for (uint64_t r0 = warp * span; r0 < a.n; r0 += warps * span) {
+        const uint32_t cnt = a.n - r0 < span ? (uint32_t)(a.n - r0) : (uint32_t)span;
+        uint32_t idx[kPosRows];
+        V v[kPosRows];
+        uint64_t p[kPosRows], val[2][kPosRows];
+        bool ok[kPosRows];
+#pragma unroll
+        for (int u = 0; u < kPosRows; ++u) {
+            idx[u] = lane + 32 * u < cnt ? lane + 32 * u : 0;
+            v[u] = gmem_ld<W>(a.base + r0 * W, idx[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < kPosRows; ++u) {
+            p[u] = CHECKED ? v[u] * a.inv : v[u];
+            ok[u] = p[u] < a.sz;
+            if (!ok[u]) {
+                if (lane + 32 * u < cnt) a.drops.add(r0 + idx[u], 0);
+                p[u] = 0;  // (the column has a row: sz > 0)
+            }
+        }
+        gather_rows(a.t2c, p, val[1]);
+        if (!FETCH) {
+            if (CHECKED && a.h1c.data == a.base) {  // a mirrored list: the head is the OID itself
+#pragma unroll
+                for (int u = 0; u < kPosRows; ++u) val[0][u] = v[u];
+            } else {
+                load_rows(a.h1c, r0, idx, val[0]);
+            }
+            if (CHECKED && a.head_err) {
+#pragma unroll
+                for (int u = 0; u < kPosRows; ++u)
+                    if (val[0][u] * a.h1c.ainv > a.h1c.umax && lane + 32 * u < cnt) a.herr.add(r0 + idx[u]);
+            }
+        }
+        if (CHECKED && a.t2enc) {
+#pragma unroll
+            for (int u = 0; u < kPosRows; ++u) {
+                // fetchjoinAN's check has no cast: 16-bit codes are multiplied as 32-bit ints
+                const bool bad = FETCH && a.w2 == 2
+                                     ? (int32_t)(uint32_t)(val[1][u] * a.t2c.ainv) > (int32_t)a.t2c.umax
+                                     : mulw(val[1][u], a.t2c.ainv, a.w2) > a.t2c.umax;
+                if (bad && ok[u] && lane + 32 * u < cnt) a.drops.add(r0 + idx[u], 1);
+            }
+        }
+        if (a.reenc) {
+#pragma unroll
+            for (int u = 0; u < kPosRows; ++u) {
+                if (!FETCH) val[0][u] = dec_if(a.h1c, val[0][u], a.fh);
+                val[1][u] = dec_if(a.t2c, val[1][u], a.ft);
+            }
+        }
+        auto store = [&](void* o, int w, const uint64_t (&x)[kPosRows]) {
+            auto st = [&](auto* q) {
+                q += r0 + lane;
+#pragma unroll
+                for (int u = 0; u < kPosRows; ++u)
+                    if (lane + 32 * u < cnt) q[32 * u] = x[u];
+            };
+            if (w == 8) st((uint64_t*)o);
+            else if (w == 4) st((uint32_t*)o);
+            else if (w == 2) st((uint16_t*)o);
+            else st((uint8_t*)o);
+        };
+        if (!FETCH) store(a.oh, a.ohw, val[0]);
+        store(a.ot, a.otw, val[1]);
+    }
+}
+
+// Where the one-pass form pays and applies: more rows than one block's
+// compaction takes (8,192), room for every row, and a column to fetch from.
+inline bool pos_one_pass(uint64_t n, uint64_t cap, uint64_t sz) {
+    return n > 32 * short_k(8) * (uint64_t)kOneBlockTiles && n <= cap && sz > 0;
+}
+
+constexpr int kPosHead = 30, kPosDrops = 31, kPosCounters = 33;  // counters
+
+// Runs the one-pass form; *kept = rows kept.  Returns AHEAD_UNSUPPORTED when
+// too many rows are dropped and the compaction has to run.  `dense_head`: every
+// head is known to read as corrupt, so its vector is made by a column check.
+template <bool CHECKED, bool FETCH>
+int run_pos_join(OpScope& s, PosArgs& a, const ahead_col* head, uint64_t aoid, bool dense_head, ahead_errvec* eh,
+                 ahead_errvec* e0, ahead_errvec* e1, uint64_t* kept) {
+    const uint64_t n = a.n;
+    const size_t check = a.head_err ? colcheck_scratch(n) : 0;
+    int rc = s.reserve(drop_scratch(n, (FETCH ? 0 : a.ohw) + a.otw) + kErrListBytes + check);
+    if (rc) return rc;
+    a.herr = err_list(s, kPosHead);
+    a.drops = drop_list(s, kPosDrops);
+    uint64_t* sorted = (uint64_t*)s.alloc(kMaxDrops * 8);
+    const bool want_head = a.head_err && eh;
+    if (dense_head) a.head_err = 0;
+    const uint64_t blocks = (n + 256 * kPosRows - 1) / (256 * kPosRows);
+    const uint32_t most = (uint32_t)s.ctx->num_sms * 32;
+    pos_join_kernel<CHECKED, FETCH><<<blocks < most ? (uint32_t)blocks : most, 256, 0, s.ctx->stream>>>(a);
+    s.launched();
+    auto check_head = [&] { run_colcheck(s, *head, n, a.h1c.ainv, a.h1c.umax, 8, aoid, eh, 1); };
+    if (want_head && dense_head) check_head();
+    rc = s.finish(kPosCounters);
+    if (rc) return rc;
+    const uint64_t k = s.counter(kPosDrops), k1 = s.counter(kPosDrops + 1);
+    if (!shift_fits(s, n, k, (FETCH ? 0 : a.ohw) + a.otw)) return AHEAD_UNSUPPORTED;
+    *kept = n - k;
+    if (e0) e0->count = k - k1;
+    if (e1) e1->count = k1;
+    if (want_head && dense_head) eh->count = s.counter(1);
+    if (k) {
+        sort_drops_kernel<<<1, 1024, 0, s.ctx->stream>>>(a.drops.rows, (uint32_t)k, sorted, (const uint64_t*)a.base,
+                                                         a.inv, aoid, edata(e0), ecap(e0), edata(e1), ecap(e1));
+        s.launched();
+        if (FETCH) launch_shift(s, n, sorted, (uint32_t)k, a.ot, a.otw);
+        else launch_shift(s, n, sorted, (uint32_t)k, a.ot, a.otw, a.oh, a.ohw);
+    }
+    if (want_head && !dense_head && !settle_err_list(s, a.herr, kPosHead, aoid, eh)) {
+        check_head();
+        rc = s.finish(2);
+        if (rc) return rc;
+        eh->count = s.counter(1);
+    }
+    return s.wait();
+}
 
 // ------------------------------------------------------------ merge joins
 struct MergeSide {
@@ -1283,6 +1434,8 @@ int ahead_gpu_hashjoin_an(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r
                 if (!okv) errs[vbo].count = s.counter(1 + vbo);
             }
         }
+        rc = s.wait();
+        if (rc) return rc;
         return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
     }
     rc = s.reserve(join_scratch(nb, np) + colcheck_scratch(nl) * 2 + colcheck_scratch(nr) * 2);
@@ -1378,7 +1531,35 @@ int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
     OpScope s(ctx);
     if (rv) {
         set_errs_present(errs, type_encoded(H1), 1, 0, type_encoded(T2));
-        int rc = s.reserve(compact_scratch<MjPosOp<true>>(n1));
+        const uint64_t sz = (uint32_t)b->count;  // BAT::size() is an oid_t
+        int rc;
+        if (pos_one_pass(n1, ocap, sz)) {
+            PosArgs pa{};
+            pa.base = (const char*)a->tail.data;
+            pa.n = n1;
+            pa.inv = a->tail.Ainv;
+            pa.sz = sz;
+            pa.h1c = h1;
+            pa.t2c = t2;
+            pa.fh = fH1;
+            pa.ft = fT2;
+            pa.oh = out->head.data;
+            pa.ot = out->tail.data;
+            pa.ohw = type_width(oH);
+            pa.otw = type_width(oT);
+            pa.reenc = reenc;
+            pa.head_err = type_encoded(H1);
+            pa.t2enc = type_encoded(T2);
+            pa.w2 = t2.width;
+            uint64_t kept = 0;
+            rc = run_pos_join<true, false>(s, pa, &a->head, aoid, h1.umax == 0, ev(errs, 0), ev(errs, 1), ev(errs, 3),
+                                           &kept);
+            if (rc != AHEAD_UNSUPPORTED) {
+                if (rc == AHEAD_OK) out->count = kept;
+                return rc;
+            }
+        }
+        rc = s.reserve(compact_scratch<MjPosOp<true>>(n1));
         if (rc) return rc;
         MjPosOp<true> op;
         op.base = (const char*)a->tail.data;
@@ -1388,7 +1569,7 @@ int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
         op.at1inv = a->tail.Ainv;
         op.ah1inv = type_encoded(H1) ? a->head.Ainv : 0;
         op.ah1max = a->head.unenc_max;
-        op.sz = (uint32_t)b->count;  // BAT::size() is an oid_t
+        op.sz = sz;
         op.fh = fH1;
         op.ft = fT2;
         op.cap = ocap;
@@ -1621,7 +1802,26 @@ int ahead_gpu_matchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, 
         return m > cap ? AHEAD_CAPACITY : AHEAD_OK;
     }
     if (T1 == AHEAD_OID && H2 == AHEAD_VOID) {
-        int rc = s.reserve(compact_scratch<MjPosOp<false>>(n1));
+        int rc;
+        if (pos_one_pass(n1, ocap, n2)) {
+            PosArgs pa{};
+            pa.base = (const char*)a->tail.data;
+            pa.n = n1;
+            pa.sz = n2;
+            pa.h1c = h1;
+            pa.t2c = t2;
+            pa.oh = out->head.data;
+            pa.ot = out->tail.data;
+            pa.ohw = type_width(type_select_of(H1));
+            pa.otw = type_width(type_select_of(T2));
+            uint64_t kept = 0;
+            rc = run_pos_join<false, false>(s, pa, nullptr, 0, false, nullptr, nullptr, nullptr, &kept);
+            if (rc != AHEAD_UNSUPPORTED) {
+                if (rc == AHEAD_OK) out->count = kept;
+                return rc;
+            }
+        }
+        rc = s.reserve(compact_scratch<MjPosOp<false>>(n1));
         if (rc) return rc;
         MjPosOp<false> op{};
         op.base = (const char*)a->tail.data;
@@ -1728,7 +1928,28 @@ int ahead_gpu_fetchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
     }
     out->count = 0;
     OpScope s(ctx);
-    int rc = s.reserve(compact_scratch<FetchOp<true>>(a->count));
+    int rc;
+    if (pos_one_pass(a->count, out->tail.data ? cap : 0, b->count)) {
+        PosArgs pa{};
+        pa.base = (const char*)a->tail.data;
+        pa.n = a->count;
+        pa.inv = a->tail.Ainv;
+        pa.sz = b->count;
+        pa.t2c = dcol(b->tail);
+        pa.ft = fac;
+        pa.ot = out->tail.data;
+        pa.otw = w;
+        pa.reenc = reenc;
+        pa.t2enc = 1;
+        pa.w2 = w;
+        uint64_t kept = 0;
+        rc = run_pos_join<true, true>(s, pa, nullptr, aoid, false, nullptr, ev(errs, 0), ev(errs, 1), &kept);
+        if (rc != AHEAD_UNSUPPORTED) {
+            if (rc == AHEAD_OK) out->count = kept;
+            return rc;
+        }
+    }
+    rc = s.reserve(compact_scratch<FetchOp<true>>(a->count));
     if (rc) return rc;
     FetchOp<true> op;
     op.base = (const char*)a->tail.data;
@@ -1771,7 +1992,23 @@ int ahead_gpu_fetchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, 
     copy_meta(&out->tail, T2, &b->tail);
     out->count = 0;
     OpScope s(ctx);
-    int rc = s.reserve(compact_scratch<FetchOp<false>>(a->count));
+    int rc;
+    if (pos_one_pass(a->count, out->tail.data ? cap : 0, b->count)) {
+        PosArgs pa{};
+        pa.base = (const char*)a->tail.data;
+        pa.n = a->count;
+        pa.sz = b->count;
+        pa.t2c = dcol(b->tail);
+        pa.ot = out->tail.data;
+        pa.otw = type_width(T2);
+        uint64_t kept = 0;
+        rc = run_pos_join<false, true>(s, pa, nullptr, 0, false, nullptr, nullptr, nullptr, &kept);
+        if (rc != AHEAD_UNSUPPORTED) {
+            if (rc == AHEAD_OK) out->count = kept;
+            return rc;
+        }
+    }
+    rc = s.reserve(compact_scratch<FetchOp<false>>(a->count));
     if (rc) return rc;
     FetchOp<false> op{};
     op.base = (const char*)a->tail.data;
