@@ -103,6 +103,7 @@ inline size_t compact_bytes(uint64_t n, uint32_t ntiles, uint32_t nchan) {
 //   void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const;  streams c >= 1
 //
 //   void begin();  optional: loads what eval and out0 need from device memory, once per thread
+//   void tile(uint32_t t);  optional: the same for each tile, before its rows
 //
 // Row layout of a tile: with VEC = 16 / W rows per vector, lane l holds in
 // vector s the rows 32 * VEC * s + VEC * l + (0 .. VEC - 1) of the tile.
@@ -113,6 +114,12 @@ AHEAD_DEV auto begin_op(Op& op, int) -> decltype(op.begin(), void()) {
 }
 template <class Op>
 AHEAD_DEV void begin_op(Op&, long) {}
+template <class Op>
+AHEAD_DEV auto begin_tile(Op& op, uint32_t tile, int) -> decltype(op.tile(tile), void()) {
+    op.tile(tile);
+}
+template <class Op>
+AHEAD_DEV void begin_tile(Op&, uint32_t, long) {}
 
 template <int W>
 AHEAD_DEV void unpack16(const uint4 q, uint64_t (&v)[16 / W]) {
@@ -385,6 +392,7 @@ __global__ void __launch_bounds__(kCThreads) classify_kernel(Op op, uint64_t n, 
     for (int k = 0; k < per && tile < cb.ntiles; ++k, tile += kCWarps) {
         const uint32_t next = k + 1 < per && tile + kCWarps < whole ? tile + kCWarps : 0;
         uint32_t word, count;
+        begin_tile(op, tile, 0);
         tile_classify<Op, K>(op, n, tile, f, next, vec, acc, word, count);
         if (lane < K) cb.words[(size_t)tile * K + lane] = word;
         if (lane < Op::NCH) cb.counts[(size_t)tile * Op::NCH + lane] = count;
@@ -510,6 +518,7 @@ __global__ void __launch_bounds__(kCThreads) emit_kernel(Op op, uint64_t n, Comp
         const uint64_t b = base;
         if (k + 1 < per) head(tile_of(k + 1));
         const uint32_t c0 = __shfl_sync(kFull, c, 0);
+        begin_tile(op, tile, 0);
         if (c0) tile_emit<Op, K>(op, n, tile, w, c0, __shfl_sync(kFull, b, 0), s_rows[warp]);
         if constexpr (NCH > 1)
             if (__any_sync(kFull, lane > 0 && c)) tile_emit_sparse<Op, K>(op, n, tile, b);
@@ -530,6 +539,7 @@ __global__ void __launch_bounds__(kOneBlockTiles * 32) compact_one_kernel(Op op,
     uint64_t acc = 0;
     Flight<Op::W, K> f;
     if ((uint64_t)(warp + 1) * (32 * K) <= n) f.load(op.base, (uint64_t)warp * (32 * K) + 16 / Op::W * lane, vec);
+    begin_tile(op, warp, 0);
     tile_classify<Op, K>(op, n, warp, f, 0, vec, acc, word, count);
     if (lane < NCH) s_cnt[lane][warp] = count;
     __syncthreads();

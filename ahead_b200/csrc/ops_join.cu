@@ -792,17 +792,49 @@ AHEAD_DEV uint64_t key_val(const DCol& c, uint64_t row) { return dec_if(c, load_
 
 // Flags (bit 0) a key that does not strictly increase -- the parallel merge
 // is exact only without one -- and (bit 1) any corrupt value in either column,
-// which decides whether error positions must be produced.
-__global__ void merge_check_kernel(MergeSide m, uint64_t n, uint32_t* flag) {
+// which decides whether error positions must be produced.  Both inputs in one
+// launch (blockIdx.y), 256 rows per warp and step, eight loads in flight per
+// lane; the key before a lane's comes from its neighbour.
+__global__ void __launch_bounds__(256) merge_check_kernel(MergeSide ma, uint64_t na, MergeSide mb, uint64_t nb,
+                                                          uint32_t* flag) {
+    constexpr int U = 8;
+    const MergeSide m = blockIdx.y ? mb : ma;
+    const uint64_t n = blockIdx.y ? nb : na;
+    // (a mirrored list is checked once)
+    const bool other = m.other_enc && !(m.key_enc && m.other.data == m.key.data && m.other.ainv == m.key.ainv &&
+                                        m.other.umax == m.key.umax);
+    const int lane = threadIdx.x & 31;
     uint32_t f = 0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t k = key_val(m.key, i);
-        if ((m.key_enc && k > m.key.umax) ||
-            (m.other_enc && dec_if(m.other, load_at(m.other, i), m.other.ainv) > m.other.umax))
-            f |= 2u;
-        if (i > 0 && key_val(m.key, i - 1) >= k) f |= 1u;
+    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t r0 = ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5) * (32 * U); r0 < n;
+         r0 += warps * (32 * U)) {
+        const uint32_t cnt = n - r0 < 32 * U ? (uint32_t)(n - r0) : 32 * U;
+        uint32_t idx[U];
+        uint64_t k[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) idx[q] = lane + 32 * q < cnt ? lane + 32 * q : 0;
+        load_rows(m.key, r0, idx, k);
+        uint64_t last = r0 ? dec_if(m.key, load_at(m.key, r0 - 1), m.key.ainv) : 0;
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            k[q] = dec_if(m.key, k[q], m.key.ainv);
+            const uint64_t up = __shfl_up_sync(kFull, k[q], 1);
+            const uint64_t before = lane ? up : last;
+            last = __shfl_sync(kFull, k[q], 31);
+            if (lane + 32 * q < cnt) {
+                if (r0 + lane + 32 * q && before >= k[q]) f |= 1u;
+                if (m.key_enc && k[q] > m.key.umax) f |= 2u;
+            }
+        }
+        if (other) {
+            load_rows(m.other, r0, idx, k);
+#pragma unroll
+            for (int q = 0; q < U; ++q)
+                if (dec_if(m.other, k[q], m.other.ainv) > m.other.umax) f |= 2u;
+        }
     }
-    if (f) atomicOr(flag, f);
+    f = __reduce_or_sync(kFull, f);
+    if (f && lane == 0) atomicOr(flag, f);
 }
 
 // Error positions of the reference's merge loop (matchjoinAN.tcc:101-136) for
@@ -823,7 +855,6 @@ struct MergeErrs {
     DCol h1, t1, h2, t2;
     uint64_t n1, n2, aoid;
     int eh1, et1, eh2, et2;
-    uint64_t last2;           // key of the last second-input row
     const uint64_t* l1m;      // device word: the last first-input key occurs in the second input
     AHEAD_DEV uint64_t lb1(uint64_t x) const {  // first-input keys below x
         uint64_t lo = 0, hi = n1;
@@ -851,7 +882,7 @@ struct MergeErrs {
             bad_a = eh1 && key_val(h1, r) > h1.umax;
             bad_b = et1 && k > t1.umax;
             if (!(bad_a || bad_b)) return 0;
-            return (k < last2 && !in2(k)) ? 1u : 0u;
+            return (k < key_val(h2, n2 - 1) && !in2(k)) ? 1u : 0u;
         }
         const uint64_t K = key_val(h2, r);
         bad_a = eh2 && K > h2.umax;
@@ -991,82 +1022,47 @@ __global__ void __launch_bounds__(kMeThreads) merge_err_write_kernel(MergeErrs m
     }
 }
 
-// Bounds of a strictly increasing key sequence: [0] first key, [1] last key.
-__global__ void isect_bounds_kernel(DCol h2, uint64_t n2, uint64_t* out) {
-    out[0] = key_val(h2, 0);
-    out[1] = key_val(h2, n2 - 1);
-}
+// Intersection of two strictly increasing key sequences: each tile of the
+// first input only meets the second input's keys from its own first key to the
+// next tile's, a stretch that merge_part_kernel finds for all tiles at once;
+// each row then searches its tile's stretch (a few hundred keys, in L1).  No
+// structure over the whole key range is built, so the range's width does not
+// matter.  While a tile's keys span at most kMergeMap values (selections of
+// ordinary shares do), the stretch marks a byte map of that span in shared
+// memory and a row's search is one byte; a wider tile searches its stretch.
+// When the second input's tail is its head (a mirrored selection), the matched
+// value is the key itself and the emit pass does not search at all.
+// At 29M and 16M plain 4-byte OIDs of 60M, a binary search over all of the
+// second input per row took 775 us to classify and 285 us to emit, a search of
+// the stretch 234 and 170; this takes 57 and 54 (180 MB read per pass), and 18 us for
+// the stretches.
+struct MergeParts {
+    DCol k1, k2;  // key columns
+    uint64_t n1, n2;
+    uint64_t* part;  // [tiles + 1] first row of the second input at or past each tile's first key
+};
+constexpr uint64_t kMergeTile = 32 * short_k(8);  // rows per tile (driving columns of 2, 4 or 8 bytes)
+constexpr uint32_t kMergeMap = 4096;
 
-// Rank structure of a strictly increasing clean key sequence over
-// [kmin, kmin + 64 * words): bit (k - kmin) is set for each key, and first[w]
-// is the index of the first key in 64-bit word w (set only for non-empty
-// words, the only ones a lookup reads).
-__global__ void isect_mark_kernel(DCol h2, uint64_t n2, uint64_t kmin, unsigned long long* bits, uint32_t* first) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n2; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t d = key_val(h2, i) - kmin;
-        const uint64_t w = d >> 6;
-        atomicOr(&bits[w], 1ull << (d & 63));
-        if (i == 0 || ((key_val(h2, i - 1) - kmin) >> 6) != w) first[w] = (uint32_t)i;
-    }
-}
-
-// Intersection of two strictly increasing clean key sequences: each row of the
-// first input looks its key up in the second, through the rank structure when
-// the second's key range is dense enough, else by binary search.
-struct IsectOp {
-    static constexpr int W = 8;
-    static constexpr int NCH = 1;
-    static constexpr bool ACC = false;
-    static constexpr bool GATHER = true;
-    static constexpr bool EMIT_V = false;
-    static constexpr int NOUT = 2;
-    const char* base;
-    uint32_t* status;
-    DCol t1c, h1c, h2c, t2c;
-    uint64_t n2, fh, ft, cap;
-    uint64_t* acc;
-    void *oh, *ot;
-    int ohw, otw, reenc;
-    const unsigned long long* bits;  // rank structure, or nullptr
-    const uint32_t* first;
-    uint64_t kmin, krange;
-    AHEAD_DEV uint64_t find(uint64_t row) const {
-        const uint64_t k = key_val(t1c, row);
-        if (bits) {
-            const uint64_t d = k - kmin;
-            if (k < kmin || d >= krange) return ~0ull;
-            const unsigned long long wv = bits[d >> 6];
-            if (!((wv >> (d & 63)) & 1ull)) return ~0ull;
-            return first[d >> 6] + __popcll(wv & ((1ull << (d & 63)) - 1ull));
-        }
-        uint64_t lo = 0, hi = n2;
+__global__ void __launch_bounds__(256) merge_part_kernel(MergeParts m, uint32_t tiles) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t > tiles) return;
+    uint64_t lo = 0, hi = m.n2;
+    if (t == tiles) {
+        lo = hi;
+    } else {
+        const uint64_t k = key_val(m.k1, (uint64_t)t * kMergeTile);
         while (lo < hi) {
             const uint64_t mid = (lo + hi) >> 1;
-            if (key_val(h2c, mid) < k) lo = mid + 1;
+            if (key_val(m.k2, mid) < k) lo = mid + 1;
             else hi = mid;
         }
-        return (lo < n2 && key_val(h2c, lo) == k) ? lo : ~0ull;
     }
-    AHEAD_DEV uint32_t eval(uint64_t, uint64_t row, uint64_t&) const { return find(row) != ~0ull ? 1u : 0u; }
-    AHEAD_DEV uint64_t out0(int k, uint64_t, uint64_t row) const {
-        if (k == 0) {
-            const uint64_t h = load_at(h1c, row);
-            return reenc ? dec_if(h1c, h, fh) : h;
-        }
-        const uint64_t t = load_at(t2c, find(row));
-        return reenc ? dec_if(t2c, t, ft) : t;
-    }
-    AHEAD_DEV uint64_t cap0() const { return cap; }
-    AHEAD_DEV void* optr(int k) const { return k == 0 ? oh : ot; }
-    AHEAD_DEV int owidth(int k) const { return k == 0 ? ohw : otw; }
-    AHEAD_DEV void emit(int, uint64_t, uint64_t, uint64_t) const {}
-};
+    m.part[t] = lo;
+}
 
-// Intersection of two strictly increasing plain key sequences (binary search
-// in the second); the driving column (the first input's keys, or its head when
-// the tail is void) is W bytes wide.
 template <int WW>
-struct IsectPlainOp {
+struct IsectOp {
     static constexpr int W = WW;
     static constexpr int NCH = 1;
     static constexpr bool ACC = false;
@@ -1074,31 +1070,180 @@ struct IsectPlainOp {
     static constexpr bool EMIT_V = false;
     static constexpr int NOUT = 2;
     const char* base;
-    uint32_t* status;
     DCol t1c, h1c, h2c, t2c;
-    uint64_t n2, cap;
+    uint64_t fh, ft, cap;
     uint64_t* acc;
     void *oh, *ot;
-    int ohw, otw;
-    AHEAD_DEV uint64_t find(uint64_t row) const {
+    int ohw, otw, reenc;
+    int mirror2;   // the second input's tail is its head: its value is key * a2
+    uint64_t a2;
+    const uint64_t* part;
+    uint64_t lo, len;  // the tile's stretch of the second input
+    AHEAD_DEV void tile(uint32_t t) {
+        lo = __ldg((const unsigned long long*)part + t);
+        len = __ldg((const unsigned long long*)part + t + 1) - lo;
+    }
+    AHEAD_DEV uint64_t find(uint64_t row) const {  // ~0: no match
         const uint64_t k = key_val(t1c, row);
-        uint64_t lo = 0, hi = n2;
-        while (lo < hi) {
-            const uint64_t mid = (lo + hi) >> 1;
-            if (key_val(h2c, mid) < k) lo = mid + 1;
-            else hi = mid;
+        uint64_t at = lo, m = len;
+        while (m >> 32) {  // (a stretch of 2^32 rows and more)
+            const uint64_t half = m >> 1;
+            if (key_val(h2c, at + half) < k) {
+                at += half + 1;
+                m -= half + 1;
+            } else {
+                m = half;
+            }
         }
-        return (lo < n2 && key_val(h2c, lo) == k) ? lo : ~0ull;
+        uint32_t a = 0, b = (uint32_t)m;
+        while (a < b) {
+            const uint32_t mid = a + (b - a) / 2;
+            if (key_val(h2c, at + mid) < k) a = mid + 1;
+            else b = mid;
+        }
+        at += a;
+        return (at < lo + len && key_val(h2c, at) == k) ? at : ~0ull;
     }
     AHEAD_DEV uint32_t eval(uint64_t, uint64_t row, uint64_t&) const { return find(row) != ~0ull ? 1u : 0u; }
-    AHEAD_DEV uint64_t out0(int k, uint64_t, uint64_t row) const {
-        return k == 0 ? load_at(h1c, row) : load_at(t2c, find(row));
+    template <class V, int U>
+    AHEAD_DEV void rows0(const V (&)[U], uint64_t row0, const uint32_t (&idx)[U], uint64_t (&x)[2][U]) const {
+        load_rows(h1c, row0, idx, x[0]);
+        if (mirror2) {
+            load_rows(t1c, row0, idx, x[1]);
+#pragma unroll
+            for (int u = 0; u < U; ++u) x[1][u] = dec_if(t1c, x[1][u], t1c.ainv) * a2;
+        } else {
+            uint64_t p[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) p[u] = find(row0 + idx[u]);
+            gather_rows(t2c, p, x[1]);
+        }
+        if (reenc) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                x[0][u] = dec_if(h1c, x[0][u], fh);
+                x[1][u] = dec_if(t2c, x[1][u], ft);
+            }
+        }
     }
     AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void* optr(int k) const { return k == 0 ? oh : ot; }
     AHEAD_DEV int owidth(int k) const { return k == 0 ? ohw : otw; }
     AHEAD_DEV void emit(int, uint64_t, uint64_t, uint64_t) const {}
 };
+
+// Pass 1 through the byte map, one warp per tile; word s of a tile is the
+// ballot of its rows 32 s ... 32 s + 31.
+template <class Op>
+__global__ void __launch_bounds__(kCThreads) merge_classify_kernel(Op op, uint64_t n, CompactBufs cb) {
+    constexpr int K = short_k(8);
+    __shared__ __align__(16) uint8_t s_map[kCWarps][kMergeMap];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint8_t* map = s_map[warp];
+    const uint32_t tile = blockIdx.x * kCWarps + warp;
+    if (tile >= cb.ntiles) return;
+    op.tile(tile);
+    const uint64_t row0 = (uint64_t)tile * kMergeTile;
+    const uint32_t m = n - row0 < kMergeTile ? (uint32_t)(n - row0) : (uint32_t)kMergeTile;
+    uint32_t idx[K];
+    uint64_t k[K];
+#pragma unroll
+    for (int s = 0; s < K; ++s) idx[s] = lane + 32 * s < m ? lane + 32 * s : m - 1;
+    load_rows(op.t1c, row0, idx, k);
+#pragma unroll
+    for (int s = 0; s < K; ++s) k[s] = dec_if(op.t1c, k[s], op.t1c.ainv);
+    const uint64_t first = __shfl_sync(kFull, k[0], 0), last = __shfl_sync(kFull, k[K - 1], 31);
+    const uint64_t span = last - first + 1;
+    uint32_t word = 0;
+    if (span && span <= kMergeMap && op.len <= kMergeMap) {
+        const uint32_t w = (uint32_t)span, len = (uint32_t)op.len;
+        for (uint32_t i = lane; i < (w + 15) / 16; i += 32) reinterpret_cast<uint4*>(map)[i] = make_uint4(0, 0, 0, 0);
+        __syncwarp();
+        for (uint32_t j0 = lane; j0 < len; j0 += 128) {
+            uint32_t at[4];
+            uint64_t x[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) at[q] = j0 + 32 * q < len ? j0 + 32 * q : j0;
+            load_rows(op.h2c, op.lo, at, x);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint64_t d = dec_if(op.h2c, x[q], op.h2c.ainv) - first;
+                if (d < w) map[d] = 1;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int s = 0; s < K; ++s) {
+            const uint64_t d = k[s] - first;  // (keys out of order: any byte of the map, the result is discarded)
+            const uint32_t b = __ballot_sync(kFull, lane + 32 * s < m && d < w && map[d < w ? d : 0]);
+            if (lane == s) word = b;
+        }
+    } else {
+#pragma unroll 1
+        for (int s = 0; s < K; ++s) {
+            const uint64_t row = row0 + lane + 32 * s;
+            const uint32_t b = __ballot_sync(kFull, lane + 32 * s < m && op.find(row) != ~0ull);
+            if (lane == s) word = b;
+        }
+    }
+    if (lane < K) cb.words[(size_t)tile * K + lane] = word;
+    const uint32_t count = __reduce_add_sync(kFull, (uint32_t)__popc(word));
+    if (lane == 0) cb.counts[tile] = count;
+}
+
+size_t merge_scratch(uint64_t n1) {
+    return compact_scratch<IsectOp<8>>(n1) + (n1 / kMergeTile + 2) * 8 + 1024;
+}
+
+// The checks (flag in counter kMergeFlag) and the intersection (total in
+// counter 0), which counts only when the flag's bit 0 stays clear.  `dw`: the
+// driving column's width, at least 2.
+constexpr int kMergeFlag = 40, kMergeCounters = 41;
+
+void run_merge(OpScope& s, const DCol& t1, const DCol& h1, const DCol& h2, const DCol& t2, uint64_t n1, uint64_t n2,
+               bool checked, int dw, int reenc, uint64_t fh, uint64_t ft, void* oh, int ohw, void* ot, int otw,
+               uint64_t cap) {
+    cudaStream_t st = s.ctx->stream;
+    MergeSide ma{t1, h1, checked && t1.enc, checked && h1.enc};
+    MergeSide mb{h2, t2, checked && h2.enc, checked && t2.enc};
+    const uint64_t most = (n1 > n2 ? n1 : n2) / 4 + 1;
+    const uint32_t cg = grid_for(most, 256), cl = (uint32_t)s.ctx->num_sms * 8;
+    merge_check_kernel<<<dim3(cg < cl ? cg : cl, 2), 256, 0, st>>>(ma, n1, mb, n2,
+                                                                   (uint32_t*)(s.d_counters + kMergeFlag));
+    const uint32_t tiles = (uint32_t)((n1 + kMergeTile - 1) / kMergeTile);
+    MergeParts mp{t1, h2, n1, n2, (uint64_t*)s.alloc(((size_t)tiles + 1) * 8)};
+    merge_part_kernel<<<(tiles + 256) / 256, 256, 0, st>>>(mp, tiles);
+    s.launched(2);
+    by_width_enc(dw, [&](auto tag) -> int {
+        IsectOp<decltype(tag)::value> op;
+        op.base = (const char*)(t1.type == AHEAD_VOID ? h1.data : t1.data);
+        op.t1c = t1;
+        op.h1c = h1;
+        op.h2c = h2;
+        op.t2c = t2;
+        op.fh = fh;
+        op.ft = ft;
+        op.cap = cap;
+        op.acc = nullptr;
+        op.oh = oh;
+        op.ot = ot;
+        op.ohw = ohw;
+        op.otw = otw;
+        op.reenc = reenc;
+        op.mirror2 = t2.type != AHEAD_VOID && t2.data == h2.data && t2.type == h2.type && t2.ainv == h2.ainv;
+        op.a2 = h2.enc ? inv_pow2(h2.ainv, 64) : 1;
+        op.part = mp.part;
+        op.lo = op.len = 0;
+        if (tiles <= kOneBlockTiles) {
+            run_compact(s, op, n1, 0);
+            return 0;
+        }
+        const CompactBufs cb = s.compact_bufs(n1, tiles, 1, 0);
+        merge_classify_kernel<<<(tiles + kCWarps - 1) / kCWarps, kCThreads, 0, st>>>(op, n1, cb);
+        s.launched(1 + launch_compact_tail(s.ctx, st, op, n1, cb));
+        return 0;
+    });
+}
 
 struct MergeSeq {
     DCol h1, t1, h2, t2;
@@ -1630,68 +1775,21 @@ int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
     }
     // general merge (gm) or (void tail, resoid head) merge (mv)
     set_errs_present(errs, type_encoded(H1), type_encoded(T1), type_encoded(H2), type_encoded(T2));
-    int rc = s.reserve(compact_scratch<IsectOp>(n1) + 256);
-    if (rc) return rc;
-    uint32_t* flag = (uint32_t*)(s.d_counters + 50);
-    if (n1 && n2) {
-        MergeSide ma{t1, h1, type_encoded(T1), type_encoded(H1)};
-        MergeSide mb{h2, t2, type_encoded(H2), type_encoded(T2)};
-        merge_check_kernel<<<grid_for(n1, 256), 256, 0, ctx->stream>>>(ma, n1, flag);
-        merge_check_kernel<<<grid_for(n2, 256), 256, 0, ctx->stream>>>(mb, n2, flag);
-        s.launched(2);
-    }
-    uint64_t hb[3] = {0, 0, 0};  // flag word, first and last key of the second input
-    if (n2) {
-        isect_bounds_kernel<<<1, 1, 0, ctx->stream>>>(h2, n2, s.d_counters + 51);
-        s.launched();
-    }
-    cudaMemcpyAsync(hb, s.d_counters + 50, 24, cudaMemcpyDeviceToHost, ctx->stream);
-    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return fail(ctx, AHEAD_CUDA_ERROR, "merge check");
-    const uint32_t hflag = (uint32_t)hb[0];
-    if (!(hflag & 1u)) {
-        if (n1 && n2) {
-            // the rank structure when the key range is at most 64 words per key
-            const uint64_t krange = hb[2] - hb[1] + 1;
-            const uint64_t words = (krange + 63) / 64;
-            const bool use_bits = n2 < (1ull << 32) && words <= 64 * n2 + 1024;
-            const uint64_t nt1 = (n1 + kMeTile - 1) / kMeTile, nt2 = (n2 + kMeTile - 1) / kMeTile;
-            const size_t err_scratch = (hflag & 2u) ? (nt1 + nt2) * 24 + 2048 : 0;
-            rc = s.reserve(compact_scratch<IsectOp>(n1) + (use_bits ? words * 12 + 512 : 0) + err_scratch);
-            if (rc) return rc;
-            IsectOp op;
-            op.bits = nullptr;
-            op.first = nullptr;
-            op.kmin = hb[1];
-            op.krange = krange;
-            if (use_bits) {
-                auto* bits = (unsigned long long*)s.alloc(words * 8);
-                auto* first = (uint32_t*)s.alloc(words * 4);
-                cudaMemsetAsync(bits, 0, words * 8, ctx->stream);
-                isect_mark_kernel<<<grid_for(n2, 256), 256, 0, ctx->stream>>>(h2, n2, hb[1], bits, first);
-                s.launched();
-                op.bits = bits;
-                op.first = first;
-            }
-            // the driving column must hold data: the tail, or the head when the tail is void
-            op.base = (const char*)(T1 == AHEAD_VOID ? a->head.data : a->tail.data);
-            op.status = s.d_status;
-            op.t1c = t1;
-            op.h1c = h1;
-            op.h2c = h2;
-            op.t2c = t2;
-            op.n2 = n2;
-            op.fh = fH1;
-            op.ft = fT2;
-            op.cap = ocap;
-            op.acc = nullptr;
-            op.oh = out->head.data;
-            op.ot = out->tail.data;
-            op.ohw = type_width(oH);
-            op.otw = type_width(oT);
-            op.reenc = reenc;
-            if (type_width(T1 == AHEAD_VOID ? H1 : T1) != 8) return fail(ctx, AHEAD_UNSUPPORTED, "merge driving width");
-            run_compact(s, op, n1, 0);
-            if (hflag & 2u) {
+    if (!n1 || !n2) return AHEAD_OK;
+    int rc;
+    const int dw = type_width(T1 == AHEAD_VOID ? H1 : T1);  // 8: the head of a void list is encoded
+    {
+        const uint64_t nt1 = (n1 + kMeTile - 1) / kMeTile, nt2 = (n2 + kMeTile - 1) / kMeTile;
+        rc = s.reserve(merge_scratch(n1) + (nt1 + nt2) * 24 + 4096);
+        if (rc) return rc;
+        run_merge(s, t1, h1, h2, t2, n1, n2, true, dw, reenc, fH1, fT2, out->head.data, type_width(oH),
+                  out->tail.data, type_width(oT), ocap);
+        rc = s.finish(kMergeCounters);
+        if (rc) return rc;
+        const uint32_t flag = (uint32_t)s.counter(kMergeFlag);
+        if (!(flag & 1u)) {
+            out->count = s.counter(0);
+            if (flag & 2u) {
                 // corrupt values in ordered inputs: the loop's error positions, per row
                 MergeErrs me;
                 me.h1 = h1;
@@ -1705,7 +1803,6 @@ int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
                 me.et1 = type_encoded(T1);
                 me.eh2 = type_encoded(H2);
                 me.et2 = type_encoded(T2);
-                me.last2 = hb[2];
                 uint64_t* l1m = (uint64_t*)s.alloc(8);
                 me.l1m = l1m;
                 merge_last_kernel<<<1, 1, 0, ctx->stream>>>(me, l1m);
@@ -1724,16 +1821,17 @@ int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
                         me, side, n, toff, edata(va), ecap(va), edata(vb), ecap(vb));
                     s.launched(3);
                 }
+                rc = s.finish(5);
+                if (rc) return rc;
+                if (errs)
+                    for (int k = 0; k < 4; ++k)
+                        if (errs[k].present) errs[k].count = s.counter(1 + k);
             }
+            return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
         }
-        rc = s.finish(5);
-        if (rc) return rc;
-        out->count = (n1 && n2) ? s.counter(0) : 0;
-        if (errs && (hflag & 2u) && n1 && n2)
-            for (int k = 0; k < 4; ++k)
-                if (errs[k].present) errs[k].count = s.counter(1 + k);
-        return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
     }
+    rc = s.reserve(0);
+    if (rc) return rc;
     MergeSeq m;
     m.h1 = h1;
     m.t1 = t1;
@@ -1845,41 +1943,15 @@ int ahead_gpu_matchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, 
     // (driving column of 2, 4 or 8 bytes); anything else replays the loop
     const int dw = type_width(T1 == AHEAD_VOID ? H1 : T1);
     if (n1 && n2 && dw >= 2) {
-        int rc = s.reserve(compact_scratch<IsectPlainOp<8>>(n1) + 256);
+        int rc = s.reserve(merge_scratch(n1));
         if (rc) return rc;
-        uint32_t* flag = (uint32_t*)(s.d_counters + 50);
-        MergeSide ma{t1, h1, 0, 0};
-        MergeSide mb{h2, t2, 0, 0};
-        merge_check_kernel<<<grid_for(n1, 256), 256, 0, ctx->stream>>>(ma, n1, flag);
-        merge_check_kernel<<<grid_for(n2, 256), 256, 0, ctx->stream>>>(mb, n2, flag);
-        s.launched(2);
-        uint32_t hflag = 0;
-        cudaMemcpyAsync(&hflag, flag, 4, cudaMemcpyDeviceToHost, ctx->stream);
-        if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return fail(ctx, AHEAD_CUDA_ERROR, "merge check");
-        if (!(hflag & 1u)) {
-            rc = s.reserve(compact_scratch<IsectPlainOp<8>>(n1) + 256);
-            if (rc) return rc;
-            rc = by_width_enc(dw, [&](auto tag) -> int {
-                constexpr int W = decltype(tag)::value;
-                IsectPlainOp<W> op{};
-                op.base = (const char*)(T1 == AHEAD_VOID ? a->head.data : a->tail.data);
-                op.status = s.d_status;
-                op.t1c = t1;
-                op.h1c = h1;
-                op.h2c = h2;
-                op.t2c = t2;
-                op.n2 = n2;
-                op.cap = ocap;
-                op.acc = nullptr;
-                op.oh = out->head.data;
-                op.ot = out->tail.data;
-                op.ohw = type_width(type_select_of(H1));
-                op.otw = type_width(type_select_of(T2));
-                run_compact(s, op, n1, 0);
-                return 0;
-            });
-            rc = s.finish(1);
-            if (rc) return rc;
+        DCol k1 = t1, k2 = h2, v1 = h1, v2 = t2;
+        k1.enc = k2.enc = v1.enc = v2.enc = 0;  // plain values
+        run_merge(s, k1, v1, k2, v2, n1, n2, false, dw, 0, 1, 1, out->head.data, type_width(type_select_of(H1)),
+                  out->tail.data, type_width(type_select_of(T2)), ocap);
+        rc = s.finish(kMergeCounters);
+        if (rc) return rc;
+        if (!(s.counter(kMergeFlag) & 1u)) {
             out->count = s.counter(0);
             return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
         }
