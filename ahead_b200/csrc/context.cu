@@ -23,7 +23,9 @@ int ahead_ctx_create(int device, void* stream, ahead_ctx** out) {
         }
         c->own_stream = true;
     }
-    if (cudaMallocHost(&c->h_stage, ahead::kStageWords * sizeof(uint64_t)) != cudaSuccess) {
+    // (mapped: publish_kernel writes it; one address on both sides under unified addressing)
+    if (cudaHostAlloc((void**)&c->h_stage, ahead::kStageWords * sizeof(uint64_t),
+                      cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
         if (c->own_stream) cudaStreamDestroy(c->stream);
         delete c;
         return AHEAD_NO_MEMORY;
@@ -44,6 +46,12 @@ void ahead_ctx_destroy(ahead_ctx* c) {
 void* ahead_ctx_stream(ahead_ctx* c) { return c ? (void*)c->stream : nullptr; }
 
 const char* ahead_ctx_last_error(ahead_ctx* c) { return c ? c->err.c_str() : "no context"; }
+
+void ahead_ctx_set_output_fn(ahead_ctx* c, ahead_output_fn fn, void* user) {
+    if (!c) return;
+    c->out_fn = fn;
+    c->out_user = user;
+}
 
 uint64_t ahead_ctx_launches(ahead_ctx* c) { return c ? c->launches : 0; }
 

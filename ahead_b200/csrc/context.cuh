@@ -18,10 +18,13 @@ struct ahead_ctx {
     bool own_stream = false;
     char* arena = nullptr;  // device scratch, reused by every call
     size_t arena_cap = 0;
-    uint64_t* h_stage = nullptr;  // pinned host words for count read-back
+    bool header_clean = false;  // the arena's status word and counters are zero
+    uint64_t* h_stage = nullptr;  // pinned host words for count read-back (device-writable)
     uint64_t launches = 0;
     int num_sms = 148;
     std::string err;
+    ahead_output_fn out_fn = nullptr;  // allocates output columns of sized calls
+    void* out_user = nullptr;
     // staging buffers of the table loader (pinned host + device text blocks),
     // kept across loads; freed with the context
     std::shared_ptr<void> loader;
@@ -51,6 +54,16 @@ inline int cuda_fail(ahead_ctx* ctx, cudaError_t e, const char* where) {
         if (_e != cudaSuccess) return ::ahead::cuda_fail((ctx), _e, #call); \
     } while (0)
 
+// Ends an operator: the status word and the first `n` counters go to the pinned
+// host words, and the header is left zero for the next call.  (A copy to the
+// host and a clear ahead of the next call's kernels cost each call 7 us more.)
+static __global__ void __launch_bounds__(kStageWords) publish_kernel(uint64_t* header, uint64_t* host, int n) {
+    const int i = threadIdx.x;
+    const uint64_t v = header[i];
+    if (i <= n) host[i] = v;
+    if (v) header[i] = 0;
+}
+
 // One operator call.  Layout of the arena: [status word + 63 counters][bump
 // region].  reserve() must be called with the call's total scratch need
 // before any pointer is handed out (it may reallocate the arena).
@@ -71,6 +84,7 @@ struct OpScope {
             if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamSynchronize");
             if (ctx->arena) cudaFree(ctx->arena);
             ctx->arena = nullptr;
+            ctx->header_clean = false;
             size_t cap = need < (64u << 20) ? (64u << 20) : need + need / 4;
             e = cudaMalloc(&ctx->arena, cap);
             if (e != cudaSuccess) {
@@ -82,8 +96,11 @@ struct OpScope {
         d_status = (uint32_t*)ctx->arena;
         d_counters = (uint64_t*)(ctx->arena + 8);
         off = 512;
-        cudaError_t e = cudaMemsetAsync(ctx->arena, 0, 512, ctx->stream);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemsetAsync");
+        if (!ctx->header_clean) {
+            cudaError_t e = cudaMemsetAsync(ctx->arena, 0, 512, ctx->stream);
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemsetAsync");
+        }
+        ctx->header_clean = false;  // (until finish() has run: a call may fail half way)
         return AHEAD_OK;
     }
 
@@ -113,6 +130,7 @@ struct OpScope {
     void launched(int n = 1) {
         ctx->launches += n;
         pending = true;
+        ctx->header_clean = false;
     }
 
     // Waits for launches made after the last finish(): a caller may read the
@@ -126,23 +144,40 @@ struct OpScope {
         return e == cudaSuccess ? AHEAD_OK : cuda_fail(ctx, e, "cudaStreamSynchronize");
     }
 
-    // Copy the status word and the first `ncounters` counters to the host and
-    // wait for the stream.  Returns the call's status.
+    // Read the status word and the first `ncounters` counters back and wait for
+    // the stream.  Returns the call's status.  The device's counters are zero
+    // from here on.
     int finish(int ncounters) {
         pending = false;
+        publish_kernel<<<1, kStageWords, 0, ctx->stream>>>((uint64_t*)ctx->arena, ctx->h_stage, ncounters);
+        ctx->launches += 1;
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
-        e = cudaMemcpyAsync(ctx->h_stage, ctx->arena, 8 + 8 * (size_t)ncounters, cudaMemcpyDeviceToHost,
-                            ctx->stream);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemcpyAsync");
         e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamSynchronize");
+        ctx->header_clean = true;
         uint32_t st = (uint32_t)ctx->h_stage[0];
         if (st & kDevStatusTimeout) return fail(ctx, AHEAD_TIMEOUT, "a bounded device wait gave up");
         if (st & kDevStatusBadInput) return fail(ctx, AHEAD_UNSUPPORTED, "input outside the supported domain");
         return AHEAD_OK;
     }
     uint64_t counter(int i) const { return ctx->h_stage[1 + i]; }
+
+    // A call whose output columns are allocated once its counts are known.
+    bool sized(const ahead_bat* out, uint64_t cap) const {
+        return ctx->out_fn && cap == AHEAD_SIZED && !out->head.data && !out->tail.data;
+    }
+    // The column's buffer of `rows` rows; false when the caller's function has none.
+    bool take(ahead_col* c, int column, uint64_t rows) {
+        c->data = ctx->out_fn(ctx->out_user, column, (rows ? rows : 1) * (uint64_t)type_width(c->type));
+        return c->data != nullptr;
+    }
+    // An output without rows: a sized call still gets its columns.
+    int empty(ahead_bat* out, uint64_t cap, bool tail) {
+        if (sized(out, cap) && (!take(&out->head, 0, 0) || (tail && !take(&out->tail, 1, 0))))
+            return fail(ctx, AHEAD_NO_MEMORY, "output allocation failed");
+        return AHEAD_OK;
+    }
 };
 
 inline DCol dcol(const ahead_col& c) {
@@ -247,14 +282,43 @@ inline int launch_compact(const ahead_ctx* ctx, cudaStream_t st, const Op& op, u
     return 3;
 }
 
+// The compaction of a sized call: counts first, then `alloc(kept)` sets the op's
+// output pointers and capacity, then the rows.  Reads `ncounters` counters back.
+template <class Op, class Alloc>
+inline int run_compact_sized(OpScope& s, Op& op, uint64_t n, int c0, int ncounters, Alloc&& alloc) {
+    const uint32_t nt = compact_tiles<Op>(n), per = tiles_per_warp(s.ctx, nt);
+    const CompactBufs cb = s.compact_bufs(n, nt, Op::NCH, c0);
+    const uint32_t grid = (nt + per * kCWarps - 1) / (per * kCWarps);
+    cudaStream_t st = s.ctx->stream;
+    auto passes = [&](auto k_tag) -> int {
+        constexpr int K = decltype(k_tag)::value;
+        classify_kernel<Op, K><<<grid, kCThreads, 0, st>>>(op, n, cb, (int)per);
+        tile_scan_kernel<<<scan_groups(nt), kScanGroup, 0, st>>>(cb);
+        s.launched(2);
+        int rc = s.finish(ncounters);
+        if (rc) return rc;
+        if (!alloc(s.counter(c0))) return fail(s.ctx, AHEAD_NO_MEMORY, "output allocation failed");
+        emit_kernel<Op, K><<<grid, kCThreads, 0, st>>>(op, n, cb, (int)per);
+        s.launched();
+        return s.wait();
+    };
+    if constexpr (!Op::GATHER)
+        if (long_tiles<Op>(n)) return passes(std::integral_constant<int, kLongK>());
+    return passes(std::integral_constant<int, short_k(Op::W)>());
+}
+
 // Passes 2 and 3 of a compaction in short tiles whose pass 1 has its own kernel.
 template <class Op>
-inline int launch_compact_tail(const ahead_ctx* ctx, cudaStream_t st, const Op& op, uint64_t n, const CompactBufs& cb) {
+inline void launch_emit(OpScope& s, const Op& op, uint64_t n, const CompactBufs& cb) {
     constexpr int K = short_k(Op::W);
-    const uint32_t per = tiles_per_warp(ctx, cb.ntiles);
-    tile_scan_kernel<<<scan_groups(cb.ntiles), kScanGroup, 0, st>>>(cb);
-    emit_kernel<Op, K><<<(cb.ntiles + per * kCWarps - 1) / (per * kCWarps), kCThreads, 0, st>>>(op, n, cb, (int)per);
-    return 2;
+    const uint32_t per = tiles_per_warp(s.ctx, cb.ntiles);
+    emit_kernel<Op, K><<<(cb.ntiles + per * kCWarps - 1) / (per * kCWarps), kCThreads, 0, s.ctx->stream>>>(op, n, cb,
+                                                                                                           (int)per);
+    s.launched();
+}
+inline void launch_scan(OpScope& s, const CompactBufs& cb) {
+    tile_scan_kernel<<<scan_groups(cb.ntiles), kScanGroup, 0, s.ctx->stream>>>(cb);
+    s.launched();
 }
 
 // A compaction of an operator call; totals land in counters [c0, c0 + NCH).

@@ -124,13 +124,15 @@ inline void run_colcheck(OpScope& s, const ahead_col& c, uint64_t n, uint64_t ai
 constexpr uint32_t kFastErrCap = 4096;
 
 // Block c sorts list c (at most kFastErrCap rows, bitonic in shared memory)
-// and writes row * aoid into the error vector, up to its capacity.
-static __global__ void __launch_bounds__(1024) sort_err_rows_kernel(const unsigned long long* cnt, const uint64_t* rows1,
-                                                             const uint64_t* rows2, uint64_t* e1, uint64_t cap1,
-                                                             uint64_t* e2, uint64_t cap2, uint64_t aoid) {
+// and writes row * aoid into the error vector, up to its capacity.  The counts
+// come from the device (`cnt`), or for one list from the host (`known`).
+static __global__ void __launch_bounds__(1024) sort_err_rows_kernel(const unsigned long long* cnt, uint64_t known,
+                                                             const uint64_t* rows1, const uint64_t* rows2, uint64_t* e1,
+                                                             uint64_t cap1, uint64_t* e2, uint64_t cap2,
+                                                             uint64_t aoid) {
     __shared__ uint64_t s_r[kFastErrCap];
     const int c = blockIdx.x;
-    const unsigned long long k = cnt[c];
+    const unsigned long long k = cnt ? cnt[c] : known;
     uint64_t* e = c == 0 ? e1 : e2;
     const uint64_t cap = c == 0 ? cap1 : cap2;
     if (k == 0 || k > kFastErrCap) return;
@@ -186,8 +188,8 @@ inline bool settle_err_list(OpScope& s, const ErrList& l, int ci, uint64_t aoid,
     if (e) {
         e->count = k;
         if (k && edata(e)) {
-            sort_err_rows_kernel<<<1, 1024, 0, s.ctx->stream>>>(l.cnt, l.rows, nullptr, edata(e), ecap(e), nullptr, 0,
-                                                                aoid);
+            sort_err_rows_kernel<<<1, 1024, 0, s.ctx->stream>>>(nullptr, k, l.rows, nullptr, edata(e), ecap(e),
+                                                                nullptr, 0, aoid);
             s.launched();
         }
     }

@@ -301,7 +301,7 @@ struct DjOp {
     const char* base;
     KeyCfg pk;
     JoinOut o;
-    const uint64_t* bounds;
+    const uint64_t* bounds;  // null: kmin and span are set
     const uint32_t* bad;
     const uint32_t* bits;
     const uint64_t* val;
@@ -310,6 +310,7 @@ struct DjOp {
     uint64_t aoid, eck, eco;
     uint64_t *ek, *eo, *acc;
     AHEAD_DEV void begin() {
+        if (!bounds) return;  // (known to the host by now)
         const uint64_t lo = ~__ldg((const unsigned long long*)bounds);
         const uint64_t m = __ldg((const unsigned long long*)bounds + 1) - lo + 1;
         kmin = (uint32_t)lo;
@@ -389,11 +390,14 @@ size_t dj_scratch(uint64_t nb, uint64_t np) {
     return limit / 8 + limit * 8 + 2 * kErrListBytes + compact_scratch<DjOp<8, true>>(np) + 4096;
 }
 
-// Builds and probes; totals in counters 0 (matches), 1 and 2 (probe errors).
-// `err_k`, `err_o`: the probe key's and the probe output column's vectors.
+// Builds, probes and reads the counters back: counter 0 matches, 1 and 2 the
+// probe's errors, kDjBad whether the hash table has to take the join.  `err_k`,
+// `err_o`: the probe key's and the probe output column's vectors.  A sized call
+// (`out` given) gets its output columns between the passes.
 template <bool AN>
-void run_direct_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk, uint64_t np, const JoinOut& o,
-                     uint64_t aoid, ahead_errvec* err_k, ahead_errvec* err_o, ErrList* kerr, ErrList* verr) {
+int run_direct_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk, uint64_t np, const JoinOut& o,
+                    uint64_t aoid, ahead_errvec* err_k, ahead_errvec* err_o, ErrList* kerr, ErrList* verr,
+                    ahead_bat* out) {
     cudaStream_t st = s.ctx->stream;
     DjBuild b;
     b.bk = bk;
@@ -434,18 +438,39 @@ void run_direct_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk
         op.acc = nullptr;
         const uint32_t nt = compact_tiles<Op>(np);
         const CompactBufs cb = s.compact_bufs(np, nt, Op::NCH, 0);
-        if (nt <= kOneBlockTiles || !dyn_smem_ready<dj_classify_kernel<Op>>(s.ctx, kDjSmem)) {
+        if (!out && nt <= kOneBlockTiles) {
             s.launched(launch_compact(s.ctx, st, op, np, cb));
-            return 0;
+            return s.finish(kDjCounters);
         }
-        const uint32_t blocks = (nt + 31) / 32;
-        dj_classify_kernel<Op><<<blocks < (uint32_t)s.ctx->num_sms ? blocks : s.ctx->num_sms, 1024, kDjSmem, st>>>(
-            op, np, cb);
-        s.launched(1 + launch_compact_tail(s.ctx, st, op, np, cb));
-        return 0;
+        if (dyn_smem_ready<dj_classify_kernel<Op>>(s.ctx, kDjSmem)) {
+            const uint32_t blocks = (nt + 31) / 32;
+            dj_classify_kernel<Op><<<blocks < (uint32_t)s.ctx->num_sms ? blocks : s.ctx->num_sms, 1024, kDjSmem,
+                                     st>>>(op, np, cb);
+        } else {
+            const uint32_t per = tiles_per_warp(s.ctx, nt);
+            classify_kernel<Op, short_k(Op::W)>
+                <<<(nt + per * kCWarps - 1) / (per * kCWarps), kCThreads, 0, st>>>(op, np, cb, (int)per);
+        }
+        s.launched();
+        launch_scan(s, cb);
+        if (out) {
+            int rc = s.finish(kDjCounters);
+            if (rc || s.counter(kDjBad)) return rc;
+            // (finish() leaves the counters zero: the emit pass gets the key bounds by value)
+            op.bounds = nullptr;
+            op.kmin = (uint32_t)~s.counter(kDjBounds);
+            op.span = (uint32_t)(s.counter(kDjBounds + 1) - ~s.counter(kDjBounds) + 1);
+            op.o.cap = s.counter(0);
+            if (!s.take(&out->head, 0, op.o.cap) || !s.take(&out->tail, 1, op.o.cap))
+                return fail(s.ctx, AHEAD_NO_MEMORY, "output allocation failed");
+            op.o.oh = out->head.data;
+            op.o.ot = out->tail.data;
+        }
+        launch_emit(s, op, np, cb);
+        return out ? s.wait() : s.finish(kDjCounters);
     };
-    if constexpr (AN) by_width_enc(pk.width, probe);
-    else by_width(pk.width, probe);
+    if constexpr (AN) return by_width_enc(pk.width, probe);
+    else return by_width(pk.width, probe);
 }
 
 size_t join_scratch(uint64_t nb, uint64_t np) {
@@ -1196,13 +1221,13 @@ size_t merge_scratch(uint64_t n1) {
 }
 
 // The checks (flag in counter kMergeFlag) and the intersection (total in
-// counter 0), which counts only when the flag's bit 0 stays clear.  `dw`: the
+// counter 0), both read back; the intersection counts only when the flag's bit 0
+// stays clear.  `dw`: the
 // driving column's width, at least 2.
 constexpr int kMergeFlag = 40, kMergeCounters = 41;
 
-void run_merge(OpScope& s, const DCol& t1, const DCol& h1, const DCol& h2, const DCol& t2, uint64_t n1, uint64_t n2,
-               bool checked, int dw, int reenc, uint64_t fh, uint64_t ft, void* oh, int ohw, void* ot, int otw,
-               uint64_t cap) {
+int run_merge(OpScope& s, const DCol& t1, const DCol& h1, const DCol& h2, const DCol& t2, uint64_t n1, uint64_t n2,
+              bool checked, int dw, int reenc, uint64_t fh, uint64_t ft, ahead_bat* out, uint64_t cap) {
     cudaStream_t st = s.ctx->stream;
     MergeSide ma{t1, h1, checked && t1.enc, checked && h1.enc};
     MergeSide mb{h2, t2, checked && h2.enc, checked && t2.enc};
@@ -1214,7 +1239,8 @@ void run_merge(OpScope& s, const DCol& t1, const DCol& h1, const DCol& h2, const
     MergeParts mp{t1, h2, n1, n2, (uint64_t*)s.alloc(((size_t)tiles + 1) * 8)};
     merge_part_kernel<<<(tiles + 256) / 256, 256, 0, st>>>(mp, tiles);
     s.launched(2);
-    by_width_enc(dw, [&](auto tag) -> int {
+    const bool sized = s.sized(out, cap);
+    return by_width_enc(dw, [&](auto tag) -> int {
         IsectOp<decltype(tag)::value> op;
         op.base = (const char*)(t1.type == AHEAD_VOID ? h1.data : t1.data);
         op.t1c = t1;
@@ -1223,25 +1249,36 @@ void run_merge(OpScope& s, const DCol& t1, const DCol& h1, const DCol& h2, const
         op.t2c = t2;
         op.fh = fh;
         op.ft = ft;
-        op.cap = cap;
+        op.cap = (out->head.data && out->tail.data) ? cap : 0;
         op.acc = nullptr;
-        op.oh = oh;
-        op.ot = ot;
-        op.ohw = ohw;
-        op.otw = otw;
+        op.oh = out->head.data;
+        op.ot = out->tail.data;
+        op.ohw = type_width(out->head.type);
+        op.otw = type_width(out->tail.type);
         op.reenc = reenc;
         op.mirror2 = t2.type != AHEAD_VOID && t2.data == h2.data && t2.type == h2.type && t2.ainv == h2.ainv;
         op.a2 = h2.enc ? inv_pow2(h2.ainv, 64) : 1;
         op.part = mp.part;
         op.lo = op.len = 0;
-        if (tiles <= kOneBlockTiles) {
+        if (tiles <= kOneBlockTiles && !sized) {
             run_compact(s, op, n1, 0);
-            return 0;
+            return s.finish(kMergeCounters);
         }
         const CompactBufs cb = s.compact_bufs(n1, tiles, 1, 0);
         merge_classify_kernel<<<(tiles + kCWarps - 1) / kCWarps, kCThreads, 0, st>>>(op, n1, cb);
-        s.launched(1 + launch_compact_tail(s.ctx, st, op, n1, cb));
-        return 0;
+        s.launched();
+        launch_scan(s, cb);
+        if (sized) {
+            int rc = s.finish(kMergeCounters);
+            if (rc || (s.counter(kMergeFlag) & 1u)) return rc;
+            op.cap = s.counter(0);
+            if (!s.take(&out->head, 0, op.cap) || !s.take(&out->tail, 1, op.cap))
+                return fail(s.ctx, AHEAD_NO_MEMORY, "output allocation failed");
+            op.oh = out->head.data;
+            op.ot = out->tail.data;
+        }
+        launch_emit(s, op, n1, cb);
+        return sized ? s.wait() : s.finish(kMergeCounters);
     });
 }
 
@@ -1520,7 +1557,7 @@ int ahead_gpu_hashjoin_an(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r
     OpScope s(ctx);
     const uint64_t nl = l->count, nr = r->count;
     const bool both = nl > 0 && nr > 0;
-    if (!both) return AHEAD_OK;
+    if (!both) return s.empty(out, cap, true);
     const bool left = side == AHEAD_HASH_LEFT;
     const uint64_t nb = left ? nl : nr, np = left ? nr : nl;
     const int bt1 = type_base_width(T1), bh2 = type_base_width(H2);
@@ -1558,8 +1595,8 @@ int ahead_gpu_hashjoin_an(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r
     // error vectors of the probe's key and output column, and the build's
     const int vpk = left ? 2 : 1, vpo = left ? 3 : 0, vbk = left ? 1 : 2, vbo = left ? 0 : 3;
     ErrList kerr, verr;
-    run_direct_join<true>(s, bk, nb, pk, np, o, aoid, ev(errs, vpk), ev(errs, vpo), &kerr, &verr);
-    rc = s.finish(kDjCounters);
+    rc = run_direct_join<true>(s, bk, nb, pk, np, o, aoid, ev(errs, vpk), ev(errs, vpo), &kerr, &verr,
+                               s.sized(out, cap) ? out : nullptr);
     if (rc) return rc;
     if (!s.counter(kDjBad)) {
         out->count = s.counter(0);
@@ -1593,7 +1630,7 @@ int ahead_gpu_hashjoin_an(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r
     if (errs)
         for (int k = 0; k < 4; ++k)
             if (errs[k].present) errs[k].count = s.counter(1 + k);
-    return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
+    return out->count > cap || s.sized(out, cap) ? AHEAD_CAPACITY : AHEAD_OK;
 }
 
 int ahead_gpu_hashjoin(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r, int side, ahead_bat* out,
@@ -1610,7 +1647,7 @@ int ahead_gpu_hashjoin(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r, i
     const uint64_t nl = l->count, nr = r->count;
     const bool both = nl > 0 && nr > 0;
     const uint64_t nb = side == AHEAD_HASH_LEFT ? nl : nr, np = side == AHEAD_HASH_LEFT ? nr : nl;
-    if (!both) return AHEAD_OK;
+    if (!both) return s.empty(out, cap, true);
     const int w = type_width(T1);
     JoinOut o;
     o.fh = o.ft = 1;
@@ -1629,8 +1666,8 @@ int ahead_gpu_hashjoin(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r, i
         int rc = s.reserve(dj_scratch(nb, np));
         if (rc) return rc;
         ErrList kerr, verr;
-        run_direct_join<false>(s, bk, nb, pk, np, o, 0, nullptr, nullptr, &kerr, &verr);
-        rc = s.finish(kDjCounters);
+        rc = run_direct_join<false>(s, bk, nb, pk, np, o, 0, nullptr, nullptr, &kerr, &verr,
+                                    s.sized(out, cap) ? out : nullptr);
         if (rc) return rc;
         if (!s.counter(kDjBad)) {
             out->count = s.counter(0);
@@ -1643,7 +1680,7 @@ int ahead_gpu_hashjoin(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r, i
     rc = s.finish(1);
     if (rc) return rc;
     out->count = s.counter(0);
-    return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
+    return out->count > cap || s.sized(out, cap) ? AHEAD_CAPACITY : AHEAD_OK;
 }
 
 int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, int reenc, uint64_t ah1r,
@@ -1742,7 +1779,7 @@ int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
             errs[1].count = s.counter(2);
             if (errs[3].present) errs[3].count = s.counter(3);
         }
-        return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
+        return out->count > cap || s.sized(out, cap) ? AHEAD_CAPACITY : AHEAD_OK;
     }
     if (vv) {
         set_errs_present(errs, type_encoded(H1), 0, 0, type_encoded(T2));
@@ -1771,20 +1808,18 @@ int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
             if (errs[0].present) errs[0].count = (n1 && n2) ? s.counter(0) : 0;
             if (errs[3].present) errs[3].count = (n1 && n2) ? s.counter(1) : 0;
         }
-        return m > cap ? AHEAD_CAPACITY : AHEAD_OK;
+        return m > cap || s.sized(out, cap) ? AHEAD_CAPACITY : AHEAD_OK;
     }
     // general merge (gm) or (void tail, resoid head) merge (mv)
     set_errs_present(errs, type_encoded(H1), type_encoded(T1), type_encoded(H2), type_encoded(T2));
-    if (!n1 || !n2) return AHEAD_OK;
+    if (!n1 || !n2) return s.empty(out, cap, true);
     int rc;
     const int dw = type_width(T1 == AHEAD_VOID ? H1 : T1);  // 8: the head of a void list is encoded
     {
         const uint64_t nt1 = (n1 + kMeTile - 1) / kMeTile, nt2 = (n2 + kMeTile - 1) / kMeTile;
         rc = s.reserve(merge_scratch(n1) + (nt1 + nt2) * 24 + 4096);
         if (rc) return rc;
-        run_merge(s, t1, h1, h2, t2, n1, n2, true, dw, reenc, fH1, fT2, out->head.data, type_width(oH),
-                  out->tail.data, type_width(oT), ocap);
-        rc = s.finish(kMergeCounters);
+        rc = run_merge(s, t1, h1, h2, t2, n1, n2, true, dw, reenc, fH1, fT2, out, cap);
         if (rc) return rc;
         const uint32_t flag = (uint32_t)s.counter(kMergeFlag);
         if (!(flag & 1u)) {
@@ -1861,7 +1896,7 @@ int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
     if (errs)
         for (int k = 0; k < 4; ++k)
             if (errs[k].present) errs[k].count = s.counter(1 + k);
-    return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
+    return out->count > cap || s.sized(out, cap) ? AHEAD_CAPACITY : AHEAD_OK;
 }
 
 int ahead_gpu_matchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, ahead_bat* out, uint64_t cap) {
@@ -1897,7 +1932,7 @@ int ahead_gpu_matchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, 
         rc = s.finish(0);
         if (rc) return rc;
         out->count = m;
-        return m > cap ? AHEAD_CAPACITY : AHEAD_OK;
+        return m > cap || s.sized(out, cap) ? AHEAD_CAPACITY : AHEAD_OK;
     }
     if (T1 == AHEAD_OID && H2 == AHEAD_VOID) {
         int rc;
@@ -1937,19 +1972,18 @@ int ahead_gpu_matchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, 
         rc = s.finish(1);
         if (rc) return rc;
         out->count = n1 ? s.counter(0) : 0;
-        return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
+        return out->count > cap || s.sized(out, cap) ? AHEAD_CAPACITY : AHEAD_OK;
     }
     // merge on plain oid values: strictly increasing keys intersect in parallel
     // (driving column of 2, 4 or 8 bytes); anything else replays the loop
     const int dw = type_width(T1 == AHEAD_VOID ? H1 : T1);
-    if (n1 && n2 && dw >= 2) {
+    if (!n1 || !n2) return s.empty(out, cap, true);
+    if (dw >= 2) {
         int rc = s.reserve(merge_scratch(n1));
         if (rc) return rc;
         DCol k1 = t1, k2 = h2, v1 = h1, v2 = t2;
         k1.enc = k2.enc = v1.enc = v2.enc = 0;  // plain values
-        run_merge(s, k1, v1, k2, v2, n1, n2, false, dw, 0, 1, 1, out->head.data, type_width(type_select_of(H1)),
-                  out->tail.data, type_width(type_select_of(T2)), ocap);
-        rc = s.finish(kMergeCounters);
+        rc = run_merge(s, k1, v1, k2, v2, n1, n2, false, dw, 0, 1, 1, out, cap);
         if (rc) return rc;
         if (!(s.counter(kMergeFlag) & 1u)) {
             out->count = s.counter(0);
@@ -1976,7 +2010,7 @@ int ahead_gpu_matchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, 
     rc = s.finish(1);
     if (rc) return rc;
     out->count = s.counter(0);
-    return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
+    return out->count > cap || s.sized(out, cap) ? AHEAD_CAPACITY : AHEAD_OK;
 }
 
 int ahead_gpu_fetchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, int reenc, uint64_t atr,

@@ -73,6 +73,7 @@ template <int W, bool AN>
 int run_select(OpScope& s, const ahead_bat* in, const RangePred& p, uint64_t aoid, ahead_bat* out, uint64_t cap,
                ahead_errvec* err) {
     typedef SelectOp<W, AN> Op;
+    if (!in->count) return s.empty(out, cap, false);
     int rc = s.reserve(compact_scratch<Op>(in->count));
     if (rc) return rc;
     Op op;
@@ -89,8 +90,18 @@ int run_select(OpScope& s, const ahead_bat* in, const RangePred& p, uint64_t aoi
     op.errcap = (err && err->data) ? err->capacity : 0;
     op.acc = nullptr;
     op.pred = p;
-    run_compact<Op>(s, op, in->count, 0);
-    rc = s.finish(Op::NCH);
+    if (s.sized(out, cap)) {
+        rc = run_compact_sized(s, op, in->count, 0, Op::NCH, [&](uint64_t kept) {
+            out->count = op.cap = kept;
+            if (!s.take(&out->head, 0, kept)) return false;
+            op.out_an = (uint64_t*)out->head.data;
+            op.out_oid = (uint32_t*)out->head.data;
+            return true;
+        });
+    } else {
+        run_compact<Op>(s, op, in->count, 0);
+        rc = s.finish(Op::NCH);
+    }
     if (rc) return rc;
     out->count = s.counter(0);
     if (AN && err) err->count = s.counter(1);
@@ -698,7 +709,7 @@ int ahead_gpu_check_an(ahead_ctx* ctx, const ahead_bat* in, uint64_t ainv, uint6
                 (const char*)in->tail.data, in->count, ainv & wmask(W), unenc_max & wmask(W), cnt, rows);
             return 0;
         });
-        sort_err_rows_kernel<<<1, 1024, 0, ctx->stream>>>(cnt, rows, nullptr, edata(err), ecap(err), nullptr, 0, aoid);
+        sort_err_rows_kernel<<<1, 1024, 0, ctx->stream>>>(cnt, 0, rows, nullptr, edata(err), ecap(err), nullptr, 0, aoid);
         s.launched(2);
         rc = s.finish(1);
         if (rc) return rc;
@@ -939,7 +950,7 @@ int ahead_gpu_aggregate_mul_sum_an(ahead_ctx* ctx, const ahead_bat* a, const ahe
                 return 0;
             });
         });
-        sort_err_rows_kernel<<<2, 1024, 0, ctx->stream>>>(cnt, rows1, rows2, edata(e1), ecap(e1), edata(e2), ecap(e2),
+        sort_err_rows_kernel<<<2, 1024, 0, ctx->stream>>>(cnt, 0, rows1, rows2, edata(e1), ecap(e1), edata(e2), ecap(e2),
                                                           aoid);
         s.launched(2);
         rc = s.finish(3);

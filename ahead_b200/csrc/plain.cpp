@@ -53,6 +53,11 @@ int width_of(int type) {
     }
 }
 
+// Outputs are allocated once an operator knows its count (AHEAD_SIZED) where
+// it can, error vectors hold every row only for heads known to read as corrupt
+// (a re-encoded head keeps its void column's largest value, 0), and a BAT's
+// blocks go back as soon as no later step reads it: a query whose first joins
+// filter nothing would otherwise hold over 130 GB at 600M rows.
 // Device buffers come from a per-device memory pool through the stream-ordered
 // allocator (cudaMallocFromPoolAsync / cudaFreeAsync on the library's stream):
 // one query makes 20-30 operator calls, each with outputs sized by its inputs
@@ -62,6 +67,7 @@ int width_of(int type) {
 // largest query so far), as a caching allocator does: returning memory to the
 // device at every synchronisation point made each query map it again.
 constexpr uint64_t kPoolKeepBytes = ~uint64_t(0);
+constexpr uint64_t kKeepBytes = uint64_t(1) << 24;  // output columns up to this size stay in their block
 
 cudaMemPool_t device_pool(int dev) {
     static std::mutex mu;
@@ -124,11 +130,6 @@ struct Arena {
 
 struct Errs {
     std::vector<ahead_errvec> v;
-    uint64_t need() const {
-        uint64_t m = 0;
-        for (const auto& e : v) m = std::max(m, e.count);
-        return m;
-    }
 };
 
 struct Plain {
@@ -153,46 +154,66 @@ struct Plain {
         return view(h, b.tail, b.count);
     }
 
-    // One operator call with outputs of `cap` rows and error vectors of a small
-    // first capacity; on AHEAD_CAPACITY (or counts above the capacities) the
-    // call runs again with the sizes it reported.
+    // Whether every row of an encoded column reads as corrupt.
+    static bool dense(const ahead_col& c) {
+        return c.type >= AHEAD_RESTINY && c.type <= AHEAD_RESOID && c.unenc_max == 0;
+    }
+    static void* take_output(void* user, int, uint64_t bytes) { return static_cast<Plain*>(user)->arena.take(bytes); }
+
+    // One operator call with outputs of `cap` rows (AHEAD_SIZED: allocated by the
+    // call) and error vectors of a small first capacity, or of all rows of their
+    // input (vectors 0 and 1: the first's, 2 and 3: the second's) for those in
+    // `full`; on AHEAD_CAPACITY (or counts above the capacities) the call runs
+    // again with the sizes it reported.
     template <typename F>
-    bool run(F call, uint64_t cap, int nerr, int nout, ahead_bat* outs, Errs* errs) {
+    bool run(F call, uint64_t cap, int nerr, int nout, ahead_bat* outs, Errs* errs, uint32_t full = 0,
+             uint64_t rows_a = 0, uint64_t rows_b = 0) {
         if (rc) return false;
-        uint64_t ecap = std::min<uint64_t>(std::max<uint64_t>(cap, 1), 1u << 16);
+        const uint64_t few = cap == AHEAD_SIZED ? 1u << 16 : std::min<uint64_t>(std::max<uint64_t>(cap, 1), 1u << 16);
+        std::vector<uint64_t> ecap(nerr, few);
+        for (int i = 0; i < nerr; ++i)
+            if ((full >> i) & 1u) ecap[i] = std::max(few, i < 2 ? rows_a : rows_b);
         cap = std::max<uint64_t>(cap, 1);
         for (;;) {
+            const bool sized = cap == AHEAD_SIZED;
             for (int o = 0; o < nout; ++o) {
                 outs[o] = ahead_bat{};
+                if (sized) continue;
                 outs[o].head.data = arena.take(cap * 8);
                 outs[o].tail.data = arena.take(cap * 8);
                 if (!outs[o].head.data || !outs[o].tail.data) return fail(AHEAD_NO_MEMORY);
             }
+            void* const block[2] = {nout ? outs[0].head.data : nullptr, nout ? outs[0].tail.data : nullptr};
             if (errs) {
                 errs->v.assign(nerr, ahead_errvec{});
-                for (auto& e : errs->v) {
-                    e.data = static_cast<uint64_t*>(arena.take(ecap * 8));
-                    e.capacity = ecap;
+                for (int i = 0; i < nerr; ++i) {
+                    ahead_errvec& e = errs->v[i];
+                    e.data = static_cast<uint64_t*>(arena.take(ecap[i] * 8));
+                    e.capacity = ecap[i];
                     if (!e.data) return fail(AHEAD_NO_MEMORY);
                 }
             }
+            if (sized) ahead_ctx_set_output_fn(ctx, take_output, this);
             const int r = call(cap);
+            if (sized) ahead_ctx_set_output_fn(ctx, nullptr, nullptr);
             uint64_t need_o = 0;
             for (int o = 0; o < nout; ++o) need_o = std::max(need_o, outs[o].count);
-            const uint64_t need_e = errs ? errs->need() : 0;
-            if (r == AHEAD_CAPACITY || need_o > cap || need_e > ecap) {
-                if (need_o <= cap && need_e <= ecap) return fail(r);
-                cap = std::max(cap, need_o);
-                ecap = std::max(ecap, need_e);
-                for (int o = 0; o < nout; ++o) {
-                    arena.give_back(outs[o].head.data);
-                    arena.give_back(outs[o].tail.data);
+            bool short_e = false;
+            for (int i = 0; i < nerr; ++i) short_e |= errs->v[i].count > ecap[i];
+            if (r == AHEAD_CAPACITY || need_o > cap || short_e) {
+                if (need_o <= cap && !short_e && !sized) return fail(r);
+                if (sized && r == AHEAD_CAPACITY) cap = std::max<uint64_t>(need_o, 1);
+                else if (!sized) cap = std::max(cap, need_o);
+                for (int o = 0; o < nout; ++o) drop(outs[o]);
+                for (int i = 0; i < nerr; ++i) {
+                    arena.give_back(errs->v[i].data);
+                    ecap[i] = std::max(ecap[i], errs->v[i].count);
                 }
-                if (errs)
-                    for (auto& e : errs->v) arena.give_back(e.data);
                 continue;
             }
             if (r) return fail(r);
+            // (a selection fills only its head: its tail's block goes back at once)
+            if (!sized && nout == 1 && block[1] && outs[0].tail.data != block[1]) arena.give_back(block[1]);
             // an output far below its capacity moves into a block of its size, so
             // the next operators of the query can reuse the large one
             // (a virtual-OID column holds no data: its block goes back at once)
@@ -205,7 +226,7 @@ struct Plain {
                         c->data = nullptr;
                         continue;
                     }
-                    if (outs[o].count * 4 >= cap) continue;
+                    if (sized || cap * 8 <= kKeepBytes || outs[o].count * 4 >= cap) continue;
                     const size_t bytes = outs[o].count * (size_t)width_of(c->type);
                     void* small = arena.take(bytes);
                     if (!small) return fail(AHEAD_NO_MEMORY);
@@ -216,6 +237,11 @@ struct Plain {
             }
             return true;
         }
+    }
+    // hands a BAT's blocks back (blocks of other owners are left alone)
+    void drop(const ahead_bat& b) {
+        if (b.head.data) arena.give_back(b.head.data);
+        if (b.tail.data && b.tail.data != b.head.data) arena.give_back(b.tail.data);
     }
     bool fail(int r) {
         rc = r;
@@ -235,44 +261,59 @@ struct Plain {
         copy(h.data(), e.data, h.size() * 8, cudaMemcpyDeviceToHost);
         return h;
     }
-    void add_errs(int col, const ahead_errvec& e) {
-        std::vector<uint64_t> h = host_errs(e);
+    void add_errs(int col, const std::vector<uint64_t>& h) {
         ferr[col].insert(ferr[col].end(), h.begin(), h.end());
         std::sort(ferr[col].begin(), ferr[col].end());
     }
-    void set_errs(int col, const ahead_errvec& e) { ferr[col] = host_errs(e); }
+    // error vector `which` on the host (into *out when given); all of a call's
+    // vectors go back
+    void keep_errs(const Errs& errs, int which, std::vector<uint64_t>* out) {
+        if (!rc && out) *out = host_errs(errs.v[which]);
+        for (const auto& e : errs.v) arena.give_back(e.data);
+    }
 
     ahead_bat select_an(const ahead_bat& in, int op1, uint64_t th1, int op2, uint64_t th2, int comb,
-                        ahead_errvec* err_out) {
+                        std::vector<uint64_t>* err_out) {
         ahead_bat out{};
         Errs errs;
         run([&](uint64_t cap) {
                 return ahead_gpu_select_an(ctx, &in, op1, th1, op2, th2, comb, kAoid, &out, cap, &errs.v[0]);
             },
-            in.count, 1, 1, &out, &errs);
-        if (!rc && err_out) *err_out = errs.v[0];
+            in.count * 8 > kKeepBytes ? AHEAD_SIZED : in.count, 1, 1, &out, &errs);
+        keep_errs(errs, 0, err_out);
         return out;
     }
-    ahead_bat matchjoin_an(const ahead_bat& a, const ahead_bat& b, ahead_errvec* errs_out = nullptr) {
+    // `tail_errs`: the second input's tail errors (errs[3])
+    ahead_bat matchjoin_an(const ahead_bat& a, const ahead_bat& b, std::vector<uint64_t>* tail_errs = nullptr) {
         ahead_bat out{};
         Errs errs;
-        run([&](uint64_t cap) {
-                return ahead_gpu_matchjoin_an(ctx, &a, &b, 0, 0, 0, 0, 0, kAoid, &out, cap, errs.v.data());
+        const bool positional = b.head.type == AHEAD_VOID;
+        const uint64_t least = std::max<uint64_t>(std::min(a.count, b.count), 1);
+        const uint64_t cap = positional && a.tail.type != AHEAD_VOID ? std::max<uint64_t>(a.count, 1)
+                             : !positional && least * 8 > kKeepBytes ? AHEAD_SIZED
+                                                                     : least;
+        const uint32_t full = (dense(a.head) ? 1u : 0u) | (dense(a.tail) && !positional ? 2u : 0u) |
+                              (dense(b.head) ? 4u : 0u) | (dense(b.tail) ? 8u : 0u);
+        run([&](uint64_t c) {
+                return ahead_gpu_matchjoin_an(ctx, &a, &b, 0, 0, 0, 0, 0, kAoid, &out, c, errs.v.data());
             },
-            std::max<uint64_t>(std::min(a.count, b.count), 1), 4, 1, &out, &errs);
-        if (!rc && errs_out) std::copy(errs.v.begin(), errs.v.end(), errs_out);
+            cap, 4, 1, &out, &errs, full, a.count, b.count);
+        keep_errs(errs, 3, tail_errs);
         return out;
     }
+    // `key_errs`: the left input's key errors (errs[1])
     ahead_bat hashjoin_an(const ahead_bat& l, const ahead_bat& r, int reenc_head, int reenc_tail,
-                          ahead_errvec* errs_out = nullptr) {
+                          std::vector<uint64_t>* key_errs = nullptr) {
         ahead_bat out{};
         Errs errs;
+        const uint64_t most = std::max(l.count, r.count);
+        const uint32_t full = (dense(l.head) ? 1u : 0u) | (dense(r.tail) ? 8u : 0u);
         run([&](uint64_t cap) {
                 return ahead_gpu_hashjoin_an(ctx, &l, &r, reenc_head, kAr, kArInv, reenc_tail, kAr, kArInv,
                                              AHEAD_HASH_RIGHT, kAoid, &out, cap, errs.v.data());
             },
-            std::max(l.count, r.count), 4, 1, &out, &errs);
-        if (!rc && errs_out) std::copy(errs.v.begin(), errs.v.end(), errs_out);
+            most * 8 > kKeepBytes ? AHEAD_SIZED : most, 4, 1, &out, &errs, full, l.count, r.count);
+        keep_errs(errs, 1, key_errs);
         return out;
     }
 
@@ -280,15 +321,23 @@ struct Plain {
     // (ssbm-q11_continuous.cpp:71-79, ssbm-q13_continuous.cpp); the mirrored
     // OID list, and each selection's errors in *errs
     template <typename ColOf, typename Pred>
-    ahead_bat select_chain(int n, ColOf col_of, const Pred* preds, std::vector<ahead_errvec>* errs) {
+    ahead_bat select_chain(int n, ColOf col_of, const Pred* preds, std::vector<std::vector<uint64_t>>* errs) {
         ahead_bat sel{};
         for (int i = 0; i < n && !rc; ++i) {
             const Pred& p = preds[i];
-            ahead_errvec e{};
+            std::vector<uint64_t> e;
             ahead_bat s = select_an(col_of(p), p.op1, p.th1, p.op2, p.th2, p.comb, &e);
             if (rc) break;
-            if (errs) errs->push_back(e);
-            sel = i == 0 ? mirror_head(s) : mirror_head(matchjoin_an(sel, mirror_head(s)));
+            if (errs) errs->push_back(std::move(e));
+            if (i == 0) {
+                sel = mirror_head(s);
+            } else {
+                const ahead_bat both = matchjoin_an(sel, mirror_head(s));
+                drop(sel);
+                drop(s);
+                drop(ahead_bat{ahead_col{}, both.tail, 0});  // (only its head is used)
+                sel = mirror_head(both);
+            }
         }
         return sel;
     }
@@ -353,46 +402,53 @@ extern "C" int ahead_plain_starjoin(ahead_ctx* ctx, const ahead_sj_schema* sch, 
                 (int)preds.size(), [&](const ahead_sj_pred& p) { return dim_bat(d, sch->dim[d].attr[p.attr]); },
                 preds.data(), nullptr);
             km[d] = P.matchjoin_an(Plain::reverse(key), sel);
+            P.drop(sel);
         }
     }
+    bool grouped[4] = {false, false, false, false};
+    for (int j = 0; j < q->ngroup; ++j) grouped[q->gdim[j]] = true;
     ahead_bat joined[4]{}, s{};
     size_t first_todo = 0;
+    int last = -1;  // the dimension whose join result `s` mirrors
+    // `s` moves on: a join result no group attribute needs goes back
+    auto move_on = [&](const ahead_bat& j, int d) {
+        if (last < 0) P.drop(s);
+        else if (!grouped[last]) P.drop(joined[last]);
+        joined[d] = j;
+        s = Plain::mirror_head(j);
+        last = d;
+    };
     if (q->nfpred) {
-        std::vector<ahead_errvec> errs;
+        std::vector<std::vector<uint64_t>> errs;
         s = P.select_chain(q->nfpred, [&](const ahead_sj_fpred& p) { return lo(p.col); }, q->fpred, &errs);
         for (int k = 0; k < q->nfpred && !P.rc && k < (int)errs.size(); ++k) P.add_errs(q->fpred[k].col, errs[k]);
     } else {
         const int d0 = dims[0];
         const int void_tail = km[d0].tail.type == AHEAD_VOID;
-        ahead_errvec errs[4]{};
-        ahead_bat j = P.hashjoin_an(lo(d0), km[d0], 1, void_tail, errs);
-        if (!P.rc) P.set_errs(d0, errs[1]);
-        joined[d0] = j;
-        s = Plain::mirror_head(j);
+        move_on(P.hashjoin_an(lo(d0), km[d0], 1, void_tail, &P.ferr[d0]), d0);
         first_todo = 1;
     }
     for (size_t i = first_todo; i < dims.size() && !P.rc; ++i) {
         const int d = dims[i];
-        ahead_errvec errs[4]{};
-        ahead_bat f = P.matchjoin_an(s, lo(d), errs);
+        ahead_bat f = P.matchjoin_an(s, lo(d), &P.ferr[d]);
         if (P.rc) break;
-        P.set_errs(d, errs[3]);
         const int void_tail = km[d].tail.type == AHEAD_VOID;
-        joined[d] = P.hashjoin_an(f, km[d], void_tail, void_tail);
-        s = Plain::mirror_head(joined[d]);
+        const ahead_bat j = P.hashjoin_an(f, km[d], void_tail, void_tail);
+        P.drop(f);
+        move_on(j, d);
     }
     // measures, dropped row-consistently
     const int first = q->measure == AHEAD_SJ_MEASURE_PRICE_DISCOUNT ? AHEAD_SJ_COL_PRICE : AHEAD_SJ_COL_REVENUE;
     const int second = q->measure == AHEAD_SJ_MEASURE_PRICE_DISCOUNT ? AHEAD_SJ_COL_DISCOUNT
                        : q->measure == AHEAD_SJ_MEASURE_PROFIT      ? AHEAD_SJ_COL_SUPPLYCOST
                                                                     : -1;
-    ahead_errvec e4[4]{};
-    ahead_bat m1 = P.matchjoin_an(s, lo(first), e4);
-    if (!P.rc) P.add_errs(first, e4[3]);
+    std::vector<uint64_t> me;
+    ahead_bat m1 = P.matchjoin_an(s, lo(first), &me);
+    if (!P.rc) P.add_errs(first, me);
     ahead_bat s6 = Plain::mirror_head(m1), m2{}, mp = m1;
     if (second >= 0 && !P.rc) {
-        m2 = P.matchjoin_an(s6, lo(second), e4);
-        if (!P.rc) P.add_errs(second, e4[3]);
+        m2 = P.matchjoin_an(s6, lo(second), &me);
+        if (!P.rc) P.add_errs(second, me);
         s6 = Plain::mirror_head(m2);
         mp = P.matchjoin_an(s6, m1);
     }
@@ -414,6 +470,7 @@ extern "C" int ahead_plain_starjoin(ahead_ctx* ctx, const ahead_sj_schema* sch, 
             const int d = q->gdim[j];
             ahead_bat g = P.matchjoin_an(s6, joined[d]);
             attrs[j] = P.matchjoin_an(g, dim_bat(d, sch->dim[d].attr[q->gattr[j]]));
+            P.drop(g);
         }
         ahead_bat vals = Plain::clear_head(mp);
         if (q->measure != AHEAD_SJ_MEASURE_REVENUE && !P.rc) {

@@ -17,7 +17,7 @@ from typing import List, Optional, Tuple
 
 import numpy as np
 
-from .model import (CAPACITY, NP_DTYPE, OK, STATUS_NAMES, STR, VOID, WIDTH, Bat, CBat, CErrVec, Col, ErrVec,
+from .model import (CAPACITY, NP_DTYPE, OK, STATUS_NAMES, STR, VOID, WIDTH, Bat, CBat, CErrVec, Col, ENCODED, ErrVec,
                     ccol, col_from_c)
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -49,8 +49,8 @@ def load_library():
     lib.ahead_ctx_launches.restype = ctypes.c_uint64
     lib.ahead_ctx_stream.argtypes = [ctypes.c_void_p]
     lib.ahead_ctx_stream.restype = ctypes.c_void_p
-    lib.ahead_ctx_stream.argtypes = [ctypes.c_void_p]
-    lib.ahead_ctx_stream.restype = ctypes.c_void_p
+    lib.ahead_ctx_set_output_fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    lib.ahead_ctx_set_output_fn.restype = None
     _lib = lib
     return lib
 
@@ -110,47 +110,107 @@ def _in_bat(b: Bat) -> CBat:
                 ccol(b.tail, _ptr(b.tail.data) if b.tail.type != VOID else 0), b.count)
 
 
+# output columns up to this size stay whole behind a smaller result; a result far
+# below a larger capacity is moved out, or is allocated once its size is known
+_KEEP_BYTES = 1 << 24
+# outputs that may take this much per column are allocated once their size is known
+_SIZED_BYTES = 1 << 28
+_ERR_ROWS = 1 << 16  # rows of an error vector's first capacity (detected errors are rare)
+_SIZED = (1 << 64) - 1  # AHEAD_SIZED
+_OUTPUT_FN = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_uint64)
+
+
 class _Out:
-    def __init__(self, torch, cap: int):
-        self.cap = max(int(cap), 1)
-        self.h = torch.empty(self.cap * 8, dtype=torch.uint8, device="cuda")
-        self.t = torch.empty(self.cap * 8, dtype=torch.uint8, device="cuda")
+    """One output BAT: buffers of `cap` rows for its columns, or (sized) none
+    until the library asks for them."""
+
+    def __init__(self, torch, cap: int, tail: bool = True, sized: bool = False):
+        self.sized = sized
+        self.cap = _SIZED if sized else max(int(cap), 1)
+        self.bufs = [None, None]
         self.c = CBat()
-        self.c.head.data = self.h.data_ptr()
-        self.c.tail.data = self.t.data_ptr()
+        if not sized:
+            n = (self.cap * 8 + 15) & ~15  # (both columns 16-byte aligned)
+            if tail and n <= _KEEP_BYTES:
+                both = torch.empty(2 * n, dtype=torch.uint8, device="cuda")
+                p = both.data_ptr()
+                self.bufs = [both, both]
+                self.c.head.data, self.c.tail.data, self.at = p, p + n, n
+            else:
+                self.at = 0
+                self.bufs[0] = torch.empty(n, dtype=torch.uint8, device="cuda")
+                self.c.head.data = self.bufs[0].data_ptr()
+                if tail:
+                    self.bufs[1] = torch.empty(n, dtype=torch.uint8, device="cuda")
+                    self.c.tail.data = self.bufs[1].data_ptr()
+        else:
+            self.at = 0
 
-    def bat(self) -> Bat:
+    def bat(self, torch) -> Bat:
         n = int(self.c.count)
-
-        def col(cc, buf):
+        moved = False
+        cols = []
+        for cc, buf, at in ((self.c.head, self.bufs[0], 0), (self.c.tail, self.bufs[1], self.at)):
             if cc.type == VOID or not cc.data:
-                return col_from_c(cc, None)
-            used = buf[: n * WIDTH[cc.type]]
-            # a result far below its capacity is moved out, so the capacity-sized
-            # buffer does not stay alive with it
-            return col_from_c(cc, used.clone() if 4 * used.numel() < buf.numel() else used)
+                cols.append(col_from_c(cc, None))
+                continue
+            used = buf[at: at + n * WIDTH[cc.type]]
+            if not self.sized and self.cap * 8 > _KEEP_BYTES and 4 * used.numel() < self.cap * 8:
+                # a result far below its capacity is moved out, so the capacity-sized
+                # buffer does not stay alive with it
+                used, moved = used.clone(), True
+            cols.append(col_from_c(cc, used))
+        if moved:  # the library's stream does not wait for torch's
+            torch.cuda.current_stream().synchronize()
+        return Bat(cols[0], cols[1], n)
 
-        return Bat(col(self.c.head, self.h), col(self.c.tail, self.t), n)
+
+def _dense(c: Col) -> bool:
+    """Whether every row of an encoded column reads as corrupt: a re-encoded
+    head keeps its void column's largest value, 0."""
+    return c.type in ENCODED and c.unenc_max == 0
 
 
 class _Errs:
-    def __init__(self, torch, k: int, cap: int):
-        self.bufs = [torch.empty(max(int(cap), 1) * 8, dtype=torch.uint8, device="cuda") for _ in range(k)]
-        self.c = (CErrVec * k)()
-        for i in range(k):
-            self.c[i].data = self.bufs[i].data_ptr()
-            self.c[i].capacity = max(int(cap), 1)
+    """The error vectors of one call.  Vectors of up to _ERR_ROWS rows lie in the
+    context's buffer, which goes to the result when one of them holds anything
+    (the next call then gets another)."""
 
-    def need(self) -> int:
-        return max([int(e.count) for e in self.c] + [0])
+    def __init__(self, ops: "GpuOps", caps: List[int]):
+        self.caps = caps
+        self.bufs = [None] * len(caps)
+        self.c = (CErrVec * len(caps))()
+        base = ops._err_base()
+        for i, cap in enumerate(caps):
+            e = self.c[i]
+            if cap <= _ERR_ROWS:
+                e.data = base + i * _ERR_ROWS * 8
+            else:
+                self.bufs[i] = ops.torch.empty(cap * 8, dtype=ops.torch.uint8, device="cuda")
+                e.data = self.bufs[i].data_ptr()
+            e.capacity = cap
 
-    def vecs(self) -> List[ErrVec]:
-        out = []
+    def short(self) -> bool:
+        return any(int(e.count) > cap for e, cap in zip(self.c, self.caps))
+
+    def grown(self) -> List[int]:
+        return [max(cap, int(e.count)) for e, cap in zip(self.c, self.caps)]
+
+    def vecs(self, ops: "GpuOps") -> List[ErrVec]:
+        out, held = [], False
         for i, e in enumerate(self.c):
             if not e.present:
                 out.append(ErrVec(None, False))
-            else:
+            elif not e.count:
+                out.append(ErrVec(ops._no_errors, True))
+            elif self.bufs[i] is not None:
                 out.append(ErrVec(self.bufs[i][: int(e.count) * 8], True))
+            else:
+                at = i * _ERR_ROWS * 8
+                out.append(ErrVec(ops._err_buf[at: at + int(e.count) * 8], True))
+                held = True
+        if held:
+            ops._err_buf = None
         return out
 
 
@@ -163,6 +223,8 @@ class GpuOps:
         self.torch.cuda.set_device(device)
         stream = self.torch.cuda.current_stream(device)
         self.ctx = ctypes.c_void_p()
+        self._err_buf = self._err_at = self._output_fn = None
+        self._no_errors = self.torch.empty(0, dtype=self.torch.uint8, device="cuda")
         rc = self.lib.ahead_ctx_create(device, ctypes.c_void_p(stream.cuda_stream), ctypes.byref(self.ctx))
         if rc != OK:
             raise AheadError(rc, "ahead_ctx_create")
@@ -193,22 +255,68 @@ class GpuOps:
         if rc != OK:
             raise AheadError(rc, what, self.lib.ahead_ctx_last_error(self.ctx).decode())
 
-    def _run(self, what, call, cap: int, nerr: int, nout: int = 1):
-        """Run an operator with outputs of `cap` rows and error vectors of a
-        small first capacity (detected errors are rare); on AHEAD_CAPACITY the
-        call is repeated with the sizes it reported."""
+    def _err_base(self) -> int:
+        """The context's error-vector buffer (four vectors)."""
+        if self._err_buf is None:
+            self._err_buf = self.torch.empty(4 * _ERR_ROWS * 8, dtype=self.torch.uint8, device="cuda")
+            self._err_at = self._err_buf.data_ptr()
+        return self._err_at
+
+    def _result(self, buf, nbytes: int):
+        """The first bytes of an output buffer, moved out of a far larger one."""
+        used = buf[:nbytes]
+        if buf.numel() > _KEEP_BYTES and 4 * nbytes < buf.numel():
+            used = used.clone()
+            self.torch.cuda.current_stream().synchronize()  # the library's stream does not wait for torch's
+        return used
+
+    def _set_sized(self, out: _Out):
+        """The library asks for `out`'s columns during the next call."""
         torch = self.torch
-        ecap = min(max(int(cap), 1), 1 << 16)
+
+        def take(_user, column, nbytes):
+            try:
+                buf = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+            except Exception:
+                return None  # (AHEAD_NO_MEMORY)
+            out.bufs[column] = buf
+            return buf.data_ptr()
+
+        self._output_fn = _OUTPUT_FN(take)  # alive until the next one replaces it
+        self.lib.ahead_ctx_set_output_fn(self.ctx, self._output_fn, None)
+
+    def _run(self, what, call, cap: int, nerr: int, nout: int = 1, tail: bool = True, sized: bool = False,
+             cols=()):
+        """Run an operator with outputs of `cap` rows (sized: allocated by the
+        call when they may be large) and error vectors of a small first
+        capacity, or of all rows for the checked columns `cols` ((column, rows)
+        per vector) whose every row reads as corrupt; on AHEAD_CAPACITY the call
+        is repeated with the sizes it reported."""
+        torch = self.torch
+        cap = int(cap)
+        few = min(max(cap, 1), _ERR_ROWS)
+        ecaps = [few] * nerr
+        for i, (c, rows) in enumerate(cols):
+            if rows > few and _dense(c):
+                ecaps[i] = int(rows)
+        sized = sized and cap * 8 >= _SIZED_BYTES
         while True:
-            outs = [_Out(torch, cap) for _ in range(nout)]
-            errs = _Errs(torch, nerr, ecap) if nerr else None
+            outs = [_Out(torch, cap, tail, sized) for _ in range(nout)]
+            errs = _Errs(self, ecaps) if nerr else None
+            if sized:
+                self._set_sized(outs[0])
             rc = call(outs, errs)
-            need_o = max([int(o.c.count) for o in outs] + [0])
-            need_e = errs.need() if errs else 0
-            if rc == CAPACITY or need_o > cap or need_e > ecap:
-                if need_o <= cap and need_e <= ecap:
+            need_o = max([int(o.c.count) for o in outs]) if outs else 0
+            short = errs.short() if errs else False
+            if rc == CAPACITY or short or (need_o > cap and not sized):
+                if need_o <= cap and not short and not sized:
                     self._check(rc, what)
-                cap, ecap = max(cap, need_o, 1), max(ecap, need_e)
+                if sized and rc == CAPACITY:  # (this call cannot be sized: its count is known now)
+                    cap, sized = max(need_o, 1), False
+                else:
+                    cap = max(cap, need_o, 1)
+                if errs:
+                    ecaps = errs.grown()
                 continue
             self._check(rc, what)
             return outs, errs
@@ -221,8 +329,8 @@ class GpuOps:
                                                 ctypes.c_uint64(th2), comb, ctypes.c_uint64(aoid),
                                                 ctypes.byref(outs[0].c), ctypes.c_uint64(outs[0].cap),
                                                 ctypes.byref(errs.c[0]))
-        outs, errs = self._run("selectAN", call, b.count, 1)
-        return outs[0].bat(), errs.vecs()[0]
+        outs, errs = self._run("selectAN", call, b.count, 1, tail=False, sized=True)
+        return outs[0].bat(self.torch), errs.vecs(self)[0]
 
     def select(self, b: Bat, op1, th1, op2=0, th2=0, comb=0) -> Bat:
         def call(outs, errs):
@@ -230,8 +338,8 @@ class GpuOps:
             return self.lib.ahead_gpu_select(self.ctx, ctypes.byref(cb), op1, ctypes.c_uint64(th1), op2,
                                              ctypes.c_uint64(th2), comb, ctypes.byref(outs[0].c),
                                              ctypes.c_uint64(outs[0].cap))
-        outs, _ = self._run("select", call, b.count, 0)
-        return outs[0].bat()
+        outs, _ = self._run("select", call, b.count, 0, tail=False, sized=True)
+        return outs[0].bat(self.torch)
 
     # -- string selection over fixed-width string slots
     def _select_str(self, fn, what, strs, width: int, seqbase, op1, th1, op2, th2, comb, an: bool) -> Col:
@@ -245,11 +353,9 @@ class GpuOps:
             return fn(self.ctx, ctypes.c_void_p(strs.data_ptr()), ctypes.c_uint64(width), ctypes.c_uint64(count),
                       ctypes.c_uint64(seqbase), op1, ctypes.c_char_p(th1), op2, ctypes.c_char_p(th2), comb,
                       ctypes.byref(outs[0].c), ctypes.c_uint64(outs[0].cap))
-        outs, _ = self._run(what, call, count, 0)
+        outs, _ = self._run(what, call, count, 0, tail=False)
         o = outs[0]
-        n = int(o.c.count)
-        used = o.h[: n * (8 if an else 4)]
-        return col_from_c(o.c.head, used.clone() if 4 * used.numel() < o.h.numel() else used)
+        return col_from_c(o.c.head, self._result(o.bufs[0], int(o.c.count) * (8 if an else 4)))
 
     def select_str_an(self, strs, width: int, seqbase, op1, th1: bytes, op2=0, th2: bytes = b"", comb=0) -> Col:
         """selectAN over a string tail (selectAN_scalar.tcc:98-131, 185-222):
@@ -273,27 +379,27 @@ class GpuOps:
             raise ValueError("r_strs must be a contiguous uint8 CUDA tensor of rows of `width` bytes")
         torch.cuda.current_stream().synchronize()  # the library launches on its own stream
         cap = max(l.count, 1)
-        ecap = min(max(l.count, r.count, 1), 1 << 16)
+        ecaps = [min(max(l.count, r.count, 1), _ERR_ROWS)] * 4
         while True:
             head = torch.empty(cap * 8, dtype=torch.uint8, device="cuda")
             strs = torch.empty(cap * width + 1, dtype=torch.uint8, device="cuda")
             c = CBat()
             c.head.data = head.data_ptr()
             c.tail.data = strs.data_ptr()
-            errs = _Errs(torch, 4, ecap)
+            errs = _Errs(self, ecaps)
             rc = self.lib.ahead_gpu_hashjoin_str_an(
                 self.ctx, ctypes.byref(_in_bat(l)), ctypes.byref(_in_bat(r)), ctypes.c_void_p(r_strs.data_ptr()),
                 ctypes.c_uint64(width), int(bool(reenc_head)), ctypes.c_uint64(ah1r), ctypes.c_uint64(ah1invr), side,
                 ctypes.c_uint64(aoid), ctypes.byref(c), ctypes.c_uint64(cap), errs.c)
-            n, need_e = int(c.count), errs.need()
-            if rc == CAPACITY or n > cap or need_e > ecap:
-                if n <= cap and need_e <= ecap:
+            n, short = int(c.count), errs.short()
+            if rc == CAPACITY or n > cap or short:
+                if n <= cap and not short:
                     self._check(rc, "hashjoinAN(str)")
-                cap, ecap = max(cap, n, 1), max(ecap, need_e)
+                cap, ecaps = max(cap, n, 1), errs.grown()
                 continue
             self._check(rc, "hashjoinAN(str)")
-            hcol = col_from_c(c.head, head[: n * WIDTH[c.head.type]].clone())
-            return hcol, strs[: n * width].view(n, width).clone(), errs.vecs()
+            hcol = col_from_c(c.head, self._result(head, n * WIDTH[c.head.type]))
+            return hcol, self._result(strs, n * width).view(n, width), errs.vecs(self)
 
     def fetchjoin_str_an(self, a: Bat, strs, width: int, aoid=16089):
         """fetchjoinAN with a string tail (matchjoinAN.tcc:304-354): the
@@ -305,22 +411,21 @@ class GpuOps:
         count = strs.numel() // width
         torch.cuda.current_stream().synchronize()  # the library launches on its own stream
         cap = max(a.count, 1)
-        ecap = min(cap, 1 << 16)
+        ecaps = [min(cap, _ERR_ROWS)] * 2
         while True:
             out = torch.empty(cap * width + 1, dtype=torch.uint8, device="cuda")
             n = ctypes.c_uint64(0)
-            errs = _Errs(torch, 2, ecap)
+            errs = _Errs(self, ecaps)
             rc = self.lib.ahead_gpu_fetchjoin_str_an(self.ctx, ctypes.byref(_in_bat(a)), ctypes.c_void_p(strs.data_ptr()),
                                                      ctypes.c_uint64(width), ctypes.c_uint64(count),
                                                      ctypes.c_uint64(aoid), ctypes.c_void_p(out.data_ptr()),
                                                      ctypes.c_uint64(cap), ctypes.byref(n), errs.c)
-            need_e = errs.need()
-            if rc == CAPACITY or need_e > ecap:
-                cap, ecap = max(cap, int(n.value), 1), max(ecap, need_e)
+            if rc == CAPACITY or errs.short():
+                cap, ecaps = max(cap, int(n.value), 1), errs.grown()
                 continue
             self._check(rc, "fetchjoinAN(str)")
             k = int(n.value)
-            return out[: k * width].view(k, width).clone(), errs.vecs()
+            return self._result(out, k * width).view(k, width), errs.vecs(self)
 
     def groupby2_str_an(self, strs, width: int, grouping: Bat, ngroups: int, aoid=65117,
                         aoidinv=0x3E36D3BC8D9BC5F5, seqbase: int = 0) -> Tuple[Bat, Bat, List[ErrVec]]:
@@ -341,7 +446,7 @@ class GpuOps:
                                                       ctypes.c_uint64(aoidinv), ctypes.byref(outs[0].c),
                                                       ctypes.byref(outs[1].c), ctypes.c_uint64(outs[0].cap), errs.c)
         outs, errs = self._run("groupbyAN2(str)", call, count, 3, nout=2)
-        return outs[0].bat(), outs[1].bat(), errs.vecs()
+        return outs[0].bat(self.torch), outs[1].bat(self.torch), errs.vecs(self)
 
     def fetchjoin_str(self, a: Bat, strs, width: int):
         """fetchjoin over a string tail (Normal/matchjoin.tcc:144-160): the
@@ -363,7 +468,7 @@ class GpuOps:
                 continue
             self._check(rc, "fetchjoin(str)")
             k = int(n.value)
-            return out[: k * width].view(k, width).clone()
+            return self._result(out, k * width).view(k, width)
 
     def groupby2_str(self, strs, width: int, grouping: Bat, ngroups: int, seqbase: int = 0) -> Tuple[Bat, Bat]:
         """groupby binary over a string tail (Normal/groupby.tcc:85-121)."""
@@ -380,7 +485,7 @@ class GpuOps:
                                                    ctypes.byref(outs[0].c), ctypes.byref(outs[1].c),
                                                    ctypes.c_uint64(outs[0].cap))
         outs, _ = self._run("groupby2(str)", call, count, 0, nout=2)
-        return outs[0].bat(), outs[1].bat()
+        return outs[0].bat(self.torch), outs[1].bat(self.torch)
 
     # -- check / decode
     def check_an(self, b: Bat, ainv, unenc_max, aoid=16089) -> ErrVec:
@@ -390,7 +495,7 @@ class GpuOps:
                                                ctypes.c_uint64(unenc_max), ctypes.c_uint64(aoid),
                                                ctypes.byref(errs.c[0]))
         _, errs = self._run("checkAN", call, b.count, 1, nout=0)
-        return errs.vecs()[0]
+        return errs.vecs(self)[0]
 
     def decode_an(self, b: Bat, aoid=16089) -> Tuple[Bat, ErrVec]:
         def call(outs, errs):
@@ -399,7 +504,7 @@ class GpuOps:
                                                 ctypes.byref(outs[0].c), ctypes.c_uint64(outs[0].cap),
                                                 ctypes.byref(errs.c[0]))
         outs, errs = self._run("decodeAN", call, b.count, 1)
-        return outs[0].bat(), errs.vecs()[0]
+        return outs[0].bat(self.torch), errs.vecs(self)[0]
 
     def check_and_decode_an(self, b: Bat, aoid=16089) -> Tuple[Bat, ErrVec, ErrVec]:
         def call(outs, errs):
@@ -408,8 +513,8 @@ class GpuOps:
                                                           ctypes.byref(outs[0].c), ctypes.c_uint64(outs[0].cap),
                                                           ctypes.byref(errs.c[0]), ctypes.byref(errs.c[1]))
         outs, errs = self._run("checkAndDecodeAN", call, b.count, 2)
-        v = errs.vecs()
-        return outs[0].bat(), v[0], v[1]
+        v = errs.vecs(self)
+        return outs[0].bat(self.torch), v[0], v[1]
 
     def encode_an(self, b: Bat, A) -> Bat:
         def call(outs, errs):
@@ -417,7 +522,7 @@ class GpuOps:
             return self.lib.ahead_gpu_encode_an(self.ctx, ctypes.byref(cb), ctypes.c_uint64(A),
                                                 ctypes.byref(outs[0].c), ctypes.c_uint64(outs[0].cap))
         outs, _ = self._run("encodeAN", call, b.count, 0)
-        return outs[0].bat()
+        return outs[0].bat(self.torch)
 
     # -- joins
     def hashjoin_an(self, l: Bat, r: Bat, reenc_head=False, ah1r=1, ah1invr=1, reenc_tail=False, at2r=1,
@@ -429,16 +534,17 @@ class GpuOps:
                                                   ctypes.c_uint64(at2r), ctypes.c_uint64(at2invr), side,
                                                   ctypes.c_uint64(aoid), ctypes.byref(outs[0].c),
                                                   ctypes.c_uint64(outs[0].cap), errs.c)
-        outs, errs = self._run("hashjoinAN", call, max(l.count, r.count), 4)
-        return outs[0].bat(), errs.vecs()
+        outs, errs = self._run("hashjoinAN", call, max(l.count, r.count), 4, sized=True,
+                               cols=((l.head, l.count), (l.tail, l.count), (r.head, r.count), (r.tail, r.count)))
+        return outs[0].bat(self.torch), errs.vecs(self)
 
     def hashjoin(self, l: Bat, r: Bat, side=1) -> Bat:
         def call(outs, errs):
             cl, cr = _in_bat(l), _in_bat(r)
             return self.lib.ahead_gpu_hashjoin(self.ctx, ctypes.byref(cl), ctypes.byref(cr), side,
                                                ctypes.byref(outs[0].c), ctypes.c_uint64(outs[0].cap))
-        outs, _ = self._run("hashjoin", call, max(l.count, r.count), 0)
-        return outs[0].bat()
+        outs, _ = self._run("hashjoin", call, max(l.count, r.count), 0, sized=True)
+        return outs[0].bat(self.torch)
 
     def matchjoin_an(self, a: Bat, b: Bat, reenc=False, ah1r=0, ah1invr=0, at2r=0, at2invr=0,
                      aoid=16089) -> Tuple[Bat, List[ErrVec]]:
@@ -449,17 +555,23 @@ class GpuOps:
                                                    ctypes.c_uint64(at2r), ctypes.c_uint64(at2invr),
                                                    ctypes.c_uint64(aoid), ctypes.byref(outs[0].c),
                                                    ctypes.c_uint64(outs[0].cap), errs.c)
-        # at most one output row per row of the smaller input (a retry covers the rest)
-        outs, errs = self._run("matchjoinAN", call, max(min(a.count, b.count), 1), 4)
-        return outs[0].bat(), errs.vecs()
+        # a positional join keeps at most its list's rows, a merge of ordered inputs
+        # the smaller input's (a retry covers the rest)
+        positional = b.head.type == VOID and a.tail.type != VOID
+        cap = a.count if positional else min(a.count, b.count)
+        outs, errs = self._run("matchjoinAN", call, max(cap, 1), 4, sized=b.head.type != VOID,
+                               cols=((a.head, a.count), (a.tail, a.count), (b.head, b.count), (b.tail, b.count)))
+        return outs[0].bat(self.torch), errs.vecs(self)
 
     def matchjoin(self, a: Bat, b: Bat) -> Bat:
         def call(outs, errs):
             ca, cb = _in_bat(a), _in_bat(b)
             return self.lib.ahead_gpu_matchjoin(self.ctx, ctypes.byref(ca), ctypes.byref(cb),
                                                 ctypes.byref(outs[0].c), ctypes.c_uint64(outs[0].cap))
-        outs, _ = self._run("matchjoin", call, max(a.count, b.count), 0)
-        return outs[0].bat()
+        positional = b.head.type == VOID and a.tail.type != VOID
+        cap = a.count if positional else max(a.count, b.count)
+        outs, _ = self._run("matchjoin", call, max(cap, 1), 0, sized=b.head.type != VOID)
+        return outs[0].bat(self.torch)
 
     def fetchjoin_an(self, a: Bat, b: Bat, reenc=False, atr=1, atrinv=1, aoid=16089) -> Tuple[Bat, List[ErrVec]]:
         def call(outs, errs):
@@ -468,8 +580,8 @@ class GpuOps:
                                                    ctypes.c_uint64(atr), ctypes.c_uint64(atrinv),
                                                    ctypes.c_uint64(aoid), ctypes.byref(outs[0].c),
                                                    ctypes.c_uint64(outs[0].cap), errs.c)
-        outs, errs = self._run("fetchjoinAN", call, a.count, 2)
-        return outs[0].bat(), errs.vecs()
+        outs, errs = self._run("fetchjoinAN", call, a.count, 2, cols=((a.tail, 0), (b.tail, a.count)))
+        return outs[0].bat(self.torch), errs.vecs(self)
 
     def fetchjoin(self, a: Bat, b: Bat) -> Bat:
         def call(outs, errs):
@@ -477,7 +589,7 @@ class GpuOps:
             return self.lib.ahead_gpu_fetchjoin(self.ctx, ctypes.byref(ca), ctypes.byref(cb),
                                                 ctypes.byref(outs[0].c), ctypes.c_uint64(outs[0].cap))
         outs, _ = self._run("fetchjoin", call, a.count, 0)
-        return outs[0].bat()
+        return outs[0].bat(self.torch)
 
     # -- grouping and aggregation
     def groupby_an(self, b: Bat, aoid=65117, aoidinv=0x3E36D3BC8D9BC5F5) -> Tuple[Bat, Bat, List[ErrVec]]:
@@ -487,7 +599,7 @@ class GpuOps:
                                                  ctypes.c_uint64(aoidinv), ctypes.byref(outs[0].c),
                                                  ctypes.byref(outs[1].c), ctypes.c_uint64(outs[0].cap), errs.c)
         outs, errs = self._run("groupbyAN", call, b.count, 2, nout=2)
-        return outs[0].bat(), outs[1].bat(), errs.vecs()
+        return outs[0].bat(self.torch), outs[1].bat(self.torch), errs.vecs(self)
 
     def groupby2_an(self, b: Bat, grouping: Bat, ngroups: int, aoid=65117,
                     aoidinv=0x3E36D3BC8D9BC5F5) -> Tuple[Bat, Bat, List[ErrVec]]:
@@ -498,7 +610,7 @@ class GpuOps:
                                                   ctypes.c_uint64(aoidinv), ctypes.byref(outs[0].c),
                                                   ctypes.byref(outs[1].c), ctypes.c_uint64(outs[0].cap), errs.c)
         outs, errs = self._run("groupbyAN2", call, b.count, 3, nout=2)
-        return outs[0].bat(), outs[1].bat(), errs.vecs()
+        return outs[0].bat(self.torch), outs[1].bat(self.torch), errs.vecs(self)
 
     def aggregate_sum_grouped_an(self, b: Bat, grouping: Bat, ngroups: int, result_type=9, ar=65117,
                                  arinv=0x3E36D3BC8D9BC5F5, aoid=65117) -> Tuple[Bat, List[ErrVec]]:
@@ -510,7 +622,7 @@ class GpuOps:
                                                                ctypes.c_uint64(aoid), ctypes.byref(outs[0].c),
                                                                errs.c)
         outs, errs = self._run("aggregate_sum_groupedAN", call, max(b.count, ngroups, 1), 3)
-        return outs[0].bat(), errs.vecs()
+        return outs[0].bat(self.torch), errs.vecs(self)
 
     def aggregate_mul_sum_an(self, a: Bat, b: Bat, result_type=9, init=0, ra=65117,
                              rainv=0x3E36D3BC8D9BC5F5, aoid=16089) -> Tuple[int, List[ErrVec]]:
@@ -523,7 +635,7 @@ class GpuOps:
                                                            ctypes.c_uint64(rainv), ctypes.c_uint64(aoid),
                                                            ctypes.byref(tot), errs.c)
         _, errs = self._run("aggregate_mul_sumAN", call, max(a.count, b.count), 2, nout=0)
-        return int(tot.value), errs.vecs()
+        return int(tot.value), errs.vecs(self)
 
     def aggregate_mul_sum(self, a: Bat, b: Bat, result_type=4, init=0) -> int:
         tot = ctypes.c_uint64(0)
@@ -540,7 +652,7 @@ class GpuOps:
             return self.lib.ahead_gpu_groupby(self.ctx, ctypes.byref(cb), ctypes.byref(outs[0].c),
                                               ctypes.byref(outs[1].c), ctypes.c_uint64(outs[0].cap))
         outs, _ = self._run("groupby", call, b.count, 0, nout=2)
-        return outs[0].bat(), outs[1].bat()
+        return outs[0].bat(self.torch), outs[1].bat(self.torch)
 
     def groupby2(self, b: Bat, grouping: Bat, ngroups: int) -> Tuple[Bat, Bat]:
         def call(outs, errs):
@@ -549,7 +661,7 @@ class GpuOps:
                                                ctypes.byref(outs[0].c), ctypes.byref(outs[1].c),
                                                ctypes.c_uint64(outs[0].cap))
         outs, _ = self._run("groupby2", call, b.count, 0, nout=2)
-        return outs[0].bat(), outs[1].bat()
+        return outs[0].bat(self.torch), outs[1].bat(self.torch)
 
     def aggregate_sum_grouped(self, b: Bat, grouping: Bat, ngroups: int, result_type=4) -> Bat:
         def call(outs, errs):
@@ -558,7 +670,7 @@ class GpuOps:
                                                             ctypes.c_uint64(ngroups), result_type,
                                                             ctypes.byref(outs[0].c))
         outs, _ = self._run("aggregate_sum_grouped", call, max(ngroups, 1), 0)
-        return outs[0].bat()
+        return outs[0].bat(self.torch)
 
     def aggregate_sum(self, b: Bat, result_type=4) -> int:
         tot = ctypes.c_uint64(0)
@@ -573,7 +685,7 @@ class GpuOps:
             return self.lib.ahead_gpu_arithmetic(self.ctx, op, result_type, ctypes.byref(ca), ctypes.byref(cb),
                                                  ctypes.byref(outs[0].c))
         outs, _ = self._run("arithmetic", call, max(a.count, 1), 0)
-        return outs[0].bat()
+        return outs[0].bat(self.torch)
 
     def arithmetic_an(self, op, result_type, a: Bat, b: Bat, ar, arinv, aoid=16089) -> Tuple[Bat, List[ErrVec]]:
         def call(outs, errs):
@@ -582,4 +694,4 @@ class GpuOps:
                                                     ctypes.c_uint64(ar), ctypes.c_uint64(arinv),
                                                     ctypes.c_uint64(aoid), ctypes.byref(outs[0].c), errs.c)
         outs, errs = self._run("arithmeticAN", call, max(a.count, 1), 4)
-        return outs[0].bat(), errs.vecs()
+        return outs[0].bat(self.torch), errs.vecs(self)

@@ -54,6 +54,19 @@ uint64_t ahead_ctx_launches(ahead_ctx* ctx);
  * the first operator that needed scratch). */
 uint64_t ahead_ctx_scratch_bytes(ahead_ctx* ctx);
 const char* ahead_status_string(int status);
+/* Output columns of exactly the size a call needs: with a function set, a call
+ * of ahead_gpu_select(_an), ahead_gpu_hashjoin(_an) or ahead_gpu_matchjoin(_an)
+ * that passes cap = AHEAD_SIZED and null output data counts its rows first,
+ * then asks the function for each output column it fills (column 0: head, 1:
+ * tail; device memory, 16-byte aligned, NULL: AHEAD_NO_MEMORY), and stores the
+ * pointers in `out`.  A call whose inputs need another path (repeated join
+ * keys, unordered merge inputs, positional joins) returns AHEAD_CAPACITY with
+ * the exact count instead and has written no rows.  The function runs on the
+ * calling thread, during the call.  No reference counterpart: its operators
+ * grow vectors. */
+#define AHEAD_SIZED UINT64_MAX
+typedef void* (*ahead_output_fn)(void* user, int column, uint64_t bytes);
+void ahead_ctx_set_output_fn(ahead_ctx* ctx, ahead_output_fn fn, void* user);
 
 /* ------------------------------------------------------------- selection */
 /* selectAN<Op>(arg, th, AOID) and selectAN<Op1,Op2,Comb>(arg, th1, th2, AOID)
