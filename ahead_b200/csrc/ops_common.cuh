@@ -274,17 +274,20 @@ static __global__ void __launch_bounds__(1024) sort_drops_kernel(const uint64_t*
     }
 }
 
-// Moves the rows of one or two columns down over the k dropped ones, in place.
-// A chunk of 2048 rows (4096 of up to 4 bytes) moves by at most k of its rows:
-// the rows whose place lies in their own chunk go there directly, once all of
-// the chunk is in registers; the few that go to the chunk before wait in `edge`
-// (k per chunk) for shift_edges_kernel.  Together they read and write each row
-// behind the first dropped one once.  A chunk's loads are issued before it looks
-// for its place in the list, which the whole block does with one load per entry.
-// 60M 4-byte values move in 88 us (480 MB, 5.5 TB/s); with a binary search ahead
-// of the loads, or the rows spilled to local memory, it took 106 and 141.
+// Moves the rows of one or two columns (4-byte aligned) down over the k dropped
+// ones, in place.  A chunk of 16 KB moves by at most k of its rows: the rows
+// whose place lies in their own chunk go there directly, once all of the chunk
+// has been read; the few that go to the chunk before wait in `edge` (k per chunk)
+// for shift_edges_kernel.  Together they read and write each row behind the first
+// dropped one once.  A chunk's loads are issued before it looks for its place in
+// the list, which the whole block does with one load per entry.  1- and 2-byte
+// rows are read and written as words shifted to their place: 150M 2-byte values
+// move in 76 us (600 MB; checkAndDecodeAN with 3 flips, from 459 us with a row at
+// a time and a result copied to its size to 313).  60M 4-byte values move in 88 us
+// (480 MB, 5.5 TB/s); with a binary search ahead of the loads, or the rows spilled
+// to local memory, it took 106 and 141.
 constexpr uint32_t kShiftChunk = 2048;
-constexpr uint32_t shift_chunk(int w) { return w == 8 ? kShiftChunk : 2 * kShiftChunk; }
+constexpr uint32_t shift_chunk(int w) { return kShiftChunk * (8 / w); }
 
 template <int W>
 struct UIntOf {
@@ -314,11 +317,56 @@ __global__ void __launch_bounds__(256, 8) shift_rows_kernel(ShiftCols s) {
     typedef typename UIntOf<W>::type T;
     constexpr uint32_t C = shift_chunk(W);
     constexpr uint32_t U = C / 256;
-    __shared__ T s_v[C];
     const int col = blockIdx.y;
     const uint64_t c0 = (uint64_t)blockIdx.x * C;
     T* p = (T*)(col ? s.data[1] : s.data[0]) + c0;
     const uint32_t m = s.n - c0 < C ? (uint32_t)(s.n - c0) : C, t = threadIdx.x;
+    if constexpr (W < 4) {  // (by words: a row at a time is as many loads and stores of a quarter or half of the bytes)
+        constexpr uint32_t P = 4 / W, UW = C / P / 256;
+        __shared__ __align__(16) uint32_t s_w[C / P + 1];
+        uint32_t x[UW];
+#pragma unroll
+        for (uint32_t u = 0; u < UW; ++u) {
+            const uint32_t r = (u * 256 + t) * P;
+            x[u] = 0;
+            if (r + P <= m) {
+                x[u] = reinterpret_cast<const uint32_t*>(p)[u * 256 + t];
+            } else {
+                for (uint32_t i = 0; r + i < m; ++i) x[u] |= (uint32_t)p[r + i] << (8 * W * i);
+            }
+        }
+        uint32_t lo = 0, hi = 0;
+        for (uint32_t i0 = 0; i0 < s.k; i0 += 256) {
+            const uint64_t r = i0 + t < s.k ? __ldg((const unsigned long long*)s.sorted + i0 + t) : ~0ull;
+            lo += __syncthreads_count(r < c0);
+            hi += __syncthreads_count(r < c0 + m);
+        }
+        if (hi == 0) return;
+#pragma unroll
+        for (uint32_t u = 0; u < UW; ++u) s_w[u * 256 + t] = x[u];
+        if (t == 0) s_w[C / P] = 0;
+        __syncthreads();
+        const T* s_r = reinterpret_cast<const T*>(s_w);
+        T* e = (T*)(col ? s.edge[1] : s.edge[0]) + (uint64_t)blockIdx.x * s.k;
+        if (lo == hi) {
+            for (uint32_t r = t; r < lo && r < m; r += 256) e[lo - 1 - r] = s_r[r];
+            const uint32_t left = m > lo ? m - lo : 0, by = lo % P;  // rows that stay in the chunk
+            for (uint32_t j = t; j < left / P; j += 256) {
+                const uint32_t at = j + lo / P;
+                reinterpret_cast<uint32_t*>(p)[j] = __funnelshift_r(s_w[at], s_w[at + 1], 8 * W * by);
+            }
+            for (uint32_t r = (left / P) * P + t; r < left; r += 256) p[r] = s_r[lo + r];
+            return;
+        }
+        for (uint32_t r = t; r < m; r += 256) {
+            const uint32_t d = drops_below(s.sorted, lo, hi, c0 + r);
+            if (d < hi && __ldg((const unsigned long long*)s.sorted + d) == c0 + r) continue;
+            if (r >= d) p[r - d] = s_r[r];
+            else e[d - 1 - r] = s_r[r];
+        }
+        return;
+    }
+    __shared__ T s_v[W < 4 ? 1 : C];
     typename std::conditional<W == 8, uint64_t, uint32_t>::type v[U];
     if (m == C) {
 #pragma unroll

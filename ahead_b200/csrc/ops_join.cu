@@ -768,6 +768,7 @@ constexpr int kPosHead = 30, kPosDrops = 31, kPosCounters = 33;  // counters
 template <bool CHECKED, bool FETCH>
 int run_pos_join(OpScope& s, PosArgs& a, const ahead_col* head, uint64_t aoid, bool dense_head, ahead_errvec* eh,
                  ahead_errvec* e0, ahead_errvec* e1, uint64_t* kept) {
+    if (((uintptr_t)a.oh | (uintptr_t)a.ot) & 3) return AHEAD_UNSUPPORTED;  // (narrow gaps are closed by words)
     const uint64_t n = a.n;
     const size_t check = a.head_err ? colcheck_scratch(n) : 0;
     int rc = s.reserve(drop_scratch(n, (FETCH ? 0 : a.ohw) + a.otw) + kErrListBytes + check);

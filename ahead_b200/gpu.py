@@ -286,7 +286,7 @@ class GpuOps:
         self.lib.ahead_ctx_set_output_fn(self.ctx, self._output_fn, None)
 
     def _run(self, what, call, cap: int, nerr: int, nout: int = 1, tail: bool = True, sized: bool = False,
-             cols=()):
+             cols=(), sized_bytes: int = _SIZED_BYTES):
         """Run an operator with outputs of `cap` rows (sized: allocated by the
         call when they may be large) and error vectors of a small first
         capacity, or of all rows for the checked columns `cols` ((column, rows)
@@ -299,7 +299,7 @@ class GpuOps:
         for i, (c, rows) in enumerate(cols):
             if rows > few and _dense(c):
                 ecaps[i] = int(rows)
-        sized = sized and cap * 8 >= _SIZED_BYTES
+        sized = sized and cap * 8 >= sized_bytes
         while True:
             outs = [_Out(torch, cap, tail, sized) for _ in range(nout)]
             errs = _Errs(self, ecaps) if nerr else None
@@ -512,7 +512,9 @@ class GpuOps:
             return self.lib.ahead_gpu_check_and_decode_an(self.ctx, ctypes.byref(cb), ctypes.c_uint64(aoid),
                                                           ctypes.byref(outs[0].c), ctypes.c_uint64(outs[0].cap),
                                                           ctypes.byref(errs.c[0]), ctypes.byref(errs.c[1]))
-        outs, errs = self._run("checkAndDecodeAN", call, b.count, 2)
+        # (buffers of the values' width: narrow ones would be moved out of wide ones)
+        outs, errs = self._run("checkAndDecodeAN", call, b.count, 2, sized=True,
+                               sized_bytes=_KEEP_BYTES if WIDTH[b.tail.type] <= 4 else _SIZED_BYTES)
         v = errs.vecs(self)
         return outs[0].bat(self.torch), v[0], v[1]
 

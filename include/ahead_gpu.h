@@ -61,9 +61,10 @@ const char* ahead_status_string(int status);
  * tail; device memory, 16-byte aligned, NULL: AHEAD_NO_MEMORY), and stores the
  * pointers in `out`.  A call whose inputs need another path (repeated join
  * keys, unordered merge inputs, positional joins) returns AHEAD_CAPACITY with
- * the exact count instead and has written no rows.  The function runs on the
- * calling thread, during the call.  No reference counterpart: its operators
- * grow vectors. */
+ * the exact count instead and has written no rows.
+ * ahead_gpu_check_and_decode_an asks for columns of its input's length.  The
+ * function runs on the calling thread, during the call.  No reference
+ * counterpart: its operators grow vectors. */
 #define AHEAD_SIZED UINT64_MAX
 typedef void* (*ahead_output_fn)(void* user, int column, uint64_t bytes);
 void ahead_ctx_set_output_fn(ahead_ctx* ctx, ahead_output_fn fn, void* user);
