@@ -27,8 +27,8 @@
 //     fact kernel, a finalize kernel (per query the non-empty groups sorted
 //     by first row) and a pack kernel (sorts the error log and packs errors
 //     and groups into one contiguous result area).  Every launch reads the
-//     batch descriptor from device memory, so one captured graph per slot
-//     serves every batch;
+//     batch descriptor from device memory, so one captured graph per slot and
+//     launch sequence (sj_kind) serves every batch;
 //   - the fact kernel: a persistent grid; each thread owns 8 rows of a
 //     2048-row tile and walks the dimensions in stages (all 8 rows' loads of
 //     a stage are in flight together); a foreign key is loaded only while some
@@ -104,6 +104,7 @@ struct SjDimDev {
     uint64_t cmagic;
     const unsigned long long* acc;  // [kAccEntries] accept masks by record
     uint64_t fk_ainv, kmin, krange;
+    uint32_t fk_a, pad_a;           // the multiplier A = (A^-1)^-1 mod 2^32
     unsigned long long joins, first;  // queries joining / joining first
     // join index slot of this dimension (1 or 2: the first or second word of
     // a fact row's entry; 0: not indexed), read by the indexed cube scans
@@ -143,14 +144,16 @@ struct SjHdr {
     unsigned long long raw[kMaxQ];      // ungrouped queries: sum of code products
     unsigned long long nonempty[4];     // per dimension: queries accepting >= 1 row
     unsigned long long errcnt, status, exccnt, unseen;
-    unsigned long long fkept;  // rows the fact-predicate prefilter kept
+    unsigned long long fkept;  // the prefilter's list: entries taken, chunk ends included
+    unsigned long long rkept;  // the same for the refining pass's
+    unsigned long long fbad;  // rows with a corrupt code the filters met
     // groups per query (counted by the compact kernel); ~0: the packed area
     // could not take them  (zeroed by the clear kernel up to here)
     unsigned long long ngroups[kMaxQ];
     unsigned long long off[kMaxQ];      // offset of each query's groups in packed
     unsigned long long nerr, packed_len;  // sorted errors at packed[0, nerr); words used
 };
-constexpr int kHdrClearWords = kMaxQ + 4 + 5 + kMaxQ;
+constexpr int kHdrClearWords = kMaxQ + 4 + 5 + 1 + 1 + kMaxQ;
 
 struct SjBatch {
     SjDimDev dim[4];
@@ -224,17 +227,26 @@ struct SjBatch {
     const unsigned long long* facc;
     const RangePred* fpr;  // [query * 2 + c] the predicates themselves, for corrupt codes
     unsigned long long fq[2], mrev, mprof;
-    // the prefilter (per-row strategy): flist_on 1 -- every query has a fact
-    // predicate: the rows a query's predicates can keep, or whose fact codes
-    // are corrupt; 2 -- no query has one and every query joins dimension
-    // flist_dim first: the rows that dimension accepts for a query, or whose
-    // foreign key is corrupt.  In flist[0, fkept) when they fit flist_cap.
-    uint32_t* flist;
-    uint64_t flist_cap;
-    uint32_t flist_on, flist_dim;
-    // flist_on 2: bit k set when some query of the batch accepts key offset k
-    // of dimension flist_dim (null: the prefilter reads the masks themselves)
-    uint32_t* pfmap;
+    // the row lists (per-row strategy).  flist_on 1: every query has a fact
+    // predicate; flist[0] holds the rows whose quantity and discount pass some
+    // query's; 2: no query has one and every query joins dimension flist_dim
+    // first; flist[0] holds the rows whose key that dimension accepts for some
+    // query.  In both, only those whose key the next dimension flist_next (4:
+    // none) accepts as well; flist[1]: of those (ref_on) the rows whose key
+    // ref_dim accepts, too (every query joins these two, in join order).  fbad:
+    // the rows with a corrupt code that a filter met (the per-row pass reports
+    // them).
+    uint32_t* flist[2];
+    uint64_t flist_cap[2];
+    uint32_t* fbad;
+    uint32_t flist_on, flist_dim, flist_next;
+    uint32_t ref_on, ref_dim, flist_pad;
+    uint32_t flist_chunk[2];  // entries a warp takes of a list at a time
+    // bit k set when some query of the batch accepts key offset k of the dimension;
+    // the words of it that the filters hold: the map itself, or a bit per 2^pffold keys
+    uint32_t* pfmap[4];
+    uint32_t* pfsmall[4];
+    uint32_t pffold[4], pfwords[4];
 };
 static_assert(sizeof(SjBatch) % 8 == 0, "SjBatch is copied in 8-byte words");
 static_assert(sizeof(SjQDev) % 8 == 0, "SjQDev is copied in 8-byte words");
@@ -256,267 +268,489 @@ __device__ __forceinline__ uint32_t pick4(uint32_t a0, uint32_t a1, uint32_t a2,
     return d == 0 ? a0 : d == 1 ? a1 : d == 2 ? a2 : a3;
 }
 
-// The prefilter of a per-row batch (SjBatch::flist_on), appending to flist --
-// in no particular order: the per-row pass adds sums, lowers first rows and
-// logs errors, none of which depends on row order -- the rows that pass:
-//  1: every query has a fact predicate: the rows that some query's selectAN on
-//     quantity / discount keeps, or whose code of such a column is corrupt (the
-//     per-row pass reports it, and selects the row when the code itself passes);
-//  2: no query has one, and every query joins dimension flist_dim first: the
-//     rows whose foreign key that dimension accepts for some query (the accept
-//     masks of the batch's accept pass), or whose foreign key is corrupt (the
-//     first join reports it).
-// Any other row is rejected by every query before anything is reported, so it
-// joins nothing and reports nothing.  Its cost is a column or two per row,
-// instead of the per-row pass's ~110 instructions for a rejected row.
-constexpr int kPfRows = 16;  // rows per thread and tile
+// The row lists of a per-row batch (SjBatch::flist_on): the prefilter scans the
+// rows for those that can matter, and a refining pass drops the ones a third
+// dimension rejects, so that the per-row pass -- about 110 instructions and several
+// dependent gathers a row -- walks only rows that pass every filtered join.
+// Lists are in no particular order: the per-row pass adds sums, lowers first
+// rows and logs errors, none of which depends on row order.
+//  - prefilter, fact predicates (flist_on 1): the rows that some query's selectAN
+//    on quantity / discount keeps;
+//  - prefilter, first join (2): the rows whose foreign key dimension flist_dim
+//    accepts for some query (every query joins it first);
+//  - of either, those whose key the next dimension flist_next accepts, too;
+//  - refining pass: the listed rows whose key dimension ref_dim accepts.
+//    The dimensions go in join order and every query joins each: a row that a
+//    dimension rejects for all queries joins nothing after it and reports
+//    nothing after it.
+// A row whose code is corrupt at any of these goes to `fbad` instead: the
+// per-row pass reports it, with whatever else it finds there.  Being listed
+// promises nothing: the per-row pass evaluates a listed row from the start,
+// each query for itself and its own prefix.
 constexpr uint64_t kFlistMaxRows = 1ull << 28;  // the row list's capacity (1 GiB); more kept rows: every row is scanned
+constexpr uint64_t kFbadCap = 1u << 20;
 // the first-join prefilter runs when the rows its dimension accepts are
-// expected (uniform attribute values) to be at most this share of the rows
+// expected (uniform attribute values) to be at most this share of the rows, a
+// further filter when they are at most that share of the rows left
 constexpr double kPrefilterMaxShare = 0.25;
+constexpr double kRefineMaxShare = 0.5;
+// rows from which the lists are made (single programs over 1.2M rows: 134-174 us
+// without, 151-188 with; over 4M: 160-253 and 159-220), and listed rows from
+// which a third filter runs (each pass first copies up to 208 KB of a map)
+constexpr uint64_t kListMinRows = 1ull << 21;
+constexpr double kRefineMinRows = 1 << 19;
+// words of shared memory for the accepted keys' bitmaps (1.7M keys), or for the
+// fact predicates' table and one bitmap
+constexpr uint32_t kPfSmem = 208 * 1024, kPfRoom = kPfSmem / 4, kFactWords = 256 * 256 / 32;
+// list entries a warp takes at a time: about a sixteenth of what it is expected
+// to list in all (fewer atomics on one word), and no more than is worth skipping
+constexpr uint32_t kListChunk = 512, kListChunkMin = 64;
 
-// Each thread takes a run of kPfRows consecutive rows of a tile: one 16-byte
-// load per 8 two-byte codes or 2 foreign-key codes, all of a run's loads (and
-// then all of its record and mask gathers) in flight together.  One row per
-// thread and step had kept a few bytes per thread in flight and ran at a
-// fifth of the copy bandwidth.
-__device__ __forceinline__ void pf_load16(const uint16_t* __restrict__ col, uint64_t r0, uint64_t nmax, bool vec,
-                                          uint32_t (&w)[kPfRows / 2]) {
-    static_assert(kPfRows % 8 == 0, "runs of whole 16-byte words");
-    if (vec && r0 + kPfRows <= nmax) {
-        const uint4* p = reinterpret_cast<const uint4*>(col + r0);
-#pragma unroll
-        for (int k = 0; k < kPfRows / 8; ++k) {
-            const uint4 x = __ldg(p + k);
-            w[4 * k] = x.x;
-            w[4 * k + 1] = x.y;
-            w[4 * k + 2] = x.z;
-            w[4 * k + 3] = x.w;
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < kPfRows / 2; ++k) {
-            const uint64_t r = r0 + 2 * k;
-            const uint32_t lo = r < nmax ? __ldg(col + r) : 0u, hi = r + 1 < nmax ? __ldg(col + r + 1) : 0u;
-            w[k] = lo | hi << 16;
-        }
-    }
+// One step of folding: bit i of the result is set when bit 2i or 2i + 1 of x is.
+AHEAD_DEV uint32_t fold_bits(uint32_t x) {
+    x = (x | (x >> 1)) & 0x55555555u;
+    x = (x | (x >> 1)) & 0x33333333u;
+    x = (x | (x >> 2)) & 0x0f0f0f0fu;
+    x = (x | (x >> 4)) & 0x00ff00ffu;
+    return (x | (x >> 8)) & 0xffffu;
 }
 
-// The first-join prefilter's accepted keys (flist_on 2): bit k of pfmap set
-// when the batch's accept mask of key offset k of dimension flist_dim is not
-// empty -- by key offset in row mode, else through the key's record.  One bit
-// a key keeps the table in L1 (supplier: 25 KB at 2M rows; customer: 375 KB
-// at 3M), where the masks themselves (8 bytes a key or record, behind a 4-byte
-// record) made the prefilter one L2 request per row.
+// Bit k of a dimension's map set when the batch's accept mask of key offset k is
+// not empty -- by key offset in row mode, else through the key's record -- for
+// the dimensions the lists filter by (blockIdx.y).  And, where the map does not
+// fit the filters' shared memory, the folded map: a bit for 2^pffold keys.  A
+// warp makes four words or one folded word at a time: the masks of 128 keys are
+// in flight together.
 __global__ void sj_pfmap_kernel(const SjBatch* __restrict__ bp) {
-    if (bp->strategy != kStratRows || bp->flist_on != 2 || !bp->pfmap) return;
-    const SjDimDev& D = bp->dim[bp->flist_dim & 3];
+    const uint32_t d = blockIdx.y;
+    if (bp->strategy != kStratRows || !bp->flist_on || !bp->pfmap[d]) return;
+    const SjDimDev& D = bp->dim[d];
     const uint64_t krange = D.krange, words = krange / 32 + 1;
-    uint32_t* map = bp->pfmap;
+    const uint32_t fold = bp->pffold[d], per = 1u << fold, span = per > 4 ? per : 4;
+    uint32_t *map = bp->pfmap[d], *folded = bp->pfsmall[d];
     const int lane = threadIdx.x & 31;
     const uint64_t w0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t wstride = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t w = w0; w < words; w += wstride) {  // (warp-uniform)
-        const uint64_t k = w * 32 + lane;
-        unsigned long long m = 0;
-        if (k < krange) m = D.accr ? __ldg(D.accr + k) : __ldg(D.acc + __ldg(D.rec + k));
-        const unsigned bits = __ballot_sync(0xffffffffu, m != 0);
-        if (lane == 0) map[w] = bits;
+    for (uint64_t w = w0 * span; w < words; w += wstride * span) {  // (warp-uniform)
+        uint32_t acc = 0;
+        for (uint32_t j = 0; j < span; j += 4) {
+            uint32_t bits[4];
+            unsigned long long m[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint64_t k = (w + j + i) * 32 + lane;
+                m[i] = 0;
+                if (k < krange) m[i] = D.accr ? __ldg(D.accr + k) : __ldg(D.acc + __ldg(D.rec + k));
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) bits[i] = __ballot_sync(kFull, m[i] != 0);
+            if (lane == 0 && w + j < words)  // (a map ends on a 16-byte boundary)
+                *reinterpret_cast<uint4*>(map + w + j) = make_uint4(bits[0], bits[1], bits[2], bits[3]);
+            if (!fold) continue;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                uint32_t x = bits[i], at = (j + i) & (per - 1);
+                for (uint32_t f = 0; f < fold && f < 5; ++f) x = fold_bits(x);
+                acc |= x << (fold <= 5 ? at * (32u >> fold) : at >> (fold - 5));
+                if (at == per - 1) {
+                    if (lane == 0) folded[(w + j + i) >> fold] = acc;
+                    acc = 0;
+                }
+            }
+        }
     }
 }
 
-// 8 warps a block, at most 80 registers a thread: three blocks an SM
-__global__ void __launch_bounds__(kSjThreads, 3) sj_prefilter_kernel(const SjBatch* __restrict__ bp) {
-    __shared__ unsigned long long s_acc[512];
-    __shared__ uint64_t s_n[kMaxQ];
-    // a tile's kept rows are staged here and appended with one global atomic
-    // per tile (one per warp and row slot had serialised on the counter)
-    __shared__ uint32_t s_rows[kPfRows * kSjThreads];
-    __shared__ uint32_t s_cnt;
-    __shared__ unsigned long long s_base;
-    // fact predicates, every query alive: bit vd of word vq * 8 + vd / 32 set
-    // when a row with decoded quantity vq and discount vd passes some query
-    __shared__ uint32_t s_T[256 * 256 / 32];
+// A warp's place in a list: it takes whole chunks of entries (one atomic per
+// chunk or more, not per warp and step) and fills what it leaves of the last
+// one with kNoRow, which every reader skips.
+struct ListOut {
+    uint32_t* list;
+    uint32_t cap, chunk;  // entries; a power of two, at most kListChunk
+    unsigned long long* count;
+    uint32_t cur = 0, left = 0;
+    AHEAD_DEV ListOut(uint32_t* l, uint64_t c, uint32_t ch, unsigned long long* n)
+        : list(l), cap((uint32_t)c), chunk(ch), count(n) {}
+    // appends row(bit) for each set bit of every lane's mask
+    template <class F>
+    AHEAD_DEV void append(uint32_t mask, F row) {
+        const int lane = threadIdx.x & 31;
+        const uint32_t cnt = (uint32_t)__popc(mask), incl = warp_incl_scan(cnt);
+        const uint32_t total = __shfl_sync(kFull, incl, 31);
+        if (!total) return;
+        uint32_t next = 0, got = 0;
+        if (total > left) {
+            got = (total - left + chunk - 1) & ~(chunk - 1);
+            unsigned long long at = 0;
+            if (lane == 0) at = atomicAdd(count, (unsigned long long)got);
+            at = __shfl_sync(kFull, at, 0);
+            // (past the capacity the list is not used: its count says so)
+            next = at + got <= cap ? (uint32_t)at : kNoRow;
+        }
+        if (next != kNoRow || total <= left) {
+            uint32_t off = incl - cnt;
+            uint32_t *const here = list + cur, *const there = list + next - left;
+            for (uint32_t m = mask; m; m &= m - 1, ++off) *((off < left ? here : there) + off) = row(__ffs(m) - 1);
+        }
+        if (total > left) {
+            cur = next + (total - left);
+            left = next == kNoRow ? 0u : got - (total - left);
+        } else {
+            cur += total;
+            left -= total;
+        }
+    }
+    AHEAD_DEV void finish() {
+        for (uint32_t i = threadIdx.x & 31; i < left; i += 32) list[cur + i] = kNoRow;
+    }
+};
+
+// (rare) appends every lane's rows with a corrupt code
+template <class F>
+AHEAD_DEV void append_bad(const SjBatch* bp, uint32_t mask, F row) {
+    if (!__any_sync(kFull, mask != 0)) return;
+    const uint32_t cnt = (uint32_t)__popc(mask), incl = warp_incl_scan(cnt);
+    unsigned long long base = 0;
+    if ((threadIdx.x & 31) == 31) base = atomicAdd(&bp->hdr->fbad, (unsigned long long)incl);
+    base = __shfl_sync(kFull, base, 31) + incl - cnt;
+    for (; mask; mask &= mask - 1, ++base)
+        if (base < kFbadCap) bp->fbad[base] = row(__ffs(mask) - 1);
+}
+
+// A dimension's accepted keys, in shared memory; a bitmap that does not fit (all
+// but customer's at scale factor 100 do) folded, so that test() keeps a superset
+// and exact() asks the bitmap itself, through L2, about the few rows that every
+// other filter kept.  (Half of the lookups in L2 instead took 507 us per 100M
+// rows; a bitmap shared by two blocks of a cluster took as long.)  test() takes
+// eight codes at once: their table words are loaded together.  A code is clean
+// exactly when its low product d = c * A^-1 mod 2^32 encodes back to it (d * A =
+// c): two multiplies instead of a 64-bit one.
+struct KeyMap {
+    const uint32_t* map;
+    const uint32_t* s;  // (in shared memory)
+    uint32_t fold, kmin, krange, ainv, A;
+    // by the whole block; a barrier follows before the first test()
+    AHEAD_DEV void load(const SjBatch* bp, uint32_t d, uint32_t* to) {
+        const SjDimDev& D = bp->dim[d];
+        map = bp->pfmap[d];
+        fold = bp->pffold[d];
+        kmin = (uint32_t)D.kmin;
+        krange = (uint32_t)D.krange;
+        ainv = (uint32_t)D.fk_ainv;
+        A = D.fk_a;
+        s = to;
+        const uint32_t n = bp->pfwords[d] / 4;
+        const uint4* from = reinterpret_cast<const uint4*>(bp->pfsmall[d]);
+        for (uint32_t i = threadIdx.x; i < n; i += 4 * blockDim.x) {
+            uint4 x[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (i + k * blockDim.x < n) x[k] = __ldg(from + i + k * blockDim.x);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (i + k * blockDim.x < n) reinterpret_cast<uint4*>(to)[i + k * blockDim.x] = x[k];
+        }
+    }
+    // of the eight codes (those set in `live`), the accepted and the corrupt
+    AHEAD_DEV void test(const unsigned long long (&c)[8], uint32_t live, uint32_t& keep, uint32_t& bad) const {
+        uint32_t idx[8], word[8], in = 0, clean = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t d = (uint32_t)c[k] * ainv;
+            idx[k] = d - kmin;
+            if ((uint64_t)d * A == c[k]) {
+                clean |= 1u << k;
+                if (idx[k] < krange) in |= 1u << k;
+            }
+            idx[k] >>= fold;
+        }
+        in &= live;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            word[k] = 0;
+            if ((in >> k) & 1u) word[k] = s[idx[k] >> 5];
+        }
+        keep = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) keep |= ((word[k] >> (idx[k] & 31)) & 1u) << k;
+        bad = live & ~clean;
+    }
+    // of eight rows that test() kept, those the whole bitmap accepts
+    template <class R>
+    AHEAD_DEV uint32_t exact(const unsigned long long* fk, R row, uint32_t keep) const {
+        if (!__any_sync(kFull, keep != 0)) return 0;
+        uint32_t idx[8], out = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if ((keep >> k) & 1u) idx[k] = (uint32_t)__ldg(fk + row(k)) * ainv - kmin;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if ((keep >> k) & 1u) out |= ((__ldg(map + (idx[k] >> 5)) >> (idx[k] & 31)) & 1u) << k;
+        return out;
+    }
+};
+
+// The prefilter: one block of 32 warps per SM, so that the accepted keys' bitmaps
+// are in shared memory once per SM; a warp takes kPfGroup steps of 512 consecutive
+// rows at a time, so that a list's neighbours are a column's neighbours for the
+// passes that gather by it.  The second column is read in the same step, where the
+// first filter keeps a row of a pair: at a fifth of the rows that is most of its
+// sectors, and a pass of its own over the list took 265 us more than the 229 of
+// the first (now 410 together).  Bound by instructions and the latency of dependent
+// lookups (1.5 GB in 410 us).  Measured at 100M rows: supplier then part (200K and
+// 1.4M keys) 410 us; customer (3M keys, folded) then supplier 544; quantity and
+// discount then date 350-370.  One filter through L1, with a list tile per block,
+// took 429, 561 and 293, and left five to twenty times the rows to the per-row
+// pass: a batch took 1.22 ms (two dimensions), 1.57 (three) and 0.83 (fact
+// predicates), now 0.65, 1.01 and 0.71.
+constexpr uint64_t kPfStep = 512, kPfGroup = 8;
+__global__ void __launch_bounds__(1024, 1) sj_prefilter_kernel(const SjBatch* __restrict__ bp) {
+    extern __shared__ __align__(16) uint32_t s_map[];  // [kPfSmem / 4]: the bitmap, or the fact predicates' table
     if (__ldg(&bp->strategy) != kStratRows || !__ldg(&bp->flist_on)) return;  // (block-uniform)
-    const uint32_t nq = bp->nq;
-    for (int i = threadIdx.x; i < 512; i += blockDim.x) s_acc[i] = __ldg(bp->facc + i);
-    if (threadIdx.x < nq) s_n[threadIdx.x] = bp->q[threadIdx.x].nrows;
-    __syncthreads();
-    const unsigned long long fq0 = bp->fq[0], fq1 = bp->fq[1];
-    unsigned long long fall = 0;  // the queries with rows
-    for (uint32_t q = 0; q < nq; ++q)
-        if (s_n[q]) fall |= 1ull << q;
-    const unsigned long long A0 = fall & fq0, A1 = fall & fq1;
-    if (bp->flist_on == 1) {  // (block-uniform)
+    const int lane = threadIdx.x & 31;
+    const uint64_t nmax = bp->nmax, warps = (uint64_t)gridDim.x * 32;
+    const uint64_t whole = nmax / kPfStep, steps = (nmax + kPfStep - 1) / kPfStep;
+    // few rows: single steps, so that every warp gets some
+    const uint64_t group = steps >= 2 * kPfGroup * warps ? kPfGroup : 1;
+    uint64_t t = ((threadIdx.x >> 5) + blockIdx.x * 32ull) * group;  // this step, then the one after it
+    auto after = [&](uint64_t x) { return (x + 1) % group ? x + 1 : x + 1 + (warps - 1) * group; };
+    ListOut out(bp->flist[0], bp->flist_cap[0], bp->flist_chunk[0], &bp->hdr->fkept);
+    // the second filter: the next join's key column, read where the first one
+    // keeps a row of a 16-byte pair
+    const uint32_t d2 = bp->flist_next;
+    const bool two = d2 < 4;
+    KeyMap km2{};
+    const char* fk2 = nullptr;
+    bool vec2 = false;
+    if (two) {
+        km2.load(bp, d2, s_map + kPfRoom - bp->pfwords[d2]);
+        fk2 = reinterpret_cast<const char*>(bp->dim[d2].fk);
+        vec2 = (reinterpret_cast<uintptr_t>(fk2) & 15) == 0;
+    }
+    // of eight rows -- four pairs from pair(0..3) on -- those both filters keep
+    auto second = [&](auto pair, bool inside, uint32_t& keep, uint32_t& bad) {
+        if (!__any_sync(kFull, keep != 0)) return;
+        unsigned long long c[8];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            c[2 * s] = c[2 * s + 1] = 0;
+            if (!((keep >> (2 * s)) & 3u)) continue;
+            if (inside) {
+                uint64_t x[2];
+                unpack16<8>(Flight<8, 8>::get(fk2, pair(s), vec2), x);
+                c[2 * s] = x[0];
+                c[2 * s + 1] = x[1];
+            } else {
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    if ((keep >> (2 * s + k)) & 1u)
+                        c[2 * s + k] = __ldg(reinterpret_cast<const unsigned long long*>(fk2) + pair(s) + k);
+            }
+        }
+        uint32_t k2, b2;
+        km2.test(c, keep, k2, b2);
+        bad |= b2;
+        keep = k2;
+        if (km2.fold)
+            keep = km2.exact(reinterpret_cast<const unsigned long long*>(fk2),
+                             [&](int k) { return pair(k >> 1) + (uint64_t)(k & 1); }, keep);
+    };
+    if (bp->flist_on == 2) {
+        const uint32_t d = bp->flist_dim & 3;
+        KeyMap km;
+        km.load(bp, d, s_map);
+        __syncthreads();
+        const char* fk = reinterpret_cast<const char*>(bp->dim[d].fk);
+        const bool vec = (reinterpret_cast<uintptr_t>(fk) & 15) == 0;
+        typedef Flight<8, 8> F;  // eight rows per lane in flight: half of a step ahead
+        F f;
+        if (t < whole) f.load(fk, t * kPfStep + 2 * lane, vec);
+        for (; t < steps; t = after(t)) {
+            const uint64_t r0 = t * kPfStep + 2 * lane, next = after(t);
+            uint32_t keep = 0, bad = 0;
+            auto row = [&](int bit) { return (uint32_t)r0 + 64u * (uint32_t)(bit >> 1) + (uint32_t)(bit & 1); };
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                unsigned long long c[8];
+                uint32_t live = 0xff, k8, b8;
+                if (t < whole) {
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        uint64_t x[2];
+                        unpack16<8>(f.q[s], x);
+                        c[2 * s] = x[0];
+                        c[2 * s + 1] = x[1];
+                        if (h == 0) f.q[s] = F::get(fk, r0 + 256 + 64 * s, vec);
+                        else if (next < whole) f.q[s] = F::get(fk, next * kPfStep + 2 * lane + 64 * s, vec);
+                    }
+                } else {
+                    live = 0;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        c[k] = 0;
+                        if (row(8 * h + k) < nmax) {
+                            live |= 1u << k;
+                            c[k] = __ldg(reinterpret_cast<const unsigned long long*>(fk) + row(8 * h + k));
+                        }
+                    }
+                }
+                km.test(c, live, k8, b8);
+                if (two) second([&](int s) { return (uint64_t)row(8 * h + 2 * s); }, t < whole, k8, b8);
+                if (km.fold)
+                    k8 = km.exact(reinterpret_cast<const unsigned long long*>(fk),
+                                  [&](int k) { return row(8 * h + k); }, k8);
+                keep |= k8 << (8 * h);
+                bad |= b8 << (8 * h);
+            }
+            out.append(keep, row);
+            append_bad(bp, bad, row);
+        }
+    } else {
+        // bit vd of word vq * 8 + vd / 32: a row with decoded quantity vq and
+        // discount vd passes some query (a column no query selects on: 0)
+        __shared__ unsigned long long s_acc[512];
+        for (int i = threadIdx.x; i < 512; i += blockDim.x) s_acc[i] = __ldg(bp->facc + i);
+        __syncthreads();
+        unsigned long long fall = 0;  // the queries with rows
+        for (uint32_t q = 0; q < bp->nq; ++q)
+            if (bp->q[q].nrows) fall |= 1ull << q;
+        const unsigned long long A0 = fall & bp->fq[0], A1 = fall & bp->fq[1];
         for (int w = threadIdx.x; w < 256 * 256 / 32; w += blockDim.x) {
             const unsigned long long mq = fall & (s_acc[w >> 3] | ~A0);
             uint32_t bits = 0;
             for (int k = 0; k < 32; ++k)
                 if (mq & (s_acc[256 + (w & 7) * 32 + k] | ~A1)) bits |= 1u << k;
-            s_T[w] = bits;
+            s_map[w] = bits;
         }
         __syncthreads();
-    }
-    const uint16_t* qty = bp->qty;
-    const uint16_t* disc = bp->disc;
-    const uint32_t qa = (uint32_t)bp->qty_ainv, da = (uint32_t)bp->disc_ainv;
-    const uint64_t nmax = bp->nmax, cap = bp->flist_cap;
-    uint32_t* list = bp->flist;
-    const bool by_dim = bp->flist_on == 2;
-    const SjDimDev& D = bp->dim[bp->flist_dim & 3];
-    const unsigned long long* fk = D.fk;
-    const uint32_t* rec = D.rec;
-    const unsigned long long *dacc = D.acc, *accr = D.accr;
-    const uint64_t fk_ainv = D.fk_ainv, kmin = D.kmin, krange = D.krange;
-    const uint32_t* pfmap = bp->pfmap;
-    unsigned long long* kept = &bp->hdr->fkept;
-    const int lane = threadIdx.x & 31;
-    // 16-byte loads need 16-byte aligned columns (a run starts at a multiple of
-    // kPfRows rows); any other column is read code by code
-    const bool vec_fk = (reinterpret_cast<uintptr_t>(fk) & 15) == 0;
-    const bool vec_q = (reinterpret_cast<uintptr_t>(qty) & 15) == 0;
-    const bool vec_d = (reinterpret_cast<uintptr_t>(disc) & 15) == 0;
-    constexpr uint64_t kTile = (uint64_t)kPfRows * kSjThreads;
-    const uint64_t ntiles = (nmax + kTile - 1) / kTile;
-    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint64_t t0 = tile * kTile;
-        if (threadIdx.x == 0) s_cnt = 0;
-        __syncthreads();
-        unsigned long long full = 0, part = 0;  // queries alive for the whole tile / ending inside it
-        for (uint32_t q = 0; q < nq; ++q) {
-            if (s_n[q] >= t0 + kTile) full |= 1ull << q;
-            else if (s_n[q] > t0) part |= 1ull << q;
-        }
-        const uint64_t r0 = t0 + (uint64_t)threadIdx.x * kPfRows;  // this thread's run
-        // the queries a row of the run is alive for (recomputed where used: a
-        // run's sixteen masks would hold 32 registers)
-        auto alive = [&](int j) -> unsigned long long {
-            const uint64_t row = r0 + j;
-            if (row >= nmax) return 0ull;
-            unsigned long long m = full;
-            for (unsigned long long p = part; p; p &= p - 1) {
-                const int q = __ffsll(p) - 1;
-                if (row < s_n[q]) m |= 1ull << q;
-            }
-            return m;
+        const char* qty = reinterpret_cast<const char*>(bp->qty);
+        const char* disc = reinterpret_cast<const char*>(bp->disc);
+        const bool vq16 = (reinterpret_cast<uintptr_t>(qty) & 15) == 0, vd16 = (reinterpret_cast<uintptr_t>(disc) & 15) == 0;
+        const uint32_t qa = (uint32_t)bp->qty_ainv, da = (uint32_t)bp->disc_ainv;
+        const bool rq = A0 != 0, rd = A1 != 0;
+        // (an unread column's codes are 0: decoded 0, never corrupt)
+        auto test = [&](uint32_t q, uint32_t d, int at, uint32_t& keep, uint32_t& bad) {
+            const uint32_t v = (q * qa) & 0xffffu, w = (d * da) & 0xffffu;
+            const bool ok = (v | w) <= 0xffu;
+            const uint32_t word = s_map[ok ? (v << 3) | (w >> 5) : 0u];
+            if (ok && ((word >> (w & 31)) & 1u)) keep |= 1u << at;
+            if (!ok) bad |= 1u << at;
         };
-        uint32_t km = 0;  // bit j: row r0 + j is kept
-        if (by_dim) {
-            // the first join, as the per-row pass takes it: the truncated key
-            // probes even when corrupt, and a corrupt key is reported; the run
-            // in two halves of 8 keys (64 bytes of loads in flight a thread)
-            constexpr int kH = kPfRows / 2;
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-                const uint64_t rh = r0 + (uint64_t)h * kH;
-                unsigned long long c[kH];
-                if (vec_fk && rh + kH <= nmax) {
-                    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(fk + rh);
+        const uint4 none = make_uint4(0, 0, 0, 0);
+        uint4 fq[2] = {none, none}, fd[2] = {none, none};
+        auto load = [&](uint64_t t) {
 #pragma unroll
-                    for (int k = 0; k < kH / 2; ++k) {
-                        const ulonglong2 x = __ldg(p + k);
-                        c[2 * k] = x.x;
-                        c[2 * k + 1] = x.y;
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < kH; ++j) c[j] = rh + j < nmax ? __ldg(fk + rh + j) : 0ull;
-                }
-                uint32_t rv[kH];
-                uint32_t bad = 0;  // bit j: row rh + j's key is corrupt
-                if (pfmap) {
-                    // a key some query accepts: the row is kept for every query
-                    // alive on it (one not accepting it drops it again in the
-                    // per-row pass, which reports nothing before its first join)
-                    uint32_t sh[kH / 4] = {};  // each key's bit in its word, a byte a row
-#pragma unroll
-                    for (int j = 0; j < kH; ++j) {
-                        const uint64_t dec = c[j] * fk_ainv;
-                        const uint64_t idx = (dec & 0xffffffffull) - kmin;
-                        if (dec > 0xffffffffull) bad |= 1u << j;
-                        rv[j] = rh + j < nmax && idx < krange ? __ldg(pfmap + (idx >> 5)) : 0u;
-                        sh[j >> 2] |= (uint32_t)(idx & 31) << ((j & 3) * 8);
-                    }
-#pragma unroll
-                    for (int j = 0; j < kH; ++j)
-                        if (((rv[j] >> ((sh[j >> 2] >> ((j & 3) * 8)) & 31u)) & 1u) || ((bad >> j) & 1u))
-                            if (alive(h * kH + j)) km |= 1u << (h * kH + j);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < kH; ++j) {
-                        const uint64_t dec = c[j] * fk_ainv;
-                        const uint64_t idx = (dec & 0xffffffffull) - kmin;
-                        if (dec > 0xffffffffull) bad |= 1u << j;
-                        rv[j] = rh + j < nmax && idx < krange ? (accr ? (uint32_t)idx + 1u : __ldg(rec + idx)) : 0u;
-                    }
-#pragma unroll
-                    for (int j = 0; j < kH; ++j) {
-                        const unsigned long long a = alive(h * kH + j);
-                        if (!a) continue;
-                        const unsigned long long acc =
-                            accr ? (rv[j] ? __ldg(accr + rv[j] - 1u) : 0ull) : __ldg(dacc + rv[j]);
-                        if ((a & acc) != 0 || ((bad >> j) & 1u)) km |= 1u << (h * kH + j);
-                    }
-                }
+            for (int s = 0; s < 2; ++s) {
+                const uint64_t r = t * kPfStep + 256 * s + 8 * lane;  // two vectors of 8 codes per column and lane
+                if (rq) fq[s] = Flight<2, 8>::get(qty, r, vq16);
+                if (rd) fd[s] = Flight<2, 8>::get(disc, r, vd16);
             }
-        } else {
-            // (a column no alive query selects on is not read)
-            const unsigned long long live = r0 < nmax ? full | part : 0ull;
-            uint32_t qw[kPfRows / 2], dw[kPfRows / 2];
-            if (live & fq0) pf_load16(qty, r0, nmax, vec_q, qw);
-            if (live & fq1) pf_load16(disc, r0, nmax, vec_d, dw);
-            if (part == 0 && full == fall && r0 + kPfRows <= nmax) {
-                // every query alive on the whole run: one table bit a row (a
-                // corrupt code, above 255 decoded, is kept and never looked up)
+        };
+        if (t < whole) load(t);
+        for (; t < steps; t = after(t)) {
+            const uint64_t r0 = t * kPfStep + 8 * lane, next = after(t);
+            uint32_t keep = 0, bad = 0;
+            auto row = [&](int bit) { return (uint32_t)r0 + 256u * (uint32_t)(bit >> 3) + (uint32_t)(bit & 7); };
+            if (t < whole) {
+                const uint4 q0 = fq[0], q1 = fq[1], d0 = fd[0], d1 = fd[1];
+                if (next < whole) load(next);
+                uint64_t q[8], d[8];
 #pragma unroll
-                for (int j = 0; j < kPfRows; ++j) {
-                    const uint32_t vq = A0 ? (((qw[j >> 1] >> ((j & 1) * 16)) & 0xffffu) * qa) & 0xffffu : 0u;
-                    const uint32_t vd = A1 ? (((dw[j >> 1] >> ((j & 1) * 16)) & 0xffffu) * da) & 0xffffu : 0u;
-                    if ((vq | vd) > 0xffu || ((s_T[(vq << 3) | (vd >> 5)] >> (vd & 31)) & 1u)) km |= 1u << j;
-                }
-            } else
+                for (int s = 0; s < 2; ++s) {
+                    unpack16<2>(s ? q1 : q0, q);
+                    unpack16<2>(s ? d1 : d0, d);
 #pragma unroll
-            for (int j = 0; j < kPfRows; ++j) {
-                const unsigned long long a = alive(j);
-                if (!a) continue;
-                unsigned long long m = a;
-                bool bad = false;
-                if (a & fq0) {
-                    const uint32_t v = (((qw[j >> 1] >> ((j & 1) * 16)) & 0xffffu) * qa) & 0xffffu;
-                    if (v > 0xffu) bad = true;
-                    else m &= s_acc[v] | ~(a & fq0);
+                    for (int k = 0; k < 8; ++k) test((uint32_t)q[k], (uint32_t)d[k], 8 * s + k, keep, bad);
                 }
-                if (a & fq1) {
-                    const uint32_t v = (((dw[j >> 1] >> ((j & 1) * 16)) & 0xffffu) * da) & 0xffffu;
-                    if (v > 0xffu) bad = true;
-                    else m &= s_acc[256 + v] | ~(a & fq1);
-                }
-                if (bad || m != 0) km |= 1u << j;
+            } else {
+                for (int b = 0; b < 16; ++b)
+                    if (row(b) < nmax)
+                        test(rq ? __ldg(bp->qty + row(b)) : 0u, rd ? __ldg(bp->disc + row(b)) : 0u, b, keep, bad);
             }
-        }
-        // the warp's kept rows, one shared atomic per warp: exclusive offsets
-        // by an inclusive scan of the threads' counts
-        const uint32_t cnt = (uint32_t)__popc(km);
-        uint32_t incl = cnt;
+            if (two) {
+                uint32_t k16 = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t k8 = (keep >> (8 * h)) & 0xff, b8 = 0;
+                    second([&](int s) { return (uint64_t)row(8 * h + 2 * s); }, t < whole, k8, b8);
+                    k16 |= k8 << (8 * h);
+                    bad |= b8 << (8 * h);
+                }
+                keep = k16;
+            }
+            out.append(keep, row);
+            append_bad(bp, bad, row);
         }
-        uint32_t wbase = 0;
-        if (lane == 31 && incl) wbase = atomicAdd(&s_cnt, incl);
-        wbase = __shfl_sync(0xffffffffu, wbase, 31);
-        uint32_t pos = wbase + incl - cnt;
-        for (uint32_t m = km; m; m &= m - 1) s_rows[pos++] = (uint32_t)(r0 + (uint64_t)(__ffs(m) - 1));
-        __syncthreads();
-        const uint32_t nt = s_cnt;
-        if (threadIdx.x == 0 && nt) s_base = atomicAdd(kept, (unsigned long long)nt);
-        __syncthreads();
-        for (uint32_t j = threadIdx.x; j < nt; j += blockDim.x)
-            if (s_base + j < cap) list[s_base + j] = s_rows[j];
-        __syncthreads();  // (s_rows and s_cnt are reused by the next tile)
     }
+    out.finish();
+}
+
+// The list the per-row pass reads: the last one that fits its capacity; false:
+// none does.
+struct ListView {
+    const uint32_t* list;
+    uint64_t n;
+};
+AHEAD_DEV bool first_list(const SjBatch& b, ListView& v) {
+    const SjHdr* h = b.hdr;
+    if (!b.flist_on || h->fkept > b.flist_cap[0] || h->fbad > kFbadCap) return false;
+    v = ListView{b.flist[0], h->fkept};
+    return true;
+}
+AHEAD_DEV bool last_list(const SjBatch& b, ListView& v) {
+    if (!first_list(b, v)) return false;
+    if (b.ref_on && b.hdr->rkept <= b.flist_cap[1]) v = ListView{b.flist[1], b.hdr->rkept};
+    return true;
+}
+
+// The third filter: eight listed rows per lane, their keys gathered together
+// while the next step's list entries are on their way.  The gathers bound it:
+// 143 us for 4M rows listed of 100M, an eighth of them kept.
+__global__ void __launch_bounds__(1024, 1) sj_refine_kernel(const SjBatch* __restrict__ bp) {
+    extern __shared__ __align__(16) uint32_t s_map[];
+    if (__ldg(&bp->strategy) != kStratRows || !__ldg(&bp->ref_on)) return;
+    ListView in;
+    if (!first_list(*bp, in)) return;  // (block-uniform)
+    const uint32_t d = bp->ref_dim & 3;
+    const int lane = threadIdx.x & 31;
+    const uint64_t nmax = bp->nmax, warps = (uint64_t)gridDim.x * 32, steps = (in.n + 255) / 256;
+    uint64_t t = blockIdx.x * 32ull + (threadIdx.x >> 5);
+    uint4 e[2];
+    auto load = [&](uint64_t step) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {  // (a list's length is a multiple of kListChunkMin)
+            const uint64_t at = step * 256 + 128 * s + 4 * lane;
+            e[s] = at < in.n ? __ldg(reinterpret_cast<const uint4*>(in.list + at)) : make_uint4(kNoRow, kNoRow, kNoRow, kNoRow);
+        }
+    };
+    if (t < steps) load(t);
+    KeyMap km;
+    km.load(bp, d, s_map);
+    __syncthreads();
+    const unsigned long long* fk = bp->dim[d].fk;
+    ListOut out(bp->flist[1], bp->flist_cap[1], bp->flist_chunk[1], &bp->hdr->rkept);
+    for (; t < steps; t += warps) {
+        const uint32_t r[8] = {e[0].x, e[0].y, e[0].z, e[0].w, e[1].x, e[1].y, e[1].z, e[1].w};
+        unsigned long long c[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) c[k] = r[k] < nmax ? __ldg(fk + r[k]) : 0ull;
+        if (t + warps < steps) load(t + warps);
+        uint32_t keep = 0, bad = 0, live = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (r[k] < nmax) live |= 1u << k;
+        km.test(c, live, keep, bad);
+        auto row = [&](int b) {
+            uint32_t v = r[0];
+#pragma unroll
+            for (int k = 1; k < 8; ++k) v = b == k ? r[k] : v;
+            return v;
+        };
+        if (km.fold) keep = km.exact(fk, row, keep);
+        out.append(keep, row);
+        append_bad(bp, bad, row);
+    }
+    out.finish();
 }
 
 template <int kSjRows, int kSjBlocksPerSm>
@@ -542,11 +776,11 @@ __global__ void __launch_bounds__(kSjThreads, kSjBlocksPerSm) sj_fact_kernel(con
     if (threadIdx.x < b.nq) s_n[threadIdx.x] = s_q[threadIdx.x].nrows;
     __syncthreads();
     const uint32_t nsm = b.nsm;
-    // over the prefilter's row list when it ran and its rows fit the list,
-    // else over the rows themselves (block-uniform)
-    const unsigned long long nkept = b.flist_on ? b.hdr->fkept : 0ull;
-    const bool listed = b.flist_on && nkept <= b.flist_cap;
-    const uint64_t nitems = listed ? nkept : b.nmax;
+    // over the last row list that fits, and the rows with a corrupt code, else
+    // over the rows themselves (block-uniform)
+    ListView lv{nullptr, 0};
+    const bool listed = last_list(b, lv);
+    const uint64_t nitems = listed ? lv.n + b.hdr->fbad : b.nmax;
     const uint32_t ntiles = (uint32_t)((nitems + kSjTile - 1) / kSjTile);
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const uint64_t t0 = (uint64_t)tile * kSjTile;
@@ -567,7 +801,10 @@ __global__ void __launch_bounds__(kSjThreads, kSjBlocksPerSm) sj_fact_kernel(con
 #pragma unroll
         for (int i = 0; i < kSjRows; ++i) {
             const uint64_t idx = t0 + (uint64_t)i * kSjThreads + threadIdx.x;
-            rowv[i] = !listed ? idx : idx < nitems ? (uint64_t)__ldg(b.flist + idx) : b.nmax;
+            rowv[i] = !listed ? idx
+                      : idx < lv.n ? (uint64_t)__ldg(lv.list + idx)
+                      : idx < nitems ? (uint64_t)__ldg(b.fbad + (idx - lv.n))
+                                     : b.nmax;
         }
         unsigned long long alive[kSjRows];
         uint32_t at[kSjRows][4];
@@ -2237,6 +2474,17 @@ SjLayout sj_layout() {
 }  // namespace
 
 // ------------------------------------------------------------------ engine
+// A captured launch sequence: one per kind of batch (sj_kind).
+struct SjGraph {
+    cudaGraphExec_t exec = nullptr;
+    cudaGraph_t src = nullptr;                    // the captured graph `exec` was made from
+    cudaGraphNode_t cube_node[2] = {};            // its cube-scan nodes (phase 0, 1)
+    cudaKernelNodeParams cube_kp[2] = {};
+    int launches = 0;
+    bool local = false;  // a local half (up to the export)
+};
+enum { kKindCube, kKindRows, kKindList, kKindRefined, kKinds };
+
 struct SjSlot {
     char* dev = nullptr;                     // device area (SjLayout)
     char* h_up = nullptr;                    // pinned upload staging [0, L.upload)
@@ -2246,10 +2494,7 @@ struct SjSlot {
     cudaEvent_t f0 = nullptr, f1 = nullptr;  // around the fact kernel (graph event nodes)
     cudaEvent_t hdr_done = nullptr;          // the header read-back finished (copy stream)
     cudaStream_t copy = nullptr;             // this slot's result read-back, overlapping the other slot's batch
-    cudaGraphExec_t graph = nullptr;
-    cudaGraph_t gsrc = nullptr;                   // the captured graph `graph` was made from
-    cudaGraphNode_t cube_node[2] = {};            // its cube-scan nodes (phase 0, 1)
-    cudaKernelNodeParams cube_kp[2] = {};
+    SjGraph graph[kKinds];
     bool busy = false;
     uint64_t ticket = 0;
     // what collection needs from the plan
@@ -2267,16 +2512,16 @@ struct SjSlot {
     unsigned long long* xlog = nullptr;
     size_t xcap = 0;  // groups the area holds
     bool local_pending = false;
-    bool graph_local = false;  // the captured graph is a local half (up to the export)
 };
 
-// Release a slot's captured graph (it is captured again on its next use).
+inline void sj_drop_graph(SjGraph& G) {
+    if (G.exec) cudaGraphExecDestroy(G.exec);
+    if (G.src) cudaGraphDestroy(G.src);
+    G = SjGraph();
+}
+// Release a slot's captured graphs (each is captured again on its next use).
 inline void sj_drop_graph(SjSlot& S) {
-    if (S.graph) cudaGraphExecDestroy(S.graph);
-    if (S.gsrc) cudaGraphDestroy(S.gsrc);
-    S.graph = nullptr;
-    S.gsrc = nullptr;
-    S.cube_node[0] = S.cube_node[1] = nullptr;
+    for (SjGraph& G : S.graph) sj_drop_graph(G);
 }
 
 struct ahead_sj_engine {
@@ -2298,10 +2543,12 @@ struct ahead_sj_engine {
     // join index (null: none): ixfmt 1: slot 1 [fact_rows], then slot 2
     // [fact_rows]; ixfmt 2: one packed word per row (layout ixp)
     // the prefilter's row list (per-row batches; allocated with the engine for
-    // fact tables of at least 2^20 rows, shared by the slots)
-    uint32_t* flist = nullptr;
-    uint64_t flist_cap = 0;
-    uint32_t* pfmap = nullptr;  // the first-join prefilter's accepted keys, one bit a key (the largest dimension)
+    // fact tables of at least kListMinRows rows, shared by the slots)
+    uint32_t* flist[2] = {nullptr, nullptr};
+    uint64_t flist_cap[2] = {0, 0};
+    uint32_t* fbad = nullptr;      // [kFbadCap]
+    uint32_t* pfmap = nullptr;     // the dimensions' accepted keys, one bit a key
+    uint64_t pfmap_at[5] = {};     // word offset of each dimension's, and of their folded copies
     unsigned long long* fidx = nullptr;
     int ixfmt = 0;
     SjIxPacking ixp{};
@@ -2330,6 +2577,11 @@ struct ahead_sj_engine {
 };
 
 namespace {
+
+void sj_free_lists(ahead_sj_engine* e) {
+    for (uint32_t** p : {&e->flist[0], &e->flist[1], &e->fbad, &e->pfmap})
+        if (*p) cudaFree(*p), *p = nullptr;
+}
 
 // The buffers the batches share (stream-ordered).  Growing one waits for the
 // device and frees, which stalls a pipelined caller, so sj_prepare sizes them
@@ -2577,6 +2829,11 @@ int sj_prepare(ahead_sj_engine* e) {
         if (cudaFuncSetAttribute(kSjFact[v], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFactSmem) !=
             cudaSuccess)
             return AHEAD_CUDA_ERROR;
+    if (cudaFuncSetAttribute(sj_prefilter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPfSmem) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(sj_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPfSmem) !=
+            cudaSuccess)
+        return AHEAD_CUDA_ERROR;
     if (cudaFuncSetAttribute(sj_contract_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFactSmem) !=
         cudaSuccess)
         return AHEAD_CUDA_ERROR;
@@ -2616,14 +2873,29 @@ int sj_prepare(ahead_sj_engine* e) {
         for (int d = 0; d < 4; ++d) al = al && ((uintptr_t)e->sch.fk[d].data & 15) == 0;
         e->vec_ok = al;
     }
-    // the prefilter's row list (when the device memory is short, no prefilter)
-    if (e->sch.fact_rows >= (1ull << 20)) {
-        const uint64_t cap = std::min<uint64_t>(e->sch.fact_rows, kFlistMaxRows);
-        if (cudaMalloc(&e->flist, cap * 4) == cudaSuccess) e->flist_cap = cap;
-        else cudaGetLastError(), e->flist = nullptr;  // (not sticky)
+    // the row lists (when the device memory is short, no prefilter)
+    if (e->sch.fact_rows >= kListMinRows) {
+        // (a refined list holds at most half of the rows it was made from, or it
+        // is not used; chunk ends of every warp besides)
+        const uint64_t ends = (uint64_t)e->ctx->num_sms * 32 * kListChunk;
+        const uint64_t cap = std::min<uint64_t>(e->sch.fact_rows + ends, kFlistMaxRows) & ~(uint64_t)(kListChunk - 1);
         uint64_t words = 0;
-        for (int d = 0; d < 4; ++d) words = std::max<uint64_t>(words, e->dim[d].krange / 32 + 1);
-        if (e->flist && cudaMalloc(&e->pfmap, words * 4) != cudaSuccess) cudaGetLastError(), e->pfmap = nullptr;
+        bool fits = true;
+        for (int d = 0; d < 4; ++d) {
+            e->pfmap_at[d] = words;
+            words += (e->dim[d].krange / 32 + 1 + 3) & ~3ull;  // (each on a 16-byte boundary)
+            fits = fits && e->dim[d].krange < (1ull << 32) - 64 && e->dim[d].kmin < (1ull << 32) &&
+                   inv_pow2(e->sch.fk[d].Ainv, 64) < (1ull << 32);
+        }
+        e->pfmap_at[4] = words;
+        e->flist_cap[0] = cap;
+        e->flist_cap[1] = (cap / 2 + ends) & ~(uint64_t)(kListChunk - 1);
+        if (!fits || cudaMalloc(&e->flist[0], e->flist_cap[0] * 4) != cudaSuccess ||
+            cudaMalloc(&e->flist[1], e->flist_cap[1] * 4) != cudaSuccess ||
+            cudaMalloc(&e->fbad, kFbadCap * 4) != cudaSuccess || cudaMalloc(&e->pfmap, words * 2 * 4) != cudaSuccess) {
+            cudaGetLastError();  // (not sticky)
+            sj_free_lists(e);
+        }
     }
     const int rc = sj_build_index(e, -1);
     if (rc == AHEAD_OK && e->fidx && e->vec_ok)
@@ -2800,6 +3072,7 @@ int sj_plan(ahead_sj_engine* e, const ahead_sj_query* qs, int nq, SjSlot& S) {
         B.dim[d].code = e->dim[d].code;
         B.dim[d].acc = reinterpret_cast<const unsigned long long*>(S.dev + L.acc) + (size_t)d * kAccEntries;
         B.dim[d].fk_ainv = sch.fk[d].Ainv;
+        B.dim[d].fk_a = (uint32_t)inv_pow2(sch.fk[d].Ainv, 64);
         B.dim[d].kmin = e->dim[d].kmin;
         B.dim[d].krange = e->dim[d].krange;
         B.dim[d].joins = joins[d];
@@ -2995,15 +3268,24 @@ int sj_plan(ahead_sj_engine* e, const ahead_sj_query* qs, int nq, SjSlot& S) {
             B.fast = 1;
         }
     }
-    // the prefilter: a per-row batch over at least 2^20 rows whose every query
+    // the row lists: a per-row batch over at least kListMinRows rows whose every query
     // selects on quantity or discount (1), or whose queries have no fact
-    // predicate and all join one dimension first (2)
-    B.flist = nullptr;
-    B.flist_cap = 0;
+    // predicate and all join one dimension first (2); then the dimensions that
+    // follow in join order, while every query joins them and they drop enough
     B.flist_on = 0;
     B.flist_dim = 0;
-    B.pfmap = nullptr;
-    if (B.strategy == kStratRows && nmax >= (1ull << 20) && !order.empty()) {
+    B.flist_next = 4;
+    B.ref_on = B.ref_dim = 0;
+    for (int d = 0; d < 4; ++d) {
+        B.pfmap[d] = B.pfsmall[d] = nullptr;
+        B.pffold[d] = B.pfwords[d] = 0;
+    }
+    for (int i = 0; i < 2; ++i) {
+        B.flist[i] = e->flist[i];
+        B.flist_cap[i] = e->flist_cap[i];
+    }
+    B.fbad = e->fbad;
+    if (B.strategy == kStratRows && nmax >= kListMinRows && !order.empty() && e->pfmap) {
         bool all_fact = true, no_fact = true;
         unsigned long long om = 0;
         for (int qi : order) {
@@ -3012,45 +3294,91 @@ int sj_plan(ahead_sj_engine* e, const ahead_sj_query* qs, int nq, SjSlot& S) {
             no_fact = no_fact && !f;
             om |= 1ull << qi;
         }
-        int mode = all_fact ? 1 : 0;
-        for (int d = 0; d < 4 && !mode; ++d)
-            if (no_fact && (first[d] & om) == om) {
-                // the share of rows the first join keeps, summed over the queries:
-                // per query the product over its predicates on d of the share of
-                // the attribute's values (min..max, sampled beyond 2^16) it accepts
-                double share = 0.0;
-                for (int qi : order) {
-                    double q = 1.0;
-                    for (int k = 0; k < qs[qi].npred; ++k) {
-                        const ahead_sj_pred& p = qs[qi].pred[k];
-                        if (p.dim != d) continue;
-                        const ahead_col& c = sch.dim[d].attr[p.attr];
-                        const uint64_t wm = wmask(type_width(c.type));
-                        const RangePred rp = RangePred::make(p.op1, p.th1, p.op2, p.th2, p.comb, wm);
-                        const uint64_t lo = e->dim[d].amin[p.attr], hi = e->dim[d].amax[p.attr];
-                        if (hi < lo) continue;
-                        const uint64_t n = hi - lo + 1, step = n > (1u << 16) ? n / (1u << 16) : 1;
-                        uint64_t hit = 0, seen = 0;
-                        for (uint64_t v = lo; v <= hi && seen < (1u << 16); v += step, ++seen)
-                            hit += rp((v * c.A) & wm) ? 1 : 0;
-                        q *= seen ? (double)hit / (double)seen : 1.0;
-                    }
-                    share += q;
+        // the share of rows a join keeps, summed over the queries: per query the
+        // product over its predicates on d of the share of the attribute's values
+        // (min..max, sampled beyond 2^16) it accepts
+        auto share_of = [&](int d) {
+            double share = 0.0;
+            for (int qi : order) {
+                double q = 1.0;
+                for (int k = 0; k < qs[qi].npred; ++k) {
+                    const ahead_sj_pred& p = qs[qi].pred[k];
+                    if (p.dim != d) continue;
+                    const ahead_col& c = sch.dim[d].attr[p.attr];
+                    const uint64_t wm = wmask(type_width(c.type));
+                    const RangePred rp = RangePred::make(p.op1, p.th1, p.op2, p.th2, p.comb, wm);
+                    const uint64_t lo = e->dim[d].amin[p.attr], hi = e->dim[d].amax[p.attr];
+                    if (hi < lo) continue;
+                    const uint64_t n = hi - lo + 1, step = n > (1u << 16) ? n / (1u << 16) : 1;
+                    uint64_t hit = 0, seen = 0;
+                    for (uint64_t v = lo; v <= hi && seen < (1u << 16); v += step, ++seen)
+                        hit += rp((v * c.A) & wm) ? 1 : 0;
+                    q *= seen ? (double)hit / (double)seen : 1.0;
                 }
-                if (share <= kPrefilterMaxShare) {
-                    mode = 2;
-                    B.flist_dim = (uint32_t)d;
-                }
-                break;  // (one dimension is every query's first)
+                share += q;
             }
-        if (mode) {
-            if (e->flist) {  // (allocated with the engine; without it every row is scanned)
-                B.flist = e->flist;
-                B.flist_cap = e->flist_cap;
-                B.flist_on = (uint32_t)mode;
-                if (mode == 2) B.pfmap = e->pfmap;
+            return share;
+        };
+        // rows expected in the lists, and the chunks warps take of them
+        double rows = (double)nmax;
+        auto chunk_of = [&](double kept) {
+            const double per = kept / ((double)e->ctx->num_sms * 32 * 16);
+            uint32_t c = kListChunkMin;
+            while (c < kListChunk && c < per) c <<= 1;
+            return c;
+        };
+        // d's map, and folded so that it fits
+        auto place = [&](int d) {
+            B.pfmap[d] = B.pfsmall[d] = e->pfmap + e->pfmap_at[d];
+            B.pfwords[d] = ((uint32_t)e->dim[d].krange / 32 + 4) & ~3u;  // (each on a 16-byte boundary)
+        };
+        auto fit = [&](int d, uint32_t room) {
+            const uint32_t words = B.pfwords[d];
+            while (B.pfwords[d] > room) {
+                ++B.pffold[d];
+                B.pfwords[d] = (((words - 1) >> B.pffold[d]) + 4) & ~3u;
+                B.pfsmall[d] = e->pfmap + e->pfmap_at[4] + e->pfmap_at[d];
+            }
+        };
+        int k0 = 0;  // the join order's next dimension
+        if (all_fact) {
+            B.flist_on = 1;
+            rows *= 0.1;
+        } else if (no_fact) {
+            for (; k0 < 4 && !joins[join_dim(k0)]; ++k0) {}
+            if (k0 < 4 && (first[join_dim(k0)] & om) == om && share_of(join_dim(k0)) <= kPrefilterMaxShare) {
+                B.flist_on = 2;
+                B.flist_dim = (uint32_t)join_dim(k0);
+                place(join_dim(k0));
+                rows *= share_of(join_dim(k0));
+                ++k0;
             }
         }
+        B.flist_chunk[0] = chunk_of(rows);
+        for (int k = k0; B.flist_on && k < 4 && !B.ref_on; ++k) {
+            const int d = join_dim(k);
+            if (!joins[d]) continue;
+            if ((joins[d] & om) != om || share_of(d) > kRefineMaxShare) break;
+            if (B.flist_next < 4 && rows < kRefineMinRows) break;
+            rows *= share_of(d);
+            place(d);
+            if (B.flist_next == 4) {
+                B.flist_next = (uint32_t)d;
+                B.flist_chunk[0] = chunk_of(rows);
+            } else {
+                B.ref_on = 1;
+                B.ref_dim = (uint32_t)d;
+                B.flist_chunk[1] = chunk_of(rows);
+                fit(d, kPfRoom);
+            }
+        }
+        // the prefilter's maps share its shared memory, half each if need be
+        if (B.flist_next < 4) {
+            const int a = (int)B.flist_dim, b = (int)B.flist_next;
+            const uint32_t other = B.flist_on == 1 ? kFactWords : std::min<uint32_t>(B.pfwords[a], kPfRoom / 2);
+            fit(b, kPfRoom - other);
+        }
+        if (B.flist_on == 2) fit((int)B.flist_dim, kPfRoom - (B.flist_next < 4 ? B.pfwords[B.flist_next] : 0));
     }
     S.strategy = B.strategy;
     S.cube_variant = e->cube_variant;
@@ -3071,14 +3399,23 @@ int sj_plan(ahead_sj_engine* e, const ahead_sj_query* qs, int nq, SjSlot& S) {
     return AHEAD_OK;
 }
 
-// The kernels of one batch (captured once per slot, or launched directly);
-// `local`: the local half of a fact-sharded batch, up to the export.
-void sj_launch(ahead_sj_engine* e, SjSlot& S, bool capturing, bool local) {
+// The launch sequence a planned batch takes: a kernel that would find nothing to
+// do is not in it (an empty launch costs 2-3 us on the device: ten of them were a
+// tenth of a single query over 2M rows, 207 us against 184).
+int sj_kind(const SjBatch& b) {
+    return b.strategy == kStratCube ? kKindCube : !b.flist_on ? kKindRows : !b.ref_on ? kKindList : kKindRefined;
+}
+
+// The kernels of one batch (captured once per slot and kind, or launched
+// directly); `local`: the local half of a fact-sharded batch, up to the export.
+// Returns the launches.
+int sj_launch(ahead_sj_engine* e, SjSlot& S, bool capturing, bool local) {
     cudaStream_t st = e->ctx->stream;
     const SjLayout L = sj_layout();
     const SjBatch* bp = reinterpret_cast<const SjBatch*>(S.dev + L.batch);
     const AcceptQ* aq = reinterpret_cast<const AcceptQ*>(S.dev + L.aq);
-    const int sms = e->ctx->num_sms;
+    const SjBatch& hb = *reinterpret_cast<const SjBatch*>(S.h_up + L.batch);
+    const int sms = e->ctx->num_sms, kind = sj_kind(hb);
     sj_clear_kernel<<<sms * 2, 256, 0, st>>>(bp);
     SjPackAll pk;
     for (int d = 0; d < 4; ++d) pk.d[d] = e->dim[d].pack;
@@ -3090,33 +3427,42 @@ void sj_launch(ahead_sj_engine* e, SjSlot& S, bool capturing, bool local) {
     // inside a capture the records become event nodes of the graph
     const unsigned int rf = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
     cudaEventRecordWithFlags(S.f0, st, rf);
-    const int v = e->variant;
-    sj_pfmap_kernel<<<sms * 2, 256, 0, st>>>(bp);
-    sj_prefilter_kernel<<<sms * 3, kSjThreads, 0, st>>>(bp);  // (its launch bounds: three blocks an SM)
-    kSjFact[v]<<<sms * kSjVarBlocks[v], kSjThreads, kFactSmem, st>>>(bp);
-    // (wide grids: both kernels are chains of dependent loads per element)
-    sj_code_kernel<<<dim3(sms * 8, 4), 256, 0, st>>>(bp);
-    const int cv = e->cube_variant;
-    // the cube scan takes the descriptor by value (a graph's copy is updated per batch)
-    const SjBatch& hb = *reinterpret_cast<const SjBatch*>(S.h_up + L.batch);
-    const CubeShape& cs = kCubeShapes[cv];
-    cs.fn<<<sms * cs.blocks_per_sm, kSjThreads, 0, st>>>(hb, 0);
-    sj_unseen_kernel<<<sms * 16, 256, 0, st>>>(bp);
-    cs.fn<<<sms * cs.blocks_per_sm, kSjThreads, 0, st>>>(hb, 1);
-    cudaEventRecordWithFlags(S.f1, st, rf);
-    sj_exc_kernel<<<64, kSjThreads, 0, st>>>(bp);
-    sj_contract_kernel<<<sms * 3, kSjThreads, kFactSmem, st>>>(bp);  // (3 blocks fit an SM: 62 KB of shared memory each)
-    n += 9;
+    if (kind == kKindList || kind == kKindRefined) {
+        sj_pfmap_kernel<<<dim3(sms * 2, 4), 256, 0, st>>>(bp);
+        sj_prefilter_kernel<<<sms, 1024, kPfSmem, st>>>(bp);
+        n += 2;
+    }
+    if (kind == kKindRefined) {
+        sj_refine_kernel<<<sms, 1024, kPfSmem, st>>>(bp);
+        n += 1;
+    }
+    if (kind == kKindCube) {
+        // (wide grids: both kernels are chains of dependent loads per element)
+        sj_code_kernel<<<dim3(sms * 8, 4), 256, 0, st>>>(bp);
+        // the cube scan takes the descriptor by value (a graph's copy is updated per batch)
+        const CubeShape& cs = kCubeShapes[e->cube_variant];
+        cs.fn<<<sms * cs.blocks_per_sm, kSjThreads, 0, st>>>(hb, 0);
+        sj_unseen_kernel<<<sms * 16, 256, 0, st>>>(bp);
+        cs.fn<<<sms * cs.blocks_per_sm, kSjThreads, 0, st>>>(hb, 1);
+        cudaEventRecordWithFlags(S.f1, st, rf);
+        sj_exc_kernel<<<64, kSjThreads, 0, st>>>(bp);
+        sj_contract_kernel<<<sms * 3, kSjThreads, kFactSmem, st>>>(bp);  // (3 blocks fit an SM: 62 KB of shared memory each)
+        n += 6;
+    } else {
+        const int v = e->variant;
+        kSjFact[v]<<<sms * kSjVarBlocks[v], kSjThreads, kFactSmem, st>>>(bp);
+        cudaEventRecordWithFlags(S.f1, st, rf);
+        n += 1;
+    }
     if (local) {
         sj_export_kernel<<<sms * 2, 256, 0, st>>>(bp, S.xsum, S.xfirst, S.xflag, S.xlog, e->shard_lo);
-        e->ctx->launches += n + 1;
-        return;
+        return n + 1;
     }
     sj_compact_kernel<<<sms * 2, 256, 0, st>>>(bp);
     sj_finalize_kernel<<<kMaxQ, 1024, 0, st>>>(bp);
     sj_pack_kernel<<<kMaxQ, 1024, kPackSmem * 8, st>>>(bp);
     sj_emit_kernel<<<dim3(8, kMaxQ), 256, 0, st>>>(bp);
-    e->ctx->launches += n + 4;
+    return n + 4;
 }
 
 int sj_finish_submit(ahead_sj_engine* e, SjSlot& S, uint64_t* ticket);
@@ -3153,13 +3499,16 @@ int sj_submit(ahead_sj_engine* e, const ahead_sj_query* qs, int nq, int use_grap
     cudaStream_t st = e->ctx->stream;
     const SjLayout L = sj_layout();
     cudaMemcpyAsync(S.dev, S.h_up, L.upload, cudaMemcpyHostToDevice, st);
-    if (use_graph && S.graph && S.graph_local != local) sj_drop_graph(S);  // captured for the other form
-    if (use_graph && !S.graph) {
-        S.graph_local = local;
+    SjBatch* hb = reinterpret_cast<SjBatch*>(S.h_up + L.batch);
+    const int kind = sj_kind(*hb);
+    SjGraph& G = S.graph[kind];
+    if (use_graph && G.exec && G.local != local) sj_drop_graph(G);  // captured for the other form
+    if (use_graph && !G.exec) {
+        G.local = local;
         cudaGraph_t g;
         if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
             return fail(e->ctx, AHEAD_CUDA_ERROR, "graph capture");
-        sj_launch(e, S, true, local);
+        G.launches = sj_launch(e, S, true, local);
         if (cudaStreamEndCapture(st, &g) != cudaSuccess) return fail(e->ctx, AHEAD_CUDA_ERROR, "graph capture");
         // the cube-scan nodes, whose by-value descriptor each batch replaces
         size_t nn = 0;
@@ -3174,36 +3523,35 @@ int sj_submit(ahead_sj_engine* e, const ahead_sj_query* qs, int nq, int use_grap
             if (cudaGraphKernelNodeGetParams(nd, &kp) != cudaSuccess) continue;
             if (kp.func != reinterpret_cast<void*>(kCubeShapes[e->cube_variant].fn)) continue;
             const int ph = *static_cast<const int*>(kp.kernelParams[1]);
-            if (ph < 0 || ph > 1 || S.cube_node[ph]) continue;
-            S.cube_node[ph] = nd;
-            S.cube_kp[ph] = kp;
+            if (ph < 0 || ph > 1 || G.cube_node[ph]) continue;
+            G.cube_node[ph] = nd;
+            G.cube_kp[ph] = kp;
             ++found;
         }
-        const cudaError_t ie = found == 2 ? cudaGraphInstantiate(&S.graph, g, 0) : cudaErrorInvalidValue;
+        const cudaError_t ie = found == (kind == kKindCube ? 2 : 0) ? cudaGraphInstantiate(&G.exec, g, 0)
+                                                                    : cudaErrorInvalidValue;
+        G.src = g;
         if (ie != cudaSuccess) {
-            cudaGraphDestroy(g);
-            S.graph = nullptr;
-            S.cube_node[0] = S.cube_node[1] = nullptr;
+            G.exec = nullptr;
+            sj_drop_graph(G);
             return fail(e->ctx, AHEAD_CUDA_ERROR, "graph instantiate");
         }
-        S.gsrc = g;
     }
     cudaEventRecord(S.e0, st);
     if (use_graph) {
-        SjBatch* hb = reinterpret_cast<SjBatch*>(S.h_up + L.batch);
-        for (int ph = 0; ph < 2; ++ph) {
+        for (int ph = 0; ph < 2 && G.cube_node[ph]; ++ph) {
             int phase = ph;
             void* args[2] = {hb, &phase};
-            cudaKernelNodeParams kp = S.cube_kp[ph];
+            cudaKernelNodeParams kp = G.cube_kp[ph];
             kp.kernelParams = args;
             kp.extra = nullptr;
-            const cudaError_t pe = cudaGraphExecKernelNodeSetParams(S.graph, S.cube_node[ph], &kp);
+            const cudaError_t pe = cudaGraphExecKernelNodeSetParams(G.exec, G.cube_node[ph], &kp);
             if (pe != cudaSuccess) return cuda_fail(e->ctx, pe, "star join graph update");
         }
-        cudaGraphLaunch(S.graph, st);
-        e->ctx->launches += local ? 12 : 15;
+        cudaGraphLaunch(G.exec, st);
+        e->ctx->launches += G.launches;
     } else {
-        sj_launch(e, S, false, local);
+        e->ctx->launches += sj_launch(e, S, false, local);
     }
     if (local) {  // the final half follows the exchange (sj_submit_final)
         const cudaError_t le = cudaGetLastError();
@@ -3409,8 +3757,7 @@ void ahead_sj_destroy(ahead_sj_engine* e) {
     if (e->exc) cudaFree(e->exc);
     if (e->unseen) cudaFree(e->unseen);
     if (e->fidx) cudaFree(e->fidx);
-    if (e->flist) cudaFree(e->flist);
-    if (e->pfmap) cudaFree(e->pfmap);
+    sj_free_lists(e);
     delete e;
 }
 
