@@ -196,6 +196,31 @@ inline bool settle_err_list(OpScope& s, const ErrList& l, int ci, uint64_t aoid,
     return true;
 }
 
+// Rows 2p and 2p + 1 of a column in one load (`vec`: its data is aligned to two rows).
+template <int W>
+AHEAD_DEV void load_pair(const char* data, uint64_t p, bool vec, uint64_t (&x)[2]) {
+    if (vec) {
+        if constexpr (W == 8) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4*>(data) + p);
+            x[0] = (uint64_t)q.y << 32 | q.x;
+            x[1] = (uint64_t)q.w << 32 | q.z;
+        } else if constexpr (W == 4) {
+            const uint2 q = __ldg(reinterpret_cast<const uint2*>(data) + p);
+            x[0] = q.x;
+            x[1] = q.y;
+        } else {
+            static_assert(W == 2, "two-, four- and eight-byte columns");
+            const uint32_t q = __ldg(reinterpret_cast<const uint32_t*>(data) + p);
+            x[0] = q & 0xffffu;
+            x[1] = q >> 16;
+        }
+    } else {
+        x[0] = gmem_ld<W>(data, 2 * p);
+        x[1] = gmem_ld<W>(data, 2 * p + 1);
+    }
+}
+inline bool pair_aligned(const void* p, int w) { return (uintptr_t)p % (2 * w) == 0; }
+
 // ---------------------------------------------- rows dropped now and then
 // checkAndDecodeAN and the positional joins drop a row only when its code, OID
 // or fetched value is corrupt, which is rare.  So one pass writes every row's
