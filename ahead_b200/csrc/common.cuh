@@ -223,7 +223,6 @@ AHEAD_DEV uint64_t warp_sum64(uint64_t v) {
 
 // Device-side status word bits (written with atomicOr, read by the host).
 enum : uint32_t {
-    kDevStatusTimeout = 1u,      // a bounded spin gave up
     kDevStatusCapacity = 2u,     // an output did not fit
     kDevStatusDupKey = 4u,       // a build side had duplicate keys (fused paths only)
     kDevStatusBadInput = 8u,     // an input outside the supported domain

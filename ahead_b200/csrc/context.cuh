@@ -157,7 +157,6 @@ struct OpScope {
         if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamSynchronize");
         ctx->header_clean = true;
         uint32_t st = (uint32_t)ctx->h_stage[0];
-        if (st & kDevStatusTimeout) return fail(ctx, AHEAD_TIMEOUT, "a bounded device wait gave up");
         if (st & kDevStatusBadInput) return fail(ctx, AHEAD_UNSUPPORTED, "input outside the supported domain");
         return AHEAD_OK;
     }
