@@ -1104,10 +1104,14 @@ struct IsectOp {
     int mirror2;   // the second input's tail is its head: its value is key * a2
     uint64_t a2;
     const uint64_t* part;
+    const uint32_t* flag;  // merge_check_kernel's
     uint64_t lo, len;  // the tile's stretch of the second input
+    // Keys out of order have stretches that start behind their end, and a search
+    // that misses a marked key: then no tile has a stretch, so that nothing is
+    // searched, kept or gathered, and the replayed loop makes the result.
     AHEAD_DEV void tile(uint32_t t) {
         lo = __ldg((const unsigned long long*)part + t);
-        len = __ldg((const unsigned long long*)part + t + 1) - lo;
+        len = (__ldg(flag) & 1u) ? 0 : __ldg((const unsigned long long*)part + t + 1) - lo;
     }
     AHEAD_DEV uint64_t find(uint64_t row) const {  // ~0: no match
         const uint64_t k = key_val(t1c, row);
@@ -1200,7 +1204,7 @@ __global__ void __launch_bounds__(kCThreads) merge_classify_kernel(Op op, uint64
         __syncwarp();
 #pragma unroll
         for (int s = 0; s < K; ++s) {
-            const uint64_t d = k[s] - first;  // (keys out of order: any byte of the map, the result is discarded)
+            const uint64_t d = k[s] - first;
             const uint32_t b = __ballot_sync(kFull, lane + 32 * s < m && d < w && map[d < w ? d : 0]);
             if (lane == s) word = b;
         }
@@ -1260,6 +1264,7 @@ int run_merge(OpScope& s, const DCol& t1, const DCol& h1, const DCol& h2, const 
         op.mirror2 = t2.type != AHEAD_VOID && t2.data == h2.data && t2.type == h2.type && t2.ainv == h2.ainv;
         op.a2 = h2.enc ? inv_pow2(h2.ainv, 64) : 1;
         op.part = mp.part;
+        op.flag = (const uint32_t*)(s.d_counters + kMergeFlag);
         op.lo = op.len = 0;
         if (tiles <= kOneBlockTiles && !sized) {
             run_compact(s, op, n1, 0);
