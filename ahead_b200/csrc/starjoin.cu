@@ -146,14 +146,15 @@ struct SjHdr {
     unsigned long long errcnt, status, exccnt, unseen;
     unsigned long long fkept;  // the prefilter's list: entries taken, chunk ends included
     unsigned long long rkept;  // the same for the refining pass's
-    unsigned long long fbad;  // rows with a corrupt code the filters met
+    unsigned long long fbad;  // rows with a corrupt code the prefilter met
+    unsigned long long rbad;  // the same for the refining pass's
     // groups per query (counted by the compact kernel); ~0: the packed area
     // could not take them  (zeroed by the clear kernel up to here)
     unsigned long long ngroups[kMaxQ];
     unsigned long long off[kMaxQ];      // offset of each query's groups in packed
     unsigned long long nerr, packed_len;  // sorted errors at packed[0, nerr); words used
 };
-constexpr int kHdrClearWords = kMaxQ + 4 + 5 + 1 + 1 + kMaxQ;
+constexpr int kHdrClearWords = kMaxQ + 4 + 5 + 1 + 1 + 1 + kMaxQ;
 
 struct SjBatch {
     SjDimDev dim[4];
@@ -405,14 +406,14 @@ struct ListOut {
     }
 };
 
-// (rare) appends every lane's rows with a corrupt code
+// (rare) appends every lane's rows with a corrupt code to fbad, from `at` on
 template <class F>
-AHEAD_DEV void append_bad(const SjBatch* bp, uint32_t mask, F row) {
+AHEAD_DEV void append_bad(const SjBatch* bp, unsigned long long* count, uint64_t at, uint32_t mask, F row) {
     if (!__any_sync(kFull, mask != 0)) return;
     const uint32_t cnt = (uint32_t)__popc(mask), incl = warp_incl_scan(cnt);
     unsigned long long base = 0;
-    if ((threadIdx.x & 31) == 31) base = atomicAdd(&bp->hdr->fbad, (unsigned long long)incl);
-    base = __shfl_sync(kFull, base, 31) + incl - cnt;
+    if ((threadIdx.x & 31) == 31) base = atomicAdd(count, (unsigned long long)incl);
+    base = __shfl_sync(kFull, base, 31) + at + incl - cnt;
     for (; mask; mask &= mask - 1, ++base)
         if (base < kFbadCap) bp->fbad[base] = row(__ffs(mask) - 1);
 }
@@ -603,7 +604,7 @@ __global__ void __launch_bounds__(1024, 1) sj_prefilter_kernel(const SjBatch* __
                 bad |= b8 << (8 * h);
             }
             out.append(keep, row);
-            append_bad(bp, bad, row);
+            append_bad(bp, &bp->hdr->fbad, 0, bad, row);
         }
     } else {
         // bit vd of word vq * 8 + vd / 32: a row with decoded quantity vq and
@@ -679,27 +680,31 @@ __global__ void __launch_bounds__(1024, 1) sj_prefilter_kernel(const SjBatch* __
                 keep = k16;
             }
             out.append(keep, row);
-            append_bad(bp, bad, row);
+            append_bad(bp, &bp->hdr->fbad, 0, bad, row);
         }
     }
     out.finish();
 }
 
-// The list the per-row pass reads: the last one that fits its capacity; false:
-// none does.
+// The list the per-row pass reads, the last one that fits its capacity, and with
+// it the rows with a corrupt code that the filters up to that list met (the
+// refining pass leaves the ones it met in the first list as well); false: no
+// list fits.  first_list() reads nothing that the refining pass writes.
 struct ListView {
     const uint32_t* list;
-    uint64_t n;
+    uint64_t n, nbad;  // the list's entries, and those of fbad
 };
 AHEAD_DEV bool first_list(const SjBatch& b, ListView& v) {
     const SjHdr* h = b.hdr;
     if (!b.flist_on || h->fkept > b.flist_cap[0] || h->fbad > kFbadCap) return false;
-    v = ListView{b.flist[0], h->fkept};
+    v = ListView{b.flist[0], h->fkept, h->fbad};
     return true;
 }
 AHEAD_DEV bool last_list(const SjBatch& b, ListView& v) {
     if (!first_list(b, v)) return false;
-    if (b.ref_on && b.hdr->rkept <= b.flist_cap[1]) v = ListView{b.flist[1], b.hdr->rkept};
+    const SjHdr* h = b.hdr;
+    if (b.ref_on && h->rkept <= b.flist_cap[1] && h->fbad + h->rbad <= kFbadCap)
+        v = ListView{b.flist[1], h->rkept, h->fbad + h->rbad};
     return true;
 }
 
@@ -748,7 +753,7 @@ __global__ void __launch_bounds__(1024, 1) sj_refine_kernel(const SjBatch* __res
         };
         if (km.fold) keep = km.exact(fk, row, keep);
         out.append(keep, row);
-        append_bad(bp, bad, row);
+        append_bad(bp, &bp->hdr->rbad, in.nbad, bad, row);
     }
     out.finish();
 }
@@ -778,9 +783,9 @@ __global__ void __launch_bounds__(kSjThreads, kSjBlocksPerSm) sj_fact_kernel(con
     const uint32_t nsm = b.nsm;
     // over the last row list that fits, and the rows with a corrupt code, else
     // over the rows themselves (block-uniform)
-    ListView lv{nullptr, 0};
+    ListView lv{nullptr, 0, 0};
     const bool listed = last_list(b, lv);
-    const uint64_t nitems = listed ? lv.n + b.hdr->fbad : b.nmax;
+    const uint64_t nitems = listed ? lv.n + lv.nbad : b.nmax;
     const uint32_t ntiles = (uint32_t)((nitems + kSjTile - 1) / kSjTile);
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const uint64_t t0 = (uint64_t)tile * kSjTile;
