@@ -770,13 +770,13 @@ int run_pos_join(OpScope& s, PosArgs& a, const ahead_col* head, uint64_t aoid, b
                  ahead_errvec* e0, ahead_errvec* e1, uint64_t* kept) {
     if (((uintptr_t)a.oh | (uintptr_t)a.ot) & 3) return AHEAD_UNSUPPORTED;  // (narrow gaps are closed by words)
     const uint64_t n = a.n;
-    const size_t check = a.head_err ? colcheck_scratch(n) : 0;
+    const bool want_head = a.head_err && eh;
+    const size_t check = want_head ? colcheck_scratch(n) : 0;
     int rc = s.reserve(drop_scratch(n, (FETCH ? 0 : a.ohw) + a.otw) + kErrListBytes + check);
     if (rc) return rc;
     a.herr = err_list(s, kPosHead);
     a.drops = drop_list(s, kPosDrops);
     uint64_t* sorted = (uint64_t*)s.alloc(kMaxDrops * 8);
-    const bool want_head = a.head_err && eh;
     if (dense_head) a.head_err = 0;
     const uint64_t blocks = (n + 256 * kPosRows - 1) / (256 * kPosRows);
     const uint32_t most = (uint32_t)s.ctx->num_sms * 32;
@@ -800,6 +800,10 @@ int run_pos_join(OpScope& s, PosArgs& a, const ahead_col* head, uint64_t aoid, b
         else launch_shift(s, n, sorted, (uint32_t)k, a.ot, a.otw, a.oh, a.ohw);
     }
     if (want_head && !dense_head && !settle_err_list(s, a.herr, kPosHead, aoid, eh)) {
+        // (the gaps' edges may have taken the scratch up to its end: the check, behind
+        // them in the stream, starts over in it)
+        rc = s.reserve(check);
+        if (rc) return rc;
         check_head();
         rc = s.finish(2);
         if (rc) return rc;
