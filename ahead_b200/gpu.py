@@ -286,7 +286,7 @@ class GpuOps:
         self.lib.ahead_ctx_set_output_fn(self.ctx, self._output_fn, None)
 
     def _run(self, what, call, cap: int, nerr: int, nout: int = 1, tail: bool = True, sized: bool = False,
-             cols=(), sized_bytes: int = _SIZED_BYTES):
+             cols=(), sized_bytes: Optional[int] = None):
         """Run an operator with outputs of `cap` rows (sized: allocated by the
         call when they may be large) and error vectors of a small first
         capacity, or of all rows for the checked columns `cols` ((column, rows)
@@ -299,7 +299,7 @@ class GpuOps:
         for i, (c, rows) in enumerate(cols):
             if rows > few and _dense(c):
                 ecaps[i] = int(rows)
-        sized = sized and cap * 8 >= sized_bytes
+        sized = sized and cap * 8 >= (_SIZED_BYTES if sized_bytes is None else sized_bytes)
         while True:
             outs = [_Out(torch, cap, tail, sized) for _ in range(nout)]
             errs = _Errs(self, ecaps) if nerr else None
@@ -514,7 +514,7 @@ class GpuOps:
                                                           ctypes.byref(errs.c[0]), ctypes.byref(errs.c[1]))
         # (buffers of the values' width: narrow ones would be moved out of wide ones)
         outs, errs = self._run("checkAndDecodeAN", call, b.count, 2, sized=True,
-                               sized_bytes=_KEEP_BYTES if WIDTH[b.tail.type] <= 4 else _SIZED_BYTES)
+                               sized_bytes=_KEEP_BYTES if WIDTH[b.tail.type] <= 4 else None)
         v = errs.vecs(self)
         return outs[0].bat(self.torch), v[0], v[1]
 
