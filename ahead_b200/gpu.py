@@ -282,8 +282,13 @@ class GpuOps:
             out.bufs[column] = buf
             return buf.data_ptr()
 
-        self._output_fn = _OUTPUT_FN(take)  # alive until the next one replaces it
+        self._output_fn = _OUTPUT_FN(take)
         self.lib.ahead_ctx_set_output_fn(self.ctx, self._output_fn, None)
+
+    def _end_sized(self):
+        """The call is over: its columns belong to the result alone."""
+        self.lib.ahead_ctx_set_output_fn(self.ctx, None, None)
+        self._output_fn = None
 
     def _run(self, what, call, cap: int, nerr: int, nout: int = 1, tail: bool = True, sized: bool = False,
              cols=(), sized_bytes: Optional[int] = None):
@@ -305,7 +310,12 @@ class GpuOps:
             errs = _Errs(self, ecaps) if nerr else None
             if sized:
                 self._set_sized(outs[0])
-            rc = call(outs, errs)
+                try:
+                    rc = call(outs, errs)
+                finally:
+                    self._end_sized()
+            else:
+                rc = call(outs, errs)
             need_o = max([int(o.c.count) for o in outs]) if outs else 0
             short = errs.short() if errs else False
             if rc == CAPACITY or short or (need_o > cap and not sized):
