@@ -64,3 +64,11 @@ const char* ahead_status_string(int s) {
 }
 
 }  // extern "C"
+
+namespace ahead {
+// plain.cpp: its own output function for the length of a call, then the caller's again.
+void swap_output_fn(ahead_ctx* c, ahead_output_fn& fn, void*& user) {
+    std::swap(c->out_fn, fn);
+    std::swap(c->out_user, user);
+}
+}  // namespace ahead

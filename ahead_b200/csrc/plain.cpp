@@ -36,6 +36,10 @@
 
 #include "../../include/ahead_gpu.h"
 
+namespace ahead {
+void swap_output_fn(ahead_ctx* c, ahead_output_fn& fn, void*& user);  // context.cu
+}
+
 namespace {
 
 constexpr uint64_t kAoid = 16089;
@@ -193,9 +197,11 @@ struct Plain {
                     if (!e.data) return fail(AHEAD_NO_MEMORY);
                 }
             }
-            if (sized) ahead_ctx_set_output_fn(ctx, take_output, this);
+            ahead_output_fn fn = take_output;
+            void* user = this;
+            if (sized) ahead::swap_output_fn(ctx, fn, user);
             const int r = call(cap);
-            if (sized) ahead_ctx_set_output_fn(ctx, nullptr, nullptr);
+            if (sized) ahead::swap_output_fn(ctx, fn, user);  // (the caller's function stays set)
             uint64_t need_o = 0;
             for (int o = 0; o < nout; ++o) need_o = std::max(need_o, outs[o].count);
             bool short_e = false;
