@@ -1357,6 +1357,17 @@ __global__ void merge_seq_kernel(MergeSeq m, uint64_t* counters) {
     for (int v = 0; v < 4; ++v) counters[1 + v] = ne[v];
 }
 
+// A sized call's columns for the replayed loop: each row it keeps takes one of
+// either input, so the shorter one's length always fits, and a count of them
+// would be the whole loop run twice.
+int seq_columns(OpScope& s, ahead_bat* out, uint64_t n1, uint64_t n2, uint64_t& cap) {
+    if (!s.sized(out, cap)) return AHEAD_OK;
+    cap = n1 < n2 ? n1 : n2;
+    if (!s.take(&out->head, 0, cap) || !s.take(&out->tail, 1, cap))
+        return fail(s.ctx, AHEAD_NO_MEMORY, "output allocation failed");
+    return AHEAD_OK;
+}
+
 __global__ void zip_kernel(DCol h1, DCol t2, uint64_t p1, uint64_t p2, uint64_t m, int reenc, uint64_t fh, uint64_t ft,
                            void* oh, int ohw, void* ot, int otw, uint64_t cap) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m && i < cap;
@@ -1877,6 +1888,8 @@ int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
     }
     rc = s.reserve(0);
     if (rc) return rc;
+    rc = seq_columns(s, out, n1, n2, cap);
+    if (rc) return rc;
     MergeSeq m;
     m.h1 = h1;
     m.t1 = t1;
@@ -1887,7 +1900,7 @@ int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
     m.fh = fH1;
     m.ft = fT2;
     m.aoid = aoid;
-    m.cap = ocap;
+    m.cap = (out->head.data && out->tail.data) ? cap : 0;
     for (int k = 0; k < 4; ++k) {
         m.e[k] = edata(ev(errs, k));
         m.ecap[k] = ecap(ev(errs, k));
@@ -1906,7 +1919,7 @@ int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
     if (errs)
         for (int k = 0; k < 4; ++k)
             if (errs[k].present) errs[k].count = s.counter(1 + k);
-    return out->count > cap || s.sized(out, cap) ? AHEAD_CAPACITY : AHEAD_OK;
+    return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
 }
 
 int ahead_gpu_matchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, ahead_bat* out, uint64_t cap) {
@@ -2002,6 +2015,8 @@ int ahead_gpu_matchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, 
     }
     int rc = s.reserve(0);
     if (rc) return rc;
+    rc = seq_columns(s, out, n1, n2, cap);
+    if (rc) return rc;
     MergeSeq m{};
     m.h1 = h1;
     m.t1 = t1;
@@ -2009,7 +2024,7 @@ int ahead_gpu_matchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, 
     m.t2 = t2;
     m.n1 = n1;
     m.n2 = n2;
-    m.cap = ocap;
+    m.cap = (out->head.data && out->tail.data) ? cap : 0;
     m.oh = out->head.data;
     m.ot = out->tail.data;
     m.ohw = type_width(type_select_of(H1));
@@ -2020,7 +2035,7 @@ int ahead_gpu_matchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, 
     rc = s.finish(1);
     if (rc) return rc;
     out->count = s.counter(0);
-    return out->count > cap || s.sized(out, cap) ? AHEAD_CAPACITY : AHEAD_OK;
+    return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
 }
 
 int ahead_gpu_fetchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, int reenc, uint64_t atr,

@@ -155,7 +155,8 @@ class _Out:
                 cols.append(col_from_c(cc, None))
                 continue
             used = buf[at: at + n * WIDTH[cc.type]]
-            if not self.sized and self.cap * 8 > _KEEP_BYTES and 4 * used.numel() < self.cap * 8:
+            room = buf.numel() if self.sized else self.cap * 8
+            if room > _KEEP_BYTES and 4 * used.numel() < room:
                 # a result far below its capacity is moved out, so the capacity-sized
                 # buffer does not stay alive with it
                 used, moved = used.clone(), True
