@@ -191,10 +191,14 @@ __global__ void __launch_bounds__(256) probe_emit_kernel(const ProbeSlot* __rest
 // 1.6M keys), where 32 lanes' lookups cost a few bank conflicts, not 32 L2
 // requests; only the matches touch the value array in L2.
 //
-// Three things send the join to the hash table instead, found by the build
+// Two things send the join to the hash table instead, found by the build
 // kernels and read back with the counts: a key range above the limit (2^24 at
-// most: the value array then stays near L2's size), or a repeated key; and
-// 8-byte raw codes as keys are not tried (multiples of A: far too wide).
+// most: the value array then stays near L2's size), or a repeated key.  The probe
+// passes see it on the device and read nothing, which leaves some 40 us of
+// launches ahead of the table (60M probe rows, one key of 320K repeated: 1.38 ms a
+// call, 1.39 by the table alone; 30M against 3M keys of a wide range 1.95 and
+// 1.92).  Not tried: more build rows than the limit, and 8-byte raw codes as
+// keys (multiples of A: far too wide).
 // At 60M probe rows against 320K of 800K keys: hash probe 512 + 559 us (one
 // 16-byte slot request to L2 per row, then thread-serial output) and 110 us of
 // separate column checks, against 15 us to build, 123 to classify and 219 to emit
@@ -207,6 +211,9 @@ inline uint64_t dj_limit(uint64_t nb, uint64_t np) {
     const uint64_t l = (1ull << 20) + 64 * nb + np;
     return (l < kDjMaxSpan ? l : kDjMaxSpan) & ~31ull;
 }
+
+// More rows than the range has keys: some key repeats.
+inline bool dj_possible(uint64_t nb, uint64_t np) { return nb <= dj_limit(nb, np); }
 
 struct DjBuild {
     KeyCfg bk;
@@ -269,6 +276,7 @@ __global__ void __launch_bounds__(256) dj_insert_kernel(DjBuild b) {
     }
     const uint64_t rounds = (b.nb + stride - 1) / stride;
     for (uint64_t r = 0; r < rounds; ++r) {
+        if (r && __any_sync(kFull, *(volatile uint32_t*)b.bad != 0)) return;  // (the hash table has the join)
         const uint64_t i = r * stride + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
         const bool live = i < b.nb;
         uint64_t d = 0;
@@ -366,6 +374,11 @@ __global__ void __launch_bounds__(1024, 1) dj_classify_kernel(Op op, uint64_t n,
     const bool vec = ((uintptr_t)op.base & 15) == 0;
     op.begin();
     const uint32_t whole = (uint32_t)(n / (32 * K)), nw = gridDim.x * 32;
+    if (!op.span) {  // the hash table has the join: the probe column is not read, and no tile keeps a row
+        const uint64_t words = (uint64_t)cb.ntiles * Op::NCH;
+        for (uint64_t i = blockIdx.x * 1024ull + threadIdx.x; i < words; i += gridDim.x * 1024ull) cb.counts[i] = 0;
+        return;
+    }
     uint32_t tile = blockIdx.x * 32 + (threadIdx.x >> 5);
     Flight<Op::W, K> f;
     if (tile < whole) f.load(op.base, (uint64_t)tile * (32 * K) + 16 / Op::W * lane, vec);
@@ -481,9 +494,9 @@ size_t join_scratch(uint64_t nb, uint64_t np) {
 }
 
 // Build on `bk` (nb rows), probe with `pk` (np rows); the output total lands
-// in counter `ci`.
-void run_hash_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk, uint64_t np, const JoinOut& o,
-                   int ci) {
+// in counter 0.  A sized call (`out` given) reads the total back once the matches
+// are counted, gets its columns, and has the total in out->count.
+int run_hash_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk, uint64_t np, JoinOut o, ahead_bat* out) {
     cudaStream_t st = s.ctx->stream;
     const uint32_t cap = ht_capacity(nb);
     HashTab h;
@@ -519,22 +532,32 @@ void run_hash_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk, 
     ProbeSlot* pt = (ProbeSlot*)s.alloc((size_t)(cap + 1) * sizeof(ProbeSlot));
     ht_pack_kernel<<<grid_for(cap + 1, 256), 256, 0, st>>>(h, pt, cap + 1, direct);
     s.launched(6);
-    if (!np) return;
     const uint32_t nt = (uint32_t)((np + kProbeTile - 1) / kProbeTile);
     CompactBufs pb;
     pb.words = nullptr;
     pb.counts = (uint32_t*)s.alloc((size_t)nt * 4);
     pb.offsets = (uint64_t*)s.alloc((size_t)nt * 8);
     pb.gbase = (uint64_t*)s.alloc((size_t)scan_groups(nt) * 8);
-    pb.totals = s.d_counters + ci;
+    pb.totals = s.d_counters;
     pb.done = sb.done;
     pb.ntiles = nt;
     pb.nchan = 1;
     const uint32_t pg = nt < (uint32_t)g ? nt : (uint32_t)g;
     probe_count_kernel<<<pg, 256, 0, st>>>(pt, h.mask, direct, pk, np, pslot, pb);
     tile_scan_kernel<<<scan_groups(nt), kScanGroup, 0, st>>>(pb);
+    s.launched(2);
+    if (out) {
+        const int rc = s.finish(1);
+        if (rc) return rc;
+        out->count = o.cap = s.counter(0);
+        if (!s.take(&out->head, 0, o.cap) || !s.take(&out->tail, 1, o.cap))
+            return fail(s.ctx, AHEAD_NO_MEMORY, "output allocation failed");
+        o.oh = out->head.data;
+        o.ot = out->tail.data;
+    }
     probe_emit_kernel<<<pg, 256, 0, st>>>(pt, h.rows, np, pslot, pb, o);
-    s.launched(3);
+    s.launched();
+    return AHEAD_OK;
 }
 
 bool small_res(int t) { return t == AHEAD_RESTINY || t == AHEAD_RESSHORT || t == AHEAD_RESINT; }
@@ -1611,15 +1634,19 @@ int ahead_gpu_hashjoin_an(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r
         if (k == 3 && eT2)
             run_colcheck(s, r->tail, nr, AT2Inv, r->tail.unenc_max & wmask(wt2e), wt2e, aoid, ev(errs, 3), 4);
     };
-    int rc = s.reserve(dj_scratch(nb, np));
-    if (rc) return rc;
     // error vectors of the probe's key and output column, and the build's
     const int vpk = left ? 2 : 1, vpo = left ? 3 : 0, vbk = left ? 1 : 2, vbo = left ? 0 : 3;
     ErrList kerr, verr;
-    rc = run_direct_join<true>(s, bk, nb, pk, np, o, aoid, ev(errs, vpk), ev(errs, vpo), &kerr, &verr,
-                               s.sized(out, cap) ? out : nullptr);
-    if (rc) return rc;
-    if (!s.counter(kDjBad)) {
+    int rc = AHEAD_OK;
+    const bool direct = dj_possible(nb, np);
+    if (direct) {
+        rc = s.reserve(dj_scratch(nb, np));
+        if (rc) return rc;
+        rc = run_direct_join<true>(s, bk, nb, pk, np, o, aoid, ev(errs, vpk), ev(errs, vpo), &kerr, &verr,
+                                   s.sized(out, cap) ? out : nullptr);
+        if (rc) return rc;
+    }
+    if (direct && !s.counter(kDjBad)) {
         out->count = s.counter(0);
         if (errs) {
             errs[vpk].count = s.counter(1);
@@ -1643,15 +1670,20 @@ int ahead_gpu_hashjoin_an(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r
     }
     rc = s.reserve(join_scratch(nb, np) + colcheck_scratch(nl) * 2 + colcheck_scratch(nr) * 2);
     if (rc) return rc;
-    run_hash_join(s, bk, nb, pk, np, o, 0);
-    for (int k = 0; k < 4; ++k) check(k);
+    const bool sized = s.sized(out, cap);
+    // (build columns that the bitmap form has just found clean are not read again)
+    const bool clean_key = direct && !s.counter(kDjBuildKey), clean_val = direct && !s.counter(kDjBuildVal);
+    rc = run_hash_join(s, bk, nb, pk, np, o, sized ? out : nullptr);
+    if (rc) return rc;
+    for (int k = 0; k < 4; ++k)
+        if (!(clean_key && k == vbk) && !(clean_val && k == vbo)) check(k);
     rc = s.finish(5);
     if (rc) return rc;
-    out->count = s.counter(0);
+    if (!sized) out->count = s.counter(0);
     if (errs)
         for (int k = 0; k < 4; ++k)
             if (errs[k].present) errs[k].count = s.counter(1 + k);
-    return out->count > cap || s.sized(out, cap) ? AHEAD_CAPACITY : AHEAD_OK;
+    return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
 }
 
 int ahead_gpu_hashjoin(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r, int side, ahead_bat* out,
@@ -1683,7 +1715,7 @@ int ahead_gpu_hashjoin(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r, i
     o.probe_is_head = side != AHEAD_HASH_LEFT;
     o.pcol = dcol(side == AHEAD_HASH_LEFT ? r->tail : l->head);
     o.bcol = dcol(side == AHEAD_HASH_LEFT ? l->head : r->tail);
-    if (w < 8) {  // (8-byte keys are raw codes)
+    if (w < 8 && dj_possible(nb, np)) {  // (8-byte keys are raw codes)
         int rc = s.reserve(dj_scratch(nb, np));
         if (rc) return rc;
         ErrList kerr, verr;
@@ -1697,11 +1729,14 @@ int ahead_gpu_hashjoin(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r, i
     }
     int rc = s.reserve(join_scratch(nb, np));
     if (rc) return rc;
-    run_hash_join(s, bk, nb, pk, np, o, 0);
+    const bool sized = s.sized(out, cap);
+    rc = run_hash_join(s, bk, nb, pk, np, o, sized ? out : nullptr);
+    if (rc) return rc;
+    if (sized) return s.wait();
     rc = s.finish(1);
     if (rc) return rc;
     out->count = s.counter(0);
-    return out->count > cap || s.sized(out, cap) ? AHEAD_CAPACITY : AHEAD_OK;
+    return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
 }
 
 int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, int reenc, uint64_t ah1r,

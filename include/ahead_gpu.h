@@ -59,11 +59,10 @@ const char* ahead_status_string(int status);
  * that passes cap = AHEAD_SIZED and null output data counts its rows first,
  * then asks the function for each output column it fills (column 0: head, 1:
  * tail; device memory, 16-byte aligned, NULL: AHEAD_NO_MEMORY), and stores the
- * pointers in `out`.  A call that cannot be sized (repeated join keys, a
- * positional join) returns AHEAD_CAPACITY with the exact count instead and has
- * written no rows.  ahead_gpu_check_and_decode_an asks for columns of its
- * input's length, a merge of keys out of order for the shorter input's.  The
- * function runs on the calling thread, during the call.  ahead_plain_starjoin
+ * pointers in `out`.  A positional join cannot be sized: it returns
+ * AHEAD_CAPACITY with the exact count and has written no rows.
+ * ahead_gpu_check_and_decode_an asks for columns of its input's length, a merge
+ * of keys out of order for the shorter input's.  The function runs on the calling thread, during the call.  ahead_plain_starjoin
  * sets one of its own for its operator calls and leaves the caller's set.  No
  * reference counterpart: its operators grow vectors. */
 #define AHEAD_SIZED UINT64_MAX
