@@ -30,12 +30,57 @@ AHEAD_DEV uint64_t gb_key(const GbKey& k, uint64_t row) {
     return ((t & k.lmask) * (k.ngroups & k.lmask) + (g & k.lmask)) & k.lmask;
 }
 
-__global__ void gb_insert_kernel(HashTab h, GbKey k, uint64_t n, uint32_t* slot_of, uint32_t* first) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t s = ht_insert(h, gb_key(k, i));
-        slot_of[i] = s;
-        if ((uint32_t)i < first[s]) atomicMin(&first[s], (uint32_t)i);  // (a stale word is only larger)
+// A row's first look at the table takes the key word and the first row of the
+// slot its key hashes to together (the slot is the key's own for nearly all
+// rows), and a thread has U rows' looks in flight: at 12M rows of 70,000 dates the
+// call took 555 us with a look at a time.  CHECK: the columns' AN checks
+// ride along, corrupt rows go to short lists.
+template <bool CHECK, int U>
+__global__ void __launch_bounds__(256) gb_insert_kernel(HashTab h, GbKey k, uint64_t n, uint64_t gmax,
+                                                        uint32_t* slot_of, uint32_t* first, ErrList terr,
+                                                        ErrList gerr) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i0 < n; i0 += U * stride) {
+        uint64_t key[U], seen[U];
+        uint32_t slot[U], row[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint64_t i = i0 + u * stride < n ? i0 + u * stride : i0;
+            if (CHECK && i0 + u * stride < n) {
+                if (dec_if(k.tail, load_at(k.tail, i), k.tail.ainv) > k.tail.umax) terr.add(i);
+                if (k.binary && load_at(k.grp, i) * k.gainv > gmax) gerr.add(i);
+            }
+            key[u] = gb_key(k, i);
+            slot[u] = ht_mix(key[u]) & h.mask;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            seen[u] = h.keys[slot[u]];
+            row[u] = first[slot[u]];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint64_t i = i0 + u * stride;
+            if (i >= n) break;
+            if (seen[u] != key[u] || key[u] == kEmptyKey) {
+                slot[u] = ht_insert(h, key[u]);
+                row[u] = first[slot[u]];
+            }
+            slot_of[i] = slot[u];
+            if ((uint32_t)i < row[u]) atomicMin(&first[slot[u]], (uint32_t)i);  // (a stale word is only larger)
+        }
     }
+}
+
+// Four rows a thread once every thread of the grid has them; fewer rows spread thinner.
+template <bool CHECK>
+void launch_gb_insert(const OpScope& s, const HashTab& h, const GbKey& k, uint64_t n, uint64_t gmax, uint32_t* slot_of,
+                      uint32_t* first, const ErrList& terr, const ErrList& gerr) {
+    const uint32_t grid = grid_for(n, 256);
+    if (n >= (1u << 22))
+        gb_insert_kernel<CHECK, 4><<<grid, 256, 0, s.ctx->stream>>>(h, k, n, gmax, slot_of, first, terr, gerr);
+    else
+        gb_insert_kernel<CHECK, 1><<<grid, 256, 0, s.ctx->stream>>>(h, k, n, gmax, slot_of, first, terr, gerr);
 }
 
 // Rows that are the first row of their group, in row order; the rank of such
@@ -98,7 +143,13 @@ __global__ void gb_assign_kernel(const uint32_t* slot_of, const uint32_t* first,
 // (insert 22.8 and 46.2: 8 and 16 bytes a row at 4.2 TB/s, bound by HBM and
 // the L1 gathers).  The columns' AN checks ride along: corrupt rows go to short
 // lists.  A key at or above `limit` raises `over`, and the hash table takes the
-// call.
+// call: when a seed row has one, the grid's passes return at once.  What the
+// attempt costs then (20-30 us: clearing the table, the seed, four empty launches,
+// a wait) the table's insert pass gives back where it checks columns or many rows
+// share a group.  12M rows, 40 wide keys 345 us (980 by the table alone before),
+// 3M wide keys 1,200 (1,365), 70,000 dates 570 (557); unencoded 307 (909),
+// 1,140 (1,285) and 525 (491); 1M rows, 250,000 wide keys: 147 (173), unencoded
+// 138 (128).
 constexpr uint32_t kGbMinLimit = 1u << 16, kGbMaxLimit = 1u << 22;
 constexpr uint32_t kGbSort = 4096;  // groups ranked by one block's sort; more are ranked by the compaction
 constexpr uint32_t kGbSeedRows = 4096;
@@ -152,8 +203,8 @@ template <bool TENC>
 __global__ void __launch_bounds__(1024) small_gb_seed_kernel(SmallGb g) {
     const uint64_t m = g.n < kGbSeedRows ? g.n : kGbSeedRows;
     for (uint64_t i = threadIdx.x; i < m; i += blockDim.x) {
+        if (*(volatile uint32_t*)g.over) return;
         g.slot_of[i] = small_gb_row<TENC>(g, i, load_at(g.k.tail, i), g.k.binary ? load_at(g.k.grp, i) : 0);
-        __syncwarp();
     }
 }
 
@@ -181,6 +232,7 @@ AHEAD_DEV void load4(const DCol& c, uint64_t i, bool vec, uint64_t (&v)[4]) {
 template <int TW, int GW, bool TENC>
 __global__ void __launch_bounds__(256) small_gb_insert_kernel(SmallGb g, bool vec) {
     const uint64_t r0 = kGbSeedRows, m = (g.n - r0) / 4, stride = (uint64_t)gridDim.x * blockDim.x;
+    if (*(volatile uint32_t*)g.over) return;  // (a seed row's key: the hash table has the call)
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += stride) {
         const uint64_t row = r0 + 4 * i;
         uint64_t t[4], gv[4] = {0, 0, 0, 0};
@@ -484,6 +536,22 @@ int run_groupby(ahead_ctx* ctx, const ahead_bat* in, const ahead_bat* grouping, 
     auto check_grp = [&] {
         run_colcheck(s, grouping->tail, n, grouping->tail.Ainv, grouping->tail.unenc_max, 8, aoid, ev(errs, 2), 3);
     };
+    // the error vectors from the lists the insert pass filled, once the counters are read back
+    auto settle = [&](const ErrList& terr, const ErrList& gerr) -> int {
+        const bool ok_t = settle_err_list(s, terr, kGbTail, aoid, ev(errs, 1));
+        const bool ok_g = !binary || settle_err_list(s, gerr, kGbGrp, aoid, ev(errs, 2));
+        if (!ok_t || !ok_g) {  // a column with many corrupt codes
+            int r = s.reserve(2 * colcheck_scratch(n));
+            if (r) return r;
+            if (!ok_t) check_tail();
+            if (!ok_g) check_grp();
+            r = s.finish(4);
+            if (r) return r;
+            if (errs && !ok_t) errs[1].count = s.counter(2);
+            if (errs && !ok_g) errs[2].count = s.counter(3);
+        }
+        return s.wait();
+    };
     auto first_op = [&](const uint32_t* slot_of, const uint32_t* first, uint32_t* gid_of_slot) {
         FirstOp op;
         op.base = (const char*)slot_of;
@@ -516,29 +584,18 @@ int run_groupby(ahead_ctx* ctx, const ahead_bat* in, const ahead_bat* grouping, 
                 s.launched();
             }
         }
-        const bool ok_t = settle_err_list(s, g.terr, kGbTail, aoid, ev(errs, 1));
-        const bool ok_g = !binary || settle_err_list(s, g.gerr, kGbGrp, aoid, ev(errs, 2));
-        if (!ok_t || !ok_g) {  // a column with many corrupt codes
-            rc = s.reserve(2 * colcheck_scratch(n));
-            if (rc) return rc;
-            if (!ok_t) check_tail();
-            if (!ok_g) check_grp();
-            rc = s.finish(4);
-            if (rc) return rc;
-            if (errs && !ok_t) errs[1].count = s.counter(2);
-            if (errs && !ok_g) errs[2].count = s.counter(3);
-        }
         firsts->count = groups;
-        rc = s.wait();
+        rc = settle(g.terr, g.gerr);
         if (rc) return rc;
         return (n > cap || groups > cap) ? AHEAD_CAPACITY : AHEAD_OK;
     }
     // keys beyond the first-row table: the hash table
     const uint32_t cap_slots = ht_capacity(n);
     rc = s.reserve((size_t)(cap_slots + 1) * (8 + 4 + 4) + n * 4 + compact_scratch<FirstOp>(n) +
-                   3 * colcheck_scratch(n) + 4096);
+                   3 * colcheck_scratch(n) + 2 * kErrListBytes + 4096);
     if (rc) return rc;
     cudaStream_t st = ctx->stream;
+    const ErrList terr = err_list(s, kGbTail), gerr = err_list(s, kGbGrp);
     HashTab h{};
     h.mask = cap_slots - 1;
     h.keys = (uint64_t*)s.alloc((size_t)(cap_slots + 1) * 8);
@@ -547,23 +604,19 @@ int run_groupby(ahead_ctx* ctx, const ahead_bat* in, const ahead_bat* grouping, 
     uint32_t* slot_of = (uint32_t*)s.alloc(n * 4);
     cudaMemsetAsync(h.keys, 0xff, (size_t)(cap_slots + 1) * 8, st);
     cudaMemsetAsync(first, 0xff, (size_t)(cap_slots + 1) * 4, st);
-    gb_insert_kernel<<<grid_for(n, 256), 256, 0, st>>>(h, k, n, slot_of, first);
+    launch_gb_insert<true>(s, h, k, n, binary ? grouping->tail.unenc_max : 0, slot_of, first, terr, gerr);
     run_compact(s, first_op(slot_of, first, gid_of_slot), n, 0);
     if (gids->tail.data)
         gb_assign_kernel<<<grid_for(n, 256), 256, 0, st>>>(slot_of, first, gid_of_slot, n, aoid, binary,
                                                             (uint64_t*)gids->tail.data, cap);
     s.launched(2);
     check_head();
-    check_tail();
-    if (binary) check_grp();
-    rc = s.finish(4);
+    rc = s.finish(kGbCounters);
     if (rc) return rc;
     firsts->count = s.counter(0);
-    if (errs) {
-        if (eH) errs[0].count = s.counter(1);
-        errs[1].count = s.counter(2);
-        if (binary) errs[2].count = s.counter(3);
-    }
+    if (errs && eH) errs[0].count = s.counter(1);
+    rc = settle(terr, gerr);
+    if (rc) return rc;
     return (n > cap || firsts->count > cap) ? AHEAD_CAPACITY : AHEAD_OK;
 }
 
@@ -677,7 +730,7 @@ int run_groupby_plain(ahead_ctx* ctx, const ahead_bat* in, const ahead_bat* grou
     uint32_t* slot_of = (uint32_t*)s.alloc(n * 4);
     cudaMemsetAsync(h.keys, 0xff, (size_t)(cap_slots + 1) * 8, st);
     cudaMemsetAsync(first, 0xff, (size_t)(cap_slots + 1) * 4, st);
-    gb_insert_kernel<<<grid_for(n, 256), 256, 0, st>>>(h, k, n, slot_of, first);
+    launch_gb_insert<false>(s, h, k, n, 0, slot_of, first, ErrList{}, ErrList{});
     run_compact(s, first_op(slot_of, first, gid_of_slot), n, 0);
     if (gids->tail.data)
         gb_assign_plain_kernel<<<grid_for(n, 256), 256, 0, st>>>(slot_of, gid_of_slot, n, (uint32_t*)gids->tail.data,
