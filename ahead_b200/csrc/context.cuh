@@ -88,6 +88,7 @@ struct OpScope {
             size_t cap = need < (64u << 20) ? (64u << 20) : need + need / 4;
             e = cudaMalloc(&ctx->arena, cap);
             if (e != cudaSuccess) {
+                cudaGetLastError();  // (not sticky: the caller may do with less)
                 ctx->arena_cap = 0;
                 return fail(ctx, AHEAD_NO_MEMORY, "scratch arena allocation failed");
             }

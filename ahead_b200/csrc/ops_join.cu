@@ -786,7 +786,8 @@ inline bool pos_one_pass(uint64_t n, uint64_t cap, uint64_t sz) {
 constexpr int kPosHead = 30, kPosDrops = 31, kPosCounters = 33;  // counters
 
 // Runs the one-pass form; *kept = rows kept.  Returns AHEAD_UNSUPPORTED when
-// too many rows are dropped and the compaction has to run.  `dense_head`: every
+// too many rows are dropped, or the device memory is short, and the compaction
+// has to run.  `dense_head`: every
 // head is known to read as corrupt, so its vector is made by a column check.
 template <bool CHECKED, bool FETCH>
 int run_pos_join(OpScope& s, PosArgs& a, const ahead_col* head, uint64_t aoid, bool dense_head, ahead_errvec* eh,
@@ -796,7 +797,7 @@ int run_pos_join(OpScope& s, PosArgs& a, const ahead_col* head, uint64_t aoid, b
     const bool want_head = a.head_err && eh;
     const size_t check = want_head ? colcheck_scratch(n) : 0;
     int rc = s.reserve(drop_scratch(n, (FETCH ? 0 : a.ohw) + a.otw) + kErrListBytes + check);
-    if (rc) return rc;
+    if (rc) return rc == AHEAD_NO_MEMORY ? AHEAD_UNSUPPORTED : rc;  // (the compaction needs a tenth of it)
     a.herr = err_list(s, kPosHead);
     a.drops = drop_list(s, kPosDrops);
     uint64_t* sorted = (uint64_t*)s.alloc(kMaxDrops * 8);
@@ -1638,10 +1639,13 @@ int ahead_gpu_hashjoin_an(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r
     const int vpk = left ? 2 : 1, vpo = left ? 3 : 0, vbk = left ? 1 : 2, vbo = left ? 0 : 3;
     ErrList kerr, verr;
     int rc = AHEAD_OK;
-    const bool direct = dj_possible(nb, np);
+    bool direct = dj_possible(nb, np);
     if (direct) {
         rc = s.reserve(dj_scratch(nb, np));
-        if (rc) return rc;
+        if (rc && rc != AHEAD_NO_MEMORY) return rc;
+        direct = !rc;  // (device memory short: the table may need less)
+    }
+    if (direct) {
         rc = run_direct_join<true>(s, bk, nb, pk, np, o, aoid, ev(errs, vpk), ev(errs, vpo), &kerr, &verr,
                                    s.sized(out, cap) ? out : nullptr);
         if (rc) return rc;
@@ -1715,9 +1719,14 @@ int ahead_gpu_hashjoin(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r, i
     o.probe_is_head = side != AHEAD_HASH_LEFT;
     o.pcol = dcol(side == AHEAD_HASH_LEFT ? r->tail : l->head);
     o.bcol = dcol(side == AHEAD_HASH_LEFT ? l->head : r->tail);
-    if (w < 8 && dj_possible(nb, np)) {  // (8-byte keys are raw codes)
-        int rc = s.reserve(dj_scratch(nb, np));
-        if (rc) return rc;
+    int rc = AHEAD_OK;
+    bool direct = w < 8 && dj_possible(nb, np);  // (8-byte keys are raw codes)
+    if (direct) {
+        rc = s.reserve(dj_scratch(nb, np));
+        if (rc && rc != AHEAD_NO_MEMORY) return rc;
+        direct = !rc;
+    }
+    if (direct) {
         ErrList kerr, verr;
         rc = run_direct_join<false>(s, bk, nb, pk, np, o, 0, nullptr, nullptr, &kerr, &verr,
                                     s.sized(out, cap) ? out : nullptr);
@@ -1727,7 +1736,7 @@ int ahead_gpu_hashjoin(ahead_ctx* ctx, const ahead_bat* l, const ahead_bat* r, i
             return out->count > cap ? AHEAD_CAPACITY : AHEAD_OK;
         }
     }
-    int rc = s.reserve(join_scratch(nb, np));
+    rc = s.reserve(join_scratch(nb, np));
     if (rc) return rc;
     const bool sized = s.sized(out, cap);
     rc = run_hash_join(s, bk, nb, pk, np, o, sized ? out : nullptr);

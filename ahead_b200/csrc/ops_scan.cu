@@ -862,10 +862,12 @@ int ahead_gpu_check_and_decode_an(ahead_ctx* ctx, const ahead_bat* in, uint64_t 
         // ones 56 and 82 (the gaps are three more launches and a synchronisation).
         const uint64_t n = in->count;
         const int ow = type_width(ut), w = type_width(t);
-        if (((uintptr_t)in->tail.data % 16) == 0 && ((uintptr_t)out->tail.data % 16) == 0 && out->tail.data &&
-            n >= kDecodeInPlace && n <= cap) {
-            int rc = s.reserve(drop_scratch(n, ow));
-            if (rc) return rc;
+        const bool in_place = ((uintptr_t)in->tail.data % 16) == 0 && ((uintptr_t)out->tail.data % 16) == 0 &&
+                              out->tail.data && n >= kDecodeInPlace && n <= cap;
+        // (an eighth of the output; with the device memory short, the compaction needs a bit a row)
+        int rc = in_place ? s.reserve(drop_scratch(n, ow)) : AHEAD_NO_MEMORY;
+        if (rc && rc != AHEAD_NO_MEMORY) return rc;
+        if (!rc) {
             const DropList drops = drop_list(s, 0);
             uint64_t* sorted = (uint64_t*)s.alloc(kMaxDrops * 8);
             const uint64_t blocks = (n * w / 16 + 511) / 512;
