@@ -181,21 +181,6 @@ struct RangePred {
     }
 };
 
-// ----------------------------------------------------------------- memory order
-AHEAD_DEV uint64_t ld_acquire(const uint64_t* p) {
-    uint64_t v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-AHEAD_DEV void st_release(uint64_t* p, uint64_t v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-AHEAD_DEV uint32_t ld_acquire32(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
 // ----------------------------------------------------------------- warp scans
 AHEAD_DEV uint32_t warp_incl_scan(uint32_t v) {
     const int lane = threadIdx.x & 31;
@@ -221,11 +206,7 @@ AHEAD_DEV uint64_t warp_sum64(uint64_t v) {
     return v;
 }
 
-// Device-side status word bits (written with atomicOr, read by the host).
-enum : uint32_t {
-    kDevStatusCapacity = 2u,     // an output did not fit
-    kDevStatusDupKey = 4u,       // a build side had duplicate keys (fused paths only)
-    kDevStatusBadInput = 8u,     // an input outside the supported domain
-};
+// Status bit of the star engine's header (set with atomicOr, read by the host).
+constexpr uint32_t kDevStatusCapacity = 2u;  // an output did not fit
 
 }  // namespace ahead

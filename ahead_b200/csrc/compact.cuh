@@ -100,7 +100,7 @@ inline size_t compact_bytes(uint64_t n, uint32_t ntiles, uint32_t nchan) {
 //   void put0(int k, uint64_t pos, uint64_t val) const;    store it at pos < cap0()
 //   void rows0(v[U], row0, idx[U], val[NOUT][U]) const;    optional: the outputs of U kept
 //                               rows row0 + idx[u] at once, so that their loads overlap
-//   void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const;  streams c >= 1
+//   void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const;  streams c >= 1, if there are any
 //
 //   void begin();  optional: loads what eval and out0 need from device memory, once per thread
 //   void tile(uint32_t t);  optional: the same for each tile, before its rows

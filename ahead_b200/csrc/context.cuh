@@ -18,7 +18,7 @@ struct ahead_ctx {
     bool own_stream = false;
     char* arena = nullptr;  // device scratch, reused by every call
     size_t arena_cap = 0;
-    bool header_clean = false;  // the arena's status word and counters are zero
+    bool header_clean = false;  // the arena's counters are zero
     uint64_t* h_stage = nullptr;  // pinned host words for count read-back (device-writable)
     uint64_t launches = 0;
     int num_sms = 148;
@@ -54,8 +54,8 @@ inline int cuda_fail(ahead_ctx* ctx, cudaError_t e, const char* where) {
         if (_e != cudaSuccess) return ::ahead::cuda_fail((ctx), _e, #call); \
     } while (0)
 
-// Ends an operator: the status word and the first `n` counters go to the pinned
-// host words, and the header is left zero for the next call.  (A copy to the
+// Ends an operator: the first `n` counters (words 1 to n) go to the pinned host
+// words, and the header is left zero for the next call.  (A copy to the
 // host and a clear ahead of the next call's kernels cost each call 7 us more.)
 static __global__ void __launch_bounds__(kStageWords) publish_kernel(uint64_t* header, uint64_t* host, int n) {
     const int i = threadIdx.x;
@@ -64,13 +64,12 @@ static __global__ void __launch_bounds__(kStageWords) publish_kernel(uint64_t* h
     if (v) header[i] = 0;
 }
 
-// One operator call.  Layout of the arena: [status word + 63 counters][bump
+// One operator call.  Layout of the arena: [a spare word, 63 counters][bump
 // region].  reserve() must be called with the call's total scratch need
 // before any pointer is handed out (it may reallocate the arena).
 struct OpScope {
     ahead_ctx* ctx;
     size_t off = 0;
-    uint32_t* d_status = nullptr;
     uint64_t* d_counters = nullptr;  // [kStageWords - 1]
     int rc = AHEAD_OK;
     bool pending = false;  // launches since the last wait
@@ -94,7 +93,6 @@ struct OpScope {
             }
             ctx->arena_cap = cap;
         }
-        d_status = (uint32_t*)ctx->arena;
         d_counters = (uint64_t*)(ctx->arena + 8);
         off = 512;
         if (!ctx->header_clean) {
@@ -145,9 +143,8 @@ struct OpScope {
         return e == cudaSuccess ? AHEAD_OK : cuda_fail(ctx, e, "cudaStreamSynchronize");
     }
 
-    // Read the status word and the first `ncounters` counters back and wait for
-    // the stream.  Returns the call's status.  The device's counters are zero
-    // from here on.
+    // Read the first `ncounters` counters back and wait for the stream.  The
+    // device's counters are zero from here on.
     int finish(int ncounters) {
         pending = false;
         publish_kernel<<<1, kStageWords, 0, ctx->stream>>>((uint64_t*)ctx->arena, ctx->h_stage, ncounters);
@@ -157,8 +154,6 @@ struct OpScope {
         e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamSynchronize");
         ctx->header_clean = true;
-        uint32_t st = (uint32_t)ctx->h_stage[0];
-        if (st & kDevStatusBadInput) return fail(ctx, AHEAD_UNSUPPORTED, "input outside the supported domain");
         return AHEAD_OK;
     }
     uint64_t counter(int i) const { return ctx->h_stage[1 + i]; }

@@ -20,14 +20,13 @@
 //     current, and caches it); creating a context on the device drops the
 //     cached address, so a device reset between contexts is safe, but a
 //     context must not be used across a reset of its device;
-//   * every call copies its status to the host and waits for its stream, so
+//   * every call copies its count to the host and waits for its stream, so
 //     a call blocks and is never usable inside stream capture;
 //   * the scratch is one buffer per device: calls must not overlap on a device
 //     (one stream, or wait for the previous call to return -- each call
 //     returns only after its stream has finished); overlapping calls race;
-//   * what must start at zero: the status word and the counters (first 512
-//     bytes); each call clears them with cudaMemsetAsync on the context's
-//     stream before its kernels run.
+//   * what must start at zero: the counters (first 512 bytes); each call clears
+//     them with cudaMemsetAsync on the context's stream before its kernels run.
 // Results are those of ahead_gpu_check_an (checkAN, encdecAN_scalar.tcc:
 // 69-94): the positions row * AOID of the codes whose decoded value exceeds the
 // largest unencoded value.  The reference has no such entry point.
@@ -44,7 +43,7 @@ constexpr uint64_t kNoAllocMaxRows = 1ull << 24;
 constexpr uint32_t kNoAllocTiles = (uint32_t)(kLongColumn / (32 * short_k(8)));
 static_assert(kNoAllocMaxRows / (32 * kLongK) <= kNoAllocTiles, "long tiles need no more");
 constexpr size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
-constexpr size_t kHeadBytes = 512;  // status word (8 B) + counters
+constexpr size_t kHeadBytes = 512;  // counters, behind a spare word
 constexpr size_t kWordsBytes = align256((size_t)(kNoAllocMaxRows / 8));
 constexpr size_t kCountsBytes = align256((size_t)kNoAllocTiles * 4);
 constexpr size_t kOffsetsBytes = align256((size_t)kNoAllocTiles * 8);
@@ -96,7 +95,6 @@ int check_noalloc(ahead_ctx* ctx, unsigned char* scratch, const ahead_bat* in, u
     typedef CheckOp<W> Op;
     const uint64_t n = in->count;
     cudaStream_t st = ctx->stream;
-    uint32_t* status = reinterpret_cast<uint32_t*>(scratch);
     uint64_t* counters = reinterpret_cast<uint64_t*>(scratch + 8);
     cudaError_t e = cudaMemsetAsync(scratch, 0, kHeadBytes, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemsetAsync");
@@ -113,7 +111,6 @@ int check_noalloc(ahead_ctx* ctx, unsigned char* scratch, const ahead_bat* in, u
         cb.nchan = Op::NCH;
         Op op;
         op.base = (const char*)in->tail.data;
-        op.status = status;
         op.ainv = ainv & wmask(W);
         op.umax = unenc_max & wmask(W);
         op.aoid = aoid;
@@ -124,12 +121,12 @@ int check_noalloc(ahead_ctx* ctx, unsigned char* scratch, const ahead_bat* in, u
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
-    uint64_t h[2] = {0, 0};  // status word, error count (pageable host copy: no pinned buffer)
-    e = cudaMemcpyAsync(h, scratch, sizeof h, cudaMemcpyDeviceToHost, st);
+    uint64_t errors = 0;  // (pageable host copy: no pinned buffer)
+    e = cudaMemcpyAsync(&errors, counters, sizeof errors, cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemcpyAsync");
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamSynchronize");
-    if (err) err->count = n ? h[1] : 0;
+    if (err) err->count = n ? errors : 0;
     return AHEAD_OK;
 }
 

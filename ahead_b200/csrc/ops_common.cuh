@@ -48,7 +48,6 @@ struct CheckOp {
     static constexpr bool ACC = false;
     static constexpr bool GATHER = false;
     const char* base;
-    uint32_t* status;
     uint64_t ainv, umax, aoid, errcap;
     uint64_t* err;
     uint64_t* acc;
@@ -61,9 +60,6 @@ struct CheckOp {
     AHEAD_DEV uint64_t cap0() const { return errcap; }
     AHEAD_DEV void* optr(int) const { return err; }
     AHEAD_DEV int owidth(int) const { return 8; }
-    AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
-        if (pos < errcap) err[pos] = row * aoid;
-    }
 };
 
 
@@ -79,7 +75,6 @@ struct ColCheckOp {
     static constexpr bool EMIT_V = false;
     static constexpr int NOUT = 1;
     const char* base;
-    uint32_t* status;
     uint64_t ainv, umax, aoid, errcap, wmaskenc;
     uint64_t* err;
     uint64_t* acc;
@@ -88,9 +83,6 @@ struct ColCheckOp {
     AHEAD_DEV uint64_t cap0() const { return errcap; }
     AHEAD_DEV void* optr(int) const { return err; }
     AHEAD_DEV int owidth(int) const { return 8; }
-    AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
-        if (pos < errcap) err[pos] = row * aoid;
-    }
 };
 
 inline size_t colcheck_scratch(uint64_t n) { return compact_scratch<ColCheckOp<8>>(n); }
@@ -103,7 +95,6 @@ inline void run_colcheck(OpScope& s, const ahead_col& c, uint64_t n, uint64_t ai
         constexpr int W = decltype(tag)::value;
         ColCheckOp<W> op;
         op.base = (const char*)c.data;
-        op.status = s.d_status;
         op.ainv = ainv;
         op.umax = umax;
         op.aoid = aoid;

@@ -93,7 +93,6 @@ struct FirstOp {
     static constexpr bool EMIT_V = false;
     static constexpr int NOUT = 1;
     const char* base;
-    uint32_t* status;
     const uint32_t* first;
     uint32_t* gid_of_slot;
     DCol head;
@@ -113,7 +112,6 @@ struct FirstOp {
             firsts[pos] = (decode_head ? dec_if(head, h, head.ainv) : h) * aoid;
         }
     }
-    AHEAD_DEV void emit(int, uint64_t, uint64_t, uint64_t) const {}
 };
 
 // Encoded group id of every row.  The binary group-by's dictionary stores the
@@ -555,7 +553,6 @@ int run_groupby(ahead_ctx* ctx, const ahead_bat* in, const ahead_bat* grouping, 
     auto first_op = [&](const uint32_t* slot_of, const uint32_t* first, uint32_t* gid_of_slot) {
         FirstOp op;
         op.base = (const char*)slot_of;
-        op.status = s.d_status;
         op.first = first;
         op.gid_of_slot = gid_of_slot;
         op.head = hc;
@@ -635,7 +632,6 @@ struct FirstPlainOp {
     static constexpr bool EMIT_V = false;
     static constexpr int NOUT = 1;
     const char* base;
-    uint32_t* status;
     const uint32_t* first;
     uint32_t* gid_of_slot;
     DCol head;
@@ -650,7 +646,6 @@ struct FirstPlainOp {
         gid_of_slot[s] = (uint32_t)pos;
         if (pos < cap) firsts[pos] = (uint32_t)load_at(head, row);
     }
-    AHEAD_DEV void emit(int, uint64_t, uint64_t, uint64_t) const {}
 };
 
 __global__ void gb_assign_plain_kernel(const uint32_t* slot_of, const uint32_t* gid_of_slot, uint64_t n,
@@ -689,7 +684,6 @@ int run_groupby_plain(ahead_ctx* ctx, const ahead_bat* in, const ahead_bat* grou
     auto first_op = [&](const uint32_t* slot_of, const uint32_t* first, uint32_t* gid_of_slot) {
         FirstPlainOp op;
         op.base = (const char*)slot_of;
-        op.status = s.d_status;
         op.first = first;
         op.gid_of_slot = gid_of_slot;
         op.head = dcol(in->head);
@@ -1020,7 +1014,6 @@ int ahead_gpu_groupby2_str_an(ahead_ctx* ctx, const char* strs, uint64_t width, 
         vh.seqbase = seqbase;
         FirstOp op;
         op.base = (const char*)slot_of;
-        op.status = s.d_status;
         op.first = first;
         op.gid_of_slot = gid_of_slot;
         op.head = dcol(vh);
@@ -1078,7 +1071,6 @@ int ahead_gpu_groupby2_str(ahead_ctx* ctx, const char* strs, uint64_t width, uin
         vh.seqbase = seqbase;
         FirstPlainOp op;
         op.base = (const char*)slot_of;
-        op.status = s.d_status;
         op.first = first;
         op.gid_of_slot = gid_of_slot;
         op.head = dcol(vh);

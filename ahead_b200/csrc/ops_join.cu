@@ -482,8 +482,13 @@ int run_direct_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk,
         launch_emit(s, op, np, cb);
         return out ? s.wait() : s.finish(kDjCounters);
     };
-    if constexpr (AN) return by_width_enc(pk.width, probe);
-    else return by_width(pk.width, probe);
+    if constexpr (AN) {
+        return by_width_enc(pk.width, probe);
+    } else {  // (8-byte raw codes do not come here)
+        if (pk.width == 1) return probe(std::integral_constant<int, 1>());
+        if (pk.width == 2) return probe(std::integral_constant<int, 2>());
+        return probe(std::integral_constant<int, 4>());
+    }
 }
 
 size_t join_scratch(uint64_t nb, uint64_t np) {
@@ -588,7 +593,6 @@ struct MjPosOp {
     static constexpr bool EMIT_V = true;
     static constexpr int NOUT = 2;
     const char* base;
-    uint32_t* status;
     DCol h1c, t2c;
     uint64_t at1inv, ah1inv, ah1max, sz, fh, ft, cap, aoid, ec1, ec2, ec4;
     uint64_t *e1, *e2, *e4, *acc;
@@ -643,7 +647,6 @@ struct FetchOp {
     static constexpr bool EMIT_V = true;
     static constexpr int NOUT = 1;
     const char* base;
-    uint32_t* status;
     DCol t2c;
     uint64_t at1inv, at2inv, at2max, vsz, fac, cap, aoid, ec1, ec2;
     uint64_t *e1, *e2, *acc;
@@ -1187,7 +1190,6 @@ struct IsectOp {
     AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void* optr(int k) const { return k == 0 ? oh : ot; }
     AHEAD_DEV int owidth(int k) const { return k == 0 ? ohw : otw; }
-    AHEAD_DEV void emit(int, uint64_t, uint64_t, uint64_t) const {}
 };
 
 // Pass 1 through the byte map, one warp per tile; word s of a tile is the
@@ -1461,7 +1463,6 @@ struct FetchStrOp {
     static constexpr bool EMIT_V = true;
     static constexpr int NOUT = 1;
     const char* base;
-    uint32_t* status;
     uint64_t ainv, count, aoid, cap, errcap;
     uint32_t* rows;
     uint64_t* err;
@@ -1471,8 +1472,8 @@ struct FetchStrOp {
     AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void* optr(int) const { return rows; }
     AHEAD_DEV int owidth(int) const { return 4; }
-    AHEAD_DEV void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const {
-        if (c == 1 && pos < errcap) err[pos] = row * aoid;
+    AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
+        if (pos < errcap) err[pos] = row * aoid;
     }
 };
 
@@ -1486,7 +1487,6 @@ struct FetchStrPlainOp {
     static constexpr bool EMIT_V = true;
     static constexpr int NOUT = 1;
     const char* base;
-    uint32_t* status;
     uint64_t count, cap;
     uint32_t* rows;
     uint64_t* acc;
@@ -1495,7 +1495,6 @@ struct FetchStrPlainOp {
     AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void* optr(int) const { return rows; }
     AHEAD_DEV int owidth(int) const { return 4; }
-    AHEAD_DEV void emit(int, uint64_t, uint64_t, uint64_t) const {}
 };
 
 // The slots of a compacted row list, into `out` (the second step of both string fetch-joins).
@@ -1810,7 +1809,6 @@ int ahead_gpu_matchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
         if (rc) return rc;
         MjPosOp<true> op;
         op.base = (const char*)a->tail.data;
-        op.status = s.d_status;
         op.h1c = h1;
         op.t2c = t2;
         op.at1inv = a->tail.Ainv;
@@ -2025,7 +2023,6 @@ int ahead_gpu_matchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, 
         if (rc) return rc;
         MjPosOp<false> op{};
         op.base = (const char*)a->tail.data;
-        op.status = s.d_status;
         op.h1c = h1;
         op.t2c = t2;
         op.sz = n2;
@@ -2128,7 +2125,6 @@ int ahead_gpu_fetchjoin_an(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* 
     if (rc) return rc;
     FetchOp<true> op;
     op.base = (const char*)a->tail.data;
-    op.status = s.d_status;
     op.t2c = dcol(b->tail);
     op.at1inv = a->tail.Ainv;
     op.at2inv = b->tail.Ainv & wmask(w);
@@ -2187,7 +2183,6 @@ int ahead_gpu_fetchjoin(ahead_ctx* ctx, const ahead_bat* a, const ahead_bat* b, 
     if (rc) return rc;
     FetchOp<false> op{};
     op.base = (const char*)a->tail.data;
-    op.status = s.d_status;
     op.t2c = dcol(b->tail);
     op.vsz = b->count;
     op.fac = 1;
@@ -2220,7 +2215,6 @@ int ahead_gpu_fetchjoin_str_an(ahead_ctx* ctx, const ahead_bat* a, const char* s
     uint32_t* rows = (uint32_t*)s.alloc((n ? n : 1) * 4);
     FetchStrOp op;
     op.base = (const char*)a->tail.data;
-    op.status = s.d_status;
     op.ainv = a->tail.Ainv;
     op.count = count;
     op.aoid = aoid;
@@ -2252,7 +2246,6 @@ int ahead_gpu_fetchjoin_str(ahead_ctx* ctx, const ahead_bat* a, const char* strs
     uint32_t* rows = (uint32_t*)s.alloc((n ? n : 1) * 4);
     FetchStrPlainOp op;
     op.base = (const char*)a->tail.data;
-    op.status = s.d_status;
     op.count = count;
     op.cap = n;
     op.rows = rows;

@@ -23,7 +23,6 @@ struct SelectOp {
     static constexpr bool ACC = false;
     static constexpr bool GATHER = false;
     const char* base;
-    uint32_t* status;
     uint64_t seqbase, ainv, umax, aoid, cap, errcap;
     uint64_t* out_an;
     uint32_t* out_oid;
@@ -56,16 +55,8 @@ struct SelectOp {
             return b;
         }
     }
-    AHEAD_DEV void emit(int c, uint64_t pos, uint64_t, uint64_t row) const {
-        const uint32_t oid = (uint32_t)(seqbase + row);
-        if (c == 0) {
-            if (pos < cap) {
-                if (AN) out_an[pos] = (uint64_t)oid * kResoidAMax;
-                else out_oid[pos] = oid;
-            }
-        } else if (pos < errcap) {
-            err[pos] = row * aoid;
-        }
+    AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
+        if (pos < errcap) err[pos] = row * aoid;
     }
 };
 
@@ -78,7 +69,6 @@ int run_select(OpScope& s, const ahead_bat* in, const RangePred& p, uint64_t aoi
     if (rc) return rc;
     Op op;
     op.base = (const char*)in->tail.data;
-    op.status = s.d_status;
     op.seqbase = in->head.seqbase;
     op.ainv = in->tail.Ainv & wmask(W);
     op.umax = in->tail.unenc_max & wmask(W);
@@ -177,7 +167,6 @@ int run_select_str(ahead_ctx* ctx, const char* strs, uint64_t width, uint64_t co
     }
     Op op;  // over the flag bytes: A^-1 = 1 and maximum 0xFF, so no flag is ever reported as corrupt
     op.base = (const char*)flags;
-    op.status = s.d_status;
     op.seqbase = seqbase;
     op.ainv = 1;
     op.umax = 0xFF;
@@ -242,7 +231,6 @@ struct CadVoidOp {
     static constexpr bool ACC = false;
     static constexpr bool GATHER = false;
     const char* base;
-    uint32_t* status;
     void* out;
     int ow;
     uint64_t ainv, umax, aoid, cap, errcap;
@@ -257,12 +245,8 @@ struct CadVoidOp {
     AHEAD_DEV uint64_t cap0() const { return cap; }
     AHEAD_DEV void* optr(int) const { return out; }
     AHEAD_DEV int owidth(int) const { return ow; }
-    AHEAD_DEV void emit(int c, uint64_t pos, uint64_t v, uint64_t row) const {
-        if (c == 0) {
-            if (pos < cap) store_at(out, ow, pos, mulw(v, ainv, W));
-        } else if (pos < errcap) {
-            err[pos] = row * aoid;
-        }
+    AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
+        if (pos < errcap) err[pos] = row * aoid;
     }
 };
 
@@ -276,7 +260,6 @@ struct CadGenOp {
     static constexpr bool ACC = false;
     static constexpr bool GATHER = false;
     const char* base;
-    uint32_t* status;
     DCol hc, tc;
     void *oh, *ot;
     int ohw, otw;
@@ -297,13 +280,8 @@ struct CadGenOp {
         const bool hok = !hc.enc || dh <= hc.umax, tok = dt <= tc.umax;
         return (hok && tok ? 1u : 0u) | (hok ? 0u : 2u) | (tok ? 0u : 4u);
     }
-    AHEAD_DEV void emit(int c, uint64_t pos, uint64_t t, uint64_t row) const {
-        if (c == 0) {
-            if (pos < cap) {
-                store_at(oh, ohw, pos, dec_if(hc, load_at(hc, row), hc.ainv));
-                store_at(ot, otw, pos, mulw(t, tc.ainv, W));
-            }
-        } else if (c == 1) {
+    AHEAD_DEV void emit(int c, uint64_t pos, uint64_t, uint64_t row) const {
+        if (c == 1) {
             if (pos < ecap_h) err_h[pos] = row * aoid;
         } else if (pos < ecap_t) {
             err_t[pos] = row * aoid;
@@ -319,7 +297,6 @@ struct DecodeOp {
     static constexpr bool ACC = false;
     static constexpr bool GATHER = false;
     const char* base;
-    uint32_t* status;
     DCol hc, tc;
     void *oh, *ot;
     int ohw, otw;
@@ -338,9 +315,6 @@ struct DecodeOp {
         store_at(ot, otw, row, d);
         return d > tc.umax ? 1u : 0u;
     }
-    AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
-        if (pos < errcap) err[pos] = row * aoid;
-    }
 };
 
 // ------------------------------------------------------------ mul-sum
@@ -353,7 +327,6 @@ struct MulSumOp {
     static constexpr bool ACC = true;
     static constexpr bool GATHER = false;
     const char* base;
-    uint32_t* status;
     DCol ac, bc;
     uint64_t aoid, ecap1, ecap2;
     uint64_t *e1, *e2;
@@ -369,12 +342,8 @@ struct MulSumOp {
         s += a * b;
         return (mulw(a, ac.ainv, W) > ac.umax ? 1u : 0u) | (mulw(b, bc.ainv, bc.width) > bc.umax ? 2u : 0u);
     }
-    AHEAD_DEV void emit(int c, uint64_t pos, uint64_t, uint64_t row) const {
-        if (c == 0) {
-            if (pos < ecap1) e1[pos] = row * aoid;
-        } else if (pos < ecap2) {
-            e2[pos] = row * aoid;
-        }
+    AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
+        if (pos < ecap2) e2[pos] = row * aoid;
     }
 };
 
@@ -546,7 +515,6 @@ struct ArithOp {
     static constexpr bool ACC = false;
     static constexpr bool GATHER = false;
     const char* base;
-    uint32_t* status;
     DCol ac, bc;
     uint64_t ar, aoid, ecap1, ecap2;
     uint64_t *e1, *e2;
@@ -572,12 +540,8 @@ struct ArithOp {
         store_at(out, ow, row, v);
         return (t1 > ac.umax ? 1u : 0u) | (t2 > bc.umax ? 2u : 0u);
     }
-    AHEAD_DEV void emit(int c, uint64_t pos, uint64_t, uint64_t row) const {
-        if (c == 0) {
-            if (pos < ecap1) e1[pos] = row * aoid;
-        } else if (pos < ecap2) {
-            e2[pos] = row * aoid;
-        }
+    AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
+        if (pos < ecap2) e2[pos] = row * aoid;
     }
 };
 
@@ -652,7 +616,6 @@ int restiny_promoted_check(ahead_ctx* ctx, const uint16_t* codes, uint64_t n, ui
     }
     Op op;
     op.base = (const char*)flags;
-    op.status = s.d_status;
     op.seqbase = 0;
     op.ainv = 1;
     op.umax = 0;  // every set flag is an error row
@@ -782,7 +745,6 @@ int ahead_gpu_check_an(ahead_ctx* ctx, const ahead_bat* in, uint64_t ainv, uint6
         if (rc) return rc;
         Op op;
         op.base = (const char*)in->tail.data;
-        op.status = s.d_status;
         op.ainv = ainv & wmask(W);
         op.umax = unenc_max & wmask(W);
         op.aoid = aoid;
@@ -816,7 +778,6 @@ int ahead_gpu_decode_an(ahead_ctx* ctx, const ahead_bat* in, uint64_t aoid, ahea
         if (rc) return rc;
         Op op;
         op.base = (const char*)in->tail.data;
-        op.status = s.d_status;
         op.hc = dcol(in->head);
         op.tc = dcol(in->tail);
         op.oh = out->head.data;
@@ -907,7 +868,6 @@ int ahead_gpu_check_and_decode_an(ahead_ctx* ctx, const ahead_bat* in, uint64_t 
             if (rc) return rc;
             Op op;
             op.base = (const char*)in->tail.data;
-            op.status = s.d_status;
             op.out = out->tail.data;
             op.ow = type_width(ut);
             op.ainv = in->tail.Ainv & wmask(W);
@@ -936,7 +896,6 @@ int ahead_gpu_check_and_decode_an(ahead_ctx* ctx, const ahead_bat* in, uint64_t 
         if (rc) return rc;
         Op op;
         op.base = (const char*)in->tail.data;
-        op.status = s.d_status;
         op.hc = dcol(in->head);
         op.tc = dcol(in->tail);
         op.oh = out->head.data;
@@ -1038,7 +997,6 @@ int ahead_gpu_aggregate_mul_sum_an(ahead_ctx* ctx, const ahead_bat* a, const ahe
         if (rc) return rc;
         Op op;
         op.base = (const char*)a->tail.data;
-        op.status = s.d_status;
         op.ac = dcol(a->tail);
         op.bc = dcol(b->tail);
         op.aoid = aoid;
@@ -1133,7 +1091,6 @@ int ahead_gpu_arithmetic_an(ahead_ctx* ctx, int op, int result_type, const ahead
         if (rc) return rc;
         Op o;
         o.base = (const char*)a->tail.data;
-        o.status = s.d_status;
         o.ac = dcol(a->tail);
         o.bc = dcol(b->tail);
         o.ar = ar;
