@@ -734,7 +734,7 @@ __global__ void __launch_bounds__(256) pos_join_kernel(PosArgs a) {
         }
         gather_rows(a.t2c, p, val[1]);
         if (!FETCH) {
-            if (CHECKED && a.h1c.data == a.base) {  // a mirrored list: the head is the OID itself
+            if (CHECKED && a.h1c.type != AHEAD_VOID && a.h1c.data == a.base) {  // a mirrored list: the head is the OID itself
 #pragma unroll
                 for (int u = 0; u < kPosRows; ++u) val[0][u] = v[u];
             } else {
