@@ -104,7 +104,7 @@ struct SjDimDev {
     uint64_t cmagic;
     const unsigned long long* acc;  // [kAccEntries] accept masks by record
     uint64_t fk_ainv, kmin, krange;
-    uint32_t fk_a, pad_a;           // the multiplier A = (A^-1)^-1 mod 2^32
+    uint32_t fk_a;                  // the multiplier A = (A^-1)^-1 mod 2^32
     unsigned long long joins, first;  // queries joining / joining first
     // join index slot of this dimension (1 or 2: the first or second word of
     // a fact row's entry; 0: not indexed), read by the indexed cube scans
@@ -241,7 +241,7 @@ struct SjBatch {
     uint64_t flist_cap[2];
     uint32_t* fbad;
     uint32_t flist_on, flist_dim, flist_next;
-    uint32_t ref_on, ref_dim, flist_pad;
+    uint32_t ref_on, ref_dim;
     uint32_t flist_chunk[2];  // entries a warp takes of a list at a time
     // bit k set when some query of the batch accepts key offset k of the dimension;
     // the words of it that the filters hold: the map itself, or a bit per 2^pffold keys
