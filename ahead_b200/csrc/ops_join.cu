@@ -5,16 +5,19 @@
 // cast to the unencoded base type, probe in probe-row order and emit every match
 // in build order (lib/column_operators/AN/hashjoinAN.tcc:54-223).  Unique keys
 // of a bounded range (a dimension's keys) index a bitmap and a value array
-// directly, and the probe is a compaction; anything else takes the hash table
-// of hash.cuh.  Rows with detected errors are still built and probed, exactly
-// as in the reference; the four error vectors are checks of the four inputs.
+// directly, and the probe is a compaction; anything else, and a call with too
+// little device memory for these, takes the hash table of hash.cuh.  Rows with
+// detected errors are still built and probed, exactly as in the reference; the
+// four error vectors are checks of the four inputs.
 //
-// Positional match/fetch joins are compactions over the OID list with a gather
-// (matchjoinAN.tcc:226-354).  The merge matchjoin (matchjoinAN.tcc:46-144) is
-// an intersection when both inputs are strictly increasing and clean (the
-// common case: two selection vectors); otherwise the reference's merge loop is
-// replayed step by step on the device so that every error push (including its
-// repeated checks of the same row) is reproduced.
+// Positional match/fetch joins (matchjoinAN.tcc:226-354) gather once per OID,
+// write every row to its own place and close the gaps of the few rows they drop;
+// short lists, many dropped rows and short device memory take a compaction over
+// the list.  The merge matchjoin (matchjoinAN.tcc:46-144) is an intersection when
+// the keys of both inputs strictly increase (the common case: two selection
+// vectors), with the error positions of corrupt values derived per row; keys out
+// of order replay the reference's merge loop step by step on the device, so that
+// every error push (including its repeated checks of the same row) is reproduced.
 #include "hash.cuh"
 #include "ops_common.cuh"
 

@@ -1,11 +1,13 @@
 // ops_scan.cu -- streaming AN operators: selectAN / select, checkAN,
 // decodeAN, checkAndDecodeAN, encodeAN, aggregate_mul_sum(AN), arithmeticAN.
 //
-// Each operator is one pass over its input columns through the compaction
-// kernel of compact.cuh: the AN check is fused into the load (multiply by
-// A^-1 mod 2^w, compare with the largest valid value), predicates are
-// evaluated on the codes, and kept rows and error positions are written in
-// scan order.
+// The AN check is fused into the load (multiply by A^-1 mod 2^w, compare with the
+// largest valid value) and predicates are evaluated on the codes.  Selections go
+// through the compaction of compact.cuh, which writes kept rows and error
+// positions in scan order.  Operators that keep every row (checkAN, the sums,
+// arithmeticAN) read their columns once and list the rare corrupt rows; the
+// compaction makes the vectors when a list overflows.  A large checkAndDecodeAN
+// decodes every row to its own place and then closes the gaps of the corrupt ones.
 #include <cstring>
 
 #include "ops_common.cuh"

@@ -62,9 +62,10 @@ const char* ahead_status_string(int status);
  * pointers in `out`.  A positional join cannot be sized: it returns
  * AHEAD_CAPACITY with the exact count and has written no rows.
  * ahead_gpu_check_and_decode_an asks for columns of its input's length, a merge
- * of keys out of order for the shorter input's.  The function runs on the calling thread, during the call.  ahead_plain_starjoin
- * sets one of its own for its operator calls and leaves the caller's set.  No
- * reference counterpart: its operators grow vectors. */
+ * of keys out of order for the shorter input's.  The function runs on the calling
+ * thread, during the call.  ahead_plain_starjoin sets one of its own for its
+ * operator calls and leaves the caller's set.  No reference counterpart: its
+ * operators grow vectors. */
 #define AHEAD_SIZED UINT64_MAX
 typedef void* (*ahead_output_fn)(void* user, int column, uint64_t bytes);
 void ahead_ctx_set_output_fn(ahead_ctx* ctx, ahead_output_fn fn, void* user);
