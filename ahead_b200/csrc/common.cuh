@@ -181,6 +181,15 @@ struct RangePred {
     }
 };
 
+// A word through L1, for flags and minima that other warps raise or lower meanwhile:
+// a stale value only shows an earlier state.  (A volatile read goes to L2, where the
+// reads of all warps queue on the one word behind each other and behind its writes.)
+AHEAD_DEV uint32_t ld_ca(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 // ----------------------------------------------------------------- warp scans
 AHEAD_DEV uint32_t warp_incl_scan(uint32_t v) {
     const int lane = threadIdx.x & 31;

@@ -167,12 +167,6 @@ struct SmallGb {
     ErrList terr, gerr;
 };
 
-AHEAD_DEV uint32_t ld_ca(const uint32_t* p) {  // cached: a stale word only shows a later row, or none
-    uint32_t v;
-    asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
-
 template <bool TENC>
 AHEAD_DEV uint32_t small_gb_row(const SmallGb& g, uint64_t row, uint64_t tv, uint64_t gv) {
     const uint64_t t = TENC ? mulw(tv, g.k.tail.ainv, g.k.tail.width) : tv;

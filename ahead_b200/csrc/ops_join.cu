@@ -271,6 +271,8 @@ __global__ void __launch_bounds__(256) dj_bounds_kernel(DjBuild b) {
 
 // Sets each key's bit and value.  Neighbouring lanes hold neighbouring keys
 // (dimension tables are in key order), so the lanes of one word share one atomic.
+// Once a key has repeated the warps stop, and no more of them write the word: 3M rows
+// of 200K keys took 575 us with volatile reads of it next to every warp's write.
 __global__ void __launch_bounds__(256) dj_insert_kernel(DjBuild b) {
     const uint64_t kmin = b.kmin(), span = b.span(), stride = (uint64_t)gridDim.x * blockDim.x;
     if (span > b.limit) {
@@ -279,7 +281,7 @@ __global__ void __launch_bounds__(256) dj_insert_kernel(DjBuild b) {
     }
     const uint64_t rounds = (b.nb + stride - 1) / stride;
     for (uint64_t r = 0; r < rounds; ++r) {
-        if (r && __any_sync(kFull, *(volatile uint32_t*)b.bad != 0)) return;  // (the hash table has the join)
+        if (__any_sync(kFull, ld_ca(b.bad) != 0)) return;  // (the hash table has the join)
         const uint64_t i = r * stride + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
         const bool live = i < b.nb;
         uint64_t d = 0;
@@ -294,7 +296,7 @@ __global__ void __launch_bounds__(256) dj_insert_kernel(DjBuild b) {
         const uint32_t set = __reduce_or_sync(peers, bit);
         if (live && (threadIdx.x & 31) == __ffs(peers) - 1) {
             const uint32_t old = atomicOr(&b.bits[word], set);
-            if ((old & set) || __popc(set) != __popc(peers)) *b.bad = 1;  // a key twice
+            if (((old & set) || __popc(set) != __popc(peers)) && !ld_ca(b.bad)) *b.bad = 1;  // a key twice
         }
     }
 }
