@@ -422,44 +422,10 @@ AHEAD_DEV uint64_t block_scan_1024(uint64_t x, uint64_t* s_part, uint64_t* total
     return r;
 }
 
-// Pass 2: each block scans the counts of 1024 consecutive tiles per stream
-// (exclusive, within the group; three streams' counts of at most 1024 share a
-// 64-bit word, 21 bits each) and writes the group totals to gbase; the last
-// block to finish turns those into exclusive group offsets, a warp per stream
-// while they are few.  (As two kernels, each scanning stream after stream, this
-// took 10-14 us of every operator with up to a few thousand tiles.)
-static __global__ void __launch_bounds__(kScanGroup) tile_scan_kernel(CompactBufs cb) {
-    __shared__ uint64_t s_part[33];
-    __shared__ bool s_last;
-    const uint32_t nch = cb.nchan, ng = scan_groups(cb.ntiles);
-    const uint32_t t = blockIdx.x * kScanGroup + threadIdx.x;
-    for (uint32_t c0 = 0; c0 < nch; c0 += 3) {
-        const uint32_t m = nch - c0 < 3 ? nch - c0 : 3;
-        const uint64_t part = m == 1 ? ~0ull : (1ull << 21) - 1;  // (a single stream's counts may be larger)
-        uint64_t x = 0;
-        if (t < cb.ntiles)
-            for (uint32_t c = 0; c < m; ++c) x |= (uint64_t)cb.counts[(size_t)t * nch + c0 + c] << (21 * c);
-        uint64_t total;
-        const uint64_t ex = block_scan_1024(x, s_part, &total);
-        if (t < cb.ntiles)
-            for (uint32_t c = 0; c < m; ++c) cb.offsets[(size_t)t * nch + c0 + c] = (ex >> (21 * c)) & part;
-        if (threadIdx.x < m) {
-            const uint64_t tot = (total >> (21 * threadIdx.x)) & part;
-            cb.gbase[(size_t)blockIdx.x * nch + c0 + threadIdx.x] = ng == 1 ? 0 : tot;
-            if (ng == 1) cb.totals[c0 + threadIdx.x] = tot;
-        }
-    }
-    if (ng == 1) return;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        s_last = atomicAdd(cb.done, 1u) == gridDim.x - 1;
-        if (s_last) *cb.done = 0;
-        __threadfence();
-    }
-    __syncthreads();
-    if (!s_last) return;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// The group totals in gbase to exclusive group offsets, by one block of 1024: a
+// warp per stream while they are few.
+AHEAD_DEV void scan_group_totals(const CompactBufs& cb, uint64_t* s_part) {
+    const uint32_t nch = cb.nchan, ng = scan_groups(cb.ntiles), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (ng <= 128) {
         if (warp >= nch) return;
         uint64_t carry = 0;
@@ -486,6 +452,63 @@ static __global__ void __launch_bounds__(kScanGroup) tile_scan_kernel(CompactBuf
         }
         if (threadIdx.x == 0) cb.totals[c] = carry;
     }
+}
+
+// Pass 2: each block scans the counts of 1024 consecutive tiles per stream
+// (exclusive, within the group; three streams' counts of at most 1024 share a
+// 64-bit word, 21 bits each) and writes the group totals to gbase; the last
+// block to finish turns those into exclusive group offsets.  (As two kernels, each
+// scanning stream after stream, this took 10-14 us of every operator with up to a
+// few thousand tiles.)  From kScanSplit groups on -- the slots of a large hash table
+// only: a compaction of 2^30 rows has that many -- the offsets get a launch of their
+// own: each block's fence and count took 96 us of 8M slots, 55 without.
+constexpr uint32_t kScanSplit = 1024;
+
+static __global__ void __launch_bounds__(kScanGroup) group_scan_kernel(CompactBufs cb) {
+    __shared__ uint64_t s_part[33];
+    scan_group_totals(cb, s_part);
+}
+
+static __global__ void __launch_bounds__(kScanGroup) tile_scan_kernel(CompactBufs cb) {
+    __shared__ uint64_t s_part[33];
+    __shared__ bool s_last;
+    const uint32_t nch = cb.nchan, ng = scan_groups(cb.ntiles);
+    const uint32_t t = blockIdx.x * kScanGroup + threadIdx.x;
+    for (uint32_t c0 = 0; c0 < nch; c0 += 3) {
+        const uint32_t m = nch - c0 < 3 ? nch - c0 : 3;
+        const uint64_t part = m == 1 ? ~0ull : (1ull << 21) - 1;  // (a single stream's counts may be larger)
+        uint64_t x = 0;
+        if (t < cb.ntiles)
+            for (uint32_t c = 0; c < m; ++c) x |= (uint64_t)cb.counts[(size_t)t * nch + c0 + c] << (21 * c);
+        uint64_t total;
+        const uint64_t ex = block_scan_1024(x, s_part, &total);
+        if (t < cb.ntiles)
+            for (uint32_t c = 0; c < m; ++c) cb.offsets[(size_t)t * nch + c0 + c] = (ex >> (21 * c)) & part;
+        if (threadIdx.x < m) {
+            const uint64_t tot = (total >> (21 * threadIdx.x)) & part;
+            cb.gbase[(size_t)blockIdx.x * nch + c0 + threadIdx.x] = ng == 1 ? 0 : tot;
+            if (ng == 1) cb.totals[c0 + threadIdx.x] = tot;
+        }
+    }
+    if (ng == 1 || ng >= kScanSplit) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(cb.done, 1u) == gridDim.x - 1;
+        if (s_last) *cb.done = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_last) scan_group_totals(cb, s_part);
+}
+
+// Launches pass 2; returns the number of launches.
+inline int scan_tiles(cudaStream_t st, const CompactBufs& cb) {
+    const uint32_t ng = scan_groups(cb.ntiles);
+    tile_scan_kernel<<<ng, kScanGroup, 0, st>>>(cb);
+    if (ng < kScanSplit) return 1;
+    group_scan_kernel<<<1, kScanGroup, 0, st>>>(cb);
+    return 2;
 }
 
 // Pass 3, `per` tiles per warp; the next tile's header and words are loaded

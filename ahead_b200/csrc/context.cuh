@@ -265,16 +265,13 @@ inline int launch_compact(const ahead_ctx* ctx, cudaStream_t st, const Op& op, u
     auto passes = [&](auto k_tag) {
         constexpr int K = decltype(k_tag)::value;
         classify_kernel<Op, K><<<grid, kCThreads, 0, st>>>(op, n, cb, (int)per);
-        tile_scan_kernel<<<scan_groups(nt), kScanGroup, 0, st>>>(cb);
+        const int scans = scan_tiles(st, cb);
         emit_kernel<Op, K><<<grid, kCThreads, 0, st>>>(op, n, cb, (int)per);
+        return 2 + scans;
     };
     if constexpr (!Op::GATHER)
-        if (long_tiles<Op>(n)) {
-            passes(std::integral_constant<int, kLongK>());
-            return 3;
-        }
-    passes(std::integral_constant<int, short_k(Op::W)>());
-    return 3;
+        if (long_tiles<Op>(n)) return passes(std::integral_constant<int, kLongK>());
+    return passes(std::integral_constant<int, short_k(Op::W)>());
 }
 
 // The compaction of a sized call: counts first, then `alloc(kept)` sets the op's
@@ -288,8 +285,7 @@ inline int run_compact_sized(OpScope& s, Op& op, uint64_t n, int c0, int ncounte
     auto passes = [&](auto k_tag) -> int {
         constexpr int K = decltype(k_tag)::value;
         classify_kernel<Op, K><<<grid, kCThreads, 0, st>>>(op, n, cb, (int)per);
-        tile_scan_kernel<<<scan_groups(nt), kScanGroup, 0, st>>>(cb);
-        s.launched(2);
+        s.launched(1 + scan_tiles(st, cb));
         int rc = s.finish(ncounters);
         if (rc) return rc;
         if (!alloc(s.counter(c0))) return fail(s.ctx, AHEAD_NO_MEMORY, "output allocation failed");
@@ -312,8 +308,7 @@ inline void launch_emit(OpScope& s, const Op& op, uint64_t n, const CompactBufs&
     s.launched();
 }
 inline void launch_scan(OpScope& s, const CompactBufs& cb) {
-    tile_scan_kernel<<<scan_groups(cb.ntiles), kScanGroup, 0, s.ctx->stream>>>(cb);
-    s.launched();
+    s.launched(scan_tiles(s.ctx->stream, cb));
 }
 
 // A compaction of an operator call; totals land in counters [c0, c0 + NCH).

@@ -533,7 +533,7 @@ int run_hash_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk, u
     sb.done = (uint32_t*)(s.d_counters + kScanDone);
     sb.ntiles = cap + 1;
     sb.nchan = 1;
-    tile_scan_kernel<<<scan_groups(cap + 1), kScanGroup, 0, st>>>(sb);
+    launch_scan(s, sb);
     ht_offsets_kernel<<<grid_for(cap + 1, 256), 256, 0, st>>>(h, sb);
     ht_fill_kernel<<<grid_for(nb, 256), 256, 0, st>>>(h, slot_of, nb);
     ht_order_kernel<<<grid_for(cap + 1, 256), 256, 0, st>>>(h, cap + 1);
@@ -541,7 +541,7 @@ int run_hash_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk, u
     const bool direct = nb < (uint64_t)(kDirect - 1);
     ProbeSlot* pt = (ProbeSlot*)s.alloc((size_t)(cap + 1) * sizeof(ProbeSlot));
     ht_pack_kernel<<<grid_for(cap + 1, 256), 256, 0, st>>>(h, pt, cap + 1, direct);
-    s.launched(6);
+    s.launched(5);
     const uint32_t nt = (uint32_t)((np + kProbeTile - 1) / kProbeTile);
     CompactBufs pb;
     pb.words = nullptr;
@@ -554,8 +554,8 @@ int run_hash_join(OpScope& s, const KeyCfg& bk, uint64_t nb, const KeyCfg& pk, u
     pb.nchan = 1;
     const uint32_t pg = nt < (uint32_t)g ? nt : (uint32_t)g;
     probe_count_kernel<<<pg, 256, 0, st>>>(pt, h.mask, direct, pk, np, pslot, pb);
-    tile_scan_kernel<<<scan_groups(nt), kScanGroup, 0, st>>>(pb);
-    s.launched(2);
+    s.launched();
+    launch_scan(s, pb);
     if (out) {
         const int rc = s.finish(1);
         if (rc) return rc;
