@@ -228,11 +228,13 @@ constexpr uint32_t kSureDrops = 256;  // scratch for the edges of this many is a
 struct DropList {
     unsigned long long *cnt, *kind1;  // entries, and those of kind 1
     uint64_t* rows;                   // [kMaxDrops] row << 1 | kind
-    AHEAD_DEV void add(uint64_t row, uint32_t kind) const {
-        if (*(volatile unsigned long long*)cnt > kMaxDrops) return;
+    // true: more than kMaxDrops rows are dropped, so the caller's pass is for nothing
+    AHEAD_DEV bool add(uint64_t row, uint32_t kind) const {
+        if (*(volatile unsigned long long*)cnt > kMaxDrops) return true;
         const unsigned long long k = atomicAdd(cnt, 1ull);
         if (k < kMaxDrops) rows[k] = row << 1 | kind;
         if (kind) atomicAdd(kind1, 1ull);
+        return false;
     }
 };
 
