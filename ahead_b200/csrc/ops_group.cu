@@ -160,14 +160,16 @@ struct SmallGb {
     uint32_t* first;         // [limit] first row of each key
     uint32_t* gid_of_slot;   // [limit]
     uint32_t* found;         // [kGbSort] the keys that occur, in any order
-    unsigned long long* count;  // keys that occur; above kGbSort: more than that
+    unsigned long long* count;  // keys that occur
+    uint32_t* many;          // count may be too small, but above kGbSort
     uint32_t* over;          // a key did not fit
     uint32_t limit;
     int check;               // AN inputs: report corrupt codes
     ErrList terr, gerr;
 };
 
-template <bool TENC>
+// MANY: beyond kGbSort groups, which the compaction counts, a new one is not added.
+template <bool TENC, bool MANY>
 AHEAD_DEV uint32_t small_gb_row(const SmallGb& g, uint64_t row, uint64_t tv, uint64_t gv) {
     const uint64_t t = TENC ? mulw(tv, g.k.tail.ainv, g.k.tail.width) : tv;
     if (TENC && t > g.k.tail.umax) g.terr.add(row);
@@ -182,14 +184,10 @@ AHEAD_DEV uint32_t small_gb_row(const SmallGb& g, uint64_t row, uint64_t tv, uin
         return 0;
     }
     const uint32_t s = (uint32_t)key, r = (uint32_t)row;
-    if (r < ld_ca(g.first + s)) {
-        // (beyond kGbSort groups the compaction counts them: 1M groups' adds on the one
-        // word took the insert pass of 3M rows from 39 to 199 us)
-        const bool more = ld_ca((const uint32_t*)g.count) <= kGbSort;
-        if (r < *(volatile uint32_t*)(g.first + s) && atomicMin(&g.first[s], r) == kNoRow && more) {
-            const unsigned long long i = atomicAdd(g.count, 1ull);
-            if (i < kGbSort) g.found[i] = s;
-        }
+    if (r < ld_ca(g.first + s) && r < *(volatile uint32_t*)(g.first + s) && atomicMin(&g.first[s], r) == kNoRow &&
+        (!MANY || ld_ca((const uint32_t*)g.count) <= kGbSort)) {
+        const unsigned long long i = atomicAdd(g.count, 1ull);
+        if (i < kGbSort) g.found[i] = s;
     }
     return s;
 }
@@ -201,7 +199,7 @@ __global__ void __launch_bounds__(1024) small_gb_seed_kernel(SmallGb g) {
     const uint64_t m = g.n < kGbSeedRows ? g.n : kGbSeedRows;
     for (uint64_t i = threadIdx.x; i < m; i += blockDim.x) {
         if (*(volatile uint32_t*)g.over) return;
-        g.slot_of[i] = small_gb_row<TENC>(g, i, load_at(g.k.tail, i), g.k.binary ? load_at(g.k.grp, i) : 0);
+        g.slot_of[i] = small_gb_row<TENC, false>(g, i, load_at(g.k.tail, i), g.k.binary ? load_at(g.k.grp, i) : 0);
     }
 }
 
@@ -225,13 +223,10 @@ AHEAD_DEV void load4(const DCol& c, uint64_t i, bool vec, uint64_t (&v)[4]) {
     for (int q = 0; q < 4; ++q) v[q] = load_at(c, i + q);
 }
 
-// TW, GW: the tail's and the grouping's width (GW 0: unary).
-template <int TW, int GW, bool TENC>
-__global__ void __launch_bounds__(256) small_gb_insert_kernel(SmallGb g, bool vec) {
+// Rows from kGbSeedRows on, four per thread and step.
+template <int TW, int GW, bool TENC, bool MANY>
+AHEAD_DEV void small_gb_rows(const SmallGb& g, bool vec) {
     const uint64_t r0 = kGbSeedRows, m = (g.n - r0) / 4, stride = (uint64_t)gridDim.x * blockDim.x;
-    // (a seed row's key did not fit: the hash table has the call.  Through L1: nearly
-    // 10,000 warps' reads of one word at L2 took 2 to 19 us)
-    if (ld_ca(g.over)) return;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += stride) {
         const uint64_t row = r0 + 4 * i;
         uint64_t t[4], gv[4] = {0, 0, 0, 0};
@@ -239,12 +234,30 @@ __global__ void __launch_bounds__(256) small_gb_insert_kernel(SmallGb g, bool ve
         if constexpr (GW) load4<GW>(g.k.grp, row, vec, gv);
         uint32_t s[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) s[q] = small_gb_row<TENC>(g, row + q, t[q], gv[q]);
+        for (int q = 0; q < 4; ++q) s[q] = small_gb_row<TENC, MANY>(g, row + q, t[q], gv[q]);
         *reinterpret_cast<uint4*>(g.slot_of + row) = make_uint4(s[0], s[1], s[2], s[3]);
     }
     if (blockIdx.x == 0 && threadIdx.x < (g.n - r0) % 4) {
         const uint64_t row = r0 + 4 * m + threadIdx.x;
-        g.slot_of[row] = small_gb_row<TENC>(g, row, load_at(g.k.tail, row), GW ? load_at(g.k.grp, row) : 0);
+        g.slot_of[row] = small_gb_row<TENC, MANY>(g, row, load_at(g.k.tail, row), GW ? load_at(g.k.grp, row) : 0);
+    }
+}
+
+// TW, GW: the tail's and the grouping's width (GW 0: unary).  Where a quarter of the
+// seed rows opened a group, most rows may: 1M groups of 3M rows all counted on one
+// word took 199 us, 39 with the adds skipped beyond kGbSort.  The look before each add
+// is for such inputs alone: in the loop of all it cost 30M rows of 400 groups 55 us
+// instead of 50.
+template <int TW, int GW, bool TENC>
+__global__ void __launch_bounds__(256, GW ? 6 : 8) small_gb_insert_kernel(SmallGb g, bool vec) {
+    // (a seed row's key did not fit: the hash table has the call.  Through L1: nearly
+    // 10,000 warps' reads of one word at L2 took 2 to 19 us)
+    if (ld_ca(g.over)) return;
+    if (ld_ca((const uint32_t*)g.count) > kGbSeedRows / 4) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *g.many = 1;
+        small_gb_rows<TW, GW, TENC, true>(g, vec);
+    } else {
+        small_gb_rows<TW, GW, TENC, false>(g, vec);
     }
 }
 
@@ -334,8 +347,8 @@ inline size_t small_gb_scratch(uint64_t n) {
     return (size_t)gb_limit(n) * 8 + n * 4 + kGbSort * 4 + 2 * kErrListBytes + 4096;
 }
 
-// Counters 10-13 of the call: groups, `over`, corrupt tails, corrupt grouping codes.
-constexpr int kGbCount = 10, kGbOver = 11, kGbTail = 12, kGbGrp = 13, kGbCounters = 14;
+// Counters 10-14 of the call: groups, `over`, corrupt tails, corrupt grouping codes, `many`.
+constexpr int kGbCount = 10, kGbOver = 11, kGbTail = 12, kGbGrp = 13, kGbMany = 14, kGbCounters = 15;
 
 // The group-by through the first-row table: everything up to the group ids of
 // up to kGbSort groups.
@@ -354,6 +367,7 @@ SmallGb launch_small_gb(OpScope& s, const GbKey& k, uint64_t n, uint64_t gmax, c
     g.found = (uint32_t*)s.alloc(kGbSort * 4);
     g.count = (unsigned long long*)(s.d_counters + kGbCount);
     g.over = (uint32_t*)(s.d_counters + kGbOver);
+    g.many = (uint32_t*)(s.d_counters + kGbMany);
     g.check = AN;
     g.terr = err_list(s, kGbTail);
     g.gerr = err_list(s, kGbGrp);
@@ -574,16 +588,18 @@ int run_groupby(ahead_ctx* ctx, const ahead_bat* in, const ahead_bat* grouping, 
     if (!s.counter(kGbOver)) {
         uint64_t groups = s.counter(kGbCount);
         if (errs && eH) errs[0].count = s.counter(1);
-        if (groups > kGbSort) {  // ranked and counted by the compaction of the rows that are their key's first
+        if (groups > kGbSort) {  // ranked by the compaction of the rows that are their key's first
             run_compact(s, first_op(g.slot_of, g.first, g.gid_of_slot), n, 0);
             if (gids->tail.data) {
                 small_gb_assign_kernel<true, false><<<grid_for((n + 3) / 4, 256), 256, 0, ctx->stream>>>(
                     g, aoid, binary, gids->tail.data, cap);
                 s.launched();
             }
-            rc = s.finish(1);  // (leaves the lists' counters as they were read)
-            if (rc) return rc;
-            groups = s.counter(0);
+            if (s.counter(kGbMany)) {
+                rc = s.finish(1);  // (leaves the lists' counters as they were read)
+                if (rc) return rc;
+                groups = s.counter(0);
+            }
         }
         firsts->count = groups;
         rc = settle(g.terr, g.gerr);
