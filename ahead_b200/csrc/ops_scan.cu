@@ -509,49 +509,13 @@ __global__ void mul_sum_plain_kernel(DCol a, DCol b, uint64_t n, unsigned long l
 }
 
 // ------------------------------------------------------------ arithmetic
-// arithmeticAN (arithmeticAN_scalar.tcc:87-107).
-template <int WW>
-struct ArithOp {
-    static constexpr int W = WW;
-    static constexpr int NCH = 2;
-    static constexpr bool ACC = false;
-    static constexpr bool GATHER = false;
-    const char* base;
-    DCol ac, bc;
-    uint64_t ar, aoid, ecap1, ecap2;
-    uint64_t *e1, *e2;
-    void* out;
-    int ow, op;
-    uint64_t* acc;
-    static constexpr bool EMIT_V = false;
-    static constexpr int NOUT = 1;
-    AHEAD_DEV uint64_t out0(int, uint64_t, uint64_t row) const { return row * aoid; }
-    AHEAD_DEV uint64_t cap0() const { return ecap1; }
-    AHEAD_DEV void* optr(int) const { return e1; }
-    AHEAD_DEV int owidth(int) const { return 8; }
-    AHEAD_DEV uint32_t eval(uint64_t a, uint64_t row, uint64_t&) const {
-        const uint64_t t1 = mulw(a, ac.ainv, W), t2 = mulw(load_at(bc, row), bc.ainv, bc.width);
-        const uint64_t x = t1 * ar, y = t2 * ar;
-        uint64_t v;
-        switch (op) {
-            case AHEAD_ADD: v = x + y; break;
-            case AHEAD_SUB: v = x - y; break;
-            case AHEAD_MUL: v = x * y; break;
-            default: v = y ? x / y : 0; break;
-        }
-        store_at(out, ow, row, v);
-        return (t1 > ac.umax ? 1u : 0u) | (t2 > bc.umax ? 2u : 0u);
-    }
-    AHEAD_DEV void emit(int, uint64_t pos, uint64_t, uint64_t row) const {
-        if (pos < ecap2) e2[pos] = row * aoid;
-    }
-};
-
-// arithmeticAN in one pass: every row is written to its own place and the rows of
-// corrupt operands are listed (see ErrList); two neighbouring rows per thread, two
-// such pairs in flight (four took 112 registers and 73 us).  Bound by HBM: 12M
-// (resint, restiny) rows in 46 us (216 MB, 4.7 TB/s), where the compaction, which
-// runs when a list overflows, took 129 with its three launches.
+// arithmeticAN (arithmeticAN_scalar.tcc:87-107) in one pass: every row is written to
+// its own place and the rows of corrupt operands are listed (see ErrList); two
+// neighbouring rows per thread, two such pairs in flight (four took 112 registers
+// and 73 us).  Bound by HBM: 12M (resint, restiny) rows in 46 us (216 MB, 4.7 TB/s),
+// where a compaction took 129 with its three launches.  When a list overflows, only
+// the vectors are made again, by checks of the columns: 30M rows with 5,000 corrupt
+// codes 231 us (489 when a compaction also computed the rows again).
 template <int W1, int W2, bool DIV>
 __global__ void __launch_bounds__(256, DIV ? 2 : 5) arith_kernel(DCol a, DCol b, uint64_t n, int op, uint64_t ar,
                                                                  uint64_t* out, ErrList e1, ErrList e2) {
@@ -1057,6 +1021,7 @@ int ahead_gpu_arithmetic_an(ahead_ctx* ctx, int op, int result_type, const ahead
     set_meta(&out->tail, result_type, ar, arinv, type_unenc_max(result_type), 0);
     out->count = a->count;
     const uint64_t n = a->count;
+    bool ok1 = false, ok2 = false;  // whose vector the pass's list has made
     OpScope s(ctx);
     if (n && out->tail.data) {
         int rc = s.reserve(2 * kErrListBytes);
@@ -1079,41 +1044,23 @@ int ahead_gpu_arithmetic_an(ahead_ctx* ctx, int op, int result_type, const ahead
         s.launched();
         rc = s.finish(2);
         if (rc) return rc;
-        if (s.counter(0) <= kFastErrCap && s.counter(1) <= kFastErrCap) {
-            const bool some = e && s.counter(0) + s.counter(1);
-            settle_err_list(s, l1, 0, aoid, e ? &e[1] : nullptr);
-            settle_err_list(s, l2, 1, aoid, e ? &e[3] : nullptr);
-            return some ? s.wait() : AHEAD_OK;
-        }
+        const bool some = e && s.counter(0) + s.counter(1);
+        ok1 = settle_err_list(s, l1, 0, aoid, e ? &e[1] : nullptr);
+        ok2 = settle_err_list(s, l2, 1, aoid, e ? &e[3] : nullptr);
+        if (!e || (ok1 && ok2)) return some ? s.wait() : AHEAD_OK;
     }
-    return by_width_enc(type_width(T1), [&](auto tag) -> int {
-        constexpr int W = decltype(tag)::value;
-        typedef ArithOp<W> Op;
-        int rc = s.reserve(compact_scratch<Op>(a->count));
-        if (rc) return rc;
-        Op o;
-        o.base = (const char*)a->tail.data;
-        o.ac = dcol(a->tail);
-        o.bc = dcol(b->tail);
-        o.ar = ar;
-        o.aoid = aoid;
-        o.e1 = edata(e ? &e[1] : nullptr);
-        o.e2 = edata(e ? &e[3] : nullptr);
-        o.ecap1 = ecap(e ? &e[1] : nullptr);
-        o.ecap2 = ecap(e ? &e[3] : nullptr);
-        o.out = out->tail.data;
-        o.ow = type_width(result_type);
-        o.op = op;
-        o.acc = nullptr;
-        run_compact<Op>(s, o, a->count, 0);
-        rc = s.finish(2);
-        if (rc) return rc;
-        if (e) {
-            e[1].count = s.counter(0);
-            e[3].count = s.counter(1);
-        }
-        return AHEAD_OK;
-    });
+    if (!e) return AHEAD_OK;
+    // a column with many corrupt codes, or no output wanted
+    int rc = s.reserve(2 * colcheck_scratch(n));
+    if (rc) return rc;
+    const DCol ca = dcol(a->tail), cb = dcol(b->tail);
+    if (!ok1) run_colcheck(s, a->tail, n, ca.ainv, ca.umax, ca.width, aoid, &e[1], 0);
+    if (!ok2) run_colcheck(s, b->tail, n, cb.ainv, cb.umax, cb.width, aoid, &e[3], 1);
+    rc = s.finish(2);
+    if (rc) return rc;
+    if (!ok1) e[1].count = s.counter(0);
+    if (!ok2) e[3].count = s.counter(1);
+    return AHEAD_OK;
 }
 
 }  // extern "C"
