@@ -276,20 +276,7 @@ __global__ void __launch_bounds__(1024) small_gb_rank_kernel(SmallGb g, DCol hea
         s_k[i] = i < c ? ((uint64_t)g.first[s] << 32 | s) : ~0ull;
     }
     __syncthreads();
-    for (uint32_t size = 2; size <= m; size <<= 1)
-        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-                const uint32_t j = i ^ stride;
-                if (j > i) {
-                    const uint64_t x = s_k[i], y = s_k[j];
-                    if ((x > y) == ((i & size) == 0)) {
-                        s_k[i] = y;
-                        s_k[j] = x;
-                    }
-                }
-            }
-            __syncthreads();
-        }
+    sort_block(s_k, m);
     for (uint32_t i = threadIdx.x; i < c; i += blockDim.x) {
         const uint64_t x = s_k[i];
         g.gid_of_slot[(uint32_t)x] = i;
