@@ -472,9 +472,9 @@ AHEAD_DEV void scan_group_totals(const CompactBufs& cb, uint64_t* s_part) {
 // 64-bit word, 21 bits each) and writes the group totals to gbase; the last
 // block to finish turns those into exclusive group offsets.  (As two kernels, each
 // scanning stream after stream, this took 10-14 us of every operator with up to a
-// few thousand tiles.)  From kScanSplit groups on -- the slots of a large hash table
-// only: a compaction of 2^30 rows has that many -- the offsets get a launch of their
-// own: each block's fence and count took 96 us of 8M slots, 55 without.
+// few thousand tiles.)  From kScanSplit groups on -- the slots of a large hash table,
+// compactions of 2^28 rows in short tiles or 2^30 in long ones -- the offsets get a
+// launch of their own: each block's fence and count took 96 us of 8M slots, 55 without.
 constexpr uint32_t kScanSplit = 1024;
 
 static __global__ void __launch_bounds__(kScanGroup) group_scan_kernel(CompactBufs cb) {
